@@ -44,34 +44,34 @@ def _case(name, kind, n, L, **kw):
 def listed():
     return [
         # one interactive 1-NN query of a small index, host in, host out
-        _case("plain 100k x 256, 1 query", "plain", 100000, 256, leaf=2000, sigma2="0.1", nq=1, k=1, lb_sax=True,
+        _case("plain 100k x 256 / 1 query", "plain", 100000, 256, leaf=2000, sigma2="0.1", nq=1, k=1, lb_sax=True,
               host=True),
         # a workload file of 100 queries over the 1M x 256 index (leaf
         # 100,000) of the reference's own configuration, with LB_SAX
-        _case("plain 1M x 256, 100 queries", "plain", 1000000, 256, leaf=100000, fresh=True, nq=100, k=10,
+        _case("plain 1M x 256 / 100 queries", "plain", 1000000, 256, leaf=100000, fresh=True, nq=100, k=10,
               lb_sax=True),
         # a few 100-NN queries of a larger index with the default options
         # (no LB_SAX), through the host entry point
-        _case("plain 8M x 256, 16 queries, k 100", "plain", 8000000, 256, leaf=100000, fresh=True, nq=16, k=100,
+        _case("plain 8M x 256 / 16 queries / k 100", "plain", 8000000, 256, leaf=100000, fresh=True, nq=16, k=100,
               host=True),
         # long series: 64 KB rows, small leaves
-        _case("plain 100k x 16384, 12 queries", "plain", 100000, 16384, leaf=1562, sigma2="0.1", nq=12, k=10,
+        _case("plain 100k x 16384 / 12 queries", "plain", 100000, 16384, leaf=1562, sigma2="0.1", nq=12, k=10,
               lb_sax=True),
         # the index-free scan of every row, a handful of queries
-        _case("pscan 2M x 256, 4 queries", "pscan", 2000000, 256, leaf=100000, nq=4, k=10, host=True),
+        _case("pscan 2M x 256 / 4 queries", "pscan", 2000000, 256, leaf=100000, nq=4, k=10, host=True),
         # one query over a caller-owned matrix, nothing allocated
-        _case("noalloc 1M x 256, 1 query", "noalloc", 999983, 256, sigma2="0.1", nq=1, k=10),
+        _case("noalloc 1M x 256 / 1 query", "noalloc", 999983, 256, sigma2="0.1", nq=1, k=10),
         # a small service batch over a small index, host in, host out
-        _case("batch 100k x 256, 64 queries", "batch", 100000, 256, leaf=2000, sigma2="0.1", nq=64, k=1, host=True),
+        _case("batch 100k x 256 / 64 queries", "batch", 100000, 256, leaf=2000, sigma2="0.1", nq=64, k=1, host=True),
         # short embedding-like vectors: nothing prunes, odd counts
-        _case("batch 3M x 96 unit, 333 queries", "batch", 3000017, 96, leaf=8000, data="unit", sigma2="0.1", nq=333,
+        _case("batch 3M x 96 unit / 333 queries", "batch", 3000017, 96, leaf=8000, data="unit", sigma2="0.1", nq=333,
               k=10),
         # series of 1,024 points at bench.py's noise levels
-        _case("batch 1M x 1024, 512 queries", "batch", 1000000, 1024, leaf=25000, sigma2="0.1,1.0", nq=512, k=10),
+        _case("batch 1M x 1024 / 512 queries", "batch", 1000000, 1024, leaf=25000, sigma2="0.1,1.0", nq=512, k=10),
         # the longest series, batched
-        _case("batch 200k x 16384, 128 queries", "batch", 200000, 16384, leaf=1562, sigma2="0.1", nq=128, k=10),
+        _case("batch 200k x 16384 / 128 queries", "batch", 200000, 16384, leaf=1562, sigma2="0.1", nq=128, k=10),
         # bench.py's headline batch: 4,096 queries of mixed noise and k
-        _case("batch 25M x 256, 4096 queries", "batch", 25000000, 256, leaf=100000, fresh=True, nq=4096, k=0),
+        _case("batch 25M x 256 / 4096 queries", "batch", 25000000, 256, leaf=100000, fresh=True, nq=4096, k=0),
         # building an index from rows on the GPU
         _case("build 1M x 256", "build", 1000000, 256, leaf=10000),
     ]
