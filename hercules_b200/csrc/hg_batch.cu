@@ -119,16 +119,73 @@ __global__ void k_tile_norms(const float4* __restrict__ meta, uint64_t n, float4
 // kMaxK smallest are ranked exactly (hg_ed, reference order) and the k-th
 // distinct distance among them bounds the query's k-th neighbour distance
 // (more rows than k: a tighter bound, and k distinct distances despite ties).
-// squared distance of chunk c of x (8 floats) to the same chunk of q
-__device__ __forceinline__ float chunk_d2_v4(const float* q, const float* x, int c) {
-  const float4 x0 = reinterpret_cast<const float4*>(x)[2 * c], x1 = reinterpret_cast<const float4*>(x)[2 * c + 1];
-  const float4 q0 = reinterpret_cast<const float4*>(q)[2 * c], q1 = reinterpret_cast<const float4*>(q)[2 * c + 1];
-  const float qq[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-  const float xx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-  return hg_chunk_d2(qq, xx);
+constexpr int kSelThreads = 256;
+constexpr int kRankLongSeries = 4096;  // L from which the exact ranking uses 8 lanes per row
+
+// Exact distances of the rows named by the first nrank keys of `buf` (~0: no
+// row), without abandoning, into list[i] as (distance, id) keys.  A warp
+// takes 32 / kSlot rows at a time, kSlot lanes per row; a step covers 2 kSlot
+// chunks of each row, whose sums every lane of the slot adds in chunk order
+// (ts_euclidean_distance_SIMD's order), and the next step's lines are loaded
+// before the current ones are summed.  One row per warp, its 32 chunk sums
+// added one shuffle after the other, was bound by that chain: 428 us for 128
+// queries of 16,384 points (52 rows each), 58 us for 512 queries of 1,024.
+template <int kSlot>
+__device__ __forceinline__ void rank_rows(const BatchRank& a, const float* qv, const unsigned long long* buf, int nrank,
+                                          unsigned long long* list) {
+  constexpr int kLines = 2, kStep = kSlot * kLines, kRows = 32 / kSlot;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = lane / kSlot, slot_lead = lane & ~(kSlot - 1), j = lane & (kSlot - 1);
+  const int nch = a.L >> 3;
+  for (int i0 = warp * kRows; i0 < nrank; i0 += (kSelThreads / 32) * kRows) {
+    const int i = i0 + slot;
+    const unsigned long long key = i < nrank ? buf[i] : ~0ull;
+    const bool valid = key != ~0ull;
+    if (!__any_sync(HG_FULL, valid)) break;  // the keys are sorted: no row follows
+    const uint32_t row = (uint32_t)key;
+    const float4* x = reinterpret_cast<const float4*>(a.rows + (uint64_t)(valid ? row : 0u) * a.L) + 2 * j;
+    const float4* qc = reinterpret_cast<const float4*>(qv) + 2 * j;
+    float4 xv[kLines][2];
+    auto load = [&](int ch) {
+#pragma unroll
+      for (int l = 0; l < kLines; ++l)
+        if (valid && ch + kSlot * l + j < nch) {
+          xv[l][0] = x[2 * ch + 2 * kSlot * l];
+          xv[l][1] = x[2 * ch + 2 * kSlot * l + 1];
+        }
+    };
+    float d = 0.0f;
+    load(0);
+    for (int ch = 0; ch < nch; ch += kStep) {
+      float dl[kLines];
+      float4 xc[kLines][2];
+#pragma unroll
+      for (int l = 0; l < kLines; ++l) {
+        xc[l][0] = xv[l][0];
+        xc[l][1] = xv[l][1];
+      }
+      if (ch + kStep < nch) load(ch + kStep);
+#pragma unroll
+      for (int l = 0; l < kLines; ++l) {
+        const bool in = valid && ch + kSlot * l + j < nch;
+        dl[l] = 0.0f;  // past the row's end: adding 0 leaves a sum unchanged
+        if (in) {
+          const float4 q0 = qc[2 * ch + 2 * kSlot * l], q1 = qc[2 * ch + 2 * kSlot * l + 1];
+          const float qq[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+          const float xx[8] = {xc[l][0].x, xc[l][0].y, xc[l][0].z, xc[l][0].w,
+                               xc[l][1].x, xc[l][1].y, xc[l][1].z, xc[l][1].w};
+          dl[l] = hg_chunk_d2(qq, xx);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < kStep; ++t)
+        d = __fadd_rn(d, __shfl_sync(HG_FULL, dl[t / kSlot], slot_lead + (t % kSlot)));
+    }
+    if (valid && j == 0) list[i] = ((unsigned long long)__float_as_uint(d) << 32) | (uint32_t)a.ids[row];
+  }
 }
 
-constexpr int kSelThreads = 256;
+template <int kSlot>
 __global__ void __launch_bounds__(kSelThreads) k_bound_select(BatchRank a) {
   extern __shared__ unsigned long long ssel[];
   unsigned long long* buf = ssel;                    // bm_pow2 keys
@@ -156,28 +213,12 @@ __global__ void __launch_bounds__(kSelThreads) k_bound_select(BatchRank a) {
       __syncthreads();
     }
   const float* qv = a.Q + (uint64_t)q * a.L;
-  // a warp per row: lane c computes chunk c of a 32-chunk group (one
-  // coalesced load), the chunk sums are added in chunk order
-  // (ts_euclidean_distance_SIMD's order, no abandon)
-  const int lane = tid & 31, nch = a.L >> 3;
   // the 2k + 32 best slots by d~ (at most kMaxK) are ranked exactly: the k-th
   // distinct exact distance among them bounds the query's k-th neighbour
-  const int nrank = min(kMaxK, 2 * k + 32);
-  for (int i = tid >> 5; i < kWarpListCap; i += kSelThreads / 32) {
-    unsigned long long v = ~0ull;
-    if (i < nrank && i < n && buf[i] != ~0ull) {  // uniform over the warp
-      const uint32_t row = (uint32_t)buf[i];
-      const float* xr = a.rows + (uint64_t)row * a.L;
-      float d = 0.0f;
-      for (int c0 = 0; c0 < nch; c0 += 32) {
-        const float cd = c0 + lane < nch ? chunk_d2_v4(qv, xr, c0 + lane) : 0.0f;
-        const int lim = min(32, nch - c0);
-        for (int t = 0; t < lim; ++t) d = __fadd_rn(d, __shfl_sync(HG_FULL, cd, t));
-      }
-      v = ((unsigned long long)__float_as_uint(d) << 32) | (uint32_t)a.ids[row];
-    }
-    if (lane == 0) list[i] = v;
-  }
+  const int nrank = min(min(kMaxK, 2 * k + 32), n);
+  for (int i = tid; i < kWarpListCap; i += kSelThreads) list[i] = ~0ull;
+  __syncthreads();
+  rank_rows<kSlot>(a, qv, buf, nrank, list);
   __syncthreads();
   if (tid < 32) {
     // the valid keys are a prefix (rows of the sorted prefix), the rest ~0
@@ -196,24 +237,43 @@ __global__ void __launch_bounds__(kSelThreads) k_bound_select(BatchRank a) {
 
 // Steps 4-5 run in three kernels over the queries qlist[0 .. nlist) (all
 // queries when qlist is null).  Plan: each query's surviving rows (the first
-// bucket_cap of them when its bucket overflowed) are cut into at most
-// kBatchMaxSeg segments of at least kBatchSegMin rows; segments are numbered
-// over the list (exclusive prefix seg_prefix, by list position).
+// bucket_cap of them when its bucket overflowed) are cut into segments, one
+// warp's work each, numbered over the list (exclusive prefix seg_prefix, by
+// list position).  The length of a segment follows from the rows of all
+// queries: kBatchSegTarget segments in all (one more per query at most), and
+// not less than the rows a warp has in flight, so every warp of the GPU gets
+// several whether the rows are spread over many queries or belong to one.
+// (Segments of at least 256 rows, at most 64 per query, took 11.5 ms for 128
+// queries of 200k x 16384 with 430 rows each -- 256 warps, 0.28 TB/s -- and
+// 7.6 ms with short segments but still at most 64, where one query holds a
+// third of the rows; now 0.72 ms, and 1.1 ms with that query.)
 __global__ void __launch_bounds__(1024) k_rerank_plan(BatchRank a) {
   __shared__ uint32_t warp_sums[32];
   __shared__ uint32_t carry;
+  __shared__ unsigned long long s_rows;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid == 0) carry = 0;
+  if (tid == 0) {
+    carry = 0;
+    s_rows = 0;
+  }
   __syncthreads();
   const float inf = __int_as_float(0x7f800000);
   const int nlist = a.nlist_dev ? (int)*a.nlist_dev : a.nlist;
+  unsigned long long mine = 0;
+  for (int i = tid; i < nlist; i += 1024) {
+    const int q = a.qlist ? (int)a.qlist[i] : i;
+    mine += a.bound[q] < inf ? min(a.bucket_cnt[q], a.bucket_cap) : 0u;
+  }
+  if (mine) atomicAdd(&s_rows, mine);
+  __syncthreads();
+  const uint32_t in_flight = a.L >= kRankLongSeries ? 4u : 16u;
+  const uint32_t seg = max(in_flight, (uint32_t)((s_rows + kBatchSegTarget - 1) / kBatchSegTarget));
   for (int base = 0; base < nlist; base += 1024) {
     const int i = base + tid;
-    uint32_t nseg = 0, seg = 0;
+    uint32_t nseg = 0;
     if (i < nlist) {
       const int q = a.qlist ? (int)a.qlist[i] : i;
       const uint32_t n = a.bound[q] < inf ? min(a.bucket_cnt[q], a.bucket_cap) : 0u;
-      seg = max((uint32_t)kBatchSegMin, (n + kBatchMaxSeg - 1) / kBatchMaxSeg);
       nseg = (n + seg - 1) / seg;
       a.seg_rows[i] = seg;
       a.qbound[q] = __float_as_uint(a.bound[q]);
@@ -268,7 +328,7 @@ __host__ __device__ constexpr uint32_t rank_leaders() {
   return kSlot == 2 ? 0x55555555u : (kSlot == 4 ? 0x11111111u : (kSlot == 8 ? 0x01010101u : 0x00010001u));
 }
 template <int kSlot, int kLines>
-__global__ void __launch_bounds__(kRankWarps * 32) k_rerank_part(BatchRank a) {
+__global__ void __launch_bounds__(kRankWarps * 32, 4) k_rerank_part(BatchRank a) {
   __shared__ unsigned long long lists[kRankWarps][kWarpListCap];
   constexpr int kStep = kSlot * kLines;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -302,6 +362,7 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_part(BatchRank a) {
     for (int i = lane; i < kWarpListCap; i += 32) list[i] = i < c0 ? a.init[(uint64_t)q * kMaxK + i] : ~0ull;
     __syncwarp();
     int cnt = c0;
+    bool added = false;
     float T = cnt == k ? __uint_as_float((uint32_t)(list[k - 1] >> 32)) : inf;
     float B = fminf(T, __uint_as_float(ld_volatile(&a.qbound[q])));
     const uint32_t* bk = a.bucket + (uint64_t)q * a.bucket_cap;
@@ -380,13 +441,35 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_part(BatchRank a) {
         }
       }
       const bool take = finished && j == 0;
+      added = added || __any_sync(HG_FULL, take);
       warp_list_add<true>(list, cnt, T, k, &a.qbound[q], take, dist, take ? (uint32_t)a.ids[row] : 0u);
       B = fminf(B, T);
     }
-    cnt = warp_compact(list, cnt, k);
-    unsigned long long* part = a.parts + (uint64_t)item * a.kmax;
-    for (int i = lane; i < cnt; i += 32) part[i] = list[i];
-    if (lane == 0) a.part_cnt[item] = cnt;
+    // the part: the kept entries that step 2's list does not hold (the merge
+    // starts from that list; most segments add none)
+    uint32_t kept = 0;
+    if (added) {
+      cnt = warp_compact(list, cnt, k);
+      // short segments end before their list is full: the query's other
+      // segments get this one's k-th distance here
+      if (lane == 0 && cnt == k) atomicMin(&a.qbound[q], (uint32_t)(list[k - 1] >> 32));
+      unsigned long long* part = a.parts + (uint64_t)item * a.kmax;
+      const unsigned long long* start = a.init + (uint64_t)q * kMaxK;
+      for (int base = 0; base < cnt; base += 32) {
+        const unsigned long long v = base + lane < cnt ? list[base + lane] : ~0ull;
+        int lo = 0, hi = c0;  // first entry of the starting list at or above v
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (start[mid] < v) lo = mid + 1;
+          else hi = mid;
+        }
+        const bool fresh = base + lane < cnt && !(lo < c0 && start[lo] == v);
+        const uint32_t m = __ballot_sync(HG_FULL, fresh);
+        if (fresh) part[kept + __popc(m & ((1u << lane) - 1))] = v;
+        kept += (uint32_t)__popc(m);
+      }
+    }
+    if (lane == 0) a.part_cnt[item] = (int)kept;
     __syncwarp();
   }
 #pragma unroll
@@ -400,38 +483,64 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_part(BatchRank a) {
   }
 }
 
-// Merge: one warp per query folds its starting list and its parts into the
+// Merge: one block per query folds its starting list and its parts into the
 // answer (k distinct distances, lowest id per distance) and verifies it:
 //   ok 1: the filter kept every row within B_q and the k-th distance is <= B_q;
 //   ok 0: the bucket overflowed but its first rows gave k distances below
 //         B_q: B_q is lowered to the k-th, the list kept, the query retried;
 //   ok -1: neither: the plain path answers it.
+// A warp takes 32 parts at a time (a lane per part: the parts hold few
+// entries), so only queries with more than 32 parts occupy the other warps,
+// whose lists the first warp folds in at the end.  (One warp per query, one
+// part after the other, took 42 us for 64 parts, all of it load latency.)
 __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_merge(BatchRank a) {
   __shared__ unsigned long long lists[kRankWarps][kWarpListCap];
+  __shared__ int s_cnt[kRankWarps];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int pos = blockIdx.x * kRankWarps + wib;
+  const int pos = blockIdx.x;
   if (pos >= (a.nlist_dev ? (int)*a.nlist_dev : a.nlist)) return;
   const int q = a.qlist ? (int)a.qlist[pos] : pos;
   unsigned long long* list = lists[wib];
   const int k = (int)a.kq[q];
   const float inf = __int_as_float(0x7f800000);
   const int c0 = a.init_cnt[q];
-  for (int i = lane; i < kWarpListCap; i += 32) list[i] = i < c0 ? a.init[(uint64_t)q * kMaxK + i] : ~0ull;
-  __syncwarp();
-  int cnt = c0;
-  float T = cnt == k ? __uint_as_float((uint32_t)(list[k - 1] >> 32)) : inf;
-  // the segments shared the query's running k-th distance: no entry above
-  // its final value can be among the k, and every part is sorted
-  const float Tq = __uint_as_float(ld_volatile(&a.qbound[q]));
   const uint32_t p0 = a.seg_prefix[pos], p1 = a.seg_prefix[pos + 1];
-  for (uint32_t p = p0; p < p1; ++p) {
-    const int pc = max(0, min(a.part_cnt[p], a.kmax));
-    const unsigned long long* part = a.parts + (uint64_t)p * a.kmax;
+  const int nw = (int)min((uint32_t)kRankWarps, max(1u, (p1 - p0 + 31) / 32));  // warps with parts
+  if (wib < nw) {
+    for (int i = lane; i < kWarpListCap; i += 32)
+      list[i] = (wib == 0 && i < c0) ? a.init[(uint64_t)q * kMaxK + i] : ~0ull;
+    __syncwarp();
+    int cnt = wib == 0 ? c0 : 0;
+    float T = wib == 0 && cnt == k ? __uint_as_float((uint32_t)(list[k - 1] >> 32)) : inf;
+    // the segments shared the query's running k-th distance: no entry above
+    // its final value can be among the k, and every part is sorted
+    const float Tq = __uint_as_float(ld_volatile(&a.qbound[q]));
+    for (uint32_t pb = p0 + 32 * wib; pb < p1; pb += 32 * nw) {
+      const uint32_t p = pb + lane;
+      const int pc = p < p1 ? max(0, min(a.part_cnt[p], a.kmax)) : 0;
+      const unsigned long long* part = a.parts + (uint64_t)p * a.kmax;
+      for (int e = 0;; ++e) {
+        const unsigned long long v = e < pc ? part[e] : ~0ull;
+        const float d = __uint_as_float((uint32_t)(v >> 32));
+        const bool take = e < pc && d <= Tq && d <= T;
+        if (!__any_sync(HG_FULL, take)) break;  // the parts are sorted: nothing further qualifies
+        warp_list_add<true>(list, cnt, T, k, nullptr, take, d, (uint32_t)v);
+      }
+    }
+    cnt = warp_compact(list, cnt, k);
+    if (lane == 0) s_cnt[wib] = cnt;
+  }
+  __syncthreads();
+  if (wib != 0) return;
+  int cnt = s_cnt[0];
+  float T = cnt == k ? __uint_as_float((uint32_t)(list[k - 1] >> 32)) : inf;
+  for (int w = 1; w < nw; ++w) {
+    const int pc = s_cnt[w];
     for (int base = 0; base < pc; base += 32) {
-      const unsigned long long v = base + lane < pc ? part[base + lane] : ~0ull;
+      const unsigned long long v = base + lane < pc ? lists[w][base + lane] : ~0ull;
       const float d = __uint_as_float((uint32_t)(v >> 32));
-      const bool take = base + lane < pc && d <= Tq && d <= T;
-      if (!__any_sync(HG_FULL, take)) break;  // sorted: nothing further qualifies
+      const bool take = base + lane < pc && d <= T;
+      if (!__any_sync(HG_FULL, take)) break;
       warp_list_add<true>(list, cnt, T, k, nullptr, take, d, (uint32_t)v);
     }
   }
@@ -832,11 +941,14 @@ cudaError_t launch_bound_select(const BatchRank& r, cudaStream_t s) {
   if (!r.nq) return cudaSuccess;
   int n = 32;
   while (n < (int)r.bm_cap) n <<= 1;
-  static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)k_bound_select, (int)(sizeof(unsigned long long) * kBatchMaxSlots));
-  if (ea != cudaSuccess) return ea;
-  k_bound_select<<<r.nq, kSelThreads, sizeof(unsigned long long) * n, s>>>(r);
-  return cudaGetLastError();
+  auto run = [&](auto kernel, SmemLimit& attr) {
+    const cudaError_t ea = attr.ensure((const void*)kernel, (int)(sizeof(unsigned long long) * kBatchMaxSlots));
+    if (ea != cudaSuccess) return ea;
+    kernel<<<r.nq, kSelThreads, sizeof(unsigned long long) * n, s>>>(r);
+    return cudaGetLastError();
+  };
+  static SmemLimit attr_long, attr_short;
+  return r.L >= kRankLongSeries ? run(k_bound_select<8>, attr_long) : run(k_bound_select<4>, attr_short);
 }
 
 cudaError_t launch_rerank(const BatchRank& r, int part_blocks, cudaStream_t s) {
@@ -844,11 +956,11 @@ cudaError_t launch_rerank(const BatchRank& r, int part_blocks, cudaStream_t s) {
   k_rerank_plan<<<1, 1024, 0, s>>>(r);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (r.L >= 4096) k_rerank_part<8, 2><<<part_blocks, kRankWarps * 32, 0, s>>>(r);
+  if (r.L >= kRankLongSeries) k_rerank_part<8, 2><<<part_blocks, kRankWarps * 32, 0, s>>>(r);
   else k_rerank_part<2, 4><<<part_blocks, kRankWarps * 32, 0, s>>>(r);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_rerank_merge<<<nblk(r.nlist, kRankWarps), kRankWarps * 32, 0, s>>>(r);
+  k_rerank_merge<<<r.nlist, kRankWarps * 32, 0, s>>>(r);
   return cudaGetLastError();
 }
 

@@ -13,8 +13,9 @@ constexpr int kBatchTileRows = 128;   // rows per tensor-core tile (and per tile
 constexpr int kBatchQueryTile = 256;  // queries per tensor-core tile (filter pass)
 constexpr int kBatchBoundQueries = 64;  // queries per tile in the bound pass (MMA N = 64)
 constexpr int kBatchMaxSlots = 4096;  // bound slots per query (sorted in one block)
-constexpr int kBatchMaxSeg = 64;      // re-rank segments per query
-constexpr int kBatchSegMin = 256;     // rows per re-rank segment, at least
+// re-rank segments over all queries of a round, beyond one per query: five for
+// each of the 32 warps resident on each of 148 SMs
+constexpr uint32_t kBatchSegTarget = 5 * 32 * 148;
 
 // One work item of the bound pass: tiles [tile_lo, tile_hi) of the rows
 // [row_begin, row_end) (one approximate leaf) against queries

@@ -1646,7 +1646,7 @@ static hg_status ensure_batch_scratch(hg_index* ix, uint32_t nq, uint32_t bucket
     CK(dalloc(&b.seg_rows, nq));
     CK(dalloc(&b.seg_prefix, (size_t)nq + 1));
     CK(dalloc(&b.qbound, nq));
-    CK(dalloc(&b.part_cnt, (size_t)nq * hg::kBatchMaxSeg));
+    CK(dalloc(&b.part_cnt, (size_t)nq + hg::kBatchSegTarget));
     b.nq_cap = nq;
     ++b.gen;  // a captured pipeline holds the old addresses
     b.bucket_cap = 0;
@@ -1663,7 +1663,7 @@ static hg_status ensure_batch_scratch(hg_index* ix, uint32_t nq, uint32_t bucket
   }
   if (kmax > b.parts_kmax || !b.parts) {
     dfree(b.parts);
-    CK(dalloc(&b.parts, (size_t)b.nq_cap * hg::kBatchMaxSeg * kmax));
+    CK(dalloc(&b.parts, ((size_t)b.nq_cap + hg::kBatchSegTarget) * kmax));
     b.parts_kmax = kmax;
     ++b.gen;  // a captured pipeline holds the old addresses
   }
