@@ -271,6 +271,29 @@ void collect_leaves(const std::vector<Node>& nodes, int n, std::vector<int>& out
 // device index assembly
 // ---------------------------------------------------------------------------
 
+static void free_scratch(hg_index* ix) {
+  hg::QueryScratch& s = ix->s;
+  dfree(s.lb);
+  dfree(s.approx_leaf);
+  dfree(s.cand);
+  dfree(s.cand_lb);
+  dfree(s.cand_count);
+  dfree(s.unit_prefix);
+  dfree(s.counters);
+  dfree(s.bound);
+  dfree(s.parts);
+  dfree(s.part_count);
+  dfree(s.topk);
+  dfree(s.topk_count);
+  dfree(s.sax_tab);
+  dfree(s.sort_keys);
+  dfree(s.list);
+  dfree(s.stats);
+  dfree(s.err);
+  dfree(s.actl);
+  s.slots = 0;
+}
+
 static void free_device(hg_index* ix) {
   hg::DeviceIndex& d = ix->d;
   dfree(d.rows);
@@ -284,28 +307,7 @@ static void free_device(hg_index* ix) {
   dfree(d.leaf_points);
   dfree(d.leaf_sk);
   dfree(d.nodes);
-  hg::QueryScratch& s = ix->s;
-  dfree(s.q);
-  dfree(s.lb);
-  dfree(s.approx_leaf);
-  dfree(s.cand);
-  dfree(s.cand_lb);
-  dfree(s.cand_count);
-  dfree(s.unit_prefix);
-  dfree(s.counters);
-  dfree(s.bound);
-  dfree(s.parts);
-  dfree(s.part_count);
-  dfree(s.topk);
-  dfree(s.topk_count);
-  dfree(s.topk_row);
-  dfree(s.paa);
-  dfree(s.sax_tab);
-  dfree(s.sort_keys);
-  dfree(s.stats);
-  dfree(s.err);
-  dfree(s.list);
-  s.kmax = 0;
+  free_scratch(ix);
   hg::BatchData& bd = ix->bd;
   dfree(bd.xbf);
   dfree(bd.xmeta);
@@ -1046,52 +1048,66 @@ static hg_status read_impl(const char* dir, int device, hg_index** out) {
 // queries
 // ---------------------------------------------------------------------------
 
-static hg_status ensure_scratch(hg_index* ix, int k) {
+// Queries of a plain call that share each launch: up to kGroupSlots, fewer
+// where the survivor lists (one entry per row and slot) would pass
+// kGroupListBytes, but four of them whatever the collection's size.  A group
+// hides the latency of a query's chain of small kernels behind the other
+// queries' scans and fills the GPU from indexes whose leaves are too small to
+// (per query, one at a time -> in groups: 1M x 256, leaf 100,000, k = 10:
+// 139 -> 28 us; 100k x 16384: 480 -> 92 us; 8M x 256, k = 100: 800 -> 390 us).
+constexpr uint32_t kGroupSlots = 32;
+constexpr uint64_t kGroupListBytes = 512ull << 20;
+static uint32_t group_slots(const hg_index* ix, uint32_t nq) {
+  const uint64_t by_list = std::max<uint64_t>(4, kGroupListBytes / (4 * std::max<uint64_t>(ix->n, 1)));
+  const uint32_t most = (uint32_t)std::min<uint64_t>(kGroupSlots, by_list);
+  const uint32_t groups = (nq + most - 1) / most;
+  return groups ? (nq + groups - 1) / groups : 1;
+}
+
+static cudaError_t alloc_scratch(hg_index* ix, size_t slots) {
   hg::QueryScratch& s = ix->s;
-  if (s.kmax >= k && s.q) return HG_OK;
-  const int nl = (int)ix->leaves.size();
-  dfree(s.q);
-  dfree(s.lb);
-  dfree(s.approx_leaf);
-  dfree(s.cand);
-  dfree(s.cand_lb);
-  dfree(s.cand_count);
-  dfree(s.unit_prefix);
-  dfree(s.bound);
-  dfree(s.parts);
-  dfree(s.part_count);
-  dfree(s.topk);
-  dfree(s.topk_count);
-  dfree(s.paa);
-  dfree(s.sax_tab);
-  dfree(s.sort_keys);
-  dfree(s.stats);
-  dfree(s.err);
-  dfree(s.list);
-  dfree(s.counters);
-  dfree(s.actl);
-  s.nparts = hg::sm_count(ix->device) * hg::ed_blocks_per_sm((int)ix->L) * hg::kEdWarps;
-  CK(dalloc(&s.lb, nl));
-  CK(dalloc(&s.list, ix->n));
-  CK(dalloc(&s.counters, 8));
-  CK(dalloc(&s.approx_leaf, 1));
-  CK(dalloc(&s.cand, nl + 1));
-  CK(dalloc(&s.cand_lb, nl + 1));
-  CK(dalloc(&s.cand_count, 1));
-  CK(dalloc(&s.unit_prefix, nl + 2));
-  CK(dalloc(&s.bound, 1));
-  CK(dalloc(&s.parts, (size_t)s.nparts * hg::kWarpListCap));
-  CK(dalloc(&s.part_count, s.nparts));
-  CK(dalloc(&s.topk, hg::kMaxK));
-  CK(dalloc(&s.topk_count, 1));
-  CK(dalloc(&s.paa, 16));
-  CK(dalloc(&s.sax_tab, HG_PAA_SEGMENTS * HG_SAX_CARD));
-  if (nl > hg::kMaxLeavesSort) CK(dalloc(&s.sort_keys, 4 * (size_t)nl));
-  CK(dalloc(&s.stats, 8));
-  CK(dalloc(&s.err, 1));
-  CK(dalloc(&s.q, 1));
-  CK(dalloc(&s.actl, 4));
-  s.kmax = hg::kMaxK;
+  const size_t nl = ix->leaves.size();
+  s.nparts = hg::sm_count(ix->device) * hg::ed_blocks_per_sm((int)ix->L);
+  cudaError_t e = cudaSuccess;
+  auto get = [&](auto** p, size_t count) {
+    if (e == cudaSuccess) e = dalloc(p, count);
+  };
+  get(&s.lb, slots * nl);
+  get(&s.list, slots * ix->n);
+  get(&s.counters, slots * 8);
+  get(&s.approx_leaf, slots);
+  get(&s.cand, slots * (nl + 1));
+  get(&s.cand_lb, slots * (nl + 1));
+  get(&s.cand_count, slots);
+  get(&s.unit_prefix, slots * (nl + 2));
+  get(&s.bound, slots);
+  get(&s.parts, slots * s.nparts * hg::kWarpListCap);
+  get(&s.part_count, slots * s.nparts);
+  get(&s.topk, slots * hg::kMaxK);
+  get(&s.topk_count, slots);
+  get(&s.sax_tab, slots * HG_PAA_SEGMENTS * HG_SAX_CARD);
+  if (nl > (size_t)hg::kMaxLeavesSort) get(&s.sort_keys, slots * 4 * nl);
+  get(&s.stats, 8);
+  get(&s.err, 1);
+  get(&s.actl, 4);
+  if (e == cudaSuccess) s.slots = (int)slots;
+  return e;
+}
+
+// Scratch for groups of `want` queries; where the device has no room for so
+// many, for half as many, down to one (the caller reads s.slots).
+static hg_status ensure_scratch(hg_index* ix, uint32_t want) {
+  hg::QueryScratch& s = ix->s;
+  if (s.slots > 0 && want <= s.asked) return HG_OK;
+  free_scratch(ix);
+  for (uint32_t slots = want;; slots = std::max<uint32_t>(1, slots / 2)) {
+    const cudaError_t e = alloc_scratch(ix, slots);
+    if (e == cudaSuccess) break;
+    free_scratch(ix);
+    if (e != cudaErrorMemoryAllocation || slots == 1) return cuda_fail(e, "query scratch");
+    cudaGetLastError();  // the failed allocation
+  }
+  s.asked = want;  // a smaller group was all there was room for: not tried again on each call
   return HG_OK;
 }
 
@@ -1131,125 +1147,164 @@ static double drain(ProfEvents& p) {
   return ms;
 }
 
-// One query through the plain path: approximate leaf, LB_EAPCA of every
-// leaf, scan of the approximate leaf, candidates by LB, scan, merge.
-
-
-
-// One query through the plain path:
-//   route + PAA (approximate_knn_search's traversal) -> LB_EAPCA of every
-//   leaf -> exact distances of the approximate leaf -> k-th bound ->
-//   candidate leaves sorted by LB -> LB_SAX filter -> exact distances of the
-//   survivors -> merge.
-static hg_status knn_one(hg_index* ix, const float* d_q, int k, const hg_knn_opts& o, float* d_dist,
-                         int64_t* d_id, cudaStream_t st, Prof* prof, bool has_floor = false, float floor = 0.0f) {
+static hg::EdArgs scan_args(hg_index* ix, const float* d_q, int k) {
   hg::QueryScratch& s = ix->s;
-  hg::DeviceIndex& d = ix->d;
-  const int nl = (int)ix->leaves.size();
-  const int sms = hg::sm_count(ix->device);
-  const int ed_blocks = sms * hg::ed_blocks_per_sm((int)ix->L);
   hg::EdArgs e{};
-  e.rows = d.rows;
-  e.ids = d.ids;
+  e.rows = ix->d.rows;
+  e.ids = ix->d.ids;
   e.L = (int)ix->L;
-  e.leaf_start = d.leaf_start;
-  e.leaf_size = d.leaf_size;
+  e.list_stride = ix->n;
+  e.leaf_start = ix->d.leaf_start;
+  e.leaf_size = ix->d.leaf_size;
+  e.min_batch = 1;
   e.q = d_q;
   e.k = k;
   e.bound = s.bound;
   e.parts = s.parts;
   e.part_count = s.part_count;
+  e.parts_stride = (uint32_t)s.nparts;
   e.stats = s.stats;
+  return e;
+}
+
+static hg::MergeArgs merge_args(hg_index* ix, int nparts, int k, float* d_dist = nullptr, int64_t* d_id = nullptr) {
+  hg::QueryScratch& s = ix->s;
+  hg::MergeArgs m{};
+  m.parts = s.parts;
+  m.part_count = s.part_count;
+  m.parts_stride = (uint32_t)s.nparts;
+  m.nparts = nparts;
+  m.k = k;
+  m.topk = s.topk;
+  m.topk_count = s.topk_count;
+  m.bound = s.bound;
+  m.dist_out = d_dist;
+  m.id_out = d_id;
+  return m;
+}
+
+static hg::PrepArgs prep_args(hg_index* ix, const float* d_q) {
+  hg::QueryScratch& s = ix->s;
+  hg::PrepArgs p{};
+  p.q = d_q;
+  p.L = (int)ix->L;
+  p.tree = index_tree(ix);
+  p.nleaves = (int)ix->leaves.size();
+  p.seg_off = ix->d.leaf_seg_off;
+  p.points = ix->d.leaf_points;
+  p.sk = ix->d.leaf_sk;
+  p.bp = ix->d.bp;
+  p.approx_leaf = s.approx_leaf;
+  p.bound = s.bound;
+  p.topk_count = s.topk_count;
+  p.counters = s.counters;
+  return p;
+}
+
+// A group of queries (at most s.slots, consecutive at d_q) through the plain
+// path, each launch serving all of them:
+//   route, LB_EAPCA of every leaf, LB_SAX terms -> exact distances of the
+//   approximate leaf -> merge: k-th bound, candidate leaves sorted by LB ->
+//   LB_SAX filter -> exact distances of the survivors -> merge: answers.
+static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, const hg_knn_opts& o, float* d_dist,
+                           int64_t* d_id, cudaStream_t st, Prof* prof, uint64_t* launches, bool has_floor = false,
+                           float floor = 0.0f) {
+  hg::QueryScratch& s = ix->s;
+  hg::DeviceIndex& d = ix->d;
+  const int sms = hg::sm_count(ix->device);
+  const int ed_blocks = sms * hg::ed_blocks_per_sm((int)ix->L);
+  hg::EdArgs e = scan_args(ix, d_q, k);
   e.has_floor = has_floor ? 1 : 0;
   e.floor = floor;
+  auto scan = [&](int blocks) -> hg_status {
+    HCK(timed_begin(prof ? &prof->ed : nullptr, st));
+    CK(hg::launch_ed_stream(e, slots, blocks, st));
+    return timed_end(prof ? &prof->ed : nullptr, st);
+  };
   if (o.mode == HG_MODE_PSCAN) {
-    CK(hg::launch_pscan_prep(ix->n, s.cand_count, s.unit_prefix, s.bound, s.topk_count, s.counters, st));
-    e.list = nullptr;
-    e.ident_leaf = nullptr;
-    e.ident_first = 0;
+    // every query's blocks resident at once: they walk the rows from the
+    // front at the same pace, so the group reads most rows from L2
+    const int blocks = std::max(1, ed_blocks / slots);
+    CK(hg::launch_pscan_prep(s.bound, s.topk_count, slots, st));
     e.ident_count = ix->n;
-    e.head = s.counters + 0;
-    HCK(timed_begin(prof ? &prof->ed : nullptr, st));
-    CK(hg::launch_ed_stream(e, ed_blocks, st));
-    HCK(timed_end(prof ? &prof->ed : nullptr, st));
-    CK(hg::launch_merge(s.parts, s.part_count, ed_blocks, k, s.topk, s.topk_count, s.bound, s.err,
-                        st));
-  } else {
-    CK(hg::launch_query_prep(d_q, e.L, index_tree(ix), d.leaf_start, d.leaf_size, s.approx_leaf, s.paa, s.cand,
-                             s.cand_lb, s.cand_count, s.unit_prefix, s.bound, s.topk_count, s.counters, st));
-    CK(hg::launch_leaf_lb(d_q, e.L, nl, d.leaf_seg_off, d.leaf_points, d.leaf_sk, s.lb, st, s.paa, d.bp,
-                          o.use_lb_sax ? s.sax_tab : nullptr));
-    // the approximate leaf, with an unbounded k-th distance at the start
-        // two blocks per SM: the bound starts at +inf, so more warps would finish
-    // more rows of this leaf before it tightens; fewer leave HBM idle
-    const int a_blocks =
-        std::max(1, std::min(ed_blocks, o.approx_blocks > 0 ? o.approx_blocks : (int)ix->tune.approx_blocks_per_sm * sms));
-    e.list = nullptr;
-    e.ident_leaf = s.approx_leaf;
-    e.head = s.counters + 0;
-    HCK(timed_begin(prof ? &prof->ed : nullptr, st));
-    CK(hg::launch_ed_stream(e, a_blocks, st));
-    HCK(timed_end(prof ? &prof->ed : nullptr, st));
-    CK(hg::launch_merge(s.parts, s.part_count, a_blocks, k, s.topk, s.topk_count, s.bound, s.err,
-                        st));
-    CK(hg::launch_select_sort(s.lb, nl, s.bound, s.approx_leaf, d.leaf_start, d.leaf_size, s.cand, s.cand_lb,
-                              s.cand_count, s.unit_prefix, st, s.sort_keys));
-    // greedy seeding (the paper's L_max): the next approx_leaves - 1
-    // candidates in LB order, scanned before the rest so that the bound the
-    // rest is filtered against is tighter; the merge folds them in
-    const int seed = (o.mode == HG_MODE_PLAIN && o.approx_leaves > 1) ? o.approx_leaves - 1 : 0;
-    hg::FilterArgs f{};
-    f.sax = d.sax;
-    f.bp = d.bp;
-    f.L = e.L;
-    f.nrows = ix->n;
-    f.leaf_start = d.leaf_start;
-    f.leaf_size = d.leaf_size;
-    f.cand = s.cand;
-    f.cand_lb = s.cand_lb;
-    f.cand_count = s.cand_count;
-    f.unit_prefix = s.unit_prefix;
-    f.paa = s.paa;
-    f.sax_tab = s.sax_tab;
-    f.use_lbsax = o.use_lb_sax ? 1 : 0;
-    f.bound = s.bound;
-    f.list = s.list;
-    f.stats = s.stats;
-    f.err = s.err;
-    if (seed > 0) {
-      f.cand_lo = 0;
-      f.cand_hi = seed;
-      f.list_count = s.counters + 4;
-      HCK(timed_begin(prof ? &prof->filter : nullptr, st));
-      CK(hg::launch_lbsax_filter(f, sms, st));
-      HCK(timed_end(prof ? &prof->filter : nullptr, st));
-      e.list = s.list;
-      e.list_count = s.counters + 4;
-      e.ident_leaf = nullptr;
-      e.head = s.counters + 5;
-      HCK(timed_begin(prof ? &prof->ed : nullptr, st));
-      CK(hg::launch_ed_stream(e, ed_blocks, st));
-      HCK(timed_end(prof ? &prof->ed : nullptr, st));
-      CK(hg::launch_merge(s.parts, s.part_count, ed_blocks, k, s.topk, s.topk_count, s.bound, s.err, st));
-      f.cand_lo = seed;
-      f.cand_hi = 0;
-    }
-    f.list_count = s.counters + 2;
-    HCK(timed_begin(prof ? &prof->filter : nullptr, st));
-    CK(hg::launch_lbsax_filter(f, sms, st));
-    HCK(timed_end(prof ? &prof->filter : nullptr, st));
-    e.list = s.list;
-    e.list_count = s.counters + 2;
-    e.ident_leaf = nullptr;
-    e.head = s.counters + 1;
-    HCK(timed_begin(prof ? &prof->ed : nullptr, st));
-    CK(hg::launch_ed_stream(e, ed_blocks, st));
-    HCK(timed_end(prof ? &prof->ed : nullptr, st));
-    // the merge folds the approximate leaf's top-k (in topk) into the result
-    CK(hg::launch_merge(s.parts, s.part_count, ed_blocks, k, s.topk, s.topk_count, s.bound, s.err,
-                        st));
+    HCK(scan(blocks));
+    CK(hg::launch_merge(merge_args(ix, blocks, k, d_dist, d_id), slots, st));
+    *launches += 3;
+    return HG_OK;
   }
-  CK(hg::launch_emit(s.topk, s.topk_count, k, d_dist, d_id, st));
+  hg::PrepArgs p = prep_args(ix, d_q);
+  p.lb = s.lb;
+  p.sax_tab = o.use_lb_sax ? s.sax_tab : nullptr;
+  CK(hg::launch_query_prep(p, slots, st));
+  // the approximate leaf, with an unbounded k-th distance at the start: two
+  // blocks per SM, as more warps would finish more rows of this leaf before
+  // it tightens, and fewer leave HBM idle
+  const int a_blocks =
+      std::max(1, std::min(ed_blocks, o.approx_blocks > 0 ? o.approx_blocks : (int)ix->tune.approx_blocks_per_sm * sms));
+  // a warp's entries: one row per slot of its lanes for a query alone; a
+  // group keeps the GPU full by itself, so its warps take longer runs and
+  // fewer blocks stage a query and sort a list
+  e.min_batch = slots > 1 ? (ix->L >= 4096 ? 8u : 32u) : (ix->L >= 4096 ? 4u : 8u);
+  e.ident_leaf = s.approx_leaf;
+  HCK(scan(a_blocks));
+  hg::SelectArgs sel{};
+  sel.lb = s.lb;
+  sel.nleaves = (int)ix->leaves.size();
+  sel.approx_leaf = s.approx_leaf;
+  sel.leaf_start = d.leaf_start;
+  sel.leaf_size = d.leaf_size;
+  sel.cand = s.cand;
+  sel.cand_lb = s.cand_lb;
+  sel.cand_count = s.cand_count;
+  sel.unit_prefix = s.unit_prefix;
+  sel.gkeys = s.sort_keys;
+  CK(hg::launch_merge_select(merge_args(ix, a_blocks, k), sel, slots, st));
+  hg::FilterArgs f{};
+  f.sax = d.sax;
+  f.L = e.L;
+  f.nleaves = sel.nleaves;
+  f.leaf_start = d.leaf_start;
+  f.leaf_size = d.leaf_size;
+  f.cand = s.cand;
+  f.cand_lb = s.cand_lb;
+  f.cand_count = s.cand_count;
+  f.unit_prefix = s.unit_prefix;
+  f.sax_tab = s.sax_tab;
+  f.use_lbsax = o.use_lb_sax ? 1 : 0;
+  f.bound = s.bound;
+  f.list = s.list;
+  f.list_stride = ix->n;
+  f.stats = s.stats;
+  f.err = s.err;
+  e.ident_leaf = nullptr;
+  e.list = s.list;
+  // one filter block is resident per SM: a query alone takes them all, a
+  // group a share each, with some to spare for its larger queries
+  const int f_blocks = std::min(sms, std::max(1, 4 * sms / slots));
+  auto filter_scan_merge = [&](uint32_t* count, float* dist, int64_t* id) -> hg_status {
+    f.list_count = count;
+    HCK(timed_begin(prof ? &prof->filter : nullptr, st));
+    CK(hg::launch_lbsax_filter(f, slots, f_blocks, st));
+    HCK(timed_end(prof ? &prof->filter : nullptr, st));
+    e.list_count = count;
+    HCK(scan(ed_blocks));
+    // the merge folds the earlier stages' top-k into the result
+    CK(hg::launch_merge(merge_args(ix, ed_blocks, k, dist, id), slots, st));
+    *launches += 3;
+    return HG_OK;
+  };
+  // greedy seeding (the paper's L_max): the next approx_leaves - 1
+  // candidates in LB order, scanned before the rest so that the bound the
+  // rest is filtered against is tighter
+  const int seed = (o.mode == HG_MODE_PLAIN && o.approx_leaves > 1) ? o.approx_leaves - 1 : 0;
+  if (seed > 0) {
+    f.cand_hi = seed;
+    HCK(filter_scan_merge(s.counters + 4, nullptr, nullptr));
+    f.cand_lo = seed;
+    f.cand_hi = 0;
+  }
+  HCK(filter_scan_merge(s.counters + 2, d_dist, d_id));
+  *launches += 3;
   return HG_OK;
 }
 
@@ -1315,28 +1370,14 @@ static bool pq_pop(std::vector<PqEntry>& h, PqEntry* out) {
 static hg_status knn_approx_one(hg_index* ix, const float* d_q, int k, const hg_knn_opts& o, float* d_dist,
                                 int64_t* d_id, cudaStream_t st) {
   hg::QueryScratch& s = ix->s;
-  hg::DeviceIndex& d = ix->d;
   const int L = (int)ix->L;
   const int sms = hg::sm_count(ix->device);
   const int ed_blocks = sms * hg::ed_blocks_per_sm(L);
-  hg::EdArgs e{};
-  e.rows = d.rows;
-  e.ids = d.ids;
-  e.L = L;
-  e.leaf_start = d.leaf_start;
-  e.leaf_size = d.leaf_size;
-  e.q = d_q;
-  e.k = k;
-  e.bound = s.bound;
-  e.parts = s.parts;
-  e.part_count = s.part_count;
-  e.stats = s.stats;
-  e.head = s.counters + 0;
-  CK(hg::launch_query_prep(d_q, L, index_tree(ix), d.leaf_start, d.leaf_size, s.approx_leaf, s.paa, s.cand,
-                           s.cand_lb, s.cand_count, s.unit_prefix, s.bound, s.topk_count, s.counters, st));
+  hg::EdArgs e = scan_args(ix, d_q, k);
+  CK(hg::launch_query_prep(prep_args(ix, d_q), 1, st));
   e.ident_leaf = s.approx_leaf;
-  CK(hg::launch_ed_stream(e, ed_blocks, st));
-  CK(hg::launch_merge(s.parts, s.part_count, ed_blocks, k, s.topk, s.topk_count, s.bound, s.err, st));
+  CK(hg::launch_ed_stream(e, 1, ed_blocks, st));
+  CK(hg::launch_merge(merge_args(ix, ed_blocks, k), 1, st));
   std::vector<float> q(L);
   int approx = -1, cnt = 0;
   uint32_t bound_bits = 0;
@@ -1378,15 +1419,14 @@ static hg_status knn_approx_one(hg_index* ix, const float* d_q, int k, const hg_
     if (count > 1) {
       e.ident_first = first;
       e.ident_count = count - 1;
-      CK(hg::launch_ed_stream(e, ed_blocks, st));
-      CK(hg::launch_merge(s.parts, s.part_count, ed_blocks, k, s.topk, s.topk_count, s.bound,
-                          s.err, st));
+      CK(hg::launch_ed_stream(e, 1, ed_blocks, st));
+      CK(hg::launch_merge(merge_args(ix, ed_blocks, k), 1, st));
     }
     CK(hg::launch_stale_copy(flag, s.bound, stale, st));
     e.ident_first = first + count - 1;
     e.ident_count = 1;
-    CK(hg::launch_ed_stream(e, 1, st));
-    CK(hg::launch_merge(s.parts, s.part_count, 1, k, s.topk, s.topk_count, s.bound, s.err, st));
+    CK(hg::launch_ed_stream(e, 1, 1, st));
+    CK(hg::launch_merge(merge_args(ix, 1, k), 1, st));
     return HG_OK;
   };
   std::vector<PqEntry> pq;
@@ -1456,9 +1496,8 @@ static hg_status knn_rounds(hg_index* ix, const float* d_q, uint32_t k, const hg
   float floor = 0.0f;
   while (done < k) {
     const int kr = (int)std::min<uint32_t>((uint32_t)hg::kMaxK, k - done);
-    HCK(knn_one(ix, d_q, kr, o, d_dist ? d_dist + done : nullptr, d_id ? d_id + done : nullptr, st, prof, has_floor,
-                floor));
-    *launches += o.mode == HG_MODE_PSCAN ? 4 : (o.approx_leaves > 1 ? 12 : 9);
+    HCK(knn_group(ix, d_q, 1, kr, o, d_dist ? d_dist + done : nullptr, d_id ? d_id + done : nullptr, st, prof, launches,
+                  has_floor, floor));
     int cnt = 0;
     unsigned long long last = 0;
     CK(cudaMemcpyAsync(&cnt, s.topk_count, sizeof cnt, cudaMemcpyDeviceToHost, st));
@@ -1499,7 +1538,9 @@ static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t 
   if (approx && (int)k > hg::kMaxK)
     return set_error(HG_ERR_LIMIT, "hg_knn: k above 224 with epsilon or nprobes");
   CK(cudaSetDevice(ix->device));
-  HCK(ensure_scratch(ix, std::min((int)k, hg::kMaxK)));
+  // rounds and approximate searches follow one query at a time
+  const bool grouped = !approx && (int)k <= hg::kMaxK;
+  HCK(ensure_scratch(ix, grouped ? group_slots(ix, nq) : 1));
   if (!st) st = ix->stream;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1509,20 +1550,15 @@ static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t 
   Prof prof;
   CK(cudaEventRecord(e0, st));
   uint64_t launches = 0;
-  for (uint32_t i = 0; i < nq; ++i) {
+  const uint32_t per = grouped ? std::min<uint32_t>(group_slots(ix, nq), (uint32_t)ix->s.slots) : 1;
+  for (uint32_t i = 0; i < nq; i += per) {
     const float* qi = d_queries + (uint64_t)i * ix->L;
     float* di = d_dist ? d_dist + (uint64_t)i * k : nullptr;
     int64_t* ii = d_id ? d_id + (uint64_t)i * k : nullptr;
-    if (approx) {
-      HCK(knn_approx_one(ix, qi, (int)k, o, di, ii, st));
-    } else if ((int)k <= hg::kMaxK) {
-      HCK(knn_one(ix, qi, (int)k, o, di, ii, st, o.profile ? &prof : nullptr));
-      launches += o.mode == HG_MODE_PSCAN ? 4 : (o.approx_leaves > 1 ? 12 : 9);
-    } else {
-      uint64_t l = 0;
-      HCK(knn_rounds(ix, qi, k, o, di, ii, st, o.profile ? &prof : nullptr, &l));
-      launches += l;
-    }
+    Prof* pr = o.profile ? &prof : nullptr;
+    if (approx) HCK(knn_approx_one(ix, qi, (int)k, o, di, ii, st));
+    else if (grouped) HCK(knn_group(ix, qi, (int)std::min(per, nq - i), (int)k, o, di, ii, st, pr, &launches));
+    else HCK(knn_rounds(ix, qi, k, o, di, ii, st, pr, &launches));
   }
   CK(cudaEventRecord(e1, st));
   unsigned long long hs[8];
@@ -2110,7 +2146,7 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   if (nq == 0) return HG_OK;
   CK(cudaSetDevice(ix->device));
   if (!st) st = ix->stream;
-  HCK(ensure_scratch(ix, (int)kmax));
+  HCK(ensure_scratch(ix, 1));
   const bool data_built = ix->bd.xbf == nullptr;
   HCK(ensure_batch_data(ix, st));
   const uint32_t L = ix->L;
@@ -2198,7 +2234,7 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   CK(cudaEventCreate(&fb0));
   CK(cudaEventCreate(&fb1));
   CK(cudaEventRecord(fb0, st));
-  uint64_t fallbacks = 0;
+  uint64_t fallbacks = 0, fallback_launches = 0;
   hg_status fs = HG_OK;
   if (ctrl[3] > 0) {
     std::vector<int> ok(nq);
@@ -2210,8 +2246,8 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
     for (uint32_t q = 0; q < nq && fs == HG_OK; ++q) {
       if (ok[q] == 1) continue;
       ++fallbacks;
-      fs = knn_one(ix, b.qin + (uint64_t)q * L, (int)kq[q], po, b.out_dist + (uint64_t)q * kmax,
-                   b.out_id + (uint64_t)q * kmax, st, nullptr);
+      fs = knn_group(ix, b.qin + (uint64_t)q * L, 1, (int)kq[q], po, b.out_dist + (uint64_t)q * kmax,
+                     b.out_id + (uint64_t)q * kmax, st, nullptr, &fallback_launches);
     }
   }
   cudaEventRecord(fb1, st);
@@ -2265,7 +2301,7 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
     stats->rerank_ms = rerank;
     stats->fallback_ms = fallbacks ? tf : 0.0;
     stats->device_ms = t0e;
-    stats->kernel_launches = launches + (data_built ? 2 : 0) + 9 * fallbacks;
+    stats->kernel_launches = launches + (data_built ? 2 : 0) + fallback_launches;
     stats->err_mean = es[2] > 0 ? es[0] / es[2] : 0.0;
     stats->err_max = es[4];
     stats->err_over_bound = es[3] > 0 ? es[1] / es[3] : 0.0;
@@ -2815,8 +2851,12 @@ hg_status hg_leaf_lower_bounds(hg_index* ix, const float* query, float* lb_out) 
   CK(dalloc(&d_q, ix->L));
   cudaError_t e = dalloc(&d_lb, nl);
   if (e == cudaSuccess) e = cudaMemcpy(d_q, query, sizeof(float) * ix->L, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = hg::launch_leaf_lb(d_q, (int)ix->L, nl, ix->d.leaf_seg_off, ix->d.leaf_points, ix->d.leaf_sk, d_lb, ix->stream);
+  if (e == cudaSuccess) {
+    hg::PrepArgs p = prep_args(ix, d_q);
+    p.approx_leaf = nullptr;  // lower bounds only
+    p.lb = d_lb;
+    e = hg::launch_query_prep(p, 1, ix->stream);
+  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(lb_out, d_lb, sizeof(float) * nl, cudaMemcpyDeviceToHost, ix->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ix->stream);
   cudaFree(d_q);

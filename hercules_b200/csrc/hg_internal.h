@@ -51,29 +51,29 @@ struct DeviceIndex {
   int root = 0;
 };
 
-// Per-query scratch for the plain path (sized for the largest k).
+// Scratch of the plain path for `slots` queries at a time (hg_kernels.h: one
+// entry or run per slot).
 struct QueryScratch {
-  int kmax = 0;
-  int nparts = 0;
-  float* q = nullptr;             // L
+  int slots = 0;                  // 0: not allocated
+  uint32_t asked = 0;             // the slots asked for (slots of them fitted)
+  int nparts = 0;                 // lists per slot
   float* lb = nullptr;            // leaves
   int* approx_leaf = nullptr;     // 1
-  int* cand = nullptr;            // leaves
-  float* cand_lb = nullptr;       // leaves
+  int* cand = nullptr;            // leaves + 1
+  float* cand_lb = nullptr;       // leaves + 1
   int* cand_count = nullptr;      // 1
-  uint32_t* unit_prefix = nullptr;  // leaves + 1 (tiles per candidate, exclusive scan)
-  uint32_t* counters = nullptr;   // work counter, misc
+  uint32_t* unit_prefix = nullptr;  // leaves + 2 (32-row units per candidate, exclusive scan)
+  uint32_t* counters = nullptr;   // 8: [2] filter survivors, [4] the seeding stage's
   uint32_t* bound = nullptr;      // float bits of the current k-th distance bound
-  unsigned long long* parts = nullptr;  // nparts x kmax keys (d bits << 32 | id)
+  unsigned long long* parts = nullptr;  // nparts x kWarpListCap keys (d bits << 32 | id)
   int* part_count = nullptr;      // nparts
-  unsigned long long* topk = nullptr;   // kmax keys
-  int* topk_count = nullptr;
-  uint64_t* topk_row = nullptr;   // kmax leaf-ordered rows of the answers
-  float* paa = nullptr;           // 16
-  float* sax_tab = nullptr;       // 16 x 256 LB_SAX terms of the current query
+  unsigned long long* topk = nullptr;   // kMaxK keys
+  int* topk_count = nullptr;      // 1
+  float* sax_tab = nullptr;       // 16 x 256 LB_SAX terms of the query
   uint32_t* sort_keys = nullptr;  // 4 x leaves: candidate sort above kMaxLeavesSort leaves
-  unsigned long long* stats = nullptr;  // see ScanArgs
   uint32_t* list = nullptr;       // LB_SAX survivors (rows), n entries
+  // shared by the slots
+  unsigned long long* stats = nullptr;  // counters of the call (knn_device_impl)
   int* err = nullptr;             // device error flag
   uint32_t* actl = nullptr;       // approximate searches: [0] stale k-th bound bits, [1] gate flag
 };

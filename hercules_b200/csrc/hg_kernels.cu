@@ -42,10 +42,21 @@ __device__ void warp_mean_stdev(const float* v, int from, int to, float* mean, f
       cs = hg_hsum8(x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]);
       cq = hg_hsum8(x2[0], x2[1], x2[2], x2[3], x2[4], x2[5], x2[6], x2[7]);
     }
+    // eight chunks a turn, so the shuffles run ahead of the two chains of
+    // adds; a chunk past the end adds 0, which leaves the sums unchanged
     const int lim = min(32, nch - base);
-    for (int j = 0; j < lim; ++j) {
-      sum = __fadd_rn(sum, __shfl_sync(HG_FULL, cs, j));
-      sumsq = __fadd_rn(sumsq, __shfl_sync(HG_FULL, cq, j));
+    for (int j = 0; j < lim; j += 8) {
+      float s8[8], q8[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        s8[t] = __shfl_sync(HG_FULL, cs, j + t);
+        q8[t] = __shfl_sync(HG_FULL, cq, j + t);
+      }
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        sum = __fadd_rn(sum, s8[t]);
+        sumsq = __fadd_rn(sumsq, q8[t]);
+      }
     }
   }
   const float fc = (float)count;
@@ -222,34 +233,6 @@ __global__ void k_sax_rows(const float* __restrict__ rows, int L, uint64_t n, co
 // query kernels
 // ---------------------------------------------------------------------------
 
-// One warp: route the query (approximate_knn_search's traversal), compute
-// its PAA, and set the first scan phase to the approximate leaf with an
-// unbounded k-th distance.
-__global__ void k_query_prep(const float* __restrict__ q, int L, Tree t, const uint64_t* __restrict__ leaf_start,
-                             const uint32_t* __restrict__ leaf_size, int* approx_leaf, float* paa, int* cand,
-                             float* cand_lb, int* cand_count, uint32_t* unit_prefix, uint32_t* bound,
-                             int* topk_count, uint32_t* counters) {
-  const int lane = threadIdx.x & 31;
-  if (lane < 6) counters[lane] = 0;
-  const int leaf = warp_route(q, t);
-  if (lane < HG_PAA_SEGMENTS) {
-    const int per = L / HG_PAA_SEGMENTS;
-    float acc = 0.0f;
-    for (int i = 0; i < per; ++i) acc = __fadd_rn(acc, q[lane * per + i]);
-    paa[lane] = __fdiv_rn(acc, (float)per);
-  }
-  if (lane == 0) {
-    *approx_leaf = leaf;
-    cand[0] = leaf;
-    cand_lb[0] = 0.0f;
-    *cand_count = 1;
-    unit_prefix[0] = 0;
-    unit_prefix[1] = tiles_of_leaf(leaf_start[leaf], leaf_size[leaf]);
-    *bound = 0x7f800000u;  // +inf
-    *topk_count = 0;
-  }
-}
-
 __global__ void k_route_queries(const float* __restrict__ Q, int nq, int L, Tree t, int* __restrict__ leaf_out) {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= nq) return;
@@ -257,34 +240,62 @@ __global__ void k_route_queries(const float* __restrict__ Q, int nq, int L, Tree
   if ((threadIdx.x & 31) == 0) leaf_out[w] = leaf;
 }
 
-// LB_EAPCA of every leaf (a warp per leaf).  With sax_tab set, the
-// threads also write the query's LB_SAX term table for the filter:
-// sax_tab[t * 256 + s] = hg_lb_sax_lane(paa[t], s) (reference arithmetic,
-// sax.c:310-479), 4,096 entries, computed once per query.
-__global__ void k_leaf_lb(const float* __restrict__ q, int L, int nleaves, const int* __restrict__ seg_off,
-                          const short* __restrict__ points, const float* __restrict__ sk, float* __restrict__ lb,
-                          const float* __restrict__ paa, const float* __restrict__ bp, float* __restrict__ sax_tab) {
+// The start of a group of queries, grid (slots, blocks), one launch instead of
+// three on the way to the first scan: blocks y < gridDim.y - 1 compute
+// LB_EAPCA of the leaves (a warp per leaf) and, with sax_tab set, block y <
+// 16 the LB_SAX terms of segment y (sax_tab[y * 256 + s] =
+// hg_lb_sax_lane(paa[y], s), reference arithmetic, sax.c:310-479); the last
+// block routes the query (approximate_knn_search's traversal) and resets its
+// state for a scan with an unbounded k-th distance.  Bound by latency: the
+// routing is a chain of node and segment reads, one per tree level.
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads) k_query_prep(PrepArgs a) {
   extern __shared__ float qs[];
-  if (sax_tab) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < HG_PAA_SEGMENTS * HG_SAX_CARD;
-         i += gridDim.x * blockDim.x)
-      sax_tab[i] = hg_lb_sax_lane(paa[i >> 8], i & 255, bp);
-  }
-  for (int i = threadIdx.x; i < L; i += blockDim.x) qs[i] = q[i];
+  __shared__ float s_paa;
+  const uint32_t slot = blockIdx.x;
+  const float* q = a.q + (uint64_t)slot * a.L;
+  for (int i = threadIdx.x; i < a.L; i += kPrepThreads) qs[i] = q[i];
   __syncthreads();
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= nleaves) return;
-  const int off = seg_off[w], nseg = seg_off[w + 1] - off;
-  float sum = 0.0f;
-  int start = 0;
-  for (int s = 0; s < nseg; ++s) {
-    const int end = points[off + s];
-    float m, sd;
-    warp_mean_stdev(qs, start, end, &m, &sd);
-    sum = __fadd_rn(sum, hg_eapca_term(m, sd, sk + 4 * (off + s), end - start));
-    start = end;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.y == gridDim.y - 1) {
+    if (!a.approx_leaf || warp != 0) return;
+    if (lane < 8) a.counters[8 * slot + lane] = 0;
+    const int leaf = warp_route(qs, a.tree);
+    if (lane == 0) {
+      a.approx_leaf[slot] = leaf;
+      a.bound[slot] = 0x7f800000u;  // +inf
+      a.topk_count[slot] = 0;
+    }
+    return;
   }
-  if ((threadIdx.x & 31) == 0) lb[w] = sum;
+  if (a.sax_tab && blockIdx.y < HG_PAA_SEGMENTS) {
+    // paa_from_ts (sax.c:46-56): a sequential sum, one division
+    const int t = blockIdx.y, per = a.L / HG_PAA_SEGMENTS;
+    if (threadIdx.x == 0) {
+      float acc = 0.0f;
+#pragma unroll 8
+      for (int i = 0; i < per; ++i) acc = __fadd_rn(acc, qs[t * per + i]);
+      s_paa = __fdiv_rn(acc, (float)per);
+    }
+    __syncthreads();
+    static_assert(kPrepThreads == HG_SAX_CARD, "a thread per symbol");
+    a.sax_tab[(uint64_t)slot * (HG_PAA_SEGMENTS * HG_SAX_CARD) + t * HG_SAX_CARD + threadIdx.x] =
+        hg_lb_sax_lane(s_paa, threadIdx.x, a.bp);
+  }
+  if (!a.lb) return;
+  for (int w = blockIdx.y * (kPrepThreads / 32) + warp; w < a.nleaves; w += (gridDim.y - 1) * (kPrepThreads / 32)) {
+    const int off = a.seg_off[w], nseg = a.seg_off[w + 1] - off;
+    float sum = 0.0f;
+    int start = 0;
+    for (int s = 0; s < nseg; ++s) {
+      const int end = a.points[off + s];
+      float m, sd;
+      warp_mean_stdev(qs, start, end, &m, &sd);
+      sum = __fadd_rn(sum, hg_eapca_term(m, sd, a.sk + 4 * (off + s), end - start));
+      start = end;
+    }
+    if (lane == 0) a.lb[(uint64_t)slot * a.nleaves + w] = sum;
+  }
 }
 
 // Mean and stdev of every query over every distinct leaf segment (leaves
@@ -314,7 +325,7 @@ __global__ void k_query_segstats(const float* __restrict__ Q, int L, int nq, con
 
 // Leaves each query of a batch must filter: a thread per (query, leaf) sums
 // the LB_EAPCA terms of the leaf's segments in order (the plain path's
-// k_leaf_lb arithmetic, segment statistics from k_query_segstats; the terms
+// k_query_prep arithmetic, segment statistics from k_query_segstats; the terms
 // are >= 0, so the sum stops once it exceeds the limit) and keeps the leaf
 // when
 //     LB <= B_q (1 + 2^-10) + L 2^-20,
@@ -362,15 +373,17 @@ __global__ void k_leaf_keep(const float2* __restrict__ segstats, int nu, int L, 
 // empty; ordered by LB with a stable LSD radix sort (4-bit digits, 8 passes)
 // in one CTA; then the exclusive prefix of their tile counts.
 constexpr int kSortThreads = 1024;
-__global__ void __launch_bounds__(kSortThreads) k_select_sort(const float* __restrict__ lb, int nleaves,
-                                                              const uint32_t* bound, const int* approx_leaf,
-                                                              const uint64_t* __restrict__ leaf_start,
-                                                              const uint32_t* __restrict__ leaf_size, int* cand,
-                                                              float* cand_lb, int* cand_count,
-                                                              uint32_t* unit_prefix, uint32_t* gkeys) {
+__device__ void select_sort(const SelectArgs& a, uint32_t slot, float B, uint32_t* sm) {
+  const int nleaves = a.nleaves;
+  const float* __restrict__ lb = a.lb + (uint64_t)slot * nleaves;
+  const uint64_t* __restrict__ leaf_start = a.leaf_start;
+  const uint32_t* __restrict__ leaf_size = a.leaf_size;
+  int* cand = a.cand + (uint64_t)slot * (nleaves + 1);
+  float* cand_lb = a.cand_lb + (uint64_t)slot * (nleaves + 1);
+  uint32_t* unit_prefix = a.unit_prefix + (uint64_t)slot * (nleaves + 2);
   // keys and values (two buffers each) live in shared memory up to
   // kMaxLeavesSort leaves, else in gkeys (4 x nleaves words of global memory)
-  extern __shared__ uint32_t sm[];
+  uint32_t* gkeys = a.gkeys ? a.gkeys + (uint64_t)slot * 4 * nleaves : nullptr;
   uint32_t* cnt = sm;  // 16 x kSortThreads digit counts
   uint32_t* kbase = gkeys ? gkeys : sm + 16 * kSortThreads;
   const int cap = gkeys ? nleaves : kMaxLeavesSort;
@@ -381,8 +394,7 @@ __global__ void __launch_bounds__(kSortThreads) k_select_sort(const float* __res
   __shared__ uint32_t tmp[kSortThreads / 32 + 1];
   __shared__ uint32_t total;
   const int t = threadIdx.x;
-  const float B = __int_as_float((int)ld_volatile(bound));
-  const int approx = *approx_leaf;
+  const int approx = a.approx_leaf[slot];
   // 1. select the non-empty leaves within the bound, the approximate leaf
   //    excepted (it was scanned first), order preserving
   const int per = (nleaves + kSortThreads - 1) / kSortThreads;
@@ -492,20 +504,15 @@ __global__ void __launch_bounds__(kSortThreads) k_select_sort(const float* __res
   }
   if (t == 0) {
     unit_prefix[n] = total;
-    *cand_count = n;
+    a.cand_count[slot] = n;
   }
 }
 
-__global__ void k_pscan_prep(uint64_t nrows, int* cand_count, uint32_t* unit_prefix, uint32_t* bound,
-                             int* topk_count, uint32_t* counters) {
-  if (threadIdx.x < 4) counters[threadIdx.x] = 0;
-  if (threadIdx.x == 0) {
-    *cand_count = 1;
-    unit_prefix[0] = 0;
-    unit_prefix[1] = (uint32_t)((nrows + 31) >> 5);
-    *bound = 0x7f800000u;
-    *topk_count = 0;
-  }
+__global__ void k_pscan_prep(uint32_t* bound, int* topk_count, int slots) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= slots) return;
+  bound[i] = 0x7f800000u;
+  topk_count[i] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -531,7 +538,7 @@ __global__ void k_pscan_prep(uint64_t nrows, int* cand_count, uint32_t* unit_pre
 //
 // The per-row test is a certified lower bound of the reference's LB_SAX
 // (minidist_paa_to_isax_raw_SIMD, sax.c:310-479).  The query's 16 x 256
-// table of per-segment terms (k_leaf_lb, reference arithmetic) is turned,
+// table of per-segment terms (k_query_prep, reference arithmetic) is turned,
 // per block, into 8-bit terms q = floor(term * 254 / T) (rounded down at
 // every step, at most 255) against the pruning threshold
 // T = (B (1 + 2^-10) + 1e-6) / (L / 16); a row is pruned when its 16 terms
@@ -602,6 +609,15 @@ __device__ __forceinline__ bool fl_wait(uint32_t bar, uint32_t parity, volatile 
 
 __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a) {
   extern __shared__ __align__(16) unsigned char fsm[];
+  const uint32_t slot = blockIdx.x;
+  a.cand += (uint64_t)slot * (a.nleaves + 1);
+  a.cand_lb += (uint64_t)slot * (a.nleaves + 1);
+  a.cand_count += slot;
+  a.unit_prefix += (uint64_t)slot * (a.nleaves + 2);
+  a.sax_tab += (uint64_t)slot * (HG_PAA_SEGMENTS * HG_SAX_CARD);
+  a.bound += slot;
+  a.list += (uint64_t)slot * a.list_stride;
+  a.list_count += 8 * slot;
   uint32_t* qtab = reinterpret_cast<uint32_t*>(fsm);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(fsm);
@@ -617,8 +633,11 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a
   const int chi = a.cand_hi > 0 ? min(a.cand_hi, ncand) : ncand;
   const uint32_t ubase = clo < chi ? a.unit_prefix[clo] : 0u;
   const uint32_t total = clo < chi ? a.unit_prefix[chi] - ubase : 0u;
-  const uint32_t per_block = (total + gridDim.x - 1) / gridDim.x;
-  const uint32_t u0 = ubase + blockIdx.x * per_block;
+  // at least one full stage per block: fewer units leave blocks without a
+  // range, which return before they build a table
+  const uint32_t per_block = max((uint32_t)kStageUnits, (total + gridDim.y - 1) / gridDim.y);
+  if ((uint64_t)blockIdx.y * per_block >= total) return;
+  const uint32_t u0 = ubase + blockIdx.y * per_block;
   const uint32_t u1 = min(ubase + total, u0 + per_block);
   volatile int* s_c0 = reinterpret_cast<volatile int*>(fsm + kFiltSmMeta + 8);
   if (wib == kFiltConsumers) {
@@ -834,35 +853,42 @@ __global__ void __launch_bounds__(kEdThreads, kLines > 2 ? 3 : 4) k_ed_stream(Ed
   extern __shared__ float4 qs4[];  // the query, q4_bytes(L) bytes
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int slot_lead = lane & ~(kSlot - 1), j = lane & (kSlot - 1);
-  if (a.gate && *a.gate == 0) {
-    // a gated launch that did not pass: the block reports an empty list
-    if (threadIdx.x == 0) a.part_count[blockIdx.x] = 0;
-    return;
-  }
-  unsigned long long* list = lists[wib];
-  for (int i = lane; i < kWarpListCap; i += 32) list[i] = ~0ull;
-  for (int i = threadIdx.x; i < (a.L >> 2); i += blockDim.x)
-    qs4[q4_index(i >> 1, i & 1)] = reinterpret_cast<const float4*>(a.q)[i];
-  __syncthreads();
+  const uint32_t qslot = blockIdx.x;  // the query of the group
+  a.bound += qslot;
+  a.parts += ((uint64_t)qslot * a.parts_stride + blockIdx.y) * kWarpListCap;
+  a.part_count += (uint64_t)qslot * a.parts_stride + blockIdx.y;
+  if (a.list) a.list += (uint64_t)qslot * a.list_stride;
   const int nch = a.L >> 3;
   uint64_t first = a.ident_first;
   uint32_t total;
-  if (a.list) {
-    total = *a.list_count;
+  if (a.gate && *a.gate == 0) {
+    total = 0;  // a gated launch that did not pass
+  } else if (a.list) {
+    total = a.list_count[8 * qslot];
   } else if (a.ident_leaf) {
-    const int leaf = *a.ident_leaf;
+    const int leaf = a.ident_leaf[qslot];
     first = a.leaf_start[leaf];
     total = a.leaf_size[leaf];
   } else {
     total = (uint32_t)a.ident_count;
   }
-  const uint32_t nwarps = gridDim.x * W;
-  const uint32_t gw = blockIdx.x * W + wib;
+  const uint32_t nwarps = gridDim.y * W;
+  const uint32_t gw = blockIdx.y * W + wib;
   const uint32_t leaders = slot_leaders<kSlot>();
   // batch b of this warp covers entries [(gw + b * nwarps) * bs, +bs): bs
-  // spreads a short list over all warps (a few long rows keep every warp busy)
+  // spreads a short list over the warps, at least min_batch entries each
   const uint32_t per_warp = (uint32_t)(((uint64_t)total + nwarps - 1) / nwarps);
-  const uint32_t bs = per_warp < 1u ? 1u : (per_warp > 32u ? 32u : per_warp);
+  const uint32_t bs = per_warp < a.min_batch ? a.min_batch : (per_warp > 32u ? 32u : per_warp);
+  if ((uint64_t)blockIdx.y * W * bs >= total) {
+    // no entry for this block: an empty list
+    if (threadIdx.x == 0) *a.part_count = 0;
+    return;
+  }
+  unsigned long long* list = lists[wib];
+  for (int i = lane; i < kWarpListCap; i += 32) list[i] = ~0ull;
+  for (int i = threadIdx.x; i < (a.L >> 2); i += blockDim.x)
+    qs4[q4_index(i >> 1, i & 1)] = reinterpret_cast<const float4*>(a.q + (uint64_t)qslot * a.L)[i];
+  __syncthreads();
   auto entry = [&](uint32_t batch) -> uint32_t {
     const uint64_t idx = (uint64_t)batch * bs + lane;
     if ((uint32_t)lane >= bs || idx >= total) return 0xffffffffu;
@@ -1040,10 +1066,9 @@ __global__ void __launch_bounds__(kEdThreads, kLines > 2 ? 3 : 4) k_ed_stream(Ed
     }
   if (wib == 0) {
     const int bc = warp_dedup_sorted(flat, packed, a.k, 0);
-    unsigned long long* out = a.parts + (uint64_t)blockIdx.x * kWarpListCap;
-    for (int i = lane; i < bc; i += 32) out[i] = flat[i];
+    for (int i = lane; i < bc; i += 32) a.parts[i] = flat[i];
     if (lane == 0) {
-      a.part_count[blockIdx.x] = bc;
+      *a.part_count = bc;
       if (bc == a.k) atomicMin(a.bound, (uint32_t)(flat[a.k - 1] >> 32));
     }
   }
@@ -1061,103 +1086,126 @@ __global__ void __launch_bounds__(kEdThreads, kLines > 2 ? 3 : 4) k_ed_stream(Ed
   }
 }
 
-// Merges the per-block lists (and the current top-k, passed as part -1) into
-// the k smallest distinct distances, lowest id per distance.  Only entries
-// <= the final bound can belong to the answer.
+// Merges the per-block lists and the current top-k into the k smallest
+// distinct distances, lowest id per distance; returns the bound after it.
+// Only entries <= the bound can belong to the answer, and the lists are
+// sorted, so a warp per list reads a prefix of each, 32 entries at a time,
+// four lists in flight.  All of them are gathered in one go if they fit in
+// buf; if not (large k, many lists), 32 lists are merged alone, which lowers
+// the bound, and the rest is tried again.  (A thread per list with its reads
+// one after the other: 8 - 25 us per merge at k = 10, and about 150 us at
+// k = 100 with 592 lists.)
 constexpr int kMergeThreads = 1024;
-__global__ void __launch_bounds__(kMergeThreads) k_merge(const unsigned long long* __restrict__ parts,
-                                                         const int* __restrict__ part_count, int nparts, int k,
-                                                         unsigned long long* topk, int* topk_count,
-                                                         uint32_t* bound, int* err) {
-  extern __shared__ unsigned long long buf[];  // kMergeCap
-  __shared__ unsigned long long best[kMaxK];
-  __shared__ uint32_t tmp[kMergeThreads / 32 + 1];
-  __shared__ uint32_t total;
-  __shared__ int nbest;
-  const int t = threadIdx.x;
-  const uint32_t B = ld_volatile(bound);
-  // previous top-k
-  if (t == 0) nbest = *topk_count;
+__device__ float merge_parts(const MergeArgs& a, uint32_t slot, unsigned long long* buf /* kMergeCap */) {
+  __shared__ int s_n, s_best;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  constexpr int W = kMergeThreads / 32;
+  static_assert(kMaxK + W * kMaxK <= kMergeCap, "the lists of one round fit");
+  const unsigned long long* parts = a.parts + (uint64_t)slot * a.parts_stride * kWarpListCap;
+  const int* part_count = a.part_count + (uint64_t)slot * a.parts_stride;
+  unsigned long long* topk = a.topk + (uint64_t)slot * kMaxK;
+  const int k = a.k;
+  uint32_t B = ld_volatile(a.bound + slot);
+  const int n0 = a.topk_count[slot];
+  for (int i = t; i < n0; i += kMergeThreads) buf[i] = topk[i];
+  if (t == 0) s_best = n0;
   __syncthreads();
-  for (int i = t; i < kMaxK; i += kMergeThreads) best[i] = (i < nbest) ? topk[i] : ~0ull;
-  __syncthreads();
-  // count entries <= B per part (lists are sorted ascending)
-  const int per = (nparts + kMergeThreads - 1) / kMergeThreads;
-  const int p0 = min(nparts, t * per), p1 = min(nparts, p0 + per);
-  uint32_t mine = 0;
-  for (int p = p0; p < p1; ++p) {
-    const unsigned long long* l = parts + (uint64_t)p * kWarpListCap;
-    int lo = 0, hi = part_count[p];
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if ((uint32_t)(l[mid] >> 32) <= B) lo = mid + 1;
-      else hi = mid;
-    }
-    mine += lo;
-  }
-  const uint32_t start = block_exclusive_scan<kMergeThreads>(mine, tmp, &total);
-  const uint32_t M = total;
-  const int room = kMergeCap - k;
-  for (uint32_t r0 = 0; r0 < M || r0 == 0; r0 += room) {
-    // this round takes global positions [r0, r0 + room) after the current best
-    const uint32_t rem = M > r0 ? M - r0 : 0u;
-    const uint32_t m = rem < (uint32_t)room ? rem : (uint32_t)room;
-    int nsort = 32;
-    while (nsort < k + (int)m) nsort <<= 1;
-    for (int i = t; i < nsort; i += kMergeThreads) buf[i] = (i < k) ? best[i] : ~0ull;
-    __syncthreads();
-    uint32_t g = start;
-    for (int p = p0; p < p1; ++p) {
-      const unsigned long long* l = parts + (uint64_t)p * kWarpListCap;
-      const int cntp = part_count[p];
-      for (int j = 0; j < cntp; ++j) {
-        const unsigned long long v = l[j];
-        if ((uint32_t)(v >> 32) > B) break;
-        if (g >= r0 && g < r0 + room) buf[k + (g - r0)] = v;
-        ++g;
-      }
-    }
-    __syncthreads();
-    // bitonic sort of nsort keys
-    for (int size = 2; size <= nsort; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int i = t; i < nsort / 2; i += kMergeThreads) {
-          const int pos = 2 * i - (i & (stride - 1));
-          const int partner = pos + stride;
-          const bool asc = (pos & size) == 0;
-          const unsigned long long x = buf[pos], y = buf[partner];
-          if ((x > y) == asc) {
-            buf[pos] = y;
-            buf[partner] = x;
+  for (int p_lo = 0;;) {
+    const int nbest = s_best;
+    // [p_lo, p_hi): every list left, or after an overflow the next 32
+    int p_hi = a.nparts;
+    for (;;) {
+      if (t == 0) s_n = nbest;
+      __syncthreads();
+      for (int pb = p_lo + wid; pb < p_hi; pb += 4 * W) {
+        int cnt[4];
+        unsigned long long v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) cnt[u] = pb + u * W < p_hi ? part_count[pb + u * W] : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          v[u] = lane < cnt[u] ? parts[(uint64_t)(pb + u * W) * kWarpListCap + lane] : ~0ull;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          unsigned long long x = v[u];
+          for (int base = 0; base < cnt[u]; base += 32) {
+            if (base) x = base + lane < cnt[u] ? parts[(uint64_t)(pb + u * W) * kWarpListCap + base + lane] : ~0ull;
+            const bool take = base + lane < cnt[u] && (uint32_t)(x >> 32) <= B;
+            const uint32_t m = __ballot_sync(HG_FULL, take);
+            int pos = 0;
+            if (lane == 0 && m) pos = atomicAdd(&s_n, __popc(m));
+            pos = __shfl_sync(HG_FULL, pos, 0) + __popc(m & ((1u << lane) - 1));
+            if (take && pos < kMergeCap) buf[pos] = x;
+            if (m != HG_FULL) break;
           }
         }
-        __syncthreads();
       }
+      __syncthreads();
+      if (s_n <= kMergeCap) break;
+      p_hi = min(a.nparts, p_lo + W);
+      __syncthreads();
     }
-    // dedup by distance, keep k (thread 0; at most kMergeCap steps, exits at k)
-    if (t == 0) {
-      int out = 0;
-      uint32_t prev = 0;
-      for (int i = 0; i < nsort && out < k; ++i) {
-        const unsigned long long v = buf[i];
-        if (v == ~0ull) break;
-        const uint32_t d = (uint32_t)(v >> 32);
-        if (out > 0 && d == prev) continue;
-        best[out++] = v;
-        prev = d;
+    const int n = s_n;
+    if (n > nbest) {
+      int nsort = 32;
+      while (nsort < n) nsort <<= 1;
+      for (int i = n + t; i < nsort; i += kMergeThreads) buf[i] = ~0ull;
+      __syncthreads();
+      for (int size = 2; size <= nsort; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          for (int i = t; i < nsort / 2; i += kMergeThreads) {
+            const int pos = 2 * i - (i & (stride - 1));
+            const int partner = pos + stride;
+            const bool asc = (pos & size) == 0;
+            const unsigned long long x = buf[pos], y = buf[partner];
+            if ((x > y) == asc) {
+              buf[pos] = y;
+              buf[partner] = x;
+            }
+          }
+          __syncthreads();
+        }
+      if (wid == 0) {
+        const int best = warp_dedup_sorted(buf, n, k, 0);
+        if (lane == 0) s_best = best;
       }
-      for (int i = out; i < kMaxK; ++i) best[i] = ~0ull;
-      nbest = out;
+      __syncthreads();
     }
-    __syncthreads();
-    if (M == 0) break;
+    if (s_best == k) B = min(B, (uint32_t)(buf[k - 1] >> 32));
+    p_lo = p_hi;
+    if (p_lo >= a.nparts) break;
   }
-  for (int i = t; i < k; i += kMergeThreads) topk[i] = best[i];
+  const int cnt = s_best;
+  for (int i = t; i < cnt; i += kMergeThreads) topk[i] = buf[i];
   if (t == 0) {
-    *topk_count = nbest;
-    if (nbest == k) atomicMin(bound, (uint32_t)(best[k - 1] >> 32));
-    (void)err;
+    a.topk_count[slot] = cnt;
+    a.bound[slot] = B;
   }
+  if (a.dist_out || a.id_out) {
+    for (int i = t; i < k; i += kMergeThreads) {
+      const unsigned long long v = i < cnt ? buf[i] : ~0ull;
+      if (a.dist_out)
+        a.dist_out[(uint64_t)slot * k + i] = i < cnt ? __uint_as_float((uint32_t)(v >> 32)) : __int_as_float(0x7f800000);
+      if (a.id_out) a.id_out[(uint64_t)slot * k + i] = i < cnt ? (int64_t)(uint32_t)v : -1;
+    }
+  }
+  return __uint_as_float(B);
+}
+
+__global__ void __launch_bounds__(kMergeThreads) k_merge(MergeArgs a) {
+  extern __shared__ unsigned long long merge_buf[];  // kMergeCap
+  merge_parts(a, blockIdx.x, merge_buf);
+}
+
+// The merge of the approximate leaf's lists and, against the bound it gives,
+// the candidate leaves: one block per query, the two steps one after the
+// other in the same shared memory.
+__global__ void __launch_bounds__(kMergeThreads) k_merge_select(MergeArgs a, SelectArgs sel) {
+  extern __shared__ unsigned long long merge_buf[];
+  static_assert(kMergeThreads == kSortThreads, "one block does both");
+  const float B = merge_parts(a, blockIdx.x, merge_buf);
+  __syncthreads();
+  select_sort(sel, blockIdx.x, B, reinterpret_cast<uint32_t*>(merge_buf));
 }
 
 __global__ void k_emit(const unsigned long long* topk, const int* topk_count, int k, float* dist_out,
@@ -1259,31 +1307,20 @@ cudaError_t launch_sax_rows(const float* rows, int L, uint64_t n, const float* b
   return cudaGetLastError();
 }
 
-cudaError_t launch_query_prep(const float* q, int L, Tree t, const uint64_t* leaf_start,
-                              const uint32_t* leaf_size, int* approx_leaf, float* paa, int* cand,
-                              float* cand_lb, int* cand_count, uint32_t* unit_prefix, uint32_t* bound,
-                              int* topk_count, uint32_t* counters, cudaStream_t s) {
-  k_query_prep<<<1, 32, 0, s>>>(q, L, t, leaf_start, leaf_size, approx_leaf, paa, cand, cand_lb, cand_count,
-                                unit_prefix, bound, topk_count, counters);
+cudaError_t launch_query_prep(const PrepArgs& a, int slots, cudaStream_t s) {
+  static SmemLimit attr;
+  const cudaError_t ea = attr.ensure((const void*)k_query_prep, 65536);
+  if (ea != cudaSuccess) return ea;
+  unsigned blocks = a.lb ? blocks_for((uint64_t)a.nleaves * 32, kPrepThreads) : 0;
+  if (a.sax_tab && blocks < HG_PAA_SEGMENTS) blocks = HG_PAA_SEGMENTS;
+  if (blocks > 4096) blocks = 4096;  // a warp takes several leaves from 32,768 on (grid.y ends at 65,535)
+  k_query_prep<<<dim3(slots, blocks + 1), kPrepThreads, sizeof(float) * a.L, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s) {
   if (!nq) return cudaSuccess;
   k_route_queries<<<blocks_for((uint64_t)nq * 32, 128), 128, 0, s>>>(Q, nq, L, t, leaf_out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_leaf_lb(const float* q, int L, int nleaves, const int* seg_off, const short* points,
-                           const float* sk, float* lb_out, cudaStream_t s, const float* paa, const float* bp,
-                           float* sax_tab) {
-  if (!nleaves) return cudaSuccess;
-  static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)k_leaf_lb, 65536);
-  if (ea != cudaSuccess) return ea;
-  unsigned grid = blocks_for((uint64_t)nleaves * 32, 256);
-  if (sax_tab && grid < HG_PAA_SEGMENTS) grid = HG_PAA_SEGMENTS;  // 16 x 256 threads: one per table entry
-  k_leaf_lb<<<grid, 256, sizeof(float) * L, s>>>(q, L, nleaves, seg_off, points, sk, lb_out, paa, bp, sax_tab);
   return cudaGetLastError();
 }
 
@@ -1341,42 +1378,48 @@ cudaError_t launch_stale_copy(const int* flag, const uint32_t* bound, uint32_t* 
 static size_t select_smem(bool global_keys) {
   return sizeof(uint32_t) * 16 * kSortThreads + (global_keys ? 0 : sizeof(uint32_t) * 4 * kMaxLeavesSort);
 }
+constexpr size_t kMergeSmem = sizeof(unsigned long long) * kMergeCap;
 
-cudaError_t launch_select_sort(const float* lb, int nleaves, const uint32_t* bound, const int* approx_leaf,
-                               const uint64_t* leaf_start, const uint32_t* leaf_size, int* cand,
-                               float* cand_lb, int* cand_count, uint32_t* unit_prefix, cudaStream_t s,
-                               uint32_t* gkeys) {
-  const bool global_keys = nleaves > kMaxLeavesSort;
-  if (global_keys && !gkeys) return cudaErrorInvalidValue;
+cudaError_t launch_merge(const MergeArgs& a, int slots, cudaStream_t s) {
   static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)k_select_sort, (int)select_smem(false));
+  const cudaError_t ea = attr.ensure((const void*)k_merge, (int)kMergeSmem);
   if (ea != cudaSuccess) return ea;
-  k_select_sort<<<1, kSortThreads, select_smem(global_keys), s>>>(lb, nleaves, bound, approx_leaf, leaf_start,
-                                                                  leaf_size, cand, cand_lb, cand_count, unit_prefix,
-                                                                  global_keys ? gkeys : nullptr);
+  k_merge<<<slots, kMergeThreads, kMergeSmem, s>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_pscan_prep(uint64_t nrows, int* cand_count, uint32_t* unit_prefix, uint32_t* bound,
-                              int* topk_count, uint32_t* counters, cudaStream_t s) {
-  k_pscan_prep<<<1, 32, 0, s>>>(nrows, cand_count, unit_prefix, bound, topk_count, counters);
+cudaError_t launch_merge_select(const MergeArgs& a, const SelectArgs& sel, int slots, cudaStream_t s) {
+  const bool global_keys = sel.nleaves > kMaxLeavesSort;
+  if (global_keys && !sel.gkeys) return cudaErrorInvalidValue;
+  static SmemLimit attr;
+  const cudaError_t ea = attr.ensure((const void*)k_merge_select, (int)select_smem(false));
+  if (ea != cudaSuccess) return ea;
+  SelectArgs b = sel;
+  if (!global_keys) b.gkeys = nullptr;
+  const size_t ss = select_smem(global_keys);
+  k_merge_select<<<slots, kMergeThreads, ss > kMergeSmem ? ss : kMergeSmem, s>>>(a, b);
   return cudaGetLastError();
 }
 
-cudaError_t launch_lbsax_filter(const FilterArgs& a, int blocks, cudaStream_t s) {
+cudaError_t launch_pscan_prep(uint32_t* bound, int* topk_count, int slots, cudaStream_t s) {
+  k_pscan_prep<<<blocks_for(slots, 32), 32, 0, s>>>(bound, topk_count, slots);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cudaStream_t s) {
   static SmemLimit attr;
   const cudaError_t ea = attr.ensure((const void*)k_lbsax_filter, (int)lbsax_filter_smem());
   if (ea != cudaSuccess) return ea;
-  k_lbsax_filter<<<blocks, kFilterThreads, lbsax_filter_smem(), s>>>(a);
+  k_lbsax_filter<<<dim3(slots, blocks), kFilterThreads, lbsax_filter_smem(), s>>>(a);
   return cudaGetLastError();
 }
 
 template <bool kRowIds, int kLines, int kSlot>
-static cudaError_t launch_ed(const EdArgs& a, int blocks, cudaStream_t s) {
+static cudaError_t launch_ed(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
   static SmemLimit attr;
   const cudaError_t ea = attr.ensure((const void*)k_ed_stream<kRowIds, kLines, kSlot>, (int)q4_bytes(16384));
   if (ea != cudaSuccess) return ea;
-  k_ed_stream<kRowIds, kLines, kSlot><<<blocks, kEdThreads, q4_bytes(a.L), s>>>(a);
+  k_ed_stream<kRowIds, kLines, kSlot><<<dim3(slots, blocks), kEdThreads, q4_bytes(a.L), s>>>(a);
   return cudaGetLastError();
 }
 // long series (L >= 4096): few candidate rows per query, each long, so
@@ -1390,13 +1433,13 @@ static cudaError_t launch_ed(const EdArgs& a, int blocks, cudaStream_t s) {
 #ifndef HG_ED_SHORT_LINES
 #define HG_ED_SHORT_LINES 2
 #endif
-cudaError_t launch_ed_stream(const EdArgs& a, int blocks, cudaStream_t s) {
-  return a.L >= 4096 ? launch_ed<false, HG_ED_LONG_LINES, HG_ED_LONG_SLOT>(a, blocks, s)
-                     : launch_ed<false, HG_ED_SHORT_LINES, 4>(a, blocks, s);
+cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
+  return a.L >= 4096 ? launch_ed<false, HG_ED_LONG_LINES, HG_ED_LONG_SLOT>(a, slots, blocks, s)
+                     : launch_ed<false, HG_ED_SHORT_LINES, 4>(a, slots, blocks, s);
 }
-cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int blocks, cudaStream_t s) {
-  return a.L >= 4096 ? launch_ed<true, HG_ED_LONG_LINES, HG_ED_LONG_SLOT>(a, blocks, s)
-                     : launch_ed<true, HG_ED_SHORT_LINES, 4>(a, blocks, s);
+cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
+  return a.L >= 4096 ? launch_ed<true, HG_ED_LONG_LINES, HG_ED_LONG_SLOT>(a, slots, blocks, s)
+                     : launch_ed<true, HG_ED_SHORT_LINES, 4>(a, slots, blocks, s);
 }
 int ed_blocks_per_sm(int L) {
   // shared memory per block: the staged query + 8 per-warp lists of 2 KB
@@ -1406,17 +1449,6 @@ int ed_blocks_per_sm(int L) {
   const int lines = L >= 4096 ? HG_ED_LONG_LINES : HG_ED_SHORT_LINES;
   const int cap = lines > 2 ? 3 : kEdBlocksPerSm;
   return fit < 1 ? 1 : (fit < cap ? fit : cap);
-}
-
-cudaError_t launch_merge(const unsigned long long* parts, const int* part_count, int nparts, int k,
-                         unsigned long long* topk, int* topk_count, uint32_t* bound, int* err,
-                         cudaStream_t s) {
-  const int smem = sizeof(unsigned long long) * kMergeCap;
-  static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)k_merge, smem);
-  if (ea != cudaSuccess) return ea;
-  k_merge<<<1, kMergeThreads, smem, s>>>(parts, part_count, nparts, k, topk, topk_count, bound, err);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_emit(const unsigned long long* topk, const int* topk_count, int k, float* dist_out,

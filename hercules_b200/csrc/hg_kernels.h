@@ -54,25 +54,47 @@ struct Tree {
   int root;  // >= 0 internal node, < 0 the leaf ~root
 };
 
+// The kernels of the plain path serve a group of queries per launch: grid.x is
+// the query's slot in the group, and every per-query array below holds one
+// entry (or one run of the stated stride) per slot.  Slots vary fastest, so
+// the blocks of all queries of a group run side by side.
+
+// Routing, LB_EAPCA of every leaf and the LB_SAX term table.
+struct PrepArgs {
+  const float* q;        // [slot][L]
+  int L;
+  Tree tree;
+  int nleaves;
+  const int* seg_off;    // leaf envelopes (CSR)
+  const short* points;
+  const float* sk;
+  const float* bp;
+  float* lb;             // [slot][nleaves]; NULL: no lower bounds
+  float* sax_tab;        // [slot][16 x 256] LB_SAX terms; NULL: none
+  int* approx_leaf;      // [slot]; NULL: no routing, and the state below is left alone
+  uint32_t* bound;       // [slot] reset to +inf
+  int* topk_count;       // [slot] reset to 0
+  uint32_t* counters;    // [slot][8] reset to 0
+};
+
 // Stage 1 of the leaf scan: candidate leaves -> LB_SAX survivors.
 struct FilterArgs {
   const uint8_t* sax;
-  const float* bp;
   int L;
-  uint64_t nrows;
+  int nleaves;
   const uint64_t* leaf_start;
   const uint32_t* leaf_size;
-  const int* cand;
-  const float* cand_lb;
-  const int* cand_count;
-  const uint32_t* unit_prefix;  // exclusive prefix of 32-row units per candidate
-  const float* paa;
-  const float* sax_tab;  // the query's 16 x 256 LB_SAX terms (k_leaf_lb), 16-byte aligned
+  const int* cand;              // [slot][nleaves + 1]
+  const float* cand_lb;         // [slot][nleaves + 1]
+  const int* cand_count;        // [slot]
+  const uint32_t* unit_prefix;  // [slot][nleaves + 2] exclusive prefix of 32-row units per candidate
+  const float* sax_tab;  // [slot][16 x 256] the query's LB_SAX terms (k_query_prep), 16-byte aligned
   int use_lbsax;
   int cand_lo, cand_hi;  // candidates [cand_lo, cand_hi) of the sorted list; cand_hi <= 0: to the end
-  const uint32_t* bound;
-  uint32_t* list;        // surviving rows
-  uint32_t* list_count;  // must be 0 before the launch
+  const uint32_t* bound;  // [slot]
+  uint32_t* list;         // [slot][list_stride] surviving rows
+  uint64_t list_stride;
+  uint32_t* list_count;   // [slot][8]: must be 0 before the launch
   unsigned long long* stats;  // [0] rows considered [2] rows pruned by LB_SAX [3] leaves visited
   int* err;                   // set to 1 when a bounded wait ran out (may be NULL)
 };
@@ -82,23 +104,54 @@ struct EdArgs {
   const float* rows;  // leaf-ordered, row-major
   const int64_t* ids;
   int L;
-  const uint32_t* list;        // rows; NULL: the range below
-  const uint32_t* list_count;
-  const int* ident_leaf;       // range = this leaf's rows (device pointer), else
+  const uint32_t* list;        // [slot][list_stride] rows; NULL: the range below
+  uint64_t list_stride;
+  const uint32_t* list_count;  // [slot][8]
+  const int* ident_leaf;       // [slot] range = this leaf's rows (device pointer), else
   uint64_t ident_first;        //   [ident_first, ident_first + ident_count)
   uint64_t ident_count;
   const uint64_t* leaf_start;
   const uint32_t* leaf_size;
-  uint32_t* head;              // batch counter, must be 0 before the launch
-  const float* q;
+  uint32_t min_batch;          // entries a warp takes at least, 1..32: with fewer in all, blocks stay idle
+  const float* q;              // [slot][L]
   int k;
-  uint32_t* bound;             // float bits of the running k-th bound (atomicMin)
-  unsigned long long* parts;   // per-warp sorted lists (kWarpListCap stride)
-  int* part_count;
+  uint32_t* bound;             // [slot] float bits of the running k-th bound (atomicMin)
+  unsigned long long* parts;   // [slot][parts_stride] per-block sorted lists (kWarpListCap stride)
+  int* part_count;             // [slot][parts_stride]
+  uint32_t parts_stride;       // lists per slot
   unsigned long long* stats;   // [1] chunks computed [4] rows completed [5] rows started
   const int* gate;             // if set and *gate == 0, the launch scans nothing
   int has_floor;               // 1: only rows at distance > floor enter the lists (the
   float floor;                 //   answers of k above kMaxK come in rounds above it)
+};
+
+// Merge of a group's per-block lists into its running top-k, then either the
+// candidate leaves of the next stage or the answers.
+struct MergeArgs {
+  const unsigned long long* parts;  // [slot][parts_stride][kWarpListCap]
+  const int* part_count;            // [slot][parts_stride]
+  uint32_t parts_stride;
+  int nparts;
+  int k;
+  unsigned long long* topk;  // [slot][kMaxK]
+  int* topk_count;           // [slot]
+  uint32_t* bound;           // [slot]
+  float* dist_out;           // [slot][k] answers; both NULL: none written
+  int64_t* id_out;
+};
+
+// Candidate leaves of a group (LB_EAPCA within the bound, in LB order).
+struct SelectArgs {
+  const float* lb;  // [slot][nleaves]
+  int nleaves;
+  const int* approx_leaf;  // [slot]
+  const uint64_t* leaf_start;
+  const uint32_t* leaf_size;
+  int* cand;              // as in FilterArgs
+  float* cand_lb;
+  int* cand_count;
+  uint32_t* unit_prefix;
+  uint32_t* gkeys;        // [slot][4 x nleaves], needed above kMaxLeavesSort leaves
 };
 
 int sm_count(int device);
@@ -118,24 +171,14 @@ cudaError_t launch_sax_rows(const float* rows, int L, uint64_t n, const float* b
                             cudaStream_t s);
 
 // queries
-cudaError_t launch_query_prep(const float* q, int L, Tree t, const uint64_t* leaf_start,
-                              const uint32_t* leaf_size, int* approx_leaf, float* paa, int* cand,
-                              float* cand_lb, int* cand_count, uint32_t* unit_prefix, uint32_t* bound,
-                              int* topk_count, uint32_t* counters, cudaStream_t s);
+cudaError_t launch_query_prep(const PrepArgs& a, int slots, cudaStream_t s);
 cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s);
-cudaError_t launch_leaf_lb(const float* q, int L, int nleaves, const int* seg_off, const short* points,
-                           const float* sk, float* lb_out, cudaStream_t s, const float* paa = nullptr,
-                           const float* bp = nullptr, float* sax_tab = nullptr);
-// gkeys: 4 x nleaves words of global scratch, needed above kMaxLeavesSort leaves
-cudaError_t launch_select_sort(const float* lb, int nleaves, const uint32_t* bound, const int* approx_leaf,
-                               const uint64_t* leaf_start, const uint32_t* leaf_size, int* cand,
-                               float* cand_lb, int* cand_count, uint32_t* unit_prefix, cudaStream_t s,
-                               uint32_t* gkeys = nullptr);
-cudaError_t launch_pscan_prep(uint64_t nrows, int* cand_count, uint32_t* unit_prefix, uint32_t* bound,
-                              int* topk_count, uint32_t* counters, cudaStream_t s);
-cudaError_t launch_lbsax_filter(const FilterArgs& a, int blocks, cudaStream_t s);  // blocks: one per SM
+cudaError_t launch_pscan_prep(uint32_t* bound, int* topk_count, int slots, cudaStream_t s);
+// blocks: per slot
+cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cudaStream_t s);
 size_t lbsax_filter_smem();
-cudaError_t launch_ed_stream(const EdArgs& a, int blocks, cudaStream_t s);
+// blocks: per slot, at most EdArgs::parts_stride
+cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s);
 // batched path: the (leaf, query) pairs whose LB_EAPCA is within the query's
 // bound (k_leaf_keep)
 cudaError_t launch_leaf_keep(const float* Q, int L, int nq, const short* useg_start, const short* useg_end, int nu,
@@ -158,10 +201,10 @@ cudaError_t launch_stale_copy(const int* flag, const uint32_t* bound, uint32_t* 
 // resident blocks per SM of the distance stream for series length L
 int ed_blocks_per_sm(int L);
 // the same with id = row index (EdArgs::ids unused)
-cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int blocks, cudaStream_t s);
-cudaError_t launch_merge(const unsigned long long* parts, const int* part_count, int nparts, int k,
-                         unsigned long long* topk, int* topk_count, uint32_t* bound, int* err,
-                         cudaStream_t s);
+cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int slots, int blocks, cudaStream_t s);
+cudaError_t launch_merge(const MergeArgs& a, int slots, cudaStream_t s);
+// the merge, then the candidate selection against the merged bound
+cudaError_t launch_merge_select(const MergeArgs& a, const SelectArgs& sel, int slots, cudaStream_t s);
 cudaError_t launch_emit(const unsigned long long* topk, const int* topk_count, int k, float* dist_out,
                         int64_t* id_out, cudaStream_t s);
 

@@ -79,10 +79,7 @@ extern "C" HG_API hg_status hg_pscan_noalloc(const float* d_rows, uint64_t n, ui
   hg_status st = scratch_of(dev, &base);
   if (st != HG_OK) return st;
   // layout of the scratch
-  uint32_t* counters = reinterpret_cast<uint32_t*>(base + 0);          // 8
-  uint32_t* bound = reinterpret_cast<uint32_t*>(base + 64);            // 1
-  int* cand_count = reinterpret_cast<int*>(base + 128);                // 1
-  uint32_t* unit_prefix = reinterpret_cast<uint32_t*>(base + 192);     // 2
+  uint32_t* bound = reinterpret_cast<uint32_t*>(base + 0);             // 1
   int* topk_count = reinterpret_cast<int*>(base + 256);                // 1
   unsigned long long* stats = reinterpret_cast<unsigned long long*>(base + 512);  // 8
   unsigned long long* topk = reinterpret_cast<unsigned long long*>(base + 1024);  // kMaxK
@@ -91,28 +88,37 @@ extern "C" HG_API hg_status hg_pscan_noalloc(const float* d_rows, uint64_t n, ui
   static_assert(1024 + sizeof(unsigned long long) * hg::kMaxK <= 3072, "scratch layout");
   static_assert(3072 + sizeof(int) * kNoAllocParts <= kHeaderBytes, "scratch layout");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // counters, bound and list counts start from zero / +inf on every call
-  cudaError_t e = hg::launch_pscan_prep(n, cand_count, unit_prefix, bound, topk_count, counters, s);
+  // bound and top-k start from +inf / empty on every call
+  cudaError_t e = hg::launch_pscan_prep(bound, topk_count, 1, s);
   if (e == cudaSuccess) {
     hg::EdArgs a{};
     a.rows = d_rows;
-    a.ids = nullptr;
     a.L = (int)L;
-    a.list = nullptr;
-    a.ident_leaf = nullptr;
-    a.ident_first = 0;
     a.ident_count = n;
-    a.head = counters;
+    a.min_batch = 1;
     a.q = d_query;
     a.k = (int)k;
     a.bound = bound;
     a.parts = parts;
     a.part_count = part_count;
+    a.parts_stride = kNoAllocParts;
     a.stats = stats;
-    e = hg::launch_ed_stream_row_ids(a, kNoAllocBlocks, s);
+    e = hg::launch_ed_stream_row_ids(a, 1, kNoAllocBlocks, s);
   }
-  if (e == cudaSuccess) e = hg::launch_merge(parts, part_count, kNoAllocBlocks, (int)k, topk, topk_count, bound, nullptr, s);
-  if (e == cudaSuccess) e = hg::launch_emit(topk, topk_count, (int)k, d_dist_out, d_id_out, s);
+  if (e == cudaSuccess) {
+    hg::MergeArgs m{};
+    m.parts = parts;
+    m.part_count = part_count;
+    m.parts_stride = kNoAllocParts;
+    m.nparts = kNoAllocBlocks;
+    m.k = (int)k;
+    m.topk = topk;
+    m.topk_count = topk_count;
+    m.bound = bound;
+    m.dist_out = d_dist_out;
+    m.id_out = d_id_out;
+    e = hg::launch_merge(m, 1, s);
+  }
   if (e != cudaSuccess) return fail(HG_ERR_CUDA, cudaGetErrorString(e));
   return HG_OK;
 }
