@@ -44,8 +44,11 @@ constexpr int kBM = kBatchTileRows;
 // ---------------------------------------------------------------------------
 
 // One warp per output row w: the BF16 copy of source row src = idx ? idx[w] : w
-// (round to nearest) and, in FP64 rounded up, meta[src] = {|x|^2, |x~|,
-// |x - x~|, 0} (x~ the BF16 row).
+// (round to nearest) and, with kMeta, in FP64 rounded up, meta[src] = {|x|^2,
+// |x~|, |x - x~|, 0} (x~ the BF16 row).  Without the norms (a query panel,
+// whose queries have theirs) the copy is bound by memory instead of FP64
+// arithmetic.
+template <bool kMeta>
 __global__ void k_rows_to_bf16(const float* __restrict__ rows, const uint32_t* __restrict__ idx, uint64_t n,
                                const uint32_t* n_dev, int L, __nv_bfloat16* __restrict__ out,
                                float4* __restrict__ meta) {
@@ -68,12 +71,15 @@ __global__ void k_rows_to_bf16(const float* __restrict__ rows, const uint32_t* _
     const __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
     o[2 * i] = b0;
     o[2 * i + 1] = b1;
-    const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
-    acc(v.x, f0.x);
-    acc(v.y, f0.y);
-    acc(v.z, f1.x);
-    acc(v.w, f1.y);
+    if constexpr (kMeta) {
+      const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
+      acc(v.x, f0.x);
+      acc(v.y, f0.y);
+      acc(v.z, f1.x);
+      acc(v.w, f1.y);
+    }
   }
+  if constexpr (!kMeta) continue;
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) {
     a2 += __shfl_xor_sync(HG_FULL, a2, s);
@@ -608,7 +614,8 @@ __global__ void k_mark_overflow(const uint32_t* pairs_cnt, uint32_t pairs_cap, c
 // Queries grouped by approximate leaf (one block): per leaf its query count
 // and offset (counting sort; the order inside a leaf is arbitrary), each
 // query's bound slots, and the bound pass's item offsets per leaf (groups of
-// at most kBatchBoundQueries queries x chunks of btpi tiles).
+// at most kBatchBoundQueries queries x chunks of nitems[1] tiles: btpi, or
+// fewer, down to 2, until there are kBatchItemTarget items).
 constexpr int kGroupThreads = 1024;
 __global__ void __launch_bounds__(kGroupThreads) k_group_queries(const int* __restrict__ approx, int nq,
                                                                  const LeafPlan* __restrict__ plan, int nleaves,
@@ -631,6 +638,15 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_queries(const int* __re
   // thread owns a run of consecutive leaves
   const int per = (nleaves + kGroupThreads - 1) / kGroupThreads;
   const int l0 = min(tid * per, nleaves), l1 = min(l0 + per, nleaves);
+  __shared__ unsigned long long s_work;
+  if (tid == 0) s_work = 0;
+  __syncthreads();
+  unsigned long long work = 0;  // (group, tile) pairs
+  for (int l = l0; l < l1; ++l)
+    work += (unsigned long long)((cnt[l] + kBatchBoundQueries - 1) / kBatchBoundQueries) * plan[l].use_tiles;
+  if (work) atomicAdd(&s_work, work);
+  __syncthreads();
+  btpi = (uint32_t)min((unsigned long long)btpi, max(2ull, s_work / kBatchItemTarget));
   auto items_of = [&](int l) -> uint32_t {
     const uint32_t c = cnt[l], use = plan[l].use_tiles;
     if (c == 0 || use == 0) return 0u;
@@ -677,7 +693,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_queries(const int* __re
     oq += cnt[l];
     oi += items_of(l);
   }
-  if (tid == kGroupThreads - 1) *nitems = oi;
+  if (tid == kGroupThreads - 1) {
+    nitems[0] = oi;
+    nitems[1] = btpi;
+  }
   __syncthreads();
   for (int q = tid; q < nq; q += kGroupThreads) {
     const int l = approx[q];
@@ -688,13 +707,13 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_queries(const int* __re
 }
 
 // The bound pass's work items, one warp per leaf.
-__global__ void k_group_items(const LeafPlan* __restrict__ plan, int nleaves, uint32_t btpi,
+__global__ void k_group_items(const LeafPlan* __restrict__ plan, int nleaves, const uint32_t* __restrict__ nitems,
                               const uint32_t* __restrict__ leaf_qoff, const uint32_t* __restrict__ leaf_qcnt,
                               const uint32_t* __restrict__ item_off, BatchItem* items) {
   const int l = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (l >= nleaves) return;
   const LeafPlan p = plan[l];
-  const uint32_t c = leaf_qcnt[l], use = p.use_tiles;
+  const uint32_t c = leaf_qcnt[l], use = p.use_tiles, btpi = nitems[1];
   if (c == 0 || use == 0) return;
   const uint32_t per_group = (use + btpi - 1) / btpi;
   const uint32_t n = ((c + kBatchBoundQueries - 1) / kBatchBoundQueries) * per_group;
@@ -715,28 +734,40 @@ __global__ void k_group_items(const LeafPlan* __restrict__ plan, int nleaves, ui
 
 // The pruned filter's layout (one block): per leaf, its kept queries get a
 // run of the query panel (exclusive scan of the counts) and its work items
-// a run of the item list (query tiles of kBatchQueryTile x chunks of tpi
-// 128-row tiles on the global tile grid).  ctl[0] = items, ctl[1] = panel
-// rows, ctl[2] = the dense pass's query count: 0, or nq when the panel or
-// the item list would overflow (the dense pass then filters every row),
-// ctl[3] = the kept (leaf, query) pairs.
+// a run of the item list (query tiles of kBatchQueryTile x chunks of ctl[4]
+// 128-row tiles on the global tile grid: tpi, or fewer, down to tpi_min, until
+// there are kBatchItemTarget items).  ctl[0] = items, ctl[1] = panel rows,
+// ctl[2] = the dense pass's query count: 0, or nq when the panel or the item
+// list would overflow (the dense pass then filters every row), ctl[3] = the
+// kept (leaf, query) pairs.
 // pairs = sum over leaves of kept queries x leaf rows.
 __global__ void __launch_bounds__(kGroupThreads) k_group_pruned(const uint32_t* __restrict__ leaf_cnt,
                                                                 const LeafPlan* __restrict__ plan, int nleaves,
-                                                                uint32_t tpi, uint32_t panel_cap, uint32_t items_cap,
+                                                                uint32_t tpi, uint32_t tpi_min, uint32_t panel_cap,
+                                                                uint32_t items_cap,
                                                                 uint32_t nq, const uint32_t* nq_dev,
                                                                 uint32_t* leaf_poff, uint32_t* leaf_ioff,
                                                                 uint32_t* ctl, unsigned long long* pairs) {
   __shared__ unsigned long long wsum[3][32];
+  __shared__ unsigned long long s_work;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  auto items_of = [&](int l) -> unsigned long long {
+  const int per = (nleaves + kGroupThreads - 1) / kGroupThreads;
+  const int l0 = min(tid * per, nleaves), l1 = min(l0 + per, nleaves);
+  // query tiles x chunks of `chunk` row tiles of leaf l
+  auto chunks_of = [&](int l, uint32_t chunk) -> unsigned long long {
     const uint32_t c = leaf_cnt[l];
     if (c == 0 || plan[l].size == 0) return 0ull;
     const uint64_t t0 = plan[l].start / kBM, t1 = (plan[l].start + plan[l].size + kBM - 1) / kBM;
-    return (unsigned long long)((c + kBatchQueryTile - 1) / kBatchQueryTile) * ((t1 - t0 + tpi - 1) / tpi);
+    return (unsigned long long)((c + kBatchQueryTile - 1) / kBatchQueryTile) * ((t1 - t0 + chunk - 1) / chunk);
   };
-  const int per = (nleaves + kGroupThreads - 1) / kGroupThreads;
-  const int l0 = min(tid * per, nleaves), l1 = min(l0 + per, nleaves);
+  if (tid == 0) s_work = 0;
+  __syncthreads();
+  unsigned long long work = 0;
+  for (int l = l0; l < l1; ++l) work += chunks_of(l, 1);
+  if (work) atomicAdd(&s_work, work);
+  __syncthreads();
+  tpi = (uint32_t)min((unsigned long long)tpi, max((unsigned long long)tpi_min, s_work / kBatchItemTarget));
+  auto items_of = [&](int l) -> unsigned long long { return chunks_of(l, tpi); };
   unsigned long long sq = 0, si = 0, sp = 0;
   for (int l = l0; l < l1; ++l) {
     sq += leaf_cnt[l];
@@ -783,6 +814,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_pruned(const uint32_t* 
     ctl[1] = fits ? (uint32_t)tq : 0u;
     ctl[2] = fits ? 0u : (nq_dev ? *nq_dev : nq);
     ctl[3] = (uint32_t)tq;  // kept (leaf, query) pairs
+    ctl[4] = tpi;
     *pairs = fits ? tp : 0ull;
   }
 }
@@ -790,10 +822,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_pruned(const uint32_t* 
 // The pruned filter's panel list and work items, one block per leaf.
 __global__ void k_emit_pruned(const uint32_t* __restrict__ leaf_cnt, const uint32_t* __restrict__ leaf_q,
                               uint32_t stride, const uint32_t* __restrict__ leaf_poff,
-                              const uint32_t* __restrict__ leaf_ioff, const LeafPlan* __restrict__ plan, uint32_t tpi,
+                              const uint32_t* __restrict__ leaf_ioff, const LeafPlan* __restrict__ plan,
                               const uint32_t* __restrict__ ctl, uint32_t* panel_list, BatchItem* items) {
   const int l = blockIdx.x;
-  const uint32_t c = leaf_cnt[l];
+  const uint32_t c = leaf_cnt[l], tpi = ctl[4];
   if (ctl[0] == 0 || c == 0 || plan[l].size == 0) return;
   const uint32_t po = leaf_poff[l], io = leaf_ioff[l];
   for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) panel_list[po + i] = leaf_q[(uint64_t)l * stride + i];
@@ -861,7 +893,9 @@ cudaError_t launch_rows_to_bf16(const float* rows, const uint32_t* idx, uint64_t
     const uint64_t cap = 32ull * (uint64_t)sm_count(dev);
     if (blocks > cap) blocks = cap;
   }
-  k_rows_to_bf16<<<(unsigned)blocks, 256, 0, s>>>(rows, idx, n, n_dev, L, static_cast<__nv_bfloat16*>(out), meta);
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  if (meta) k_rows_to_bf16<true><<<(unsigned)blocks, 256, 0, s>>>(rows, idx, n, n_dev, L, o, meta);
+  else k_rows_to_bf16<false><<<(unsigned)blocks, 256, 0, s>>>(rows, idx, n, n_dev, L, o, meta);
   return cudaGetLastError();
 }
 
@@ -898,21 +932,21 @@ cudaError_t launch_group_queries(const int* approx, int nq, const LeafPlan* plan
                                                  item_off, nitems, global_cnt ? gcnt : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_group_items<<<nblk((uint64_t)nleaves * 32, 256), 256, 0, s>>>(plan, nleaves, btpi, leaf_qoff, leaf_qcnt,
+  k_group_items<<<nblk((uint64_t)nleaves * 32, 256), 256, 0, s>>>(plan, nleaves, nitems, leaf_qoff, leaf_qcnt,
                                                                  item_off, items);
   return cudaGetLastError();
 }
 
 cudaError_t launch_group_pruned(const uint32_t* leaf_cnt, const uint32_t* leaf_q, uint32_t stride,
-                                const LeafPlan* plan, int nleaves, uint32_t tpi, uint32_t panel_cap,
+                                const LeafPlan* plan, int nleaves, uint32_t tpi, uint32_t tpi_min, uint32_t panel_cap,
                                 uint32_t items_cap, uint32_t nq, uint32_t* leaf_poff, uint32_t* leaf_ioff,
                                 uint32_t* ctl, unsigned long long* pairs, uint32_t* panel_list, BatchItem* items,
                                 cudaStream_t s, const uint32_t* nq_dev) {
-  k_group_pruned<<<1, kGroupThreads, 0, s>>>(leaf_cnt, plan, nleaves, tpi, panel_cap, items_cap, nq, nq_dev,
+  k_group_pruned<<<1, kGroupThreads, 0, s>>>(leaf_cnt, plan, nleaves, tpi, tpi_min, panel_cap, items_cap, nq, nq_dev,
                                              leaf_poff, leaf_ioff, ctl, pairs);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || nleaves == 0) return e;
-  k_emit_pruned<<<nleaves, 256, 0, s>>>(leaf_cnt, leaf_q, stride, leaf_poff, leaf_ioff, plan, tpi, ctl, panel_list,
+  k_emit_pruned<<<nleaves, 256, 0, s>>>(leaf_cnt, leaf_q, stride, leaf_poff, leaf_ioff, plan, ctl, panel_list,
                                         items);
   return cudaGetLastError();
 }

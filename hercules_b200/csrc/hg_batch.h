@@ -107,18 +107,35 @@ struct BatchRank {
   uint32_t* heads;            // [0] segment counter
 };
 
-// n_dev (optional): the row count read on the device, at most n
+constexpr uint32_t kBatchPairBlock = 1024;  // survivor pairs a filter warp reserves at a time
+constexpr uint32_t kBatchPairWarps = 8;     // filter warps per SM that do
+
+// Work items that even out over the SMs: the filter's work lists are cut into
+// at least this many items where their tiles allow it
+constexpr uint32_t kBatchItemTarget = 8 * 148;
+
+// TMA descriptors of one BF16 query matrix: boxes of 256 and of 64 queries
+// (narrow query tiles), and of 128 (the CTA-pair filter)
+struct QueryMaps {
+  CUtensorMap q256, q64, q128;
+};
+
+// n_dev (optional): the row count read on the device, at most n; meta NULL:
+// the BF16 rows only
 cudaError_t launch_rows_to_bf16(const float* rows, const uint32_t* idx, uint64_t n, int L, void* out, float4* meta,
                                 cudaStream_t s, const uint32_t* n_dev = nullptr);
+// nitems[0]: items, nitems[1]: tiles per item (at most btpi; fewer where that
+// would leave SMs without an item)
 cudaError_t launch_group_queries(const int* approx, int nq, const LeafPlan* plan, int nleaves, uint32_t btpi,
                                  uint32_t* perm, uint32_t* slots, uint32_t* leaf_qoff, uint32_t* leaf_qcnt,
                                  uint32_t* item_off, uint32_t* nitems, BatchItem* items, cudaStream_t s,
                                  uint32_t* gcnt = nullptr);  // 2 x nleaves words above kMaxLeavesSort leaves
 // the pruned filter's query panel list and work items from the kept
 // (leaf, query) pairs (k_group_pruned, k_emit_pruned); ctl[2] = the query
-// count (*nq_dev if set, else nq) when the panel or the items do not fit
+// count (*nq_dev if set, else nq) when the panel or the items do not fit;
+// items of at most tpi tiles, at least tpi_min
 cudaError_t launch_group_pruned(const uint32_t* leaf_cnt, const uint32_t* leaf_q, uint32_t stride,
-                                const LeafPlan* plan, int nleaves, uint32_t tpi, uint32_t panel_cap,
+                                const LeafPlan* plan, int nleaves, uint32_t tpi, uint32_t tpi_min, uint32_t panel_cap,
                                 uint32_t items_cap, uint32_t nq, uint32_t* leaf_poff, uint32_t* leaf_ioff,
                                 uint32_t* ctl, unsigned long long* pairs, uint32_t* panel_list, BatchItem* items,
                                 cudaStream_t s, const uint32_t* nq_dev = nullptr);
@@ -135,9 +152,7 @@ size_t umma_filter_smem();
 size_t umma_pair_smem();
 cudaError_t launch_umma_pair(const CUtensorMap& rows_map, const CUtensorMap& q_half_map, const BatchGemm& g,
                              int blocks, cudaStream_t s);
-// q_map: boxes of 256 queries, except for the bound pass (mode 0) with L <= 256:
-// boxes of kBatchBoundQueries
-cudaError_t launch_umma_filter(const CUtensorMap& rows_map, const CUtensorMap& q_map, const BatchGemm& g, int blocks,
+cudaError_t launch_umma_filter(const CUtensorMap& rows_map, const QueryMaps& q, const BatchGemm& g, int blocks,
                                cudaStream_t s);
 cudaError_t launch_rerank(const BatchRank& r, int part_blocks, cudaStream_t s);
 // Distributes the filter's survivor pairs into per-query buckets

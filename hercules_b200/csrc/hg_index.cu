@@ -1629,6 +1629,12 @@ static hg_status encode_bf16_map(CUtensorMap* map, const void* base, uint64_t n,
   return HG_OK;
 }
 
+static hg_status encode_query_maps(hg::QueryMaps* m, const void* base, uint64_t n, uint32_t L) {
+  HCK(encode_bf16_map(&m->q256, base, n, L, hg::kBatchQueryTile));
+  HCK(encode_bf16_map(&m->q128, base, n, L, hg::kBatchQueryTile / 2));
+  return encode_bf16_map(&m->q64, base, n, L, hg::kBatchBoundQueries);
+}
+
 static hg_status ensure_batch_data(hg_index* ix, cudaStream_t st) {
   hg::BatchData& b = ix->bd;
   if (b.xbf) return HG_OK;
@@ -1689,8 +1695,10 @@ static hg_status ensure_batch_scratch(hg_index* ix, uint32_t nq, uint32_t bucket
     b.bm_cap = 0;
     b.parts_kmax = 0;
   }
-  // survivor pairs: room for 16,384 per query of the batch, at most 2^28
-  const uint32_t pairs_cap = (uint32_t)std::min<uint64_t>((uint64_t)b.nq_cap * 16384, 1ull << 28);
+  // survivor pairs: room for 16,384 per query of the batch and a block begun
+  // by every filter warp, at most 2^28
+  const uint64_t begun = (uint64_t)hg::sm_count(ix->device) * hg::kBatchPairWarps * hg::kBatchPairBlock;
+  const uint32_t pairs_cap = (uint32_t)std::min<uint64_t>((uint64_t)b.nq_cap * 16384 + begun, 1ull << 28);
   if (pairs_cap > b.pairs_cap || !b.pairs) {
     dfree(b.pairs);
     CK(dalloc(&b.pairs, pairs_cap));
@@ -1788,7 +1796,9 @@ static hg_status ensure_prune_scratch(hg_index* ix, bool* ok) {
   const uint64_t panel = std::min<uint64_t>(nl * nq, std::max<uint64_t>(nq, budget / (2 * L)));
   // items for the narrowest work item (8 tiles): chunks of every leaf x its query tiles
   const uint64_t ntiles = (ix->n + hg::kBatchTileRows - 1) / hg::kBatchTileRows;
-  const uint64_t items = (ntiles / 8 + 2 * nl) * ((nq + hg::kBatchQueryTile - 1) / hg::kBatchQueryTile);
+  // and kBatchItemTarget more where narrower ones even out a small batch
+  const uint64_t items =
+      (ntiles / 8 + 2 * nl) * ((nq + hg::kBatchQueryTile - 1) / hg::kBatchQueryTile) + hg::kBatchItemTarget;
   if (panel >= (1ull << 32) || items >= (1ull << 31)) {
     *ok = false;
     return HG_OK;
@@ -1802,13 +1812,12 @@ static hg_status ensure_prune_scratch(hg_index* ix, bool* ok) {
   CK(dalloc(&p, panel * L));
   b.panel_bf = p;
   CK(dalloc(&b.items3, items));
-  CK(dalloc(&b.pctl, 8));    // [0, 4): the first round's panel controls, [4, 8): a retry round's
+  CK(dalloc(&b.pctl, 16));   // [0, 8): the first round's panel controls, [8, 16): a retry round's
   CK(dalloc(&b.ppairs, 2));
   CK(dalloc(&b.segstats, std::max<uint64_t>((uint64_t)b.nu * nq, 1)));
   b.panel_cap = (uint32_t)panel;
   b.items3_cap = (uint32_t)items;
-  HCK(encode_bf16_map(&b.panel_map, b.panel_bf, panel, (uint32_t)L, hg::kBatchQueryTile));
-  HCK(encode_bf16_map(&b.panel_map_half, b.panel_bf, panel, (uint32_t)L, hg::kBatchQueryTile / 2));
+  HCK(encode_query_maps(&b.panel_maps, b.panel_bf, panel, (uint32_t)L));
   b.prune_nq = (uint32_t)nq;
   ++b.gen;  // a captured pipeline holds the old addresses
   return HG_OK;
@@ -1874,8 +1883,8 @@ static hg_status ensure_leaf_plan(hg_index* ix, uint64_t want, cudaStream_t st) 
 // bound pass, 1 + kBatchRetries filter rounds whose query lists are built on
 // the device (an empty round costs a few microseconds), the count of queries
 // left unverified.  Events gev[0..] mark the phases.
-static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_t bucket_cap, const CUtensorMap& qmap,
-                               const CUtensorMap& qmap_half, const CUtensorMap& qmap_bound, bool prune, cudaStream_t st,
+static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_t bucket_cap, const hg::QueryMaps& qmaps,
+                               bool prune, cudaStream_t st,
                                uint64_t* launches) {
   hg::BatchScratch& b = ix->bs;
   const uint32_t L = ix->L;
@@ -1917,7 +1926,7 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
   g.pairs_cap = b.pairs_cap;
   g.err = reinterpret_cast<int*>(b.heads + 3);
   g.queue = b.queues + 0;
-  CK(hg::launch_umma_filter(ix->bd.rows_map, L <= 256 ? qmap_bound : qmap, g, sms, st));
+  CK(hg::launch_umma_filter(ix->bd.rows_map, qmaps, g, sms, st));
   hg::BatchRank r{};
   r.rows = ix->d.rows;
   r.ids = ix->d.ids;
@@ -1953,6 +1962,10 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
   // 3a. the leaves each query must filter (LB_EAPCA within B_q), each leaf's
   // queries laid out contiguously in a BF16 panel, and the work items
   const hg::DeviceIndex& d = ix->d;
+  // the narrowest work item: a resident query tile (L <= 256) is loaded once
+  // per item, so an item has at least four row tiles; a streamed one is read
+  // for every two row tiles whatever the item's length
+  const uint32_t tpi_min = L <= 256 ? 4 : 2;
   if (prune) {
     CK(cudaMemsetAsync(b.leaf_cnt, 0, sizeof(uint32_t) * nl, st));
     CK(cudaMemsetAsync(b.ppairs, 0, sizeof(unsigned long long), st));
@@ -1961,9 +1974,9 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
                             b.prune_nq, st));
     ++*launches;
     CK(hg::launch_group_pruned(b.leaf_cnt, b.leaf_q, b.prune_nq, b.leaf_plan, nl, ix->tune.filter_tiles_per_item,
-                               b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, b.pctl, b.ppairs,
+                               tpi_min, b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, b.pctl, b.ppairs,
                                b.panel_list, b.items3, st));
-    CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, b.qmeta, st, b.pctl + 1));
+    CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, nullptr, st, b.pctl + 1));
     *launches += 4;
   }
   CK(stamp(1));
@@ -1972,9 +1985,9 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
   // screening passes run on CTA pairs (cta_group::2) where the query tile
   // stays resident (L <= 256) unless the tuning asks for one CTA per tile.
   const bool pair = ix->tune.filter_cta_pair != 2 && L <= 256;  // four resident 64-column K blocks
-  auto screen = [&](const CUtensorMap& full_map, const CUtensorMap& half_map) {
-    return pair ? hg::launch_umma_pair(ix->bd.rows_map, half_map, g, sms, st)
-                : hg::launch_umma_filter(ix->bd.rows_map, full_map, g, sms, st);
+  auto screen = [&](const hg::QueryMaps& q) {
+    return pair ? hg::launch_umma_pair(ix->bd.rows_map, q.q128, g, sms, st)
+                : hg::launch_umma_filter(ix->bd.rows_map, q, g, sms, st);
   };
   uint32_t* lists[2] = {b.qlist, b.qlist2};
   for (int round = 0; round <= kBatchRetries; ++round) {
@@ -1986,16 +1999,16 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
     }
     // a retry round prunes leaves again for its queries, against the bounds
     // the previous round lowered (a subset of the leaves kept before)
-    uint32_t* ctl = round == 0 ? b.pctl : b.pctl + 4;
+    uint32_t* ctl = round == 0 ? b.pctl : b.pctl + 8;
     if (round > 0 && prune) {
       CK(cudaMemsetAsync(b.leaf_cnt, 0, sizeof(uint32_t) * nl, st));
       CK(hg::launch_leaf_keep_list(b.segstats, b.nu, (int)L, (int)nq, d.leaf_seg_off, d.leaf_points, b.seg_uid,
                                    d.leaf_sk, d.leaf_size, nl, b.bound, b.leaf_cnt, b.leaf_q, b.prune_nq, list_in,
                                    n_dev, st));
       CK(hg::launch_group_pruned(b.leaf_cnt, b.leaf_q, b.prune_nq, b.leaf_plan, nl, ix->tune.filter_tiles_per_item,
-                                 b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, ctl, b.ppairs + 1,
+                                 tpi_min, b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, ctl, b.ppairs + 1,
                                  b.panel_list, b.items3, st, n_dev));
-      CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, b.qmeta, st, ctl + 1));
+      CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, nullptr, st, ctl + 1));
       *launches += 4;
     }
     g.errstat = round == 0 ? b.errstat : nullptr;
@@ -2014,7 +2027,7 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
       g.nq_dev = nullptr;
       g.qtile = hg::kBatchQueryTile;
       g.queue = round == 0 ? b.queues + 1 : b.queues + 5 + round;
-      CK(screen(b.panel_map, b.panel_map_half));
+      CK(screen(b.panel_maps));
       ++*launches;
     }
     g.mode = 1;
@@ -2022,7 +2035,7 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
     g.nq_dev = prune ? ctl + 2 : n_dev;
     g.qtile = round == 0 ? hg::kBatchQueryTile : 0;
     g.queue = b.queues + 2 + round;
-    CK(screen(qmap, qmap_half));
+    CK(screen(qmaps));
     CK(stamp(3 + 3 * round));
     CK(hg::launch_scatter_pairs(b.pairs, b.heads + 1, b.pairs_cap, list_in, (int)nq, n_dev, b.bucket, b.bucket_cnt,
                                 bucket_cap, st));
@@ -2156,7 +2169,8 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   const uint32_t btpi = ix->tune.bound_tiles_per_item;
   const uint32_t items_cap =
       (uint32_t)(((uint64_t)(nq + hg::kBatchBoundQueries - 1) / hg::kBatchBoundQueries + ix->leaves.size()) *
-                 ((b.plan_max_use + btpi - 1) / btpi));
+                 ((b.plan_max_use + btpi - 1) / btpi)) +
+      hg::kBatchItemTarget + nq;
   HCK(ensure_batch_scratch(ix, std::max(nq, b.nq_cap), bucket_cap, b.plan_bm_cap, items_cap, kmax));
   if (!b.ctrl) {
     CK(dalloc(&b.ctrl, 16));
@@ -2180,10 +2194,8 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   CK(cudaMemcpyAsync(b.qin, d_Q, sizeof(float) * nq * L,
                      host_io ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
   CK(cudaMemcpyAsync(b.kq, kq.data(), sizeof(uint32_t) * nq, cudaMemcpyHostToDevice, st));
-  CUtensorMap qmap, qmap_half, qmap_bound;
-  HCK(encode_bf16_map(&qmap, b.qbf, nq, L, hg::kBatchQueryTile));
-  HCK(encode_bf16_map(&qmap_half, b.qbf, nq, L, hg::kBatchQueryTile / 2));
-  HCK(encode_bf16_map(&qmap_bound, b.qbf, nq, L, hg::kBatchBoundQueries));
+  hg::QueryMaps qmaps;
+  HCK(encode_query_maps(&qmaps, b.qbf, nq, L));
   // the pipeline, captured once per shape in a CUDA graph and replayed
   bool prune = false;
   if (!o.dense_filter) HCK(ensure_prune_scratch(ix, &prune));
@@ -2197,7 +2209,7 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
     }
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-    const hg_status s = enqueue_batch(ix, nq, kmax, bucket_cap, qmap, qmap_half, qmap_bound, prune, st, &launches);
+    const hg_status s = enqueue_batch(ix, nq, kmax, bucket_cap, qmaps, prune, st, &launches);
     const cudaError_t ce = cudaStreamEndCapture(st, &graph);
     if (s != HG_OK) {
       if (graph) cudaGraphDestroy(graph);
@@ -2558,9 +2570,10 @@ static hg_status bf16_dots_impl(const float* d_rows, uint64_t n, uint32_t L, con
     release();
     return cuda_fail(e, "hg_bf16_dots");
   }
-  CUtensorMap xmap, qmap;
+  CUtensorMap xmap;
+  hg::QueryMaps qmaps;
   hg_status hs = encode_bf16_map(&xmap, xbf, n, L, 128);
-  if (hs == HG_OK) hs = encode_bf16_map(&qmap, qbf, nq, L, hg::kBatchQueryTile);
+  if (hs == HG_OK) hs = encode_query_maps(&qmaps, qbf, nq, L);
   if (hs != HG_OK) {
     release();
     return hs;
@@ -2581,7 +2594,7 @@ static hg_status bf16_dots_impl(const float* d_rows, uint64_t n, uint32_t L, con
   g.dots_ld = n;
   g.wait_ns = wait_ns;
   g.withhold_first_copy = withhold;
-  e = hg::launch_umma_filter(xmap, qmap, g, hg::sm_count(dev), st);
+  e = hg::launch_umma_filter(xmap, qmaps, g, hg::sm_count(dev), st);
   int herr = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -151,8 +151,7 @@ struct BatchScratch {
   uint32_t panel_cap = 0, items3_cap = 0;
   uint32_t* pctl = nullptr;              // [4] items, panel rows, dense-pass queries
   unsigned long long* ppairs = nullptr;  // (query, row) pairs of the pruned pass
-  CUtensorMap panel_map;                 // TMA descriptor of panel_bf (64 x 256 boxes)
-  CUtensorMap panel_map_half;            // the same with 64 x 128 boxes (the CTA-pair filter)
+  QueryMaps panel_maps;                  // TMA descriptors of panel_bf
   // distinct leaf segments (shared by many leaves) and the queries' mean and
   // stdev over each
   int nu = 0;

@@ -4,8 +4,9 @@
 //
 // One persistent CTA per SM, 12 warps:
 //   warp 0      TMA producer (one elected lane): row tiles (A, 128 rows x 64 K
-//               per stage) and the query tile (B, 256 queries x L, resident
-//               in shared memory for L <= 256, else streamed with A);
+//               per stage) and the query tile (B, up to 256 queries x L in
+//               boxes of 64, resident in shared memory for L <= 256, else
+//               streamed with A);
 //   warp 1      MMA issuer (one lane): per 128-row tile, L/16 MMAs of
 //               M=128, N=256, K=16 into one of two TMEM accumulators;
 //   warp 2      allocates / frees the 512 TMEM columns;
@@ -41,10 +42,18 @@ constexpr int kThreads = 384;  // 12 warps
 constexpr int kEpiThreads = 256;
 constexpr uint32_t kABytes = kUM * kUK * 2;  // 16 KB per A stage
 constexpr uint32_t kQBytes = kUN * kUK * 2;  // 32 KB per query K block
+// A query tile of at most 192 queries comes in boxes of 64 (8 KB of a K block,
+// eight 1,024-byte swizzle groups, so boxes side by side form the same tile as
+// one box of 256), and only the boxes that hold queries are copied.  A
+// streamed tile is read again for every two row tiles, and the filter is then
+// bound by the copies into shared memory: 128 queries over 200k x 16384 (59
+// kept queries per leaf) streamed 64 KB per stage of which 24 KB were not
+// wanted; the pass took 2.07 ms and now takes 1.16 ms, with shorter items.
+constexpr uint32_t kQBox = 64;
+constexpr uint32_t kQBoxBytes = kQBox * kUK * 2;
 constexpr int kResidentKB = 4;               // L <= 256: the query tile stays resident
 constexpr uint64_t kWaitNs = 2000000000ull;  // 2 s per wait
 constexpr int kErrTimeout = 1;
-constexpr uint32_t kPairBlock = 1024;        // survivor pairs reserved per warp at a time
 
 // The screening modes fold each query's threshold into the accumulator with
 // one more K = 16 MMA per tile: A_ext (128 rows x 16, every element 1) times
@@ -289,9 +298,13 @@ __device__ __forceinline__ Item item_of(const BatchGemm& a, uint32_t w, uint32_t
 // kScreen: modes 1 and 3 (else 0 and 2); kResident: L <= 256, the query tile
 // stays in shared memory (else it is streamed with the row tiles).  The
 // launcher picks the instance, so the per-stage loops carry no mode tests.
-template <bool kScreen, bool kResident, bool kBound>
+// kTail: L is not a multiple of 64, so the last K block holds fewer K = 16
+// steps (an instance of its own: a test per stage in the MMA lane's loop cost
+// the 25M x 256 pass 3%).
+template <bool kScreen, bool kResident, bool kBound, bool kTail>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_umma_filter(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmQ, BatchGemm a) {
+    k_umma_filter(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmQ,
+                  const __grid_constant__ CUtensorMap tmQ64, BatchGemm a) {
   using LY = FilterLayout<kBound>;
   extern __shared__ unsigned char umma_raw[];
   unsigned char* sm = umma_raw + ((1024 - (s2u(umma_raw) & 1023)) & 1023);
@@ -384,6 +397,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) {
     // ---------------- TMA producer
     if (lane == 0) {
+      auto load_q = [&](uint32_t dst, int kb, int q0, uint32_t boxes, uint32_t bar) {
+        if (boxes == kUN / kQBox) {
+          tma_load_2d(dst, &tmQ, kb * kUK, q0, bar);
+        } else {
+          for (uint32_t x = 0; x < boxes; ++x)
+            tma_load_2d(dst + x * kQBoxBytes, &tmQ64, kb * kUK, q0 + (int)(x * kQBox), bar);
+        }
+      };
       uint32_t g = 0, it_n = 0, q_issued = 0;
       uint32_t s_cur = 0, ph = 0;  // stage g % nst and the parity of g / nst
       bool ok = true;
@@ -398,12 +419,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         mbar_arrive(ifull_bar(sl));
         if (w >= total) break;
         const Item it = item_of(a, w, QT, ntiles, qtile, nq);
+        const uint32_t qboxes = ((uint32_t)item_n(it.qcnt, qtile) + kQBox - 1) / kQBox;
         if (resident) {
           ok = mbar_wait(qempty_bar, (it_n & 1) ^ 1, abort_flag, a.err, wns);
           if (!ok) break;
-          mbar_expect_tx(qfull_bar, (uint32_t)nkb * LY::kQBlk);
-          for (int kb = 0; kb < nkb; ++kb)
-            tma_load_2d(base + LY::kQ + kb * LY::kQBlk, &tmQ, kb * kUK, (int)it.qoff, qfull_bar);
+          mbar_expect_tx(qfull_bar, (uint32_t)nkb * qboxes * kQBoxBytes);
+          for (int kb = 0; kb < nkb; ++kb) load_q(base + LY::kQ + kb * LY::kQBlk, kb, (int)it.qoff, qboxes, qfull_bar);
           ++q_issued;
         }
         const uint32_t ngroups = it.t_hi > it.t_lo ? (it.t_hi - it.t_lo + kGroup - 1) / kGroup : 0u;
@@ -421,12 +442,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             // diagnostics: the first stage's copy withheld, so its barrier
             // phase never completes and the MMA warp's bounded wait runs out
             if (a.withhold_first_copy && g == 0) continue;
-            mbar_expect_tx(full_bar(s), kGroup * kABytes + (resident ? 0u : kQBytes));
+            mbar_expect_tx(full_bar(s), kGroup * kABytes + (resident ? 0u : qboxes * kQBoxBytes));
 #pragma unroll
             for (uint32_t gi = 0; gi < kGroup; ++gi)
               tma_load_2d(base + aBase + (s * kGroup + gi) * kABytes, &tmA, kb * kUK,
                           (int)(it.rb + (uint64_t)(t0 + gi) * kUM), full_bar(s));
-            if (!resident) tma_load_2d(base + LY::kQ + s * kQBytes, &tmQ, kb * kUK, (int)it.qoff, full_bar(s));
+            if (!resident) load_q(base + LY::kQ + s * kQBytes, kb, (int)it.qoff, qboxes, full_bar(s));
           }
         }
         if (!ok) break;
@@ -445,6 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t g = 0, tcount = 0, it_n = 0;
       uint32_t s_cur = 0, ph = 0;  // stage g % nst and the parity of g / nst
       const uint64_t dae = sw32_desc(base + LY::kAext), dbe = sw32_desc(base + LY::kBext);
+      const int last_steps = kTail ? (a.L - (nkb - 1) * kUK) / 16 : 0;  // 1..3: L is a multiple of 16
       bool ok = true;
       for (; ok; ++it_n) {
         const int sl = (int)(it_n & 1);
@@ -491,12 +513,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_fence_after();
             // K step k16 is 32 bytes on: 2 in the descriptors' address field
             const uint64_t dq = sw128_desc(base + LY::kQ + (resident ? (uint32_t)kb * LY::kQBlk : (uint32_t)s * kQBytes));
+            const int steps = kTail && kb == nkb - 1 ? last_steps : kUK / 16;
 #pragma unroll
             for (uint32_t gi = 0; gi < kGroup; ++gi) {
               const uint64_t da = sw128_desc(base + aBase + (s * kGroup + gi) * kABytes);
 #pragma unroll
               for (int k16 = 0; k16 < kUK / 16; ++k16)
-                tc_mma(d + gi * kUN, da + 2 * k16, dq + 2 * k16, idesc, (screen || kb || k16) ? 1u : 0u);
+                if (!kTail || k16 < steps)
+                  tc_mma(d + gi * kUN, da + 2 * k16, dq + 2 * k16, idesc, (screen || kb || k16) ? 1u : 0u);
             }
             tc_commit(empty_bar(s));
           }
@@ -791,7 +815,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(tempty_bar(b));
         // survivor pairs into the warp's reserved block of the pair list:
-        // plain stores, one atomic per kPairBlock pairs
+        // plain stores, one atomic per kBatchPairBlock pairs
 #pragma unroll
         for (uint32_t gi = 0; gi < kGroup; ++gi) {
         const uint64_t row = rows_g[gi];
@@ -812,10 +836,10 @@ __global__ void __launch_bounds__(kThreads, 1)
               // close the block (sentinels in its tail) and reserve the next
               for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
               uint32_t nb = 0;
-              if (lane == 0) nb = atomicAdd(a.pairs_cnt, (uint32_t)kPairBlock);
+              if (lane == 0) nb = atomicAdd(a.pairs_cnt, (uint32_t)kBatchPairBlock);
               nb = __shfl_sync(HG_FULL, nb, 0);
               pcur = nb;
-              pend = nb + kPairBlock < a.pairs_cap ? nb + kPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
+              pend = nb + kBatchPairBlock < a.pairs_cap ? nb + kBatchPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
             }
             const uint32_t slot = pcur + (uint32_t)__popc(bal & ((1u << lane) - 1));
             if (has && slot < pend) a.pairs[slot] = e;
@@ -1357,10 +1381,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (pcur + cnt > pend) {
               for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
               uint32_t nb = 0;
-              if (lane == 0) nb = atomicAdd(a.pairs_cnt, (uint32_t)kPairBlock);
+              if (lane == 0) nb = atomicAdd(a.pairs_cnt, (uint32_t)kBatchPairBlock);
               nb = __shfl_sync(HG_FULL, nb, 0);
               pcur = nb;
-              pend = nb + kPairBlock < a.pairs_cap ? nb + kPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
+              pend = nb + kBatchPairBlock < a.pairs_cap ? nb + kBatchPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
             }
             const uint32_t slot = pcur + (uint32_t)__popc(bal & ((1u << lane) - 1));
             if (has && slot < pend) a.pairs[slot] = e;
@@ -1438,18 +1462,25 @@ cudaError_t launch_umma_pair(const CUtensorMap& rows_map, const CUtensorMap& q_h
 
 size_t umma_filter_smem() { return FilterLayout<false>::kDyn; }
 
-template <bool kScreen, bool kResident, bool kBound>
-static cudaError_t launch_filter_instance(const CUtensorMap& rows_map, const CUtensorMap& q_map, const BatchGemm& g,
+template <bool kScreen, bool kResident, bool kBound, bool kTail>
+static cudaError_t launch_filter_tail(const CUtensorMap& rows_map, const QueryMaps& q, const BatchGemm& g,
                                           int grid, cudaStream_t s) {
   constexpr int smem = (int)FilterLayout<kBound>::kDyn;
   static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)k_umma_filter<kScreen, kResident, kBound>, smem);
+  const cudaError_t ea = attr.ensure((const void*)k_umma_filter<kScreen, kResident, kBound, kTail>, smem);
   if (ea != cudaSuccess) return ea;
-  k_umma_filter<kScreen, kResident, kBound><<<grid, kThreads, smem, s>>>(rows_map, q_map, g);
+  k_umma_filter<kScreen, kResident, kBound, kTail><<<grid, kThreads, smem, s>>>(rows_map, q.q256, q.q64, g);
   return cudaGetLastError();
 }
 
-cudaError_t launch_umma_filter(const CUtensorMap& rows_map, const CUtensorMap& q_map, const BatchGemm& g, int blocks,
+template <bool kScreen, bool kResident, bool kBound>
+static cudaError_t launch_filter_instance(const CUtensorMap& rows_map, const QueryMaps& q, const BatchGemm& g, int grid,
+                                          cudaStream_t s) {
+  return g.L % kUK ? launch_filter_tail<kScreen, kResident, kBound, true>(rows_map, q, g, grid, s)
+                   : launch_filter_tail<kScreen, kResident, kBound, false>(rows_map, q, g, grid, s);
+}
+
+cudaError_t launch_umma_filter(const CUtensorMap& rows_map, const QueryMaps& q, const BatchGemm& g, int blocks,
                                cudaStream_t s) {
   const uint64_t ntiles = (g.nrows + kUM - 1) / kUM;
   if (g.mode != 0 && g.qtile != 0 && g.qtile != 64 && g.qtile != 128 && g.qtile != 256) return cudaErrorInvalidValue;
@@ -1467,13 +1498,12 @@ cudaError_t launch_umma_filter(const CUtensorMap& rows_map, const CUtensorMap& q
   const bool screen = g.mode == 1 || g.mode == 3;
   const bool resident = (g.L + kUK - 1) / kUK <= kResidentKB;
   if (screen) {
-    return resident ? launch_filter_instance<true, true, false>(rows_map, q_map, g, grid, s)
-                    : launch_filter_instance<true, false, false>(rows_map, q_map, g, grid, s);
+    return resident ? launch_filter_instance<true, true, false>(rows_map, q, g, grid, s)
+                    : launch_filter_instance<true, false, false>(rows_map, q, g, grid, s);
   }
-  // the bound pass with a resident query tile: q_map has 64-query boxes
-  if (g.mode == 0 && resident) return launch_filter_instance<false, true, true>(rows_map, q_map, g, grid, s);
-  return resident ? launch_filter_instance<false, true, false>(rows_map, q_map, g, grid, s)
-                  : launch_filter_instance<false, false, false>(rows_map, q_map, g, grid, s);
+  if (g.mode == 0 && resident) return launch_filter_instance<false, true, true>(rows_map, q, g, grid, s);
+  return resident ? launch_filter_instance<false, true, false>(rows_map, q, g, grid, s)
+                  : launch_filter_instance<false, false, false>(rows_map, q, g, grid, s);
 }
 
 }  // namespace hg
