@@ -79,18 +79,19 @@ __global__ void k_rows_to_bf16(const float* __restrict__ rows, const uint32_t* _
       acc(v.w, f1.y);
     }
   }
-  if constexpr (!kMeta) continue;
+  if constexpr (kMeta) {
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    a2 += __shfl_xor_sync(HG_FULL, a2, s);
-    t2 += __shfl_xor_sync(HG_FULL, t2, s);
-    r2 += __shfl_xor_sync(HG_FULL, r2, s);
-  }
-  if (lane == 0) {
-    // FP64 sums of L non-negative terms: relative error below L 2^-53
-    const double up = 1.0 + 1e-12;
-    meta[src] = make_float4(__double2float_ru(a2 * up), __double2float_ru(sqrt(t2) * up),
-                          __double2float_ru(sqrt(r2) * up), 0.0f);
+    for (int s = 16; s > 0; s >>= 1) {
+      a2 += __shfl_xor_sync(HG_FULL, a2, s);
+      t2 += __shfl_xor_sync(HG_FULL, t2, s);
+      r2 += __shfl_xor_sync(HG_FULL, r2, s);
+    }
+    if (lane == 0) {
+      // FP64 sums of L non-negative terms: relative error below L 2^-53
+      const double up = 1.0 + 1e-12;
+      meta[src] = make_float4(__double2float_ru(a2 * up), __double2float_ru(sqrt(t2) * up),
+                              __double2float_ru(sqrt(r2) * up), 0.0f);
+    }
   }
   }
 }

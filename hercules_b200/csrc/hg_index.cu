@@ -439,6 +439,21 @@ static hg_status upload_tables(hg_index* ix) {
 
 namespace {
 
+// The tree grows on the host, the rows stay on the device: node_of holds the
+// node of every row routed so far (a leaf's members in insertion order are its
+// rows in ascending order, as rows are inserted and redistributed in order).
+// A window of rows is routed through the tree of the moment and the host
+// counts the rows into their leaves.  A leaf that fills up waits for its
+// split, and the window's later rows of that leaf wait with it; the other
+// leaves do not depend on it, so the count goes on, and at the window's end
+// all waiting leaves split together, in two device round trips (envelopes of
+// the members, then their redistribution, which also moves the waiting rows).
+// The waiting rows are counted again, until none waits.  The tree is the one
+// that splits one at a time give.  Splitting one leaf at a time and routing
+// the rest of the window again after it, with the member lists on the host,
+// took 74 ms for 1M x 256, leaf 10,000 (193 leaves; 24 ms of it routing), and
+// 1.37 s for 1M x 64, leaf 200 (8,468 leaves); this takes
+// 20 and 60 ms.
 struct BuildCtx {
   hg_index* ix;
   const float* X;  // device, n x L row-major, original order
@@ -446,178 +461,239 @@ struct BuildCtx {
   // device build scratch
   hg::DNode* d_tree = nullptr;
   size_t tree_cap = 0;
-  int* d_leaf_of = nullptr;
-  uint32_t* d_members = nullptr;
-  uint8_t* d_flags = nullptr;
+  int* d_node_of = nullptr;       // n
+  uint32_t* d_list = nullptr;     // n: rows of the leaves being split
+  uint32_t* d_count = nullptr;    // members collected and sent left per leaf, later rows
+  size_t count_cap = 0;
   int* d_keys = nullptr;
-  short* d_seg = nullptr;  // from[MAXS], to[MAXS]
-  int* h_leaf_of = nullptr;  // pinned
-  uint32_t members_cap = 0;
+  size_t keys_cap = 0;
+  unsigned char* d_round = nullptr;  // tables of a round of splits
+  size_t round_cap = 0;
   std::vector<hg::DNode> h_tree;  // node id -> routing entry (internal nodes)
+  enum State : uint32_t { kLeaf, kWaiting, kInternal };
+  struct Count {
+    uint32_t rows = 0;  // of the leaf (an internal node: when it split)
+    State state = kLeaf;
+  };
+  std::vector<Count> fill;        // by node
+  std::vector<int> win;           // node of each row of the window
+  bool tree_changed = true;
   int root_enc = ~0;
-  static constexpr uint32_t kWindow = 65536;
+  // windows double with the rows inserted, so a leaf splits about once per
+  // window; the largest bounds the rows counted again
+  static constexpr uint32_t kWindowMin = 65536, kWindowMax = 262144;
   static constexpr int kMaxSegs = 4096;
+  struct Full {
+    int nid;
+    uint32_t last;  // the row that filled the leaf
+  };
 
   ~BuildCtx() {
     dfree(d_tree);
-    dfree(d_leaf_of);
-    dfree(d_members);
-    dfree(d_flags);
+    dfree(d_node_of);
+    dfree(d_list);
+    dfree(d_count);
     dfree(d_keys);
-    dfree(d_seg);
-    if (h_leaf_of) cudaFreeHost(h_leaf_of);
+    dfree(d_round);
+  }
+
+  template <class T>
+  hg_status grow(T** p, size_t* cap, size_t want) {
+    if (want <= *cap) return HG_OK;
+    CK(cudaStreamSynchronize(st));
+    dfree(*p);
+    *cap = 0;
+    CK(dalloc(p, 2 * want));
+    *cap = 2 * want;
+    return HG_OK;
   }
 
   // During the build a leaf child is encoded ~node_id.
   hg_status sync_tree() {
-    if (h_tree.size() > tree_cap) {
-      dfree(d_tree);
-      tree_cap = std::max<size_t>(h_tree.size() * 2, 1024);
-      CK(dalloc(&d_tree, tree_cap));
-    }
+    if (!tree_changed) return HG_OK;
+    HCK(grow(&d_tree, &tree_cap, std::max<size_t>(h_tree.size(), 512)));
     CK(cudaMemcpyAsync(d_tree, h_tree.data(), sizeof(hg::DNode) * h_tree.size(), cudaMemcpyHostToDevice, st));
+    tree_changed = false;
     return HG_OK;
   }
 
   hg::Tree tree() const { return hg::Tree{d_tree, root_enc}; }
 
-  // min/max envelopes of segments [from_i, to_i) over the members
-  hg_status sketches(const uint32_t* d_mem, uint32_t count, const std::vector<short>& from,
-                     const std::vector<short>& to, std::vector<float>& out) {
-    const int ns = (int)from.size();
-    if (ns > kMaxSegs) return set_error(HG_ERR_LIMIT, "too many EAPCA segments in one node");
-    std::vector<int> init(4 * ns);
-    for (int i = 0; i < ns; ++i) {
-      init[4 * i + 0] = INT_MIN;
-      init[4 * i + 1] = INT_MAX;
-      init[4 * i + 2] = INT_MIN;
-      init[4 * i + 3] = INT_MAX;
-    }
-    CK(cudaMemcpyAsync(d_keys, init.data(), sizeof(int) * 4 * ns, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_seg, from.data(), sizeof(short) * ns, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_seg + kMaxSegs, to.data(), sizeof(short) * ns, cudaMemcpyHostToDevice, st));
-    CK(hg::launch_sketch_members(X, ix->L, d_mem, count, d_seg, d_seg + kMaxSegs, ns, d_keys, st));
-    CK(cudaMemcpyAsync(init.data(), d_keys, sizeof(int) * 4 * ns, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    out.resize(4 * ns);
-    keys_to_sketch(init.data(), ns, out.data());
-    return HG_OK;
-  }
-
-  // hercules_index_split_node (hercules_node_split.c:1043-1345) for leaf nid
-  hg_status split(int nid) {
+  // hercules_index_split_node (hercules_node_split.c:1043-1345) for each full
+  // leaf; the rows below `end` are routed, `later` of them wait, and win (whose
+  // first row is c) is brought up to date from position `from` on
+  hg_status split(const std::vector<Full>& full, uint64_t c, uint64_t end, uint64_t later, uint32_t from) {
     std::vector<Node>& nodes = ix->nodes;
-    const uint32_t count = nodes[nid].node_size;
-    // a leaf that received every row of its parent's split holds more than
-    // leaf_size rows when it splits in turn
-    if (count > members_cap) {
-      CK(cudaStreamSynchronize(st));
-      dfree(d_members);
-      dfree(d_flags);
-      members_cap = std::max(count, members_cap * 2);
-      CK(dalloc(&d_members, members_cap));
-      CK(dalloc(&d_flags, members_cap));
+    const size_t P = full.size();
+    // one upload: list start, slot of every node, size, last row and segments
+    // (vertical, then horizontal candidates) of each leaf
+    std::vector<int> seg_off(P + 1, 0);
+    uint64_t members = 0;
+    hg::SketchArgs a{};
+    for (size_t p = 0; p < P; ++p) {
+      const Node& n = nodes[full[p].nid];
+      const int ns = (int)(n.points.size() + n.hs_points.size());
+      if (ns > kMaxSegs) return set_error(HG_ERR_LIMIT, "too many EAPCA segments in one node");
+      seg_off[p + 1] = seg_off[p] + ns;
+      a.max_segs = std::max(a.max_segs, ns);
+      a.max_size = std::max(a.max_size, fill[full[p].nid].rows);
     }
-    CK(cudaMemcpyAsync(d_members, nodes[nid].members.data(), sizeof(uint32_t) * count, cudaMemcpyHostToDevice,
-                       st));
-    // vertical + horizontal sketches of the leaf over its members
-    std::vector<short> from, to;
-    for (size_t i = 0; i < nodes[nid].points.size(); ++i) {
-      from.push_back((short)seg_start(nodes[nid].points, (int)i));
-      to.push_back(nodes[nid].points[i]);
+    const size_t T = (size_t)seg_off[P], N = nodes.size();
+    const size_t o_start = 0, o_slot = o_start + 8 * P, o_size = o_slot + 4 * N, o_last = o_size + 4 * P,
+                 o_off = o_last + 4 * P, o_seg = o_off + 4 * (P + 1), bytes = (o_seg + 4 * T + 7) & ~(size_t)7;
+    const size_t o_split = bytes;  // the policies follow, written after the envelopes are known
+    std::vector<unsigned char> h(bytes);
+    uint64_t* start = reinterpret_cast<uint64_t*>(h.data() + o_start);
+    int* slot = reinterpret_cast<int*>(h.data() + o_slot);
+    uint32_t* size = reinterpret_cast<uint32_t*>(h.data() + o_size);
+    uint32_t* last = reinterpret_cast<uint32_t*>(h.data() + o_last);
+    short* seg = reinterpret_cast<short*>(h.data() + o_seg);
+    std::fill(slot, slot + N, -1);
+    memcpy(h.data() + o_off, seg_off.data(), 4 * (P + 1));
+    for (size_t p = 0; p < P; ++p) {
+      const Node& n = nodes[full[p].nid];
+      start[p] = members;
+      slot[full[p].nid] = (int)p;
+      size[p] = fill[full[p].nid].rows;
+      last[p] = full[p].last;
+      members += size[p];
+      size_t t = (size_t)seg_off[p];
+      for (const std::vector<short>* pts : {&n.points, &n.hs_points})
+        for (size_t i = 0; i < pts->size(); ++i, ++t) {
+          seg[t] = (short)seg_start(*pts, (int)i);
+          seg[T + t] = (*pts)[i];
+        }
     }
-    for (size_t i = 0; i < nodes[nid].hs_points.size(); ++i) {
-      from.push_back((short)seg_start(nodes[nid].hs_points, (int)i));
-      to.push_back(nodes[nid].hs_points[i]);
-    }
-    std::vector<float> all;
-    HCK(sketches(d_members, count, from, to, all));
-    const size_t nv = nodes[nid].points.size();
-    nodes[nid].sk.assign(all.begin(), all.begin() + 4 * nv);
-    std::vector<float> hs_sk(all.begin() + 4 * nv, all.end());
-    std::vector<short> cp = choose_split(nodes[nid], hs_sk);
-    // children (split_node_create_children, hercules_node_split.c:197-262)
-    Node l = make_leaf(cp), r = make_leaf(cp);
-    l.parent = r.parent = nid;
-    l.level = r.level = nodes[nid].level + 1;
-    l.is_left = true;
-    l.filename = filename_of(l, &nodes[nid]);
-    r.filename = filename_of(r, &nodes[nid]);
-    const int lid = (int)nodes.size(), rid = lid + 1;
-    nodes.push_back(std::move(l));
-    nodes.push_back(std::move(r));
-    Node& n = nodes[nid];
-    n.left = lid;
-    n.right = rid;
-    // redistribution in insertion order (:1294-1333)
-    CK(hg::launch_route_flags(X, ix->L, d_members, count, n.split_from, n.split_to, n.split_idx, n.split_value,
-                              d_flags, st));
-    std::vector<uint8_t> flags(count);
-    CK(cudaMemcpyAsync(flags.data(), d_flags, count, cudaMemcpyDeviceToHost, st));
+    HCK(grow(&d_round, &round_cap, bytes + sizeof(hg::SplitPolicy) * P));
+    HCK(grow(&d_count, &count_cap, 2 * P + 1));
+    HCK(grow(&d_keys, &keys_cap, 4 * T));
+    uint32_t *d_members = d_count, *d_left = d_count + P, *d_later = d_count + 2 * P;
+    const int* d_slot = reinterpret_cast<int*>(d_round + o_slot);
+    CK(cudaMemcpyAsync(d_round, h.data(), bytes, cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(d_count, 0, sizeof(uint32_t) * (2 * P + 1), st));
+    a.X = X;
+    a.L = (int)ix->L;
+    a.members = d_list;
+    a.ngroups = (int)P;
+    a.start = reinterpret_cast<uint64_t*>(d_round + o_start);
+    a.size = reinterpret_cast<uint32_t*>(d_round + o_size);
+    a.seg_off = reinterpret_cast<int*>(d_round + o_off);
+    a.seg_from = reinterpret_cast<short*>(d_round + o_seg);
+    a.seg_to = a.seg_from + T;
+    a.keys = d_keys;
+    CK(hg::launch_collect_members(d_node_of, end, d_slot, a.start, reinterpret_cast<uint32_t*>(d_round + o_last), members,
+                                  d_list, d_members, d_later, d_keys, (int)T, st));
+    CK(hg::launch_sketch(a, st));
+    std::vector<int> keys(4 * T);
+    CK(cudaMemcpyAsync(keys.data(), d_keys, sizeof(int) * 4 * T, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    Node& L = nodes[lid];
-    Node& R = nodes[rid];
-    for (uint32_t m = 0; m < count; ++m) {
-      Node& c = flags[m] ? L : R;
-      c.members.push_back(n.members[m]);
-      ++c.node_size;
+    std::vector<hg::SplitPolicy> pol(P);
+    std::vector<float> hs_sk;
+    for (size_t p = 0; p < P; ++p) {
+      const int nid = full[p].nid;
+      const size_t nv = nodes[nid].points.size(), nh = nodes[nid].hs_points.size();
+      const int* k = &keys[4 * (size_t)seg_off[p]];
+      hs_sk.resize(4 * nh);
+      nodes[nid].sk.resize(4 * nv);
+      keys_to_sketch(k, nv, nodes[nid].sk.data());
+      keys_to_sketch(k + 4 * nv, nh, hs_sk.data());
+      std::vector<short> cp = choose_split(nodes[nid], hs_sk);
+      // children (split_node_create_children, hercules_node_split.c:197-262)
+      Node l = make_leaf(cp), r = make_leaf(cp);
+      l.parent = r.parent = nid;
+      l.level = r.level = nodes[nid].level + 1;
+      l.is_left = true;
+      l.filename = filename_of(l, &nodes[nid]);
+      r.filename = filename_of(r, &nodes[nid]);
+      const int lid = (int)nodes.size(), rid = lid + 1;
+      nodes.push_back(std::move(l));
+      nodes.push_back(std::move(r));
+      Node& n = nodes[nid];
+      n.left = lid;
+      n.right = rid;
+      n.is_leaf = false;
+      n.node_size = fill[nid].rows;
+      pol[p] = hg::SplitPolicy{n.split_value, lid, rid, n.split_from, n.split_to, n.split_idx};
+      // routing entries: this node becomes internal, its parent points to it
+      if (h_tree.size() < nodes.size()) h_tree.resize(nodes.size());
+      h_tree[nid] = hg::DNode{~lid, ~rid, n.split_value, n.split_from, n.split_to, n.split_idx, 0};
+      if (n.parent < 0) root_enc = nid;
+      else {
+        hg::DNode& d = h_tree[n.parent];
+        if (d.left == ~nid) d.left = nid;
+        else d.right = nid;
+      }
     }
-    std::vector<uint32_t>().swap(n.members);
-    n.is_leaf = false;
-    // routing entries: this node becomes internal, its parent points to it
-    if (h_tree.size() < nodes.size()) h_tree.resize(nodes.size());
-    hg::DNode& d = h_tree[nid];
-    d.left = ~lid;
-    d.right = ~rid;
-    d.value = n.split_value;
-    d.from = n.split_from;
-    d.to = n.split_to;
-    d.idx = n.split_idx;
-    d.pad = 0;
-    if (n.parent < 0) root_enc = nid;
-    else {
-      hg::DNode& p = h_tree[n.parent];
-      if (p.left == ~nid) p.left = nid;
-      else p.right = nid;
+    tree_changed = true;
+    hg::SplitPolicy* d_pol = reinterpret_cast<hg::SplitPolicy*>(d_round + o_split);
+    CK(cudaMemcpyAsync(d_pol, pol.data(), sizeof(hg::SplitPolicy) * P, cudaMemcpyHostToDevice, st));
+    CK(hg::launch_split_members(X, (int)ix->L, d_node_of, d_list, members, d_later, later, d_slot, d_pol, d_left, st));
+    std::vector<uint32_t> cnt(2 * P + 1);
+    CK(cudaMemcpyAsync(cnt.data(), d_count, sizeof(uint32_t) * cnt.size(), cudaMemcpyDeviceToHost, st));
+    if (later)
+      CK(cudaMemcpyAsync(win.data() + from, d_node_of + c + from, sizeof(int) * (end - c - from), cudaMemcpyDeviceToHost,
+                         st));
+    CK(cudaStreamSynchronize(st));
+    fill.resize(nodes.size());
+    for (size_t p = 0; p < P; ++p) {
+      const uint32_t left = cnt[P + p];
+      if (cnt[p] != size[p] || left > size[p])
+        return set_error(HG_ERR_CUDA, "internal: a split lost or invented rows");
+      fill[full[p].nid].state = kInternal;
+      fill[pol[p].left].rows = left;
+      fill[pol[p].right].rows = size[p] - left;
     }
-    return sync_tree();
+    if (cnt[2 * P] != later) return set_error(HG_ERR_CUDA, "internal: a split lost or invented rows");
+    return HG_OK;
   }
 
   hg_status run() {
     std::vector<Node>& nodes = ix->nodes;
     const uint64_t n = ix->n;
     const uint32_t S = ix->leaf_size;
-    CK(dalloc(&d_leaf_of, kWindow));
-    members_cap = S + 1;
-    CK(dalloc(&d_members, members_cap));
-    CK(dalloc(&d_flags, members_cap));
-    CK(dalloc(&d_keys, 4 * kMaxSegs));
-    CK(dalloc(&d_seg, 2 * kMaxSegs));
-    CK(cudaMallocHost((void**)&h_leaf_of, sizeof(int) * kWindow));
+    CK(dalloc(&d_node_of, n));
+    CK(dalloc(&d_list, n));
     h_tree.resize(1);
-    HCK(sync_tree());
-    uint64_t c = 0;
-    while (c < n) {
-      const uint32_t w = (uint32_t)std::min<uint64_t>(kWindow, n - c);
-      CK(hg::launch_route_rows(X, ix->L, nullptr, c, w, tree(), d_leaf_of, st));
-      CK(cudaMemcpyAsync(h_leaf_of, d_leaf_of, sizeof(int) * w, cudaMemcpyDeviceToHost, st));
+    fill.resize(1);
+    std::vector<Full> full;
+    std::vector<uint32_t> waiting, again;  // window positions, ascending
+    for (uint64_t c = 0; c < n;) {
+      const uint64_t grown = std::min<uint64_t>(kWindowMax, std::max<uint64_t>(kWindowMin, c));
+      const uint32_t w = (uint32_t)std::min<uint64_t>(grown, n - c);
+      win.resize(w);
+      HCK(sync_tree());
+      CK(hg::launch_route_rows(X, (int)ix->L, c, w, tree(), d_node_of + c, st));
+      CK(cudaMemcpyAsync(win.data(), d_node_of + c, sizeof(int) * w, cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
-      uint64_t next = c + w;
-      for (uint32_t j = 0; j < w; ++j) {
-        const int nid = h_leaf_of[j];  // the kernel already decoded ~child
-        if (nid < 0 || (size_t)nid >= nodes.size() || !nodes[nid].is_leaf)
-          return set_error(HG_ERR_CUDA, "internal: routing returned a node that is not a leaf");
-        Node& leaf = nodes[nid];
-        leaf.members.push_back((uint32_t)(c + j));
-        ++leaf.node_size;
-        if (leaf.node_size >= S) {
-          HCK(split(nid));
-          next = c + j + 1;  // the rest of the window routes through the new tree
-          break;
+      bool bad = false;
+      auto insert = [&](uint32_t j) {
+        const uint32_t nid = (uint32_t)win[j];
+        if (nid >= fill.size()) {
+          bad = true;
+          return;
         }
+        Count& leaf = fill[nid];
+        if (leaf.state != kLeaf) {
+          if (leaf.state == kWaiting) waiting.push_back(j);
+          else bad = true;
+        } else if (++leaf.rows >= S) {
+          leaf.state = kWaiting;
+          full.push_back(Full{(int)nid, (uint32_t)(c + j)});
+        }
+      };
+      for (uint32_t j = 0; j < w; ++j) insert(j);
+      while (!full.empty() && !bad) {
+        HCK(split(full, c, c + w, waiting.size(), waiting.empty() ? w : waiting.front()));
+        full.clear();
+        again.swap(waiting);
+        waiting.clear();
+        for (uint32_t j : again) insert(j);
       }
-      c = next;
+      if (bad) return set_error(HG_ERR_CUDA, "internal: routing returned a node that is not a leaf");
+      c += w;
     }
+    for (size_t i = 0; i < nodes.size(); ++i)
+      if (nodes[i].is_leaf) nodes[i].node_size = fill[i].rows;
     return HG_OK;
   }
 };
@@ -626,81 +702,106 @@ struct BuildCtx {
 
 // Leaf order, file positions, leaf envelopes, the leaf-ordered tiles, iSAX
 // words and the merged internal envelopes of the written index.
-static hg_status finalize_build(hg_index* ix, const float* X, cudaStream_t st) {
+static hg_status finalize_build(hg_index* ix, const float* X, cudaStream_t st, const BuildCtx& ctx) {
   std::vector<Node>& nodes = ix->nodes;
   ix->leaves.clear();
   collect_leaves(nodes, 0, ix->leaves);
-  std::vector<uint32_t> perm;
-  perm.reserve(ix->n);
+  const size_t nl = ix->leaves.size();
   uint64_t pos = 0;
-  for (size_t i = 0; i < ix->leaves.size(); ++i) {
+  std::vector<uint64_t> at(nodes.size(), 0);  // next leaf-ordered row of each leaf
+  for (size_t i = 0; i < nl; ++i) {
     Node& lf = nodes[ix->leaves[i]];
     lf.leaf_index = (int)i;
     lf.file_pos = pos;
+    at[ix->leaves[i]] = pos;
     pos += lf.node_size;
-    perm.insert(perm.end(), lf.members.begin(), lf.members.end());
   }
   if (pos != ix->n) return set_error(HG_ERR_ARG, "internal: leaf sizes do not add up");
-  uint32_t* d_perm = nullptr;
-  CK(dalloc(&d_perm, ix->n));
-  std::unique_ptr<uint32_t, void (*)(uint32_t*)> guard(d_perm, [](uint32_t* p) { cudaFree(p); });
+  // leaf order: the rows of each leaf in ascending order
+  std::vector<uint32_t> perm(ix->n);
+  {
+    std::vector<int> node_of(ix->n);
+    CK(cudaMemcpyAsync(node_of.data(), ctx.d_node_of, sizeof(int) * ix->n, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (uint64_t r = 0; r < ix->n; ++r) perm[at[node_of[r]]++] = (uint32_t)r;
+  }
+  uint32_t* d_perm = ctx.d_list;
   CK(cudaMemcpyAsync(d_perm, perm.data(), sizeof(uint32_t) * ix->n, cudaMemcpyHostToDevice, st));
-  // leaf envelopes: vertical sketches over each leaf's members
-  int* d_keys = nullptr;
-  size_t total_segs = 0;
-  std::vector<size_t> koff(ix->leaves.size() + 1, 0);
-  for (size_t i = 0; i < ix->leaves.size(); ++i) {
-    total_segs += nodes[ix->leaves[i]].points.size();
-    koff[i + 1] = total_segs;
-  }
-  std::vector<int> keys(4 * total_segs);
-  std::vector<short> from, to;
-  for (size_t i = 0; i < ix->leaves.size(); ++i) {
-    const Node& lf = nodes[ix->leaves[i]];
-    for (size_t s = 0; s < lf.points.size(); ++s) {
-      from.push_back((short)seg_start(lf.points, (int)s));
-      to.push_back(lf.points[s]);
-      keys[4 * (koff[i] + s) + 0] = INT_MIN;
-      keys[4 * (koff[i] + s) + 1] = INT_MAX;
-      keys[4 * (koff[i] + s) + 2] = INT_MIN;
-      keys[4 * (koff[i] + s) + 3] = INT_MAX;
-    }
-  }
-  short* d_seg = nullptr;
-  CK(dalloc(&d_keys, keys.size()));
-  CK(dalloc(&d_seg, 2 * total_segs));
-  std::unique_ptr<int, void (*)(int*)> g2(d_keys, [](int* p) { cudaFree(p); });
-  std::unique_ptr<short, void (*)(short*)> g3(d_seg, [](short* p) { cudaFree(p); });
-  CK(cudaMemcpyAsync(d_keys, keys.data(), sizeof(int) * keys.size(), cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(d_seg, from.data(), sizeof(short) * total_segs, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(d_seg + total_segs, to.data(), sizeof(short) * total_segs, cudaMemcpyHostToDevice, st));
-  for (size_t i = 0; i < ix->leaves.size(); ++i) {
-    const Node& lf = nodes[ix->leaves[i]];
-    if (lf.node_size == 0) continue;
-    CK(hg::launch_sketch_members(X, ix->L, d_perm + lf.file_pos, lf.node_size, d_seg + koff[i],
-                                 d_seg + total_segs + koff[i], (int)lf.points.size(), d_keys + 4 * koff[i], st));
-  }
-  CK(cudaMemcpyAsync(keys.data(), d_keys, sizeof(int) * keys.size(), cudaMemcpyDeviceToHost, st));
   // leaf-ordered rows, ids, iSAX words
   hg::DeviceIndex& d = ix->d;
   CK(dalloc(&d.rows, (size_t)ix->n * ix->L));
   CK(hg::launch_gather_rows(X, ix->L, d_perm, ix->n, d.rows, st));
-  ix->ids.assign(perm.begin(), perm.end());
-  ix->has_ids = true;
   CK(dalloc(&d.ids, ix->n));
-  CK(cudaMemcpyAsync(d.ids, ix->ids.data(), sizeof(int64_t) * ix->n, cudaMemcpyHostToDevice, st));
+  CK(hg::launch_widen_ids(d_perm, ix->n, d.ids, st));
   CK(dalloc(&d.bp, 256));
   CK(cudaMemcpyAsync(d.bp, kHgBreakpoints, sizeof(float) * 255, cudaMemcpyHostToDevice, st));
   // padded to whole 32-row units: the LB_SAX filter bulk-copies whole units
   CK(dalloc(&d.sax, (size_t)((ix->n + 31) & ~31ull) * 16));
   CK(hg::launch_sax_rows(d.rows, ix->L, ix->n, d.bp, d.sax, st));
+  // leaf envelopes: vertical sketches over each leaf's rows, all leaves in one launch
+  std::vector<uint64_t> start(nl);
+  std::vector<uint32_t> size(nl);
+  std::vector<int> koff(nl + 1, 0);
+  hg::SketchArgs a{};
+  for (size_t i = 0; i < nl; ++i) {
+    const Node& lf = nodes[ix->leaves[i]];
+    start[i] = lf.file_pos;
+    size[i] = lf.node_size;
+    koff[i + 1] = koff[i] + (int)lf.points.size();
+    a.max_segs = std::max(a.max_segs, (int)lf.points.size());
+    a.max_size = std::max(a.max_size, lf.node_size);
+  }
+  const size_t total_segs = (size_t)koff[nl];
+  std::vector<short> seg(2 * total_segs);
+  std::vector<int> keys(4 * total_segs);
+  for (size_t i = 0; i < nl; ++i) {
+    const Node& lf = nodes[ix->leaves[i]];
+    for (size_t s = 0; s < lf.points.size(); ++s) {
+      seg[koff[i] + s] = (short)seg_start(lf.points, (int)s);
+      seg[total_segs + koff[i] + s] = lf.points[s];
+    }
+  }
+  for (size_t i = 0; i < keys.size(); ++i) keys[i] = (i & 1) ? INT_MAX : INT_MIN;
+  int *d_keys = nullptr, *d_off = nullptr;
+  short* d_seg = nullptr;
+  uint64_t* d_start = nullptr;
+  uint32_t* d_size = nullptr;
+  auto release = [](void* p) { cudaFree(p); };
+  using Guard = std::unique_ptr<void, void (*)(void*)>;
+  CK(dalloc(&d_keys, keys.size()));
+  Guard g1(d_keys, release);
+  CK(dalloc(&d_off, nl + 1));
+  Guard g2(d_off, release);
+  CK(dalloc(&d_seg, seg.size()));
+  Guard g3(d_seg, release);
+  CK(dalloc(&d_start, nl));
+  Guard g4(d_start, release);
+  CK(dalloc(&d_size, nl));
+  Guard g5(d_size, release);
+  CK(cudaMemcpyAsync(d_keys, keys.data(), sizeof(int) * keys.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_off, koff.data(), sizeof(int) * (nl + 1), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_seg, seg.data(), sizeof(short) * seg.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_start, start.data(), sizeof(uint64_t) * nl, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_size, size.data(), sizeof(uint32_t) * nl, cudaMemcpyHostToDevice, st));
+  a.X = d.rows;
+  a.L = (int)ix->L;
+  a.ngroups = (int)nl;
+  a.start = d_start;
+  a.size = d_size;
+  a.seg_off = d_off;
+  a.seg_from = d_seg;
+  a.seg_to = d_seg + total_segs;
+  a.keys = d_keys;
+  CK(hg::launch_sketch(a, st));
+  CK(cudaMemcpyAsync(keys.data(), d_keys, sizeof(int) * keys.size(), cudaMemcpyDeviceToHost, st));
+  ix->ids.assign(perm.begin(), perm.end());
+  ix->has_ids = true;
   CK(cudaStreamSynchronize(st));
-  for (size_t i = 0; i < ix->leaves.size(); ++i) {
+  for (size_t i = 0; i < nl; ++i) {
     Node& lf = nodes[ix->leaves[i]];
     if (lf.node_size == 0) continue;  // an empty leaf keeps the initial envelope
-    keys_to_sketch(&keys[4 * koff[i]], lf.points.size(), lf.sk.data());
+    keys_to_sketch(&keys[4 * (size_t)koff[i]], lf.points.size(), lf.sk.data());
   }
-  for (size_t i = 0; i < ix->leaves.size(); ++i) std::vector<uint32_t>().swap(nodes[ix->leaves[i]].members);
   // internal envelopes as the sequential writer leaves them
   for (size_t i = 0; i < ix->leaves.size(); ++i) merge_ancestors(nodes, ix->leaves[i]);
   return upload_tables(ix);
@@ -737,20 +838,17 @@ static hg_status build_impl(const float* data, int on_device, uint64_t n, uint32
   Node root = make_leaf(std::vector<short>{(short)L});
   root.filename = filename_of(root, nullptr);
   ix->nodes.push_back(std::move(root));
+  hg_status s;
   {
     BuildCtx ctx;
     ctx.ix = ix.get();
     ctx.X = X;
     ctx.st = ix->stream;
-    hg_status s = ctx.run();
-    if (s != HG_OK) {
-      free_device(ix.get());
-      cudaStreamDestroy(ix->stream);
-      return s;
-    }
+    s = ctx.run();
+    if (s == HG_OK) s = finalize_build(ix.get(), X, ix->stream, ctx);
   }
-  hg_status s = finalize_build(ix.get(), X, ix->stream);
   if (s != HG_OK) {
+    cudaStreamSynchronize(ix->stream);
     free_device(ix.get());
     cudaStreamDestroy(ix->stream);
     return s;

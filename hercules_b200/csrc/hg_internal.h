@@ -27,7 +27,6 @@ struct Node {
   int split_idx = 0;
   float split_value = 0.0f;
   uint32_t node_size = 0;
-  std::vector<uint32_t> members;  // dataset rows of a leaf, insertion order
   std::string filename;
   uint64_t file_pos = 0;
   int leaf_index = -1;

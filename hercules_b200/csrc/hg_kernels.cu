@@ -15,6 +15,32 @@
 
 namespace hg {
 
+// Adds the lanes' chunk sums 0 .. lim - 1 in chunk order, eight a turn, so the
+// shuffles run ahead of the two chains of adds; a chunk past the end adds 0,
+// which leaves the sums unchanged.
+__device__ __forceinline__ void warp_add_chunks(float cs, float cq, int lim, float& sum, float& sumsq) {
+  for (int j = 0; j < lim; j += 8) {
+    float s8[8], q8[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      s8[t] = __shfl_sync(HG_FULL, cs, j + t);
+      q8[t] = __shfl_sync(HG_FULL, cq, j + t);
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      sum = __fadd_rn(sum, s8[t]);
+      sumsq = __fadd_rn(sumsq, q8[t]);
+    }
+  }
+}
+
+__device__ __forceinline__ void segment_stats(float sum, float sumsq, int count, float* mean, float* stdev) {
+  const float fc = (float)count;
+  *mean = __fdiv_rn(sum, fc);
+  sumsq = __fsub_rn(sumsq, __fdiv_rn(__fmul_rn(sum, sum), fc));
+  *stdev = __fsqrt_rn(__fdiv_rn(sumsq, fc));
+}
+
 // Mean and stdev of v[from, to) in the order of calc_mean_stdev_SIMD: the
 // lanes compute the 8-chunk sums in parallel, then every lane accumulates
 // them in chunk order (identical warp-uniform result).
@@ -42,27 +68,9 @@ __device__ void warp_mean_stdev(const float* v, int from, int to, float* mean, f
       cs = hg_hsum8(x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]);
       cq = hg_hsum8(x2[0], x2[1], x2[2], x2[3], x2[4], x2[5], x2[6], x2[7]);
     }
-    // eight chunks a turn, so the shuffles run ahead of the two chains of
-    // adds; a chunk past the end adds 0, which leaves the sums unchanged
-    const int lim = min(32, nch - base);
-    for (int j = 0; j < lim; j += 8) {
-      float s8[8], q8[8];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        s8[t] = __shfl_sync(HG_FULL, cs, j + t);
-        q8[t] = __shfl_sync(HG_FULL, cq, j + t);
-      }
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        sum = __fadd_rn(sum, s8[t]);
-        sumsq = __fadd_rn(sumsq, q8[t]);
-      }
-    }
+    warp_add_chunks(cs, cq, min(32, nch - base), sum, sumsq);
   }
-  const float fc = (float)count;
-  *mean = __fdiv_rn(sum, fc);
-  sumsq = __fsub_rn(sumsq, __fdiv_rn(__fmul_rn(sum, sum), fc));
-  *stdev = __fsqrt_rn(__fdiv_rn(sumsq, fc));
+  segment_stats(sum, sumsq, count, mean, stdev);
 }
 
 // Walks the tree from the root (node_split_policy_route_to_left,
@@ -120,22 +128,109 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* tmp /* THREADS/32
 // build kernels
 // ---------------------------------------------------------------------------
 
-// One series per thread: walk the current tree to a leaf.
-__global__ void k_route_rows(const float* __restrict__ X, int L, const uint32_t* __restrict__ rows, uint64_t first,
-                             uint32_t count, Tree t, int* __restrict__ leaf_out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const uint64_t r = rows ? rows[i] : first + i;
-  const float* x = X + r * (uint64_t)L;
+// Mean and stdev as warp_mean_stdev, of a row in global memory: a chunk's
+// eight floats in two 16-byte loads where the segment starts on 16 bytes.
+__device__ void warp_mean_stdev_row(const float* x, int from, int to, float* mean, float* stdev) {
+  const int lane = threadIdx.x & 31;
+  const int count = to - from;
+  *mean = 0.0f;
+  *stdev = 0.0f;
+  if (count <= 0) return;
+  const float* v = x + from;
+  const bool wide = (reinterpret_cast<uintptr_t>(v) & 15) == 0;
+  const int nch = (count + 7) >> 3;
+  float sum = 0.0f, sumsq = 0.0f;
+  for (int base = 0; base < nch; base += 32) {
+    const int c = base + lane;
+    float cs = 0.0f, cq = 0.0f;
+    if (c < nch) {
+      float e[8], e2[8];
+      if (wide && c * 8 + 8 <= count) {
+        const float4 a = reinterpret_cast<const float4*>(v)[2 * c], b = reinterpret_cast<const float4*>(v)[2 * c + 1];
+        e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w;
+        e[4] = b.x; e[5] = b.y; e[6] = b.z; e[7] = b.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = c * 8 + j < count ? v[c * 8 + j] : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) e2[j] = __fmul_rn(e[j], e[j]);
+      cs = hg_hsum8(e[0], e[1], e[2], e[3], e[4], e[5], e[6], e[7]);
+      cq = hg_hsum8(e2[0], e2[1], e2[2], e2[3], e2[4], e2[5], e2[6], e2[7]);
+    }
+    warp_add_chunks(cs, cq, min(32, nch - base), sum, sumsq);
+  }
+  segment_stats(sum, sumsq, count, mean, stdev);
+}
+
+// Series up to this length are staged 32 at a time in shared memory (a pitch
+// of L + 1 floats: a lane per row reads without bank conflicts), longer ones
+// are read by a warp each.  Staged, a lane adds its own row's chunks and a
+// segment of 32 rows costs the instructions of one; a thread per row reading
+// global memory, as both cases did, touched 32 lines per load (122 us to route
+// 65,536 rows of 256, 56 us for the envelopes of 10,000; staged 20 and 9 us).
+constexpr int kStagedL = 512;
+constexpr int kStagedRows = 32;
+__host__ __device__ inline size_t staged_bytes(int L) { return sizeof(float) * kStagedRows * (size_t)(L + 1); }
+
+// `threads` threads bring rows row(0) .. row(n - 1) of X into the tile.
+template <class Row>
+__device__ __forceinline__ void stage_rows(const float* __restrict__ X, int L, int n, float* tile, int threads, Row row) {
+  const int v4 = L >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = threads >> 5;
+  for (int c = lane; c < v4; c += 32)
+    for (int r0 = warp; r0 < n; r0 += 4 * nw) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r0 + u * nw < n) v[u] = reinterpret_cast<const float4*>(X + row(r0 + u * nw) * (uint64_t)L)[c];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r0 + u * nw < n) {
+          float* d = tile + (r0 + u * nw) * (L + 1) + 4 * c;
+          d[0] = v[u].x;
+          d[1] = v[u].y;
+          d[2] = v[u].z;
+          d[3] = v[u].w;
+        }
+    }
+}
+
+// Walks the current tree to a leaf, a lane per staged row.
+__global__ void __launch_bounds__(32) k_route_staged(const float* __restrict__ X, int L, uint64_t first, uint32_t count,
+                                                     Tree t, int* __restrict__ node_of) {
+  extern __shared__ float tile[];
+  const uint32_t r0 = blockIdx.x * kStagedRows;
+  const int n = (int)min((uint32_t)kStagedRows, count - r0);
+  stage_rows(X, L, n, tile, 32, [&](int r) { return first + r0 + r; });
+  __syncwarp();
+  if ((int)threadIdx.x >= n) return;
+  const float* x = tile + threadIdx.x * (L + 1);
   int node = t.root;
   while (node >= 0) {
-    const DNode n = t.nodes[node];
+    const DNode nd = t.nodes[node];
     float m, s;
-    hg_mean_stdev(x, n.from, n.to, &m, &s);
-    const float v = n.idx ? s : m;
-    node = (v < n.value) ? n.left : n.right;
+    hg_mean_stdev(x, nd.from, nd.to, &m, &s);
+    const float v = nd.idx ? s : m;
+    node = (v < nd.value) ? nd.left : nd.right;
   }
-  leaf_out[i] = ~node;
+  node_of[r0 + threadIdx.x] = ~node;
+}
+
+// The same with a warp per row.
+__global__ void k_route_long(const float* __restrict__ X, int L, uint64_t first, uint32_t count, Tree t,
+                             int* __restrict__ node_of) {
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= count) return;
+  const float* x = X + (first + r) * (uint64_t)L;
+  int node = t.root;
+  while (node >= 0) {
+    const DNode nd = t.nodes[node];
+    float m, s;
+    warp_mean_stdev_row(x, nd.from, nd.to, &m, &s);
+    const float v = nd.idx ? s : m;
+    node = (v < nd.value) ? nd.left : nd.right;
+  }
+  if ((threadIdx.x & 31) == 0) node_of[r] = ~node;
 }
 
 // Order-preserving int image of a float for atomicMax/atomicMin.
@@ -144,54 +239,156 @@ __device__ __forceinline__ int fkey(float f) {
   return b >= 0 ? b : b ^ 0x7fffffff;
 }
 
-// Segment sketches (min/max of per-series segment mean and stdev) over a
-// member list: node_segment_sketch_update_sketch_parallel applied to every
-// member (hercules_node_split.c:86-120).  Min/max are order independent and
-// fmaxf/fminf ignore NaN, so skipping NaN gives the same envelope.
-// keys_out: nsegs x 4 ints {max mean, min mean, max stdev, min stdev}.
-__global__ void k_sketch_members(const float* __restrict__ X, int L, const uint32_t* __restrict__ members,
-                                 uint32_t count, const short* __restrict__ seg_from,
-                                 const short* __restrict__ seg_to, int nsegs, int* __restrict__ keys_out) {
-  extern __shared__ int sk[];  // nsegs x 4
-  for (int i = threadIdx.x; i < nsegs; i += blockDim.x) {
-    sk[4 * i + 0] = INT_MIN;
-    sk[4 * i + 1] = INT_MAX;
-    sk[4 * i + 2] = INT_MIN;
-    sk[4 * i + 3] = INT_MAX;
+__device__ __forceinline__ int empty_key(int i) { return (i & 1) ? INT_MAX : INT_MIN; }  // odd: minima
+
+// The rows of the leaves about to split, among the rows routed so far.
+__global__ void k_collect_members(const int* __restrict__ node_of, uint64_t end, const int* __restrict__ slot_of,
+                                  const uint64_t* __restrict__ start, const uint32_t* __restrict__ last,
+                                  uint64_t members, uint32_t* __restrict__ list, uint32_t* counts, uint32_t* later,
+                                  int* keys, int nsegs) {
+  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = t0; i < 4ull * nsegs; i += step) keys[i] = empty_key((int)(i & 1));
+  const int lane = threadIdx.x & 31;
+  const uint64_t whole = (end + 31) & ~31ull;  // whole warps to the end
+  for (uint64_t r = t0; r < whole; r += step) {
+    const int p = r < end ? slot_of[node_of[r]] : -1;
+    // -1: no row of a splitting leaf; -2: a later row; else the leaf
+    const int who = p < 0 ? -1 : (r <= last[p] ? p : -2);
+    if (!__any_sync(HG_FULL, who != -1)) continue;
+    const uint32_t same = __match_any_sync(HG_FULL, who);
+    const int leader = __ffs(same) - 1;
+    uint32_t pos = 0;
+    if (who != -1 && lane == leader) pos = atomicAdd(who == -2 ? later : &counts[who], (uint32_t)__popc(same));
+    pos = __shfl_sync(HG_FULL, pos, leader) + (uint32_t)__popc(same & ((1u << lane) - 1));
+    if (who != -1) list[(who == -2 ? members : start[who]) + pos] = (uint32_t)r;
   }
-  __syncthreads();
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < count; m += gridDim.x * blockDim.x) {
-    const float* x = X + (uint64_t)members[m] * L;
-    for (int s = 0; s < nsegs; ++s) {
-      float mean, sd;
-      hg_mean_stdev(x, seg_from[s], seg_to[s], &mean, &sd);
-      if (mean == mean) {
-        atomicMax(&sk[4 * s + 0], fkey(mean));
-        atomicMin(&sk[4 * s + 1], fkey(mean));
-      }
-      if (sd == sd) {
-        atomicMax(&sk[4 * s + 2], fkey(sd));
-        atomicMin(&sk[4 * s + 3], fkey(sd));
+}
+
+// Segment sketches (min/max of per-series segment mean and stdev) over groups
+// of rows: node_segment_sketch_update_sketch_parallel applied to every member
+// (hercules_node_split.c:86-120).  Min/max are order independent and
+// fmaxf/fminf ignore NaN, so skipping NaN gives the same envelope.
+struct SketchGroup {
+  uint64_t first;
+  uint32_t size;
+  int seg0, nsegs;
+};
+__device__ __forceinline__ SketchGroup sketch_group(const SketchArgs& a, int g) {
+  return SketchGroup{a.start[g], a.size[g], a.seg_off[g], a.seg_off[g + 1] - a.seg_off[g]};
+}
+__device__ __forceinline__ uint64_t sketch_row(const SketchArgs& a, const SketchGroup& g, uint64_t i) {
+  return a.members ? (uint64_t)a.members[g.first + i] : g.first + i;
+}
+
+constexpr int kSketchThreads = 256;
+// L <= kStagedL: grid (groups, parts); a tile of 32 rows at a time, a lane per
+// row, a warp per segment, whose extremes stay with that warp.
+__global__ void __launch_bounds__(kSketchThreads) k_sketch_staged(SketchArgs a) {
+  extern __shared__ float tile[];
+  int* sk = reinterpret_cast<int*>(tile + kStagedRows * (a.L + 1));  // [segments][4]
+  const SketchGroup g = sketch_group(a, blockIdx.x);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if ((uint64_t)blockIdx.y * kStagedRows >= g.size) return;
+  for (int i = threadIdx.x; i < 4 * g.nsegs; i += kSketchThreads) sk[i] = empty_key(i);
+  for (uint64_t t0 = (uint64_t)blockIdx.y * kStagedRows; t0 < g.size; t0 += (uint64_t)gridDim.y * kStagedRows) {
+    const int n = (int)min((uint64_t)kStagedRows, g.size - t0);
+    __syncthreads();
+    stage_rows(a.X, a.L, n, tile, kSketchThreads, [&](int r) { return sketch_row(a, g, t0 + r); });
+    __syncthreads();
+    const float* x = tile + min(lane, n - 1) * (a.L + 1);  // lanes past the rows repeat the last
+    for (int s = warp; s < g.nsegs; s += kSketchThreads / 32) {
+      float m, sd;
+      hg_mean_stdev(x, a.seg_from[g.seg0 + s], a.seg_to[g.seg0 + s], &m, &sd);
+      const int km = fkey(m), ks = fkey(sd);
+      const int k0 = __reduce_max_sync(HG_FULL, m == m ? km : INT_MIN);
+      const int k1 = __reduce_min_sync(HG_FULL, m == m ? km : INT_MAX);
+      const int k2 = __reduce_max_sync(HG_FULL, sd == sd ? ks : INT_MIN);
+      const int k3 = __reduce_min_sync(HG_FULL, sd == sd ? ks : INT_MAX);
+      if (lane == 0) {
+        sk[4 * s + 0] = max(sk[4 * s + 0], k0);
+        sk[4 * s + 1] = min(sk[4 * s + 1], k1);
+        sk[4 * s + 2] = max(sk[4 * s + 2], k2);
+        sk[4 * s + 3] = min(sk[4 * s + 3], k3);
       }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nsegs; i += blockDim.x) {
-    atomicMax(&keys_out[4 * i + 0], sk[4 * i + 0]);
-    atomicMin(&keys_out[4 * i + 1], sk[4 * i + 1]);
-    atomicMax(&keys_out[4 * i + 2], sk[4 * i + 2]);
-    atomicMin(&keys_out[4 * i + 3], sk[4 * i + 3]);
+  for (int i = threadIdx.x; i < 4 * g.nsegs; i += kSketchThreads) {
+    if (i & 1) atomicMin(&a.keys[4 * (size_t)g.seg0 + i], sk[i]);
+    else atomicMax(&a.keys[4 * (size_t)g.seg0 + i], sk[i]);
   }
 }
 
-__global__ void k_route_flags(const float* __restrict__ X, int L, const uint32_t* __restrict__ members,
-                              uint32_t count, short from, short to, int idx, float value,
-                              uint8_t* __restrict__ flags) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  float m, s;
-  hg_mean_stdev(X + (uint64_t)members[i] * L, from, to, &m, &s);
-  flags[i] = ((idx ? s : m) < value) ? 1 : 0;
+// Longer series: a warp per (row, segment).
+__global__ void __launch_bounds__(kSketchThreads) k_sketch_long(SketchArgs a) {
+  extern __shared__ int sk_long[];
+  const SketchGroup g = sketch_group(a, blockIdx.x);
+  const int lane = threadIdx.x & 31;
+  constexpr int W = kSketchThreads / 32;
+  const uint64_t items = (uint64_t)g.size * g.nsegs;
+  if ((uint64_t)blockIdx.y * W >= items) return;
+  for (int i = threadIdx.x; i < 4 * g.nsegs; i += kSketchThreads) sk_long[i] = empty_key(i);
+  __syncthreads();
+  for (uint64_t it = (uint64_t)blockIdx.y * W + (threadIdx.x >> 5); it < items; it += (uint64_t)gridDim.y * W) {
+    const uint64_t i = it / g.nsegs;
+    const int s = (int)(it - i * g.nsegs);
+    float m, sd;
+    warp_mean_stdev_row(a.X + sketch_row(a, g, i) * (uint64_t)a.L, a.seg_from[g.seg0 + s], a.seg_to[g.seg0 + s], &m, &sd);
+    if (lane == 0) {
+      if (m == m) {
+        atomicMax(&sk_long[4 * s + 0], fkey(m));
+        atomicMin(&sk_long[4 * s + 1], fkey(m));
+      }
+      if (sd == sd) {
+        atomicMax(&sk_long[4 * s + 2], fkey(sd));
+        atomicMin(&sk_long[4 * s + 3], fkey(sd));
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4 * g.nsegs; i += kSketchThreads) {
+    if (i & 1) atomicMin(&a.keys[4 * (size_t)g.seg0 + i], sk_long[i]);
+    else atomicMax(&a.keys[4 * (size_t)g.seg0 + i], sk_long[i]);
+  }
+}
+
+// The redistribution of splits (hercules_node_split.c:1294-1333), a warp per
+// row; a warp's rows are consecutive in the list, so it counts the left ones
+// of a leaf itself and adds them once.
+__global__ void k_split_members(const float* __restrict__ X, int L, int* __restrict__ node_of,
+                                const uint32_t* __restrict__ list, uint64_t members, const uint32_t* later,
+                                const int* __restrict__ slot_of, const SplitPolicy* __restrict__ splits,
+                                uint32_t* n_left) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t total = members + *later, per = (total + nw - 1) / nw;
+  int cur = -1;
+  uint32_t left = 0;
+  for (uint64_t i = w * per; i < min(total, w * per + per); ++i) {
+    const uint64_t r = list[i];
+    const int p = slot_of[node_of[r]];
+    const SplitPolicy sp = splits[p];
+    float m, s;
+    warp_mean_stdev_row(X + r * (uint64_t)L, sp.from, sp.to, &m, &s);
+    const bool l = (sp.idx ? s : m) < sp.value;
+    __syncwarp();  // every lane has read node_of[r]
+    if (lane == 0) node_of[r] = l ? sp.left : sp.right;
+    if (i < members) {
+      if (p != cur) {
+        if (lane == 0 && left) atomicAdd(&n_left[cur], left);
+        cur = p;
+        left = 0;
+      }
+      left += l ? 1u : 0u;
+    }
+  }
+  if (lane == 0 && left) atomicAdd(&n_left[cur], left);
+}
+
+__global__ void k_widen_ids(const uint32_t* __restrict__ perm, uint64_t n, int64_t* __restrict__ ids) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) ids[i] = (int64_t)perm[i];
 }
 
 // rows[r] = X[perm[r]], one thread per 16 bytes (a row is L/4 of them).
@@ -205,28 +402,30 @@ __global__ void k_gather_rows(const float* __restrict__ X, int L, const uint32_t
   reinterpret_cast<float4*>(rows + r * L)[j] = reinterpret_cast<const float4*>(X + (uint64_t)perm[r] * L)[j];
 }
 
-// iSAX word of every leaf-ordered row (sax_from_ts, sax.c:86-135).
+// iSAX word of every leaf-ordered row (sax_from_ts, sax.c:86-135): two rows
+// per warp, a lane per (row, segment), which adds its segment in order and
+// looks its symbol up.  A thread per row took 0.96 ms for 1M x 256 (1.1 TB/s),
+// its 32 rows' lines leaving L1 between two of its reads.
 __global__ void k_sax_rows(const float* __restrict__ rows, int L, uint64_t n, const float* __restrict__ bp,
                            uint8_t* __restrict__ sax) {
   __shared__ float sbp[256];
   for (int i = threadIdx.x; i < 255; i += blockDim.x) sbp[i] = bp[i];
   __syncthreads();
-  const uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t row = t / HG_PAA_SEGMENTS;
   if (row >= n) return;
   const int per = L / HG_PAA_SEGMENTS;
-  const float* x = rows + row * L;
-  uint8_t w[16];
-  for (int s = 0; s < HG_PAA_SEGMENTS; ++s) {
-    float acc = 0.0f;
-    for (int i = 0; i < per; ++i) acc = __fadd_rn(acc, x[s * per + i]);
-    w[s] = (uint8_t)hg_sax_symbol(__fdiv_rn(acc, (float)per), sbp);
+  const float* x = rows + row * L + (t % HG_PAA_SEGMENTS) * per;
+  float acc = 0.0f;
+  if (per % 4 == 0) {
+    for (int i = 0; i < per / 4; ++i) {
+      const float4 v = reinterpret_cast<const float4*>(x)[i];
+      acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+    }
+  } else {
+    for (int i = 0; i < per; ++i) acc = __fadd_rn(acc, x[i]);
   }
-  uint4 out;
-  out.x = w[0] | (w[1] << 8) | (w[2] << 16) | ((uint32_t)w[3] << 24);
-  out.y = w[4] | (w[5] << 8) | (w[6] << 16) | ((uint32_t)w[7] << 24);
-  out.z = w[8] | (w[9] << 8) | (w[10] << 16) | ((uint32_t)w[11] << 24);
-  out.w = w[12] | (w[13] << 8) | (w[14] << 16) | ((uint32_t)w[15] << 24);
-  reinterpret_cast<uint4*>(sax)[row] = out;
+  sax[t] = (uint8_t)hg_sax_symbol(__fdiv_rn(acc, (float)per), sbp);
 }
 
 // ---------------------------------------------------------------------------
@@ -1267,28 +1466,68 @@ int sm_count(int device) {
   return sms;
 }
 
-cudaError_t launch_route_rows(const float* X, int L, const uint32_t* rows, uint64_t first, uint32_t count,
-                              Tree t, int* leaf_out, cudaStream_t s) {
+cudaError_t launch_route_rows(const float* X, int L, uint64_t first, uint32_t count, Tree t, int* node_of,
+                              cudaStream_t s) {
   if (!count) return cudaSuccess;
-  k_route_rows<<<blocks_for(count, 128), 128, 0, s>>>(X, L, rows, first, count, t, leaf_out);
+  if (L <= kStagedL) {
+    static SmemLimit attr;
+    const cudaError_t ea = attr.ensure((const void*)k_route_staged, (int)staged_bytes(kStagedL));
+    if (ea != cudaSuccess) return ea;
+    k_route_staged<<<blocks_for(count, kStagedRows), 32, staged_bytes(L), s>>>(X, L, first, count, t, node_of);
+  } else {
+    k_route_long<<<blocks_for((uint64_t)count * 32, 256), 256, 0, s>>>(X, L, first, count, t, node_of);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_sketch_members(const float* X, int L, const uint32_t* members, uint32_t count,
-                                  const short* seg_from, const short* seg_to, int nsegs, int* keys_out,
-                                  cudaStream_t s) {
-  if (!count || !nsegs) return cudaSuccess;
-  unsigned b = blocks_for(count, 256);
-  if (b > 148 * 8) b = 148 * 8;
-  k_sketch_members<<<b, 256, sizeof(int) * 4 * nsegs, s>>>(X, L, members, count, seg_from, seg_to, nsegs,
-                                                           keys_out);
+cudaError_t launch_collect_members(const int* node_of, uint64_t end, const int* slot_of, const uint64_t* start,
+                                   const uint32_t* last, uint64_t members, uint32_t* list, uint32_t* counts,
+                                   uint32_t* later, int* keys, int nsegs, cudaStream_t s) {
+  const unsigned want = blocks_for(end ? end : 1, 4 * 256);
+  k_collect_members<<<want < 148 * 8 ? want : 148 * 8, 256, 0, s>>>(node_of, end, slot_of, start, last, members, list,
+                                                                    counts, later, keys, nsegs);
   return cudaGetLastError();
 }
 
-cudaError_t launch_route_flags(const float* X, int L, const uint32_t* members, uint32_t count, short from,
-                               short to, int idx, float value, uint8_t* flags, cudaStream_t s) {
-  if (!count) return cudaSuccess;
-  k_route_flags<<<blocks_for(count, 256), 256, 0, s>>>(X, L, members, count, from, to, idx, value, flags);
+cudaError_t launch_sketch(const SketchArgs& a, cudaStream_t s) {
+  const int groups = a.ngroups, segs = a.max_segs;
+  const uint32_t size = a.max_size;
+  if (!groups || !segs || !size) return cudaSuccess;
+  const bool staged = a.L <= kStagedL;
+  // parts per group: the rows of one tile (8 (row, segment) pairs) at least,
+  // and enough blocks in all for every SM
+  const uint64_t most = staged ? blocks_for(size, kStagedRows) : blocks_for((uint64_t)size * segs, kSketchThreads / 32);
+  const uint64_t fill = (148 * 8 + groups - 1) / groups;
+  const unsigned parts = (unsigned)(most < fill ? most : fill);
+  if (staged) {
+    const size_t smem = staged_bytes(a.L) + sizeof(int) * 4 * segs;
+    static SmemLimit attr;
+    const cudaError_t ea = attr.ensure((const void*)k_sketch_staged, 200 * 1024);
+    if (ea != cudaSuccess) return ea;
+    k_sketch_staged<<<dim3(groups, parts), kSketchThreads, smem, s>>>(a);
+  } else {
+    static SmemLimit attr;
+    const cudaError_t ea = attr.ensure((const void*)k_sketch_long, 200 * 1024);
+    if (ea != cudaSuccess) return ea;
+    k_sketch_long<<<dim3(groups, parts), kSketchThreads, sizeof(int) * 4 * segs, s>>>(a);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_split_members(const float* X, int L, int* node_of, const uint32_t* list, uint64_t members,
+                                 const uint32_t* later, uint64_t later_max, const int* slot_of, const SplitPolicy* splits,
+                                 uint32_t* n_left, cudaStream_t s) {
+  const uint64_t rows = members + later_max;
+  if (!rows) return cudaSuccess;
+  const unsigned want = blocks_for(rows * 32, 256);
+  k_split_members<<<want < 148 * 32 ? want : 148 * 32, 256, 0, s>>>(X, L, node_of, list, members, later, slot_of, splits,
+                                                                  n_left);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_widen_ids(const uint32_t* perm, uint64_t n, int64_t* ids, cudaStream_t s) {
+  if (!n) return cudaSuccess;
+  k_widen_ids<<<blocks_for(n, 256), 256, 0, s>>>(perm, n, ids);
   return cudaGetLastError();
 }
 
@@ -1303,7 +1542,7 @@ cudaError_t launch_gather_rows(const float* X, int L, const uint32_t* perm, uint
 cudaError_t launch_sax_rows(const float* rows, int L, uint64_t n, const float* bp, uint8_t* sax,
                             cudaStream_t s) {
   if (!n) return cudaSuccess;
-  k_sax_rows<<<blocks_for(n, 128), 128, 0, s>>>(rows, L, n, bp, sax);
+  k_sax_rows<<<blocks_for(n * HG_PAA_SEGMENTS, 256), 256, 0, s>>>(rows, L, n, bp, sax);
   return cudaGetLastError();
 }
 

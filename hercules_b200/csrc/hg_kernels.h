@@ -158,13 +158,47 @@ int sm_count(int device);
 
 
 // build
-cudaError_t launch_route_rows(const float* X, int L, const uint32_t* rows, uint64_t first, uint32_t count,
-                              Tree t, int* leaf_out, cudaStream_t s);
-cudaError_t launch_sketch_members(const float* X, int L, const uint32_t* members, uint32_t count,
-                                  const short* seg_from, const short* seg_to, int nsegs, int* keys_out,
-                                  cudaStream_t s);
-cudaError_t launch_route_flags(const float* X, int L, const uint32_t* members, uint32_t count, short from,
-                               short to, int idx, float value, uint8_t* flags, cudaStream_t s);
+// node_of[r] = the leaf row first + r reaches in the tree, r < count
+cudaError_t launch_route_rows(const float* X, int L, uint64_t first, uint32_t count, Tree t, int* node_of,
+                              cudaStream_t s);
+// The rows r < end of the leaves about to split: slot_of[node_of[r]] = p >= 0
+// puts row r <= last[p] (a member of leaf p) into list[start[p] ..) and a
+// later row (routed to it, not inserted yet) into list[members ..), in any
+// order; counts[p] and *later (0 before the launch) count them.  Also resets
+// the envelope keys of nsegs segments.
+cudaError_t launch_collect_members(const int* node_of, uint64_t end, const int* slot_of, const uint64_t* start,
+                                   const uint32_t* last, uint64_t members, uint32_t* list, uint32_t* counts,
+                                   uint32_t* later, int* keys, int nsegs, cudaStream_t s);
+// Segment envelopes of groups of rows: group g is rows start[g] .. + size[g],
+// of members if set, and segments seg_off[g] .. seg_off[g + 1].
+struct SketchArgs {
+  const float* X;
+  int L;
+  const uint32_t* members;
+  int ngroups;
+  const uint64_t* start;
+  const uint32_t* size;
+  const int* seg_off;
+  int max_segs;          // most segments of a group
+  uint32_t max_size;     // most rows of a group
+  const short* seg_from;
+  const short* seg_to;
+  int* keys;             // [segment][4] {max mean, min mean, max stdev, min stdev}, order-preserving ints
+};
+cudaError_t launch_sketch(const SketchArgs& a, cudaStream_t s);
+// The redistribution of splits: node_of of the rows in list (`members` of
+// them, then *later more) becomes a child of their leaf; n_left[p] (0 before
+// the launch) counts the members of leaf p sent left.
+struct SplitPolicy {
+  float value;
+  int left, right;
+  short from, to;
+  int idx;
+};
+cudaError_t launch_split_members(const float* X, int L, int* node_of, const uint32_t* list, uint64_t members,
+                                 const uint32_t* later, uint64_t later_max, const int* slot_of, const SplitPolicy* splits,
+                                 uint32_t* n_left, cudaStream_t s);
+cudaError_t launch_widen_ids(const uint32_t* perm, uint64_t n, int64_t* ids, cudaStream_t s);
 cudaError_t launch_gather_rows(const float* X, int L, const uint32_t* perm, uint64_t n, float* rows,
                                cudaStream_t s);
 cudaError_t launch_sax_rows(const float* rows, int L, uint64_t n, const float* bp, uint8_t* sax,
