@@ -1029,7 +1029,6 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a
 // chunks (40 float4 pairs each): chunk r of a block sits at pair r + r / 4,
 // so the slots of a warp, which sit at different 4-chunk positions, read
 // different banks.
-constexpr int kEdThreads = 256;
 __device__ __forceinline__ int q4_index(int chunk, int half) {
   const int r = chunk & 31;
   return ((chunk >> 5) * 40 + r + (r >> 2)) * 2 + half;
@@ -1041,15 +1040,22 @@ __host__ __device__ inline size_t q4_bytes(int L) { return (size_t)((L / 8 + 31)
 // flight per step, so a slot reads kSlot * kLines * 32 bytes of its row per
 // step.  Short series use 4-lane slots (8 rows per warp, 128-byte lines);
 // long series, few candidate rows per query, use wider slots.
+// kWarps: warps per block.  Eight, four blocks per SM, where the staged query
+// leaves room for four blocks; else 32 warps that share one staged query, one
+// block per SM (from about 7,900 points: at 16,384 two blocks of eight fitted,
+// and 12 queries of 100k x 16384 took 1.18 instead of 1.12 ms).
+// The allocation-free scan, which has room for 148 lists, uses 32 at any
+// length (eight warps per SM: 325 us for 1M x 256, 32: 183 us).
 template <int kSlot>
 __host__ __device__ constexpr uint32_t slot_leaders() {
   return kSlot == 32 ? 0x1u : (kSlot == 16 ? 0x10001u : (kSlot == 8 ? 0x01010101u : 0x11111111u));
 }
-template <bool kRowIds, int kLines, int kSlot>
-__global__ void __launch_bounds__(kEdThreads, kLines > 2 ? 3 : 4) k_ed_stream(EdArgs a) {
-  constexpr int W = kEdThreads / 32;
-  __shared__ unsigned long long lists[W][kWarpListCap];
-  extern __shared__ float4 qs4[];  // the query, q4_bytes(L) bytes
+template <bool kRowIds, int kLines, int kSlot, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a) {
+  constexpr int W = kWarps, kEdThreads = 32 * kWarps;
+  extern __shared__ float4 ed_smem[];
+  unsigned long long* lists = reinterpret_cast<unsigned long long*>(ed_smem);  // [W][kWarpListCap]
+  float4* qs4 = ed_smem + W * kWarpListCap / 2;                                // the query, q4_bytes(L) bytes
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int slot_lead = lane & ~(kSlot - 1), j = lane & (kSlot - 1);
   const uint32_t qslot = blockIdx.x;  // the query of the group
@@ -1083,7 +1089,7 @@ __global__ void __launch_bounds__(kEdThreads, kLines > 2 ? 3 : 4) k_ed_stream(Ed
     if (threadIdx.x == 0) *a.part_count = 0;
     return;
   }
-  unsigned long long* list = lists[wib];
+  unsigned long long* list = lists + wib * kWarpListCap;
   for (int i = lane; i < kWarpListCap; i += 32) list[i] = ~0ull;
   for (int i = threadIdx.x; i < (a.L >> 2); i += blockDim.x)
     qs4[q4_index(i >> 1, i & 1)] = reinterpret_cast<const float4*>(a.q + (uint64_t)qslot * a.L)[i];
@@ -1242,7 +1248,7 @@ __global__ void __launch_bounds__(kEdThreads, kLines > 2 ? 3 : 4) k_ed_stream(Ed
   }
   int nsort = 32;
   while (nsort < packed) nsort <<= 1;
-  unsigned long long* flat = &lists[0][0];
+  unsigned long long* flat = lists;
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kPer; ++r)
@@ -1653,42 +1659,29 @@ cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cuda
   return cudaGetLastError();
 }
 
-template <bool kRowIds, int kLines, int kSlot>
+static size_t ed_smem_bytes(int L, int warps) { return (size_t)warps * kWarpListCap * 8 + q4_bytes(L); }
+// 32-warp blocks: where fewer than four 8-warp blocks fit on an SM
+static bool ed_wide(int L) { return kEdBlocksPerSm * (ed_smem_bytes(L, kEdWarps) + 1024) > (size_t)227 * 1024; }
+
+template <bool kRowIds, int kSlot, int kWarps>
 static cudaError_t launch_ed(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
+  const auto kernel = k_ed_stream<kRowIds, 2, kSlot, kWarps>;
   static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)k_ed_stream<kRowIds, kLines, kSlot>, (int)q4_bytes(16384));
+  const cudaError_t ea = attr.ensure((const void*)kernel, (int)ed_smem_bytes(16384, kWarps));
   if (ea != cudaSuccess) return ea;
-  k_ed_stream<kRowIds, kLines, kSlot><<<dim3(slots, blocks), kEdThreads, q4_bytes(a.L), s>>>(a);
+  kernel<<<dim3(slots, blocks), 32 * kWarps, ed_smem_bytes(a.L, kWarps), s>>>(a);
   return cudaGetLastError();
 }
 // long series (L >= 4096): few candidate rows per query, each long, so
 // more lanes per row keep more of each row in flight
-#ifndef HG_ED_LONG_LINES
-#define HG_ED_LONG_LINES 2
-#endif
-#ifndef HG_ED_LONG_SLOT
-#define HG_ED_LONG_SLOT 8
-#endif
-#ifndef HG_ED_SHORT_LINES
-#define HG_ED_SHORT_LINES 2
-#endif
 cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  return a.L >= 4096 ? launch_ed<false, HG_ED_LONG_LINES, HG_ED_LONG_SLOT>(a, slots, blocks, s)
-                     : launch_ed<false, HG_ED_SHORT_LINES, 4>(a, slots, blocks, s);
+  if (ed_wide(a.L)) return launch_ed<false, 8, 32>(a, slots, blocks, s);
+  return a.L >= 4096 ? launch_ed<false, 8, kEdWarps>(a, slots, blocks, s) : launch_ed<false, 4, kEdWarps>(a, slots, blocks, s);
 }
 cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  return a.L >= 4096 ? launch_ed<true, HG_ED_LONG_LINES, HG_ED_LONG_SLOT>(a, slots, blocks, s)
-                     : launch_ed<true, HG_ED_SHORT_LINES, 4>(a, slots, blocks, s);
+  return a.L >= 4096 ? launch_ed<true, 8, 32>(a, slots, blocks, s) : launch_ed<true, 4, 32>(a, slots, blocks, s);
 }
-int ed_blocks_per_sm(int L) {
-  // shared memory per block: the staged query + 8 per-warp lists of 2 KB
-  const size_t per_block = q4_bytes(L) + (size_t)kEdWarps * kWarpListCap * 8 + 1024;
-  const int fit = (int)((size_t)227 * 1024 / per_block);
-  // registers: more than two lines per step leave room for 3 blocks
-  const int lines = L >= 4096 ? HG_ED_LONG_LINES : HG_ED_SHORT_LINES;
-  const int cap = lines > 2 ? 3 : kEdBlocksPerSm;
-  return fit < 1 ? 1 : (fit < cap ? fit : cap);
-}
+int ed_blocks_per_sm(int L) { return ed_wide(L) ? 1 : kEdBlocksPerSm; }
 
 cudaError_t launch_emit(const unsigned long long* topk, const int* topk_count, int k, float* dist_out,
                         int64_t* id_out, cudaStream_t s) {

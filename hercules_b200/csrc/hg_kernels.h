@@ -32,7 +32,7 @@ class SmemLimit {
   std::atomic<uint64_t> done_{0};
 };
 
-constexpr int kEdWarps = 8;  // warps per block of the distance stream
+constexpr int kEdWarps = 8;  // warps per block of the distance stream (32 where the staged query is large)
 constexpr int kEdBlocksPerSm = 4;  // resident blocks per SM of the distance stream
 constexpr int kWarpListCap = 256;  // per-warp candidate buffer (k <= kWarpListCap - 32)
 constexpr int kMaxK = kWarpListCap - 32;
@@ -234,7 +234,7 @@ cudaError_t launch_leaf_gate(float lb, float eps1, const uint32_t* stale, int* f
 cudaError_t launch_stale_copy(const int* flag, const uint32_t* bound, uint32_t* stale, cudaStream_t s);
 // resident blocks per SM of the distance stream for series length L
 int ed_blocks_per_sm(int L);
-// the same with id = row index (EdArgs::ids unused)
+// the same with id = row index (EdArgs::ids unused), blocks of 32 warps
 cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int slots, int blocks, cudaStream_t s);
 cudaError_t launch_merge(const MergeArgs& a, int slots, cudaStream_t s);
 // the merge, then the candidate selection against the merged bound

@@ -28,7 +28,7 @@ void hg_record_error(const char* msg);  // hg_index.cu: the text hg_last_error r
 
 namespace {
 
-// 148 blocks of 8 warps; the scan reduces its warps' lists to one
+// 148 blocks of 32 warps, one per SM; the scan reduces its warps' lists to one
 // 256-entry candidate list per block, and the merge reads those 148 lists
 constexpr int kNoAllocBlocks = 148;
 constexpr int kNoAllocParts = kNoAllocBlocks;
