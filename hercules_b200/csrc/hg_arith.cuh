@@ -57,11 +57,22 @@ HG_HD float hg_hsum8(float v0, float v1, float v2, float v3, float v4, float v5,
 // Squared distance of one 8-float chunk: (q_i - x_i)^2 per lane, then hsum8.
 HG_HD float hg_chunk_d2(const float* q, const float* x) {
   float d[8];
+#if defined(__CUDA_ARCH__)
+  // two differences and two squares per instruction, each rounded as the
+  // scalar operation; q + (-x) is q - x
 #pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    const float2 v = __fadd2_rn(make_float2(q[j], q[j + 1]), make_float2(-x[j], -x[j + 1]));
+    const float2 s = __fmul2_rn(v, v);
+    d[j] = s.x;
+    d[j + 1] = s.y;
+  }
+#else
   for (int j = 0; j < 8; ++j) {
     float v = HG_FSUB(q[j], x[j]);
     d[j] = HG_FMUL(v, v);
   }
+#endif
   return hg_hsum8(d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7]);
 }
 

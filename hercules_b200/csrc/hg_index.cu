@@ -281,6 +281,7 @@ static void free_scratch(hg_index* ix) {
   dfree(s.unit_prefix);
   dfree(s.counters);
   dfree(s.bound);
+  dfree(s.kslots);
   dfree(s.parts);
   dfree(s.part_count);
   dfree(s.topk);
@@ -1179,6 +1180,7 @@ static cudaError_t alloc_scratch(hg_index* ix, size_t slots) {
   get(&s.cand_count, slots);
   get(&s.unit_prefix, slots * (nl + 2));
   get(&s.bound, slots);
+  get(&s.kslots, slots * hg::kMaxK);
   get(&s.parts, slots * s.nparts * hg::kWarpListCap);
   get(&s.part_count, slots * s.nparts);
   get(&s.topk, slots * hg::kMaxK);
@@ -1258,6 +1260,7 @@ static hg::EdArgs scan_args(hg_index* ix, const float* d_q, int k) {
   e.q = d_q;
   e.k = k;
   e.bound = s.bound;
+  e.kslots = s.kslots;
   e.parts = s.parts;
   e.part_count = s.part_count;
   e.parts_stride = (uint32_t)s.nparts;
@@ -1294,6 +1297,7 @@ static hg::PrepArgs prep_args(hg_index* ix, const float* d_q) {
   p.bp = ix->d.bp;
   p.approx_leaf = s.approx_leaf;
   p.bound = s.bound;
+  p.kslots = s.kslots;
   p.topk_count = s.topk_count;
   p.counters = s.counters;
   return p;
@@ -1323,7 +1327,7 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
     // every query's blocks resident at once: they walk the rows from the
     // front at the same pace, so the group reads most rows from L2
     const int blocks = std::max(1, ed_blocks / slots);
-    CK(hg::launch_pscan_prep(s.bound, s.topk_count, slots, st));
+    CK(hg::launch_pscan_prep(s.bound, s.kslots, s.topk_count, slots, st));
     e.ident_count = ix->n;
     HCK(scan(blocks));
     CK(hg::launch_merge(merge_args(ix, blocks, k, d_dist, d_id), slots, st));

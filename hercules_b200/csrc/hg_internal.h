@@ -64,6 +64,7 @@ struct QueryScratch {
   uint32_t* unit_prefix = nullptr;  // leaves + 2 (32-row units per candidate, exclusive scan)
   uint32_t* counters = nullptr;   // 8: [2] filter survivors, [4] the seeding stage's
   uint32_t* bound = nullptr;      // float bits of the current k-th distance bound
+  uint32_t* kslots = nullptr;     // kMaxK: the minima behind it (EdArgs)
   unsigned long long* parts = nullptr;  // nparts x kWarpListCap keys (d bits << 32 | id)
   int* part_count = nullptr;      // nparts
   unsigned long long* topk = nullptr;   // kMaxK keys

@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_query_prep(PrepArgs a) {
   if (blockIdx.y == gridDim.y - 1) {
     if (!a.approx_leaf || warp != 0) return;
     if (lane < 8) a.counters[8 * slot + lane] = 0;
+    for (int i = lane; i < kMaxK; i += 32) a.kslots[slot * kMaxK + i] = 0x7f800000u;  // +inf
     const int leaf = warp_route(qs, a.tree);
     if (lane == 0) {
       a.approx_leaf[slot] = leaf;
@@ -707,11 +708,13 @@ __device__ void select_sort(const SelectArgs& a, uint32_t slot, float B, uint32_
   }
 }
 
-__global__ void k_pscan_prep(uint32_t* bound, int* topk_count, int slots) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= slots) return;
-  bound[i] = 0x7f800000u;
-  topk_count[i] = 0;
+__global__ void k_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count) {
+  const int slot = blockIdx.x;
+  for (int i = threadIdx.x; i < kMaxK; i += blockDim.x) kslots[slot * kMaxK + i] = 0x7f800000u;  // +inf
+  if (threadIdx.x == 0) {
+    bound[slot] = 0x7f800000u;
+    topk_count[slot] = 0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1035,6 +1038,171 @@ __device__ __forceinline__ int q4_index(int chunk, int half) {
 }
 // bytes of that layout for a series of L floats
 __host__ __device__ inline size_t q4_bytes(int L) { return (size_t)((L / 8 + 31) / 32) * 40 * 2 * 16; }
+// What this block scans: the launch's arguments moved to its query and list,
+// the rows' first index and count.  False when nothing falls to the block (its
+// list is then empty).
+template <int W>
+__device__ __forceinline__ bool ed_range(EdArgs& a, uint64_t& first, uint32_t& total, uint32_t& bs) {
+  const uint32_t qslot = blockIdx.x;  // the query of the group
+  a.bound += qslot;
+  a.kslots += (uint64_t)qslot * kMaxK;
+  a.parts += ((uint64_t)qslot * a.parts_stride + blockIdx.y) * kWarpListCap;
+  a.part_count += (uint64_t)qslot * a.parts_stride + blockIdx.y;
+  a.q += (uint64_t)qslot * a.L;
+  if (a.list) a.list += (uint64_t)qslot * a.list_stride;
+  first = a.ident_first;
+  if (a.gate && *a.gate == 0) {
+    total = 0;  // a gated launch that did not pass
+  } else if (a.list) {
+    total = a.list_count[8 * qslot];
+  } else if (a.ident_leaf) {
+    const int leaf = a.ident_leaf[qslot];
+    first = a.leaf_start[leaf];
+    total = a.leaf_size[leaf];
+  } else {
+    total = (uint32_t)a.ident_count;
+  }
+  // warp w of the launch takes entries [(w + b nwarps) bs, +bs), b = 0, 1, ..:
+  // bs spreads a short list over the warps, at least min_batch entries each
+  const uint32_t nwarps = gridDim.y * W;
+  const uint32_t per_warp = (uint32_t)(((uint64_t)total + nwarps - 1) / nwarps);
+  bs = per_warp < a.min_batch ? a.min_batch : (per_warp > 32u ? 32u : per_warp);
+  if ((uint64_t)blockIdx.y * W * bs < total) return true;
+  if (threadIdx.x == 0) *a.part_count = 0;
+  return false;
+}
+
+// The running bound of a scan.  A warp's own k-th distance is a poor bound: a
+// warp sees a few hundred rows, and the least of 4,736 warps' 10th distances
+// after 16 rows each is at the 17% quantile.  So the query also has k slots:
+// a finished row's distance goes to slot hash(distance) with a minimum, equal
+// distances share a slot, so k filled slots hold k distinct distances, and
+// their maximum bounds the k-th distinct distance of all rows finished so far
+// on the GPU (about three times its quantile).  Each block keeps a copy in
+// shared memory; a warp exchanges it with the global slots when it kept a row
+// and in every 16th turn (rarer with more warps per block and more than 32
+// slots), its block mates in others: a word that every warp reads in every turn keeps its L2 slice busy
+// longer than a scan of 2M rows takes.  Against bounds from the warps' own
+// lists alone, one query: PSCAN of 2M x 256 329 -> 230 us, of 1M x 512 429 ->
+// 269 us, the allocation-free scan of 1M x 256 200 -> 126 us.
+struct EdShared {
+  uint32_t bound;
+  uint32_t slot[kMaxK];
+};
+__device__ __forceinline__ void ed_shared_init(const EdArgs& a, EdShared& sh, int threads) {
+  for (int i = threadIdx.x; i < a.k; i += threads) sh.slot[i] = 0x7f800000u;
+  if (threadIdx.x == 0) sh.bound = ld_volatile(a.bound);
+}
+__device__ __noinline__ void ed_exchange(uint32_t* gslot, uint32_t* gbound, int k, EdShared* sh) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t gb = ld_volatile(gbound);
+  uint32_t most = 0;
+  for (int i = lane; i < k; i += 32) {
+    const uint32_t g = ld_volatile(gslot + i), s = ld_volatile(&sh->slot[i]);
+    if (s < g) atomicMin(gslot + i, s);
+    else if (g < s) atomicMin(&sh->slot[i], g);
+    most = max(most, min(g, s));
+  }
+  most = __reduce_max_sync(HG_FULL, most);
+  if (lane == 0) {
+    if (most < gb) atomicMin(gbound, most);
+    atomicMin(&sh->bound, min(most, gb));
+  }
+  __syncwarp();
+}
+// after a turn's finished rows (take, dist) are in the list: the bound to go on with
+__device__ __forceinline__ float ed_bound(const EdArgs& a, EdShared& sh, uint32_t turn, bool take, float dist, float B,
+                                          float T) {
+  if (take) {
+    const uint32_t bits = __float_as_uint(dist);
+    atomicMin(&sh.slot[__umulhi(bits * 2654435761u, (uint32_t)a.k)], bits);
+  }
+  if (__any_sync(HG_FULL, take) || ((turn + 2 * (threadIdx.x >> 5)) & (a.period - 1)) == 0) {
+    __syncwarp();
+    ed_exchange(a.kslots, a.bound, a.k, &sh);
+  }
+  return fminf(fminf(B, T), __uint_as_float(ld_volatile(&sh.bound)));
+}
+
+// The block's warp lists (each at most k entries) become one: the entries
+// within the bound are packed to the front (read to registers, a barrier,
+// written at the warp's offset), the next power of two of them sorted, the
+// first k distinct distances kept; the merge then reads one part per block.
+template <int W>
+__device__ __forceinline__ void ed_finish(const EdArgs& a, unsigned long long* lists, unsigned long long* list, int cnt,
+                                          uint32_t n_chunks, uint32_t n_done, uint32_t n_rows) {
+  constexpr int kEdThreads = 32 * W;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  cnt = warp_compact(list, cnt, a.k);
+  uint32_t B = 0;
+  if (lane == 0) {
+    if (cnt == a.k) atomicMin(a.bound, (uint32_t)(list[a.k - 1] >> 32));
+    B = ld_volatile(a.bound);
+  }
+  B = __shfl_sync(HG_FULL, B, 0);
+  __shared__ int s_cnt[W];
+  constexpr int kPer = kWarpListCap / 32;  // entries per lane of a full list
+  unsigned long long mine[kPer];
+  int within = 0;  // entries within the bound: a prefix of the sorted list
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    mine[r] = list[lane + 32 * r];
+    within += __popc(__ballot_sync(HG_FULL, lane + 32 * r < cnt && (uint32_t)(mine[r] >> 32) <= B));
+  }
+  cnt = within;
+  if (lane == 0) s_cnt[wib] = cnt;
+  __syncthreads();
+  int offset = 0, packed = 0;
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    offset += w < wib ? s_cnt[w] : 0;
+    packed += s_cnt[w];
+  }
+  int nsort = 32;
+  while (nsort < packed) nsort <<= 1;
+  unsigned long long* flat = lists;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kPer; ++r)
+    if (lane + 32 * r < cnt) flat[offset + lane + 32 * r] = mine[r];
+  for (int i = packed + (int)threadIdx.x; i < nsort; i += kEdThreads) flat[i] = ~0ull;
+  __syncthreads();
+  for (int size = 2; size <= nsort; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int i = threadIdx.x; i < nsort / 2; i += kEdThreads) {
+        const int pos = 2 * i - (i & (stride - 1));
+        const int partner = pos + stride;
+        const bool asc = (pos & size) == 0;
+        const unsigned long long x = flat[pos], y = flat[partner];
+        if ((x > y) == asc) {
+          flat[pos] = y;
+          flat[partner] = x;
+        }
+      }
+      __syncthreads();
+    }
+  if (wib == 0) {
+    const int bc = warp_dedup_sorted(flat, packed, a.k, 0);
+    for (int i = lane; i < bc; i += 32) a.parts[i] = flat[i];
+    if (lane == 0) {
+      *a.part_count = bc;
+      if (bc == a.k) atomicMin(a.bound, (uint32_t)(flat[a.k - 1] >> 32));
+    }
+  }
+  unsigned long long s_chunks = n_chunks, s_done = n_done, s_rows = n_rows;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s_chunks += __shfl_xor_sync(HG_FULL, s_chunks, o);
+    s_done += __shfl_xor_sync(HG_FULL, s_done, o);
+    s_rows += __shfl_xor_sync(HG_FULL, s_rows, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&a.stats[1], s_chunks);
+    atomicAdd(&a.stats[4], s_done);
+    atomicAdd(&a.stats[5], s_rows);
+  }
+}
+
 // kRowIds: the id of a row is its row index (a matrix without an id map).
 // kSlot: lanes per row (a slot); kLines: 32-byte chunks per lane of a row in
 // flight per step, so a slot reads kSlot * kLines * 32 bytes of its row per
@@ -1052,47 +1220,25 @@ __host__ __device__ constexpr uint32_t slot_leaders() {
 }
 template <bool kRowIds, int kLines, int kSlot, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a) {
-  constexpr int W = kWarps, kEdThreads = 32 * kWarps;
+  constexpr int W = kWarps;
   extern __shared__ float4 ed_smem[];
   unsigned long long* lists = reinterpret_cast<unsigned long long*>(ed_smem);  // [W][kWarpListCap]
   float4* qs4 = ed_smem + W * kWarpListCap / 2;                                // the query, q4_bytes(L) bytes
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int slot_lead = lane & ~(kSlot - 1), j = lane & (kSlot - 1);
-  const uint32_t qslot = blockIdx.x;  // the query of the group
-  a.bound += qslot;
-  a.parts += ((uint64_t)qslot * a.parts_stride + blockIdx.y) * kWarpListCap;
-  a.part_count += (uint64_t)qslot * a.parts_stride + blockIdx.y;
-  if (a.list) a.list += (uint64_t)qslot * a.list_stride;
   const int nch = a.L >> 3;
-  uint64_t first = a.ident_first;
-  uint32_t total;
-  if (a.gate && *a.gate == 0) {
-    total = 0;  // a gated launch that did not pass
-  } else if (a.list) {
-    total = a.list_count[8 * qslot];
-  } else if (a.ident_leaf) {
-    const int leaf = a.ident_leaf[qslot];
-    first = a.leaf_start[leaf];
-    total = a.leaf_size[leaf];
-  } else {
-    total = (uint32_t)a.ident_count;
-  }
+  uint64_t first;
+  uint32_t total, bs;
+  if (!ed_range<W>(a, first, total, bs)) return;
   const uint32_t nwarps = gridDim.y * W;
   const uint32_t gw = blockIdx.y * W + wib;
   const uint32_t leaders = slot_leaders<kSlot>();
-  // batch b of this warp covers entries [(gw + b * nwarps) * bs, +bs): bs
-  // spreads a short list over the warps, at least min_batch entries each
-  const uint32_t per_warp = (uint32_t)(((uint64_t)total + nwarps - 1) / nwarps);
-  const uint32_t bs = per_warp < a.min_batch ? a.min_batch : (per_warp > 32u ? 32u : per_warp);
-  if ((uint64_t)blockIdx.y * W * bs >= total) {
-    // no entry for this block: an empty list
-    if (threadIdx.x == 0) *a.part_count = 0;
-    return;
-  }
   unsigned long long* list = lists + wib * kWarpListCap;
   for (int i = lane; i < kWarpListCap; i += 32) list[i] = ~0ull;
-  for (int i = threadIdx.x; i < (a.L >> 2); i += blockDim.x)
-    qs4[q4_index(i >> 1, i & 1)] = reinterpret_cast<const float4*>(a.q + (uint64_t)qslot * a.L)[i];
+  for (int i = threadIdx.x; i < (a.L >> 2); i += 32 * W)
+    qs4[q4_index(i >> 1, i & 1)] = reinterpret_cast<const float4*>(a.q)[i];
+  __shared__ EdShared sh;
+  ed_shared_init(a, sh, 32 * W);
   __syncthreads();
   auto entry = [&](uint32_t batch) -> uint32_t {
     const uint64_t idx = (uint64_t)batch * bs + lane;
@@ -1113,7 +1259,7 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
 
   int cnt = 0;
   float T = __int_as_float(0x7f800000);
-  float B = __int_as_float((int)ld_volatile(a.bound));
+  float B = __uint_as_float(sh.bound);
   const float F = a.has_floor ? a.floor : -1.0f;  // distances are >= 0
   bool valid = false;  // slot-uniform
   uint32_t row = 0;
@@ -1130,7 +1276,7 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
     const int o = kSlot * l + j;
     qoff[l] = 2 * (o + (o >> 2));
   }
-  for (int iter = 1;; ++iter) {
+  for (uint32_t turn = 0;; ++turn) {
     // refill the slots without a row
     uint32_t need = __ballot_sync(HG_FULL, !valid) & leaders;
     while (need) {
@@ -1159,7 +1305,6 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
       need = __ballot_sync(HG_FULL, !valid) & leaders;
     }
     if (!__any_sync(HG_FULL, valid)) break;
-    const uint32_t bnext = ((iter & 7) == 0) ? ld_volatile(a.bound) : 0x7f800000u;
     // kLines chunks of every owned row in flight: lane j computes chunks
     // ch + kSlot l + j (l < kLines); chunks past the row's end count as 0
     float4 xv[kLines][2];
@@ -1223,72 +1368,134 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
       }
     }
     const bool take = finished && j == 0 && dist <= B && dist <= T && dist > F;
-    warp_list_add(list, cnt, T, a.k, a.bound, take, dist,
-                  take ? (kRowIds ? row : (uint32_t)a.ids[row]) : 0u);
-    B = fminf(fminf(B, T), __int_as_float((int)bnext));
+    warp_list_add<true>(list, cnt, T, a.k, a.bound, take, dist, take ? (kRowIds ? row : (uint32_t)a.ids[row]) : 0u);
+    B = ed_bound(a, sh, turn, take, dist, B, T);
   }
-  cnt = warp_compact(list, cnt, a.k);
-  if (cnt == a.k && lane == 0) atomicMin(a.bound, (uint32_t)(list[a.k - 1] >> 32));
-  // the block's warp lists (each at most k entries) become one: the
-  // entries are packed to the front (read to registers, a barrier, written
-  // at the warp's offset), the next power of two of them sorted, the first
-  // k distinct distances kept; the merge then reads one part per block
-  __shared__ int s_cnt[W];
-  if (lane == 0) s_cnt[wib] = cnt;
-  constexpr int kPer = kWarpListCap / 32;  // entries per lane of a full list
-  unsigned long long mine[kPer];
-#pragma unroll
-  for (int r = 0; r < kPer; ++r) mine[r] = list[lane + 32 * r];
+  ed_finish<W>(a, lists, list, cnt, n_chunks, n_done, n_rows);
+}
+
+// The same for a group of queries over short series: a warp takes 8 rows (4
+// lanes each) together and stays with them until the last has finished or
+// abandoned, instead of giving a free slot the next row at every step.  Lanes
+// idle more (a row of 256 points abandons after 1.5 to 2.7 of its 4 steps), but
+// a step costs far fewer instructions (no refill; one place in the query for
+// all slots, so its reads are broadcasts), which bind the scan once a group
+// keeps every warp busy: 16 queries of 8M x 256, k = 100, 6.01 -> 5.66 ms per
+// call, 100 of 1M x 256 2.91 -> 2.73, 16 of 1M x 1024 1.19 -> 1.08, 16 of 300k
+// x 2048 0.85 -> 0.77.  A query alone waits for its loads instead, and the
+// other kernel's slots never idle: allocation-free scan of 1M x 256 127 us
+// there, 145 here.  (Loading the next rows' first step early spills at 64
+// registers: 5 to 20% slower.)
+__global__ void __launch_bounds__(32 * kEdWarps, kEdBlocksPerSm) k_ed_short(EdArgs a) {
+  constexpr int W = kEdWarps, kSlot = 4, kLines = 2, kStep = kSlot * kLines, kRows = 32 / kSlot;
+  extern __shared__ float4 ed_smem[];
+  unsigned long long* lists = reinterpret_cast<unsigned long long*>(ed_smem);  // [W][kWarpListCap]
+  float4* qs = ed_smem + W * kWarpListCap / 2;                                 // the query, whole steps, zero beyond L
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int slot = lane / kSlot, slot_lead = lane & ~(kSlot - 1), j = lane & (kSlot - 1);
+  const int nch = a.L >> 3;
+  uint64_t first;
+  uint32_t total, bs;
+  if (!ed_range<W>(a, first, total, bs)) return;
+  unsigned long long* list = lists + wib * kWarpListCap;
+  for (int i = lane; i < kWarpListCap; i += 32) list[i] = ~0ull;
+  for (int i = threadIdx.x; i < 2 * ((nch + kStep - 1) / kStep) * kStep; i += 32 * W)
+    qs[i] = i < 2 * nch ? reinterpret_cast<const float4*>(a.q)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  __shared__ EdShared sh;
+  ed_shared_init(a, sh, 32 * W);
   __syncthreads();
-  int offset = 0, packed = 0;
+  const uint32_t nwarps = gridDim.y * W;
+  uint32_t batch = blockIdx.y * W + wib;  // the batch of `cur`
+  auto entry = [&](uint32_t b) -> uint32_t {
+    const uint64_t idx = (uint64_t)b * bs + lane;
+    if ((uint32_t)lane >= bs || idx >= total) return 0u;
+    return a.list ? a.list[idx] : (uint32_t)(first + idx);
+  };
+  auto count_of = [&](uint32_t b) -> uint32_t {
+    const uint64_t b0 = (uint64_t)b * bs;
+    return b0 < total ? (uint32_t)(total - b0 < bs ? total - b0 : bs) : 0u;
+  };
+  uint32_t cur = entry(batch), cur_n = count_of(batch), used = 0;  // lane i holds entry i of the batch
+  uint32_t nxt = entry(batch + nwarps), nxt_n = count_of(batch + nwarps);
+  // the next 8 rows; false: none left
+  uint32_t row = 0;
+  bool alive = false;  // slot-uniform
+  auto fetch = [&]() -> bool {
+    if (used >= cur_n) {
+      if (nxt_n == 0) return false;
+      batch += nwarps;
+      cur = nxt;
+      cur_n = nxt_n;
+      used = 0;
+      nxt = entry(batch + nwarps);
+      nxt_n = count_of(batch + nwarps);
+    }
+    row = __shfl_sync(HG_FULL, cur, (int)(used + slot) & 31);
+    alive = used + slot < cur_n;
+    used += kRows;
+    return true;
+  };
+  int cnt = 0;
+  float T = __int_as_float(0x7f800000);
+  float B = __uint_as_float(sh.bound);
+  const float F = a.has_floor ? a.floor : -1.0f;  // distances are >= 0
+  uint32_t n_chunks = 0, n_done = 0, n_rows = 0;  // this lane's (slot leaders only)
+  for (uint32_t turn = 0; fetch(); ++turn) {
+    const float4* x = reinterpret_cast<const float4*>(a.rows + (uint64_t)row * a.L) + 2 * j;
+    if (alive && j == 0) ++n_rows;
+    float dist = 0.0f;
+    for (int ch = 0;;) {
+      float4 xv[kLines][2];
+      bool in[kLines];
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    offset += w < wib ? s_cnt[w] : 0;
-    packed += s_cnt[w];
-  }
-  int nsort = 32;
-  while (nsort < packed) nsort <<= 1;
-  unsigned long long* flat = lists;
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < kPer; ++r)
-    if (lane + 32 * r < cnt) flat[offset + lane + 32 * r] = mine[r];
-  for (int i = packed + (int)threadIdx.x; i < nsort; i += kEdThreads) flat[i] = ~0ull;
-  __syncthreads();
-  for (int size = 2; size <= nsort; size <<= 1)
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < nsort / 2; i += kEdThreads) {
-        const int pos = 2 * i - (i & (stride - 1));
-        const int partner = pos + stride;
-        const bool asc = (pos & size) == 0;
-        const unsigned long long x = flat[pos], y = flat[partner];
-        if ((x > y) == asc) {
-          flat[pos] = y;
-          flat[partner] = x;
+      for (int l = 0; l < kLines; ++l) {
+        in[l] = alive && ch + kSlot * l + j < nch;
+        if (in[l]) {
+          xv[l][0] = __ldcs(x + 2 * (ch + kSlot * l));
+          xv[l][1] = __ldcs(x + 2 * (ch + kSlot * l) + 1);
         }
       }
-      __syncthreads();
-    }
-  if (wib == 0) {
-    const int bc = warp_dedup_sorted(flat, packed, a.k, 0);
-    for (int i = lane; i < bc; i += 32) a.parts[i] = flat[i];
-    if (lane == 0) {
-      *a.part_count = bc;
-      if (bc == a.k) atomicMin(a.bound, (uint32_t)(flat[a.k - 1] >> 32));
-    }
-  }
-  unsigned long long s_chunks = n_chunks, s_done = n_done, s_rows = n_rows;
+      float dl[kLines];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s_chunks += __shfl_xor_sync(HG_FULL, s_chunks, o);
-    s_done += __shfl_xor_sync(HG_FULL, s_done, o);
-    s_rows += __shfl_xor_sync(HG_FULL, s_rows, o);
+      for (int l = 0; l < kLines; ++l) {
+        const float4 q0 = qs[2 * (ch + kSlot * l + j)], q1 = qs[2 * (ch + kSlot * l + j) + 1];
+        const float qa[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        const float xa[8] = {xv[l][0].x, xv[l][0].y, xv[l][0].z, xv[l][0].w,
+                             xv[l][1].x, xv[l][1].y, xv[l][1].z, xv[l][1].w};
+        const float d = hg_chunk_d2(qa, xa);
+        dl[l] = in[l] ? d : 0.0f;  // adding 0 leaves a sum unchanged
+      }
+      float part[kStep];
+      float acc = dist;
+#pragma unroll
+      for (int t = 0; t < kStep; ++t) {
+        acc = __fadd_rn(acc, __shfl_sync(HG_FULL, dl[t / kSlot], slot_lead + (t % kSlot)));
+        part[t] = acc;
+      }
+      const bool dead = alive && acc > B;
+      if (dead && j == 0) {
+        // the reference reads up to the first chunk whose sum exceeds the
+        // bound (the partial sums never decrease)
+        uint32_t u = 1;
+#pragma unroll
+        for (int t = 0; t < kStep; ++t) u += part[t] <= B ? 1u : 0u;
+        n_chunks += (uint32_t)ch + u;
+      }
+      alive = alive && !dead;
+      dist = acc;
+      ch += kStep;
+      if (ch >= nch || !__any_sync(HG_FULL, alive)) break;
+    }
+    const bool lead = alive && j == 0;
+    if (lead) {
+      n_chunks += (uint32_t)nch;
+      ++n_done;
+    }
+    const bool take = lead && dist <= B && dist <= T && dist > F;
+    warp_list_add<true>(list, cnt, T, a.k, a.bound, take, dist, take ? (uint32_t)a.ids[row] : 0u);
+    B = ed_bound(a, sh, turn, take, dist, B, T);
   }
-  if (lane == 0) {
-    atomicAdd(&a.stats[1], s_chunks);
-    atomicAdd(&a.stats[4], s_done);
-    atomicAdd(&a.stats[5], s_rows);
-  }
+  ed_finish<W>(a, lists, list, cnt, n_chunks, n_done, n_rows);
 }
 
 // Merges the per-block lists and the current top-k into the k smallest
@@ -1646,8 +1853,8 @@ cudaError_t launch_merge_select(const MergeArgs& a, const SelectArgs& sel, int s
   return cudaGetLastError();
 }
 
-cudaError_t launch_pscan_prep(uint32_t* bound, int* topk_count, int slots, cudaStream_t s) {
-  k_pscan_prep<<<blocks_for(slots, 32), 32, 0, s>>>(bound, topk_count, slots);
+cudaError_t launch_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count, int slots, cudaStream_t s) {
+  k_pscan_prep<<<slots, 128, 0, s>>>(bound, kslots, topk_count);
   return cudaGetLastError();
 }
 
@@ -1662,24 +1869,34 @@ cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cuda
 static size_t ed_smem_bytes(int L, int warps) { return (size_t)warps * kWarpListCap * 8 + q4_bytes(L); }
 // 32-warp blocks: where fewer than four 8-warp blocks fit on an SM
 static bool ed_wide(int L) { return kEdBlocksPerSm * (ed_smem_bytes(L, kEdWarps) + 1024) > (size_t)227 * 1024; }
+constexpr int kEdShortL = 2048;  // k_ed_short up to this length, for groups
 
-template <bool kRowIds, int kSlot, int kWarps>
-static cudaError_t launch_ed(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  const auto kernel = k_ed_stream<kRowIds, 2, kSlot, kWarps>;
-  static SmemLimit attr;
-  const cudaError_t ea = attr.ensure((const void*)kernel, (int)ed_smem_bytes(16384, kWarps));
+template <class K>
+static cudaError_t launch_ed(K kernel, SmemLimit& attr, const EdArgs& args, int warps, int slots, int blocks,
+                             cudaStream_t s) {
+  const cudaError_t ea = attr.ensure((const void*)kernel, (int)ed_smem_bytes(16384, warps));
   if (ea != cudaSuccess) return ea;
-  kernel<<<dim3(slots, blocks), 32 * kWarps, ed_smem_bytes(a.L, kWarps), s>>>(a);
+  EdArgs a = args;
+  a.period = 2 * (uint32_t)warps;
+  for (int k = 32; k < a.k; k *= 2) a.period *= 2;
+  kernel<<<dim3(slots, blocks), 32 * warps, ed_smem_bytes(a.L, warps), s>>>(a);
   return cudaGetLastError();
 }
-// long series (L >= 4096): few candidate rows per query, each long, so
-// more lanes per row keep more of each row in flight
+// Groups over series of at most kEdShortL points: k_ed_short (longer rows of a
+// warp differ too much in where they abandon).  Long series (L >= 4096): few
+// candidate rows per query, each long, so more lanes per row keep more of each
+// row in flight.
 cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  if (ed_wide(a.L)) return launch_ed<false, 8, 32>(a, slots, blocks, s);
-  return a.L >= 4096 ? launch_ed<false, 8, kEdWarps>(a, slots, blocks, s) : launch_ed<false, 4, kEdWarps>(a, slots, blocks, s);
+  static SmemLimit wide, lng, mid, shrt;
+  if (slots > 1 && a.L <= kEdShortL) return launch_ed(k_ed_short, shrt, a, kEdWarps, slots, blocks, s);
+  if (ed_wide(a.L)) return launch_ed(k_ed_stream<false, 2, 8, 32>, wide, a, 32, slots, blocks, s);
+  if (a.L >= 4096) return launch_ed(k_ed_stream<false, 2, 8, kEdWarps>, lng, a, kEdWarps, slots, blocks, s);
+  return launch_ed(k_ed_stream<false, 2, 4, kEdWarps>, mid, a, kEdWarps, slots, blocks, s);
 }
 cudaError_t launch_ed_stream_row_ids(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  return a.L >= 4096 ? launch_ed<true, 8, 32>(a, slots, blocks, s) : launch_ed<true, 4, 32>(a, slots, blocks, s);
+  static SmemLimit lng, mid;
+  if (a.L >= 4096) return launch_ed(k_ed_stream<true, 2, 8, 32>, lng, a, 32, slots, blocks, s);
+  return launch_ed(k_ed_stream<true, 2, 4, 32>, mid, a, 32, slots, blocks, s);
 }
 int ed_blocks_per_sm(int L) { return ed_wide(L) ? 1 : kEdBlocksPerSm; }
 

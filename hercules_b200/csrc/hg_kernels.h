@@ -73,6 +73,7 @@ struct PrepArgs {
   float* sax_tab;        // [slot][16 x 256] LB_SAX terms; NULL: none
   int* approx_leaf;      // [slot]; NULL: no routing, and the state below is left alone
   uint32_t* bound;       // [slot] reset to +inf
+  uint32_t* kslots;      // [slot][kMaxK] reset to +inf
   int* topk_count;       // [slot] reset to 0
   uint32_t* counters;    // [slot][8] reset to 0
 };
@@ -116,9 +117,11 @@ struct EdArgs {
   const float* q;              // [slot][L]
   int k;
   uint32_t* bound;             // [slot] float bits of the running k-th bound (atomicMin)
+  uint32_t* kslots;            // [slot][kMaxK] distance bits: minima whose first k bound the k-th (atomicMin)
   unsigned long long* parts;   // [slot][parts_stride] per-block sorted lists (kWarpListCap stride)
   int* part_count;             // [slot][parts_stride]
   uint32_t parts_stride;       // lists per slot
+  uint32_t period;             // turns between two looks at kslots by one warp (set by the launcher)
   unsigned long long* stats;   // [1] chunks computed [4] rows completed [5] rows started
   const int* gate;             // if set and *gate == 0, the launch scans nothing
   int has_floor;               // 1: only rows at distance > floor enter the lists (the
@@ -207,7 +210,7 @@ cudaError_t launch_sax_rows(const float* rows, int L, uint64_t n, const float* b
 // queries
 cudaError_t launch_query_prep(const PrepArgs& a, int slots, cudaStream_t s);
 cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s);
-cudaError_t launch_pscan_prep(uint32_t* bound, int* topk_count, int slots, cudaStream_t s);
+cudaError_t launch_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count, int slots, cudaStream_t s);
 // blocks: per slot
 cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cudaStream_t s);
 size_t lbsax_filter_smem();

@@ -84,12 +84,14 @@ extern "C" HG_API hg_status hg_pscan_noalloc(const float* d_rows, uint64_t n, ui
   unsigned long long* stats = reinterpret_cast<unsigned long long*>(base + 512);  // 8
   unsigned long long* topk = reinterpret_cast<unsigned long long*>(base + 1024);  // kMaxK
   int* part_count = reinterpret_cast<int*>(base + 3072);              // kNoAllocParts
+  uint32_t* kslots = reinterpret_cast<uint32_t*>(base + 4096);         // kMaxK
   unsigned long long* parts = reinterpret_cast<unsigned long long*>(base + kHeaderBytes);
   static_assert(1024 + sizeof(unsigned long long) * hg::kMaxK <= 3072, "scratch layout");
-  static_assert(3072 + sizeof(int) * kNoAllocParts <= kHeaderBytes, "scratch layout");
+  static_assert(3072 + sizeof(int) * kNoAllocParts <= 4096, "scratch layout");
+  static_assert(4096 + sizeof(uint32_t) * hg::kMaxK <= kHeaderBytes, "scratch layout");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // bound and top-k start from +inf / empty on every call
-  cudaError_t e = hg::launch_pscan_prep(bound, topk_count, 1, s);
+  cudaError_t e = hg::launch_pscan_prep(bound, kslots, topk_count, 1, s);
   if (e == cudaSuccess) {
     hg::EdArgs a{};
     a.rows = d_rows;
@@ -99,6 +101,7 @@ extern "C" HG_API hg_status hg_pscan_noalloc(const float* d_rows, uint64_t n, ui
     a.q = d_query;
     a.k = (int)k;
     a.bound = bound;
+    a.kslots = kslots;
     a.parts = parts;
     a.part_count = part_count;
     a.parts_stride = kNoAllocParts;
