@@ -266,9 +266,13 @@ __global__ void __launch_bounds__(1024) k_rerank_plan(BatchRank a) {
   __syncthreads();
   const float inf = __int_as_float(0x7f800000);
   const int nlist = a.nlist_dev ? (int)*a.nlist_dev : a.nlist;
+  // a pair list that overflowed lost rows of any query: all of the round's
+  // count as overflowed
+  const bool lost = *a.pairs_cnt > a.pairs_cap;
   unsigned long long mine = 0;
   for (int i = tid; i < nlist; i += 1024) {
     const int q = a.qlist ? (int)a.qlist[i] : i;
+    if (lost) a.bucket_cnt[q] = max(a.bucket_cnt[q], a.bucket_cap + 1);
     mine += a.bound[q] < inf ? min(a.bucket_cnt[q], a.bucket_cap) : 0u;
   }
   if (mine) atomicAdd(&s_rows, mine);
@@ -579,7 +583,8 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_merge(BatchRank a) {
 // the filter emits them tile by tile); empty slots (~0) are skipped.
 __global__ void k_scatter_pairs(const unsigned long long* __restrict__ pairs, const uint32_t* pairs_cnt,
                                 uint32_t pairs_cap, uint32_t* __restrict__ bucket, uint32_t* bucket_cnt,
-                                uint32_t bucket_cap) {
+                                uint32_t bucket_cap, unsigned long long* stamp) {
+  stamp_start(stamp);
   const uint32_t n = min(*pairs_cnt, pairs_cap);
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -594,17 +599,6 @@ __global__ void k_scatter_pairs(const unsigned long long* __restrict__ pairs, co
     if (valid && lane == leader) pos = atomicAdd(&bucket_cnt[q], (uint32_t)__popc(same));
     pos = __shfl_sync(HG_FULL, pos, leader) + (uint32_t)__popc(same & ((1u << lane) - 1));
     if (valid && pos < bucket_cap) bucket[(uint64_t)q * bucket_cap + pos] = (uint32_t)e;
-  }
-}
-
-// The pair list overflowed: every query of the round counts as overflowed.
-__global__ void k_mark_overflow(const uint32_t* pairs_cnt, uint32_t pairs_cap, const uint32_t* qlist, int nlist,
-                                const uint32_t* nlist_dev, uint32_t* bucket_cnt, uint32_t bucket_cap) {
-  if (*pairs_cnt <= pairs_cap) return;
-  if (nlist_dev) nlist = (int)*nlist_dev;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nlist; i += gridDim.x * blockDim.x) {
-    const uint32_t q = qlist ? qlist[i] : (uint32_t)i;
-    bucket_cnt[q] = max(bucket_cnt[q], bucket_cap + 1);
   }
 }
 
@@ -849,30 +843,17 @@ __global__ void k_emit_pruned(const uint32_t* __restrict__ leaf_cnt, const uint3
   }
 }
 
-// Queries of a round (list, or 0 .. n) still to retry (ok == 0) go to out.
+// The end of a round: its queries (list, or 0 .. n) still to retry (ok == 0) go
+// to out, those that neither verified nor can be retried are counted.
 __global__ void k_collect_retry(const int* __restrict__ ok, const uint32_t* list, uint32_t n, const uint32_t* n_dev,
-                                uint32_t* out, uint32_t* out_n) {
+                                uint32_t* out, uint32_t* out_n, uint32_t* failed, unsigned long long* stamp) {
+  stamp_start(stamp);
   if (n_dev) n = *n_dev;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t q = list ? list[i] : i;
     if (ok[q] == 0) out[atomicAdd(out_n, 1u)] = q;
+    else if (ok[q] != 1) atomicAdd(failed, 1u);
   }
-}
-
-// Phase boundary of a batch: the global timer (ns) into a slot.
-__global__ void k_stamp(unsigned long long* slot) {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  *slot = t;
-}
-
-// Queries the batch did not verify (ok != 1): the plain path answers them.
-__global__ void k_count_unverified(const int* __restrict__ ok, uint32_t nq, uint32_t* out) {
-  uint32_t c = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) c += ok[i] != 1;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(HG_FULL, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -908,14 +889,10 @@ cudaError_t launch_tile_norms(const float4* meta, uint64_t n, float4* tile_meta,
 }
 
 cudaError_t launch_scatter_pairs(const unsigned long long* pairs, const uint32_t* pairs_cnt, uint32_t pairs_cap,
-                                 const uint32_t* qlist, int nlist, const uint32_t* nlist_dev, uint32_t* bucket,
-                                 uint32_t* bucket_cnt, uint32_t bucket_cap, cudaStream_t s) {
+                                 uint32_t* bucket, uint32_t* bucket_cnt, uint32_t bucket_cap,
+                                 unsigned long long* stamp, cudaStream_t s) {
   // grid-stride, enough threads in flight to hide the bucket atomics' latency
-  k_scatter_pairs<<<2048, 256, 0, s>>>(pairs, pairs_cnt, pairs_cap, bucket, bucket_cnt, bucket_cap);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || nlist == 0) return e;
-  k_mark_overflow<<<nblk(nlist, 256), 256, 0, s>>>(pairs_cnt, pairs_cap, qlist, nlist, nlist_dev, bucket_cnt,
-                                                   bucket_cap);
+  k_scatter_pairs<<<2048, 256, 0, s>>>(pairs, pairs_cnt, pairs_cap, bucket, bucket_cnt, bucket_cap, stamp);
   return cudaGetLastError();
 }
 
@@ -953,22 +930,11 @@ cudaError_t launch_group_pruned(const uint32_t* leaf_cnt, const uint32_t* leaf_q
 }
 
 cudaError_t launch_collect_retry(const int* ok, const uint32_t* list, uint32_t n, const uint32_t* n_dev,
-                                 uint32_t* out, uint32_t* out_n, cudaStream_t s) {
+                                 uint32_t* out, uint32_t* out_n, uint32_t* failed, unsigned long long* stamp,
+                                 cudaStream_t s) {
   if (!n) return cudaSuccess;
   const unsigned g = nblk(n, 256) < 1024 ? nblk(n, 256) : 1024;
-  k_collect_retry<<<g, 256, 0, s>>>(ok, list, n, n_dev, out, out_n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_stamp(unsigned long long* slot, cudaStream_t s) {
-  k_stamp<<<1, 1, 0, s>>>(slot);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_count_unverified(const int* ok, uint32_t nq, uint32_t* out, cudaStream_t s) {
-  if (!nq) return cudaSuccess;
-  const unsigned g = nblk(nq, 256) < 1024 ? nblk(nq, 256) : 1024;
-  k_count_unverified<<<g, 256, 0, s>>>(ok, nq, out);
+  k_collect_retry<<<g, 256, 0, s>>>(ok, list, n, n_dev, out, out_n, failed, stamp);
   return cudaGetLastError();
 }
 

@@ -34,6 +34,19 @@ struct LeafPlan {
   uint32_t size, use_tiles, sub, pad;
 };
 
+// Device-side control words of a batch, in one block: zeroed by one memset at
+// the start of a batch and read back by one copy.
+struct BatchCtl {
+  unsigned long long stats[8];   // BatchRank::stats
+  unsigned long long pairs[2];   // (query, row) pairs of the pruned passes: first round, retries
+  double errstat[6];             // BatchGemm::errstat of the first round
+  unsigned long long stamps[16];  // global-timer stamps: [0] start, round r: [2 + 3r] filter, [3 + 3r] re-rank, [4 + 3r] end
+  uint32_t ctrl[16];   // [0] bound items [1] their tiles [3] queries for the plain path [4 + r] queries of round r
+  uint32_t heads[4];   // [1] pair slots reserved [2] re-rank segments taken [3] error flag
+  uint32_t queues[12];  // work-item counters of the filter launches
+  uint32_t pctl[16];   // pruned panel controls: [0, 8) the first round's, [8, 16) a retry round's
+};
+
 // Arguments of the tensor-core filter (hg_umma.cu); the BF16 rows and the
 // BF16 queries (in tile order) reach it as TMA descriptors.
 struct BatchGemm {
@@ -70,6 +83,7 @@ struct BatchGemm {
   // mode 2 (diagnostics): raw dot products q~.x~, [query position][dots_ld]
   float* dots;
   uint64_t dots_ld;
+  unsigned long long* stamp;  // if set: the global timer at the launch's start
   uint64_t wait_ns;         // each bounded wait gives up after this (0: 2 s)
   int withhold_first_copy;  // diagnostics: the first operand copy is never issued
 };
@@ -89,8 +103,10 @@ struct BatchRank {
   unsigned long long* init;        // [q][kMaxK] exact keys of the bound rows
   int* init_cnt;
   const uint32_t* bucket;
-  const uint32_t* bucket_cnt;
+  uint32_t* bucket_cnt;            // raised past bucket_cap for every query when the pair list overflowed
   uint32_t bucket_cap;
+  const uint32_t* pairs_cnt;       // pair slots the filter reserved
+  uint32_t pairs_cap;
   float* dist_out;  // [q][kmax]
   int64_t* id_out;
   int* ok_out;                // 1 verified, 0 retry with the lowered bound, -1 plain path
@@ -139,10 +155,11 @@ cudaError_t launch_group_pruned(const uint32_t* leaf_cnt, const uint32_t* leaf_q
                                 uint32_t items_cap, uint32_t nq, uint32_t* leaf_poff, uint32_t* leaf_ioff,
                                 uint32_t* ctl, unsigned long long* pairs, uint32_t* panel_list, BatchItem* items,
                                 cudaStream_t s, const uint32_t* nq_dev = nullptr);
+// the round's queries (list, or 0 .. n) left to retry (ok == 0) go to out
+// (*out_n of them), those for the plain path (ok == -1) are counted in *failed
 cudaError_t launch_collect_retry(const int* ok, const uint32_t* list, uint32_t n, const uint32_t* n_dev,
-                                 uint32_t* out, uint32_t* out_n, cudaStream_t s);
-cudaError_t launch_count_unverified(const int* ok, uint32_t nq, uint32_t* out, cudaStream_t s);
-cudaError_t launch_stamp(unsigned long long* slot, cudaStream_t s);  // global-timer stamp (ns)
+                                 uint32_t* out, uint32_t* out_n, uint32_t* failed, unsigned long long* stamp,
+                                 cudaStream_t s);
 cudaError_t launch_tile_norms(const float4* meta, uint64_t n, float4* tile_meta, cudaStream_t s);
 cudaError_t launch_bound_select(const BatchRank& r, cudaStream_t s);
 size_t umma_filter_smem();
@@ -156,10 +173,9 @@ cudaError_t launch_umma_filter(const CUtensorMap& rows_map, const QueryMaps& q, 
                                cudaStream_t s);
 cudaError_t launch_rerank(const BatchRank& r, int part_blocks, cudaStream_t s);
 // Distributes the filter's survivor pairs into per-query buckets
-// (bucket_cnt[q] counts every pair of q, also beyond bucket_cap); when the
-// pair list overflowed, every query of the round is marked overflowed.
+// (bucket_cnt[q] counts every pair of q, also beyond bucket_cap).
 cudaError_t launch_scatter_pairs(const unsigned long long* pairs, const uint32_t* pairs_cnt, uint32_t pairs_cap,
-                                 const uint32_t* qlist, int nlist, const uint32_t* nlist_dev, uint32_t* bucket,
-                                 uint32_t* bucket_cnt, uint32_t bucket_cap, cudaStream_t s);
+                                 uint32_t* bucket, uint32_t* bucket_cnt, uint32_t bucket_cap,
+                                 unsigned long long* stamp, cudaStream_t s);
 
 }  // namespace hg

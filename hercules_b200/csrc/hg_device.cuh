@@ -13,6 +13,16 @@ __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {
   return *(const volatile uint32_t*)p;
 }
 
+// The global timer (ns) into *slot, by one thread of the launch: a phase
+// boundary of a batch, at the start of the phase's first kernel.
+__device__ __forceinline__ void stamp_start(unsigned long long* slot) {
+  if (slot && blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    *slot = t;
+  }
+}
+
 // --- warp candidate list -----------------------------------------------------
 // A warp keeps its candidates as 64-bit keys (distance bits << 32 | id) in a
 // shared buffer of kWarpListCap entries.  Compaction sorts the buffer

@@ -271,6 +271,13 @@ void collect_leaves(const std::vector<Node>& nodes, int n, std::vector<int>& out
 // device index assembly
 // ---------------------------------------------------------------------------
 
+static void drop_graphs(hg::BatchScratch& b) {
+  for (cudaGraphExec_t& g : b.graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 static void free_scratch(hg_index* ix) {
   hg::QueryScratch& s = ix->s;
   dfree(s.lb);
@@ -329,8 +336,7 @@ static void free_device(hg_index* ix) {
   dfree(b.bucket_cnt);
   dfree(b.pairs);
   dfree(b.ok);
-  dfree(b.stats);
-  dfree(b.heads);
+  dfree(b.ctl);
   dfree(b.qlist);
   dfree(b.seg_rows);
   dfree(b.seg_prefix);
@@ -338,7 +344,6 @@ static void free_device(hg_index* ix) {
   dfree(b.parts);
   dfree(b.part_cnt);
   dfree(b.qlist2);
-  dfree(b.ctrl);
   dfree(b.qin);
   dfree(b.out_dist);
   dfree(b.out_id);
@@ -347,10 +352,7 @@ static void free_device(hg_index* ix) {
   dfree(b.leaf_qoff);
   dfree(b.leaf_qcnt);
   dfree(b.item_off);
-  if (b.graph) cudaGraphExecDestroy(b.graph);
-  dfree(b.stamps);
-  dfree(b.errstat);
-  dfree(b.queues);
+  drop_graphs(b);
   dfree(b.leaf_cnt);
   dfree(b.leaf_q);
   dfree(b.leaf_poff);
@@ -358,8 +360,6 @@ static void free_device(hg_index* ix) {
   dfree(b.panel_list);
   dfree(b.panel_bf);
   dfree(b.items3);
-  dfree(b.pctl);
-  dfree(b.ppairs);
   dfree(b.useg_start);
   dfree(b.useg_end);
   dfree(b.seg_uid);
@@ -1813,9 +1813,8 @@ static hg_status ensure_batch_scratch(hg_index* ix, uint32_t nq, uint32_t bucket
     b.parts_kmax = kmax;
     ++b.gen;  // a captured pipeline holds the old addresses
   }
-  if (!b.stats) {
-    CK(dalloc(&b.stats, 8));
-    CK(dalloc(&b.heads, 4));
+  if (!b.ctl) {
+    CK(dalloc(&b.ctl, 1));
     ++b.gen;  // a captured pipeline holds the old addresses
   }
   if ((uint64_t)b.nq_cap * bucket_cap > (uint64_t)b.nq_cap * b.bucket_cap || !b.bucket) {
@@ -1888,8 +1887,6 @@ static hg_status ensure_prune_scratch(hg_index* ix, bool* ok) {
   dfree(b.panel_list);
   dfree(b.panel_bf);
   dfree(b.items3);
-  dfree(b.pctl);
-  dfree(b.ppairs);
   dfree(b.segstats);
   b.prune_nq = 0;
   size_t free_b = 0, total_b = 0;
@@ -1898,9 +1895,10 @@ static hg_status ensure_prune_scratch(hg_index* ix, bool* ok) {
   const uint64_t panel = std::min<uint64_t>(nl * nq, std::max<uint64_t>(nq, budget / (2 * L)));
   // items for the narrowest work item (8 tiles): chunks of every leaf x its query tiles
   const uint64_t ntiles = (ix->n + hg::kBatchTileRows - 1) / hg::kBatchTileRows;
-  // and kBatchItemTarget more where narrower ones even out a small batch
+  // and 2 kBatchItemTarget more where narrower ones even out a small batch: the
+  // item list never overflows
   const uint64_t items =
-      (ntiles / 8 + 2 * nl) * ((nq + hg::kBatchQueryTile - 1) / hg::kBatchQueryTile) + hg::kBatchItemTarget;
+      (ntiles / 8 + 2 * nl) * ((nq + hg::kBatchQueryTile - 1) / hg::kBatchQueryTile) + 2 * hg::kBatchItemTarget;
   if (panel >= (1ull << 32) || items >= (1ull << 31)) {
     *ok = false;
     return HG_OK;
@@ -1914,8 +1912,6 @@ static hg_status ensure_prune_scratch(hg_index* ix, bool* ok) {
   CK(dalloc(&p, panel * L));
   b.panel_bf = p;
   CK(dalloc(&b.items3, items));
-  CK(dalloc(&b.pctl, 16));   // [0, 8): the first round's panel controls, [8, 16): a retry round's
-  CK(dalloc(&b.ppairs, 2));
   CK(dalloc(&b.segstats, std::max<uint64_t>((uint64_t)b.nu * nq, 1)));
   b.panel_cap = (uint32_t)panel;
   b.items3_cap = (uint32_t)items;
@@ -1979,59 +1975,42 @@ static hg_status ensure_leaf_plan(hg_index* ix, uint64_t want, cudaStream_t st) 
   return HG_OK;
 }
 
-// Everything of one batch after the queries are in b.qin and their k in
-// b.kq, as one stream-ordered sequence with no host decision inside (so it
-// can be captured in a CUDA graph): routing and grouping on the device, the
-// bound pass, 1 + kBatchRetries filter rounds whose query lists are built on
-// the device (an empty round costs a few microseconds), the count of queries
-// left unverified.  Events gev[0..] mark the phases.
-static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_t bucket_cap, const hg::QueryMaps& qmaps,
-                               bool prune, cudaStream_t st,
-                               uint64_t* launches) {
+// One round of a batch, after the queries are in b.qin and their k in b.kq, as
+// one stream-ordered sequence with no host decision inside (so it can be
+// captured in a CUDA graph).  Round 0 routes and groups the queries on the
+// device and runs the bound pass; every round filters, re-ranks and lists the
+// queries left to retry.  A retry round is launched only when the one before
+// left it queries: three empty rounds of twelve kernels each cost a small
+// batch a third of its time (100k x 256, 64 queries: 300 -> 127 us on the device, with
+// the stamps, counters and overflow marks folded into the kernels beside them).
+static hg_status enqueue_round(hg_index* ix, int round, uint32_t nq, uint32_t kmax, uint32_t bucket_cap,
+                               const hg::QueryMaps& qmaps, bool prune, cudaStream_t st, uint64_t* launches) {
   hg::BatchScratch& b = ix->bs;
+  hg::BatchCtl* c = b.ctl;
+  const hg::DeviceIndex& d = ix->d;
   const uint32_t L = ix->L;
   const int sms = hg::sm_count(ix->device);
   const int nl = (int)ix->leaves.size();
-  auto stamp = [&](int i) { return hg::launch_stamp(b.stamps + i, st); };
-  CK(stamp(0));
-  CK(cudaMemsetAsync(b.ctrl, 0, sizeof(uint32_t) * 16, st));
-  CK(cudaMemsetAsync(b.heads, 0, sizeof(uint32_t) * 4, st));
-  CK(cudaMemsetAsync(b.stats, 0, sizeof(unsigned long long) * 8, st));
-  CK(cudaMemsetAsync(b.queues, 0, sizeof(uint32_t) * 12, st));
-  CK(cudaMemsetAsync(b.bm, 0xff, sizeof(unsigned long long) * nq * b.plan_bm_cap, st));
-  // 1. approximate leaves, grouping
-  CK(hg::launch_route_queries(b.qin, (int)nq, (int)L, index_tree(ix), b.approx, st));
-  CK(hg::launch_group_queries(b.approx, (int)nq, b.leaf_plan, nl, ix->tune.bound_tiles_per_item, b.qperm, b.slots,
-                              b.leaf_qoff, b.leaf_qcnt, b.item_off, b.ctrl + 0, b.items, st, b.group_cnt));
-  CK(hg::launch_rows_to_bf16(b.qin, b.qperm, nq, (int)L, b.qbf, b.qmeta, st));
-  // 2. bound pass
+  uint64_t n_launch = 0;
   hg::BatchGemm g{};
   g.L = (int)L;
   g.nrows = ix->n;
   g.xmeta = ix->bd.xmeta;
   g.tile_meta = ix->bd.tile_meta;
   g.qmeta = b.qmeta;
-  g.qperm = b.qperm;
   g.nq = (int)nq;
-  g.mode = 0;
-  g.qtile = hg::kBatchQueryTile;
-  g.items = b.items;
-  g.nitems = b.items_cap;
-  g.nitems_dev = b.ctrl + 0;
   g.bm = b.bm;
   g.bm_cap = b.plan_bm_cap;
   g.tiles_per_item = ix->tune.filter_tiles_per_item;
   filter_coefficients(L, &g.c_acc, &g.c_sq);
   g.bound = b.bound;
   g.pairs = b.pairs;
-  g.pairs_cnt = b.heads + 1;
+  g.pairs_cnt = c->heads + 1;
   g.pairs_cap = b.pairs_cap;
-  g.err = reinterpret_cast<int*>(b.heads + 3);
-  g.queue = b.queues + 0;
-  CK(hg::launch_umma_filter(ix->bd.rows_map, qmaps, g, sms, st));
+  g.err = reinterpret_cast<int*>(c->heads + 3);
   hg::BatchRank r{};
-  r.rows = ix->d.rows;
-  r.ids = ix->d.ids;
+  r.rows = d.rows;
+  r.ids = d.ids;
   r.Q = b.qin;
   r.L = (int)L;
   r.nq = (int)nq;
@@ -2046,115 +2025,121 @@ static hg_status enqueue_batch(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_
   r.bucket = b.bucket;
   r.bucket_cnt = b.bucket_cnt;
   r.bucket_cap = bucket_cap;
+  r.pairs_cnt = c->heads + 1;
+  r.pairs_cap = b.pairs_cap;
   r.dist_out = b.out_dist;
   r.id_out = b.out_id;
   r.ok_out = b.ok;
-  r.stats = b.stats;
+  r.stats = c->stats;
   r.seg_rows = b.seg_rows;
   r.seg_prefix = b.seg_prefix;
   r.qbound = b.qbound;
   r.parts = b.parts;
   r.part_cnt = b.part_cnt;
-  r.heads = b.heads + 2;
-  r.qlist = nullptr;
+  r.heads = c->heads + 2;
+  uint32_t* lists[2] = {b.qlist, b.qlist2};
+  const uint32_t* list = round == 0 ? nullptr : lists[(round - 1) & 1];
+  const uint32_t* n_dev = round == 0 ? nullptr : c->ctrl + 4 + round;
+  r.qlist = list;
   r.nlist = (int)nq;
-  r.nlist_dev = nullptr;
-  CK(hg::launch_bound_select(r, st));
-  *launches = 8;  // route, group (2), conversion, bound pass, bound selection
-  // 3a. the leaves each query must filter (LB_EAPCA within B_q), each leaf's
-  // queries laid out contiguously in a BF16 panel, and the work items
-  const hg::DeviceIndex& d = ix->d;
+  r.nlist_dev = n_dev;
   // the narrowest work item: a resident query tile (L <= 256) is loaded once
   // per item, so an item has at least four row tiles; a streamed one is read
   // for every two row tiles whatever the item's length
   const uint32_t tpi_min = L <= 256 ? 4 : 2;
-  if (prune) {
-    CK(cudaMemsetAsync(b.leaf_cnt, 0, sizeof(uint32_t) * nl, st));
-    CK(cudaMemsetAsync(b.ppairs, 0, sizeof(unsigned long long), st));
-    CK(hg::launch_leaf_keep(b.qin, (int)L, (int)nq, b.useg_start, b.useg_end, b.nu, b.segstats, d.leaf_seg_off,
-                            d.leaf_points, b.seg_uid, d.leaf_sk, d.leaf_size, nl, b.bound, b.leaf_cnt, b.leaf_q,
-                            b.prune_nq, st));
-    ++*launches;
-    CK(hg::launch_group_pruned(b.leaf_cnt, b.leaf_q, b.prune_nq, b.leaf_plan, nl, ix->tune.filter_tiles_per_item,
-                               tpi_min, b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, b.pctl, b.ppairs,
-                               b.panel_list, b.items3, st));
-    CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, nullptr, st, b.pctl + 1));
-    *launches += 4;
+  uint32_t* pctl = round == 0 ? c->pctl : c->pctl + 8;
+  if (round == 0) {
+    CK(cudaMemsetAsync(c, 0, sizeof *c, st));
+    CK(cudaMemsetAsync(b.bm, 0xff, sizeof(unsigned long long) * nq * b.plan_bm_cap, st));
+    // 1. approximate leaves, grouping
+    CK(hg::launch_route_queries(b.qin, (int)nq, (int)L, index_tree(ix), b.approx, st, b.bucket_cnt, nq,
+                                prune ? b.leaf_cnt : nullptr, prune ? (uint32_t)nl : 0u, c->stamps + 0));
+    CK(hg::launch_group_queries(b.approx, (int)nq, b.leaf_plan, nl, ix->tune.bound_tiles_per_item, b.qperm, b.slots,
+                                b.leaf_qoff, b.leaf_qcnt, b.item_off, c->ctrl + 0, b.items, st, b.group_cnt));
+    CK(hg::launch_rows_to_bf16(b.qin, b.qperm, nq, (int)L, b.qbf, b.qmeta, st));
+    // 2. bound pass
+    g.qperm = b.qperm;
+    g.mode = 0;
+    g.qtile = hg::kBatchQueryTile;
+    g.items = b.items;
+    g.nitems = b.items_cap;
+    g.nitems_dev = c->ctrl + 0;
+    g.queue = c->queues + 0;
+    CK(hg::launch_umma_filter(ix->bd.rows_map, qmaps, g, sms, st));
+    CK(hg::launch_bound_select(r, st));
+    n_launch += 6;  // route, group (2), conversion, bound pass, bound selection
+    // 3a. the leaves each query must filter (LB_EAPCA within B_q)
+    if (prune) {
+      CK(hg::launch_leaf_keep(b.qin, (int)L, (int)nq, b.useg_start, b.useg_end, b.nu, b.segstats, d.leaf_seg_off,
+                              d.leaf_points, b.seg_uid, d.leaf_sk, d.leaf_size, nl, b.bound, b.leaf_cnt, b.leaf_q,
+                              b.prune_nq, st));
+      n_launch += 2;
+    }
+  } else {
+    CK(cudaMemsetAsync(b.bucket_cnt, 0, sizeof(uint32_t) * nq, st));
+    CK(cudaMemsetAsync(c->heads + 1, 0, sizeof(uint32_t), st));
+    CK(hg::launch_rows_to_bf16(b.qin, list, nq, (int)L, b.qbf, b.qmeta, st, n_dev));
+    ++n_launch;
+    // a retry round prunes leaves again for its queries, against the bounds
+    // the previous round lowered (a subset of the leaves kept before)
+    if (prune) {
+      CK(cudaMemsetAsync(b.leaf_cnt, 0, sizeof(uint32_t) * nl, st));
+      CK(hg::launch_leaf_keep_list(b.segstats, b.nu, (int)L, (int)nq, d.leaf_seg_off, d.leaf_points, b.seg_uid,
+                                   d.leaf_sk, d.leaf_size, nl, b.bound, b.leaf_cnt, b.leaf_q, b.prune_nq, list, n_dev,
+                                   st));
+      ++n_launch;
+    }
   }
-  CK(stamp(1));
-  // 3-5. certified filter, exact re-rank, verification; queries whose bucket
+  // 3b. each leaf's queries laid out contiguously in a BF16 panel, and the
+  // work items
+  if (prune) {
+    CK(hg::launch_group_pruned(b.leaf_cnt, b.leaf_q, b.prune_nq, b.leaf_plan, nl, ix->tune.filter_tiles_per_item,
+                               tpi_min, b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, pctl,
+                               c->pairs + (round == 0 ? 0 : 1), b.panel_list, b.items3, st, n_dev));
+    CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, nullptr, st, pctl + 1));
+    n_launch += 3;
+  }
+  // 3c-5. certified filter, exact re-rank, verification; queries whose bucket
   // overflowed are retried with the bound their first survivors gave.  The
   // screening passes run on CTA pairs (cta_group::2) where the query tile
   // stays resident (L <= 256) unless the tuning asks for one CTA per tile.
   const bool pair = ix->tune.filter_cta_pair != 2 && L <= 256;  // four resident 64-column K blocks
   auto screen = [&](const hg::QueryMaps& q) {
+    ++n_launch;
     return pair ? hg::launch_umma_pair(ix->bd.rows_map, q.q128, g, sms, st)
                 : hg::launch_umma_filter(ix->bd.rows_map, q, g, sms, st);
   };
-  uint32_t* lists[2] = {b.qlist, b.qlist2};
-  for (int round = 0; round <= kBatchRetries; ++round) {
-    const uint32_t* list_in = round == 0 ? nullptr : lists[(round - 1) & 1];
-    const uint32_t* n_dev = round == 0 ? nullptr : b.ctrl + 4 + round;
-    if (round > 0) {
-      CK(hg::launch_rows_to_bf16(b.qin, list_in, nq, (int)L, b.qbf, b.qmeta, st, n_dev));
-      ++*launches;
-    }
-    // a retry round prunes leaves again for its queries, against the bounds
-    // the previous round lowered (a subset of the leaves kept before)
-    uint32_t* ctl = round == 0 ? b.pctl : b.pctl + 8;
-    if (round > 0 && prune) {
-      CK(cudaMemsetAsync(b.leaf_cnt, 0, sizeof(uint32_t) * nl, st));
-      CK(hg::launch_leaf_keep_list(b.segstats, b.nu, (int)L, (int)nq, d.leaf_seg_off, d.leaf_points, b.seg_uid,
-                                   d.leaf_sk, d.leaf_size, nl, b.bound, b.leaf_cnt, b.leaf_q, b.prune_nq, list_in,
-                                   n_dev, st));
-      CK(hg::launch_group_pruned(b.leaf_cnt, b.leaf_q, b.prune_nq, b.leaf_plan, nl, ix->tune.filter_tiles_per_item,
-                                 tpi_min, b.panel_cap, b.items3_cap, nq, b.leaf_poff, b.leaf_ioff, ctl, b.ppairs + 1,
-                                 b.panel_list, b.items3, st, n_dev));
-      CK(hg::launch_rows_to_bf16(b.qin, b.panel_list, b.panel_cap, (int)L, b.panel_bf, nullptr, st, ctl + 1));
-      *launches += 4;
-    }
-    g.errstat = round == 0 ? b.errstat : nullptr;
-    if (round == 0) CK(cudaMemsetAsync(b.errstat, 0, 5 * sizeof(double), st));
-    CK(cudaMemsetAsync(b.bucket_cnt, 0, sizeof(uint32_t) * nq, st));
-    CK(cudaMemsetAsync(b.heads + 1, 0, sizeof(uint32_t), st));
-    CK(stamp(2 + 3 * round));
-    if (prune) {
-      // the kept (leaf, query) pairs; the dense pass below runs only when
-      // the panel overflowed (its query count is then the round's, else 0)
-      g.mode = 3;
-      g.items = b.items3;
-      g.nitems = b.items3_cap;
-      g.nitems_dev = ctl + 0;
-      g.qperm = b.panel_list;
-      g.nq_dev = nullptr;
-      g.qtile = hg::kBatchQueryTile;
-      g.queue = round == 0 ? b.queues + 1 : b.queues + 5 + round;
-      CK(screen(b.panel_maps));
-      ++*launches;
-    }
-    g.mode = 1;
-    g.qperm = round == 0 ? b.qperm : list_in;
-    g.nq_dev = prune ? ctl + 2 : n_dev;
-    g.qtile = round == 0 ? hg::kBatchQueryTile : 0;
-    g.queue = b.queues + 2 + round;
-    CK(screen(qmaps));
-    CK(stamp(3 + 3 * round));
-    CK(hg::launch_scatter_pairs(b.pairs, b.heads + 1, b.pairs_cap, list_in, (int)nq, n_dev, b.bucket, b.bucket_cnt,
-                                bucket_cap, st));
-    r.qlist = list_in;
-    r.nlist = (int)nq;
-    r.nlist_dev = n_dev;
-    CK(hg::launch_rerank(r, sms * (int)ix->tune.rerank_blocks_per_sm, st));
-    CK(stamp(4 + 3 * round));
-    *launches += 9;  // filter, scatter, overflow mark, re-rank plan / segments / merge
-    if (round < kBatchRetries) {
-      CK(hg::launch_collect_retry(b.ok, list_in, nq, n_dev, lists[round & 1], b.ctrl + 4 + round + 1, st));
-      ++*launches;
-    }
+  g.errstat = round == 0 ? c->errstat : nullptr;
+  g.stamp = c->stamps + 2 + 3 * round;
+  if (prune) {
+    g.mode = 3;
+    g.items = b.items3;
+    g.nitems = b.items3_cap;
+    g.nitems_dev = pctl + 0;
+    g.qperm = b.panel_list;
+    g.nq_dev = nullptr;
+    g.qtile = hg::kBatchQueryTile;
+    g.queue = round == 0 ? c->queues + 1 : c->queues + 5 + round;
+    CK(screen(b.panel_maps));
+    g.stamp = nullptr;
   }
-  CK(hg::launch_count_unverified(b.ok, nq, b.ctrl + 3, st));
-  CK(stamp(15));
-  *launches += 2;
+  // every row against every query: without pruning, and behind it where the
+  // panel may overflow (its query count is then the round's, else 0)
+  if (!prune || (uint64_t)b.panel_cap < (uint64_t)nl * nq) {
+    g.mode = 1;
+    g.qperm = round == 0 ? b.qperm : list;
+    g.nq_dev = prune ? pctl + 2 : n_dev;
+    g.qtile = round == 0 ? hg::kBatchQueryTile : 0;
+    g.queue = c->queues + 2 + round;
+    CK(screen(qmaps));
+  }
+  CK(hg::launch_scatter_pairs(b.pairs, c->heads + 1, b.pairs_cap, b.bucket, b.bucket_cnt, bucket_cap,
+                              c->stamps + 3 + 3 * round, st));
+  CK(hg::launch_rerank(r, sms * (int)ix->tune.rerank_blocks_per_sm, st));
+  CK(hg::launch_collect_retry(b.ok, list, nq, n_dev, lists[round & 1], c->ctrl + 4 + round + 1, c->ctrl + 3,
+                              c->stamps + 4 + 3 * round, st));
+  n_launch += 5;  // scatter, re-rank plan / segments / merge, collection
+  *launches = n_launch;
   return HG_OK;
 }
 
@@ -2274,12 +2259,6 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
                  ((b.plan_max_use + btpi - 1) / btpi)) +
       hg::kBatchItemTarget + nq;
   HCK(ensure_batch_scratch(ix, std::max(nq, b.nq_cap), bucket_cap, b.plan_bm_cap, items_cap, kmax));
-  if (!b.ctrl) {
-    CK(dalloc(&b.ctrl, 16));
-    CK(dalloc(&b.stamps, 16));
-    CK(dalloc(&b.errstat, 5));
-    CK(dalloc(&b.queues, 12));
-  }
   if (!b.qlist2 || !b.qin || b.out_kmax < kmax) {
     dfree(b.qlist2);
     dfree(b.qin);
@@ -2296,52 +2275,47 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   CK(cudaMemcpyAsync(b.qin, d_Q, sizeof(float) * nq * L,
                      host_io ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
   CK(cudaMemcpyAsync(b.kq, kq.data(), sizeof(uint32_t) * nq, cudaMemcpyHostToDevice, st));
-  hg::QueryMaps qmaps;
-  HCK(encode_query_maps(&qmaps, b.qbf, nq, L));
-  // the pipeline, captured once per shape in a CUDA graph and replayed
+  // the rounds, each captured once per shape in a CUDA graph and replayed
   bool prune = false;
   if (!o.dense_filter) HCK(ensure_prune_scratch(ix, &prune));
   const uint64_t key[8] = {nq, kmax, bucket_cap, b.gen, ix->tune.filter_tiles_per_item, ix->tune.bound_tiles_per_item,
                            ix->tune.rerank_blocks_per_sm, (prune ? 2u : 1u) | (ix->tune.filter_cta_pair << 4)};
-  uint64_t launches = 0;
-  if (!b.graph || memcmp(key, b.graph_key, sizeof key) != 0) {
-    if (b.graph) {
-      cudaGraphExecDestroy(b.graph);
-      b.graph = nullptr;
-    }
-    cudaGraph_t graph = nullptr;
-    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-    const hg_status s = enqueue_batch(ix, nq, kmax, bucket_cap, qmaps, prune, st, &launches);
-    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-    if (s != HG_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return s;
-    }
-    CK(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&b.graph, graph, 0);
-    cudaGraphDestroy(graph);
-    CK(ie);
+  if (memcmp(key, b.graph_key, sizeof key) != 0) {
+    drop_graphs(b);
     memcpy(b.graph_key, key, sizeof key);
-    b.graph_launches = launches;
   }
-  launches = b.graph_launches;
-  CK(cudaGraphLaunch(b.graph, st));
-  unsigned long long hs[8], ts[16];
-  uint32_t ctrl[16];
-  uint32_t dev_err = 0;
-  double es[5];
-  uint32_t pc[4] = {0, 0, 0, 0};
-  unsigned long long pp = 0;
-  if (prune) {
-    CK(cudaMemcpyAsync(pc, b.pctl, sizeof pc, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&pp, b.ppairs, sizeof pp, cudaMemcpyDeviceToHost, st));
+  uint64_t launches = 0;
+  hg::BatchCtl hc;
+  int round = 0;
+  for (;; ++round) {
+    if (!b.graph[round]) {
+      hg::QueryMaps qmaps;
+      HCK(encode_query_maps(&qmaps, b.qbf, nq, L));
+      cudaGraph_t graph = nullptr;
+      CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
+      const hg_status s = enqueue_round(ix, round, nq, kmax, bucket_cap, qmaps, prune, st, &b.graph_launches[round]);
+      const cudaError_t ce = cudaStreamEndCapture(st, &graph);
+      if (s != HG_OK) {
+        if (graph) cudaGraphDestroy(graph);
+        return s;
+      }
+      CK(ce);
+      const cudaError_t ie = cudaGraphInstantiate(&b.graph[round], graph, 0);
+      cudaGraphDestroy(graph);
+      if (ie != cudaSuccess) b.graph[round] = nullptr;
+      CK(ie);
+    }
+    launches += b.graph_launches[round];
+    CK(cudaGraphLaunch(b.graph[round], st));
+    CK(cudaMemcpyAsync(&hc, b.ctl, sizeof hc, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    // the queries left to retry, while rounds are left
+    if (hc.heads[3] || round == kBatchRetries || hc.ctrl[4 + round + 1] == 0) break;
   }
-  CK(cudaMemcpyAsync(ts, b.stamps, sizeof ts, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(es, b.errstat, sizeof es, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(hs, b.stats, sizeof hs, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(ctrl, b.ctrl, sizeof ctrl, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&dev_err, b.heads + 3, sizeof dev_err, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  const uint32_t dev_err = hc.heads[3], *ctrl = hc.ctrl, *pc = hc.pctl;
+  const unsigned long long *hs = hc.stats, *ts = hc.stamps;
+  const double* es = hc.errstat;
+  const uint32_t unverified = ctrl[3] + ctrl[4 + round + 1];
   if (dev_err) return set_error(HG_ERR_TIMEOUT, "hg_knn_batch: a tensor-core filter wait timed out");
   // queries that did not verify: the plain path
   cudaEvent_t fb0 = nullptr, fb1 = nullptr;
@@ -2350,7 +2324,7 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   CK(cudaEventRecord(fb0, st));
   uint64_t fallbacks = 0, fallback_launches = 0;
   hg_status fs = HG_OK;
-  if (ctrl[3] > 0) {
+  if (unverified > 0) {
     std::vector<int> ok(nq);
     CK(cudaMemcpy(ok.data(), b.ok, sizeof(int) * nq, cudaMemcpyDeviceToHost));
     hg_knn_opts po{};
@@ -2389,20 +2363,18 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
     float tf = 0;
     double gemm = 0, rerank = 0;
     uint64_t pairs = 0, retried = 0;
-    const double t01 = span(0, 1);
-    for (int round = 0; round <= kBatchRetries; ++round) {
-      const double tg = span(2 + 3 * round, 3 + 3 * round), tr = span(3 + 3 * round, 4 + 3 * round);
-      const uint64_t cnt = round == 0 ? nq : ctrl[4 + round];
-      if (round > 0) retried += cnt;
-      if (cnt == 0 && round > 0) continue;
-      gemm += tg;
-      rerank += tr;
+    const double t01 = span(0, 2);
+    for (int i = 0; i <= round; ++i) {
+      const uint64_t cnt = i == 0 ? nq : ctrl[4 + i];
+      if (i > 0) retried += cnt;
+      gemm += span(2 + 3 * i, 3 + 3 * i);
+      rerank += span(3 + 3 * i, 4 + 3 * i);
       // the first filter round with pruning: the kept pairs, plus every pair if the dense
       // pass ran instead
-      pairs += (round == 0 && prune) ? pp + (uint64_t)pc[2] * ix->n : cnt * ix->n;
+      pairs += (i == 0 && prune) ? hc.pairs[0] + (uint64_t)pc[2] * ix->n : cnt * ix->n;
     }
     cudaEventElapsedTime(&tf, fb0, fb1);
-    const double t0e = span(0, 15) + (fallbacks ? tf : 0.0);
+    const double t0e = span(0, 4 + 3 * round) + (fallbacks ? tf : 0.0);
     stats->queries = nq;
     stats->rows_visited = hs[0];
     stats->chunks_loaded = hs[1];

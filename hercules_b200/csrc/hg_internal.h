@@ -106,8 +106,6 @@ struct BatchScratch {
   unsigned long long* pairs = nullptr;  // filter survivors before they are bucketed
   uint32_t pairs_cap = 0;
   int* ok = nullptr;
-  unsigned long long* stats = nullptr;
-  uint32_t* heads = nullptr;
   uint32_t parts_kmax = 0;
   uint32_t* qlist = nullptr;  // queries of a retry round
   uint32_t* seg_rows = nullptr;
@@ -116,8 +114,8 @@ struct BatchScratch {
   unsigned long long* parts = nullptr;
   int* part_cnt = nullptr;
   // device-side control of a batch
+  BatchCtl* ctl = nullptr;
   uint32_t* qlist2 = nullptr;    // second retry list (rounds alternate)
-  uint32_t* ctrl = nullptr;      // [0] bound items [3] unverified queries [4 + r] queries of round r
   float* qin = nullptr;          // the batch's queries (fixed address for the graph)
   float* out_dist = nullptr;     // the batch's answers before they are copied out
   int64_t* out_id = nullptr;
@@ -131,13 +129,11 @@ struct BatchScratch {
   uint64_t plan_want = 0;
   uint32_t plan_bm_cap = 0, plan_max_use = 0;
   uint64_t gen = 0;              // bumped whenever a buffer above moves
-  // the captured batch pipeline and the key it was captured for
-  cudaGraphExec_t graph = nullptr;
+  // the captured pipelines (the first round, and each retry round once a
+  // batch needs it) and the key they were captured for
+  cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
   uint64_t graph_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  uint64_t graph_launches = 0;   // kernels in the captured pipeline
-  unsigned long long* stamps = nullptr;  // [16] global-timer stamps at the phase boundaries
-  double* errstat = nullptr;             // [5] certified bounds of the first filter pass (BatchGemm::errstat)
-  uint32_t* queues = nullptr;            // [8] work-item counters of the filter launches
+  uint64_t graph_launches[4] = {0, 0, 0, 0};  // kernels in each
   // pruned filter: the (leaf, query) pairs LB_EAPCA keeps, their query panel
   // (each leaf's queries contiguous, BF16) and work items
   uint32_t prune_nq = 0;                 // queries the buffers hold (0: not allocated)
@@ -149,8 +145,6 @@ struct BatchScratch {
   void* panel_bf = nullptr;              // [panel_cap][L] BF16
   BatchItem* items3 = nullptr;           // [items3_cap]
   uint32_t panel_cap = 0, items3_cap = 0;
-  uint32_t* pctl = nullptr;              // [4] items, panel rows, dense-pass queries
-  unsigned long long* ppairs = nullptr;  // (query, row) pairs of the pruned pass
   QueryMaps panel_maps;                  // TMA descriptors of panel_bf
   // distinct leaf segments (shared by many leaves) and the queries' mean and
   // stdev over each

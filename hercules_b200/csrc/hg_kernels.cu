@@ -432,8 +432,16 @@ __global__ void k_sax_rows(const float* __restrict__ rows, int L, uint64_t n, co
 // query kernels
 // ---------------------------------------------------------------------------
 
-__global__ void k_route_queries(const float* __restrict__ Q, int nq, int L, Tree t, int* __restrict__ leaf_out) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The approximate leaf of every query, a warp each; the threads also zero the
+// batch's counters zero_a and zero_b (the next kernels').
+__global__ void k_route_queries(const float* __restrict__ Q, int nq, int L, Tree t, int* __restrict__ leaf_out,
+                                uint32_t* zero_a, uint32_t na, uint32_t* zero_b, uint32_t nb,
+                                unsigned long long* stamp) {
+  stamp_start(stamp);
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  for (uint32_t i = tid; i < na; i += threads) zero_a[i] = 0;
+  for (uint32_t i = tid; i < nb; i += threads) zero_b[i] = 0;
+  const int w = (int)(tid >> 5);
   if (w >= nq) return;
   const int leaf = warp_route(Q + (uint64_t)w * L, t);
   if ((threadIdx.x & 31) == 0) leaf_out[w] = leaf;
@@ -1770,9 +1778,11 @@ cudaError_t launch_query_prep(const PrepArgs& a, int slots, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s) {
+cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s,
+                                 uint32_t* zero_a, uint32_t na, uint32_t* zero_b, uint32_t nb,
+                                 unsigned long long* stamp) {
   if (!nq) return cudaSuccess;
-  k_route_queries<<<blocks_for((uint64_t)nq * 32, 128), 128, 0, s>>>(Q, nq, L, t, leaf_out);
+  k_route_queries<<<blocks_for((uint64_t)nq * 32, 128), 128, 0, s>>>(Q, nq, L, t, leaf_out, zero_a, na, zero_b, nb, stamp);
   return cudaGetLastError();
 }
 

@@ -209,7 +209,9 @@ cudaError_t launch_sax_rows(const float* rows, int L, uint64_t n, const float* b
 
 // queries
 cudaError_t launch_query_prep(const PrepArgs& a, int slots, cudaStream_t s);
-cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s);
+cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* leaf_out, cudaStream_t s,
+                                 uint32_t* zero_a = nullptr, uint32_t na = 0, uint32_t* zero_b = nullptr,
+                                 uint32_t nb = 0, unsigned long long* stamp = nullptr);
 cudaError_t launch_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count, int slots, cudaStream_t s);
 // blocks: per slot
 cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cudaStream_t s);

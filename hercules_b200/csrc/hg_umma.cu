@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   float* s_qn2 = reinterpret_cast<float*>(sm + LY::kQn2);
   volatile int* s_okw = reinterpret_cast<volatile int*>(sm + LY::kOkw);
 
+  stamp_start(a.stamp);
   const uint64_t wns = a.wait_ns ? a.wait_ns : kWaitNs;  // every bounded wait gives up after this
   const int nkb = (a.L + kUK - 1) / kUK;
   constexpr bool resident = kResident;
