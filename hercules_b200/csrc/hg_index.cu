@@ -1345,8 +1345,17 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
       std::max(1, std::min(ed_blocks, o.approx_blocks > 0 ? o.approx_blocks : (int)ix->tune.approx_blocks_per_sm * sms));
   // a warp's entries: one row per slot of its lanes for a query alone; a
   // group keeps the GPU full by itself, so its warps take longer runs and
-  // fewer blocks stage a query and sort a list
-  e.min_batch = slots > 1 ? (ix->L >= 4096 ? 8u : 32u) : (ix->L >= 4096 ? 4u : 8u);
+  // fewer blocks stage a query and sort a list.  Long rows: by the rows the
+  // group's approximate leaves may hold against the GPU's 32 warps per SM
+  // (12 queries, leaf 1,562, L = 16384: 0.93 ms at 4 entries, 1.20 at 8; 20
+  // queries, leaf 2,000, L = 4096: 0.74 at 4, 0.67 at 8)
+  if (ix->L >= 4096) {
+    const uint64_t rows = (uint64_t)slots * std::min<uint64_t>(ix->leaf_size, ix->n), warps = 32ull * sms;
+    e.few_rows = slots == 1 && 2 * rows <= warps ? 1 : 0;
+    e.min_batch = e.few_rows ? 1u : (slots > 1 && rows >= 6 * warps ? 8u : 4u);
+  } else {
+    e.min_batch = slots > 1 ? 32u : 8u;
+  }
   e.ident_leaf = s.approx_leaf;
   HCK(scan(a_blocks));
   hg::SelectArgs sel{};

@@ -1895,9 +1895,16 @@ static cudaError_t launch_ed(K kernel, SmemLimit& attr, const EdArgs& args, int 
 // Groups over series of at most kEdShortL points: k_ed_short (longer rows of a
 // warp differ too much in where they abandon).  Long series (L >= 4096): few
 // candidate rows per query, each long, so more lanes per row keep more of each
-// row in flight.
+// row in flight -- all 32 where there are fewer rows than warps (one query over
+// a leaf of a thousand rows of 64 KB reads each row in 128 dependent steps with
+// 8 lanes: 528 us, 348 us with 32; with rows for every warp 8 lanes are faster,
+// PSCAN of 60k x 16384 619 us against 1,007).
 cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  static SmemLimit wide, lng, mid, shrt;
+  static SmemLimit wide, lng, mid, shrt, few_wide, few_lng;
+  if (a.few_rows) {
+    if (ed_wide(a.L)) return launch_ed(k_ed_stream<false, 1, 32, 32>, few_wide, a, 32, slots, blocks, s);
+    return launch_ed(k_ed_stream<false, 1, 32, kEdWarps>, few_lng, a, kEdWarps, slots, blocks, s);
+  }
   if (slots > 1 && a.L <= kEdShortL) return launch_ed(k_ed_short, shrt, a, kEdWarps, slots, blocks, s);
   if (ed_wide(a.L)) return launch_ed(k_ed_stream<false, 2, 8, 32>, wide, a, 32, slots, blocks, s);
   if (a.L >= 4096) return launch_ed(k_ed_stream<false, 2, 8, kEdWarps>, lng, a, kEdWarps, slots, blocks, s);

@@ -114,6 +114,7 @@ struct EdArgs {
   const uint64_t* leaf_start;
   const uint32_t* leaf_size;
   uint32_t min_batch;          // entries a warp takes at least, 1..32: with fewer in all, blocks stay idle
+  int few_rows;                // 1: one query, fewer rows than half the warps of the GPU: a warp per row
   const float* q;              // [slot][L]
   int k;
   uint32_t* bound;             // [slot] float bits of the running k-th bound (atomicMin)

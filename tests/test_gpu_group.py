@@ -40,6 +40,9 @@ def indexes(hg, oracle_mod, gpu_available):
     (40000, 64, 30000, 7, 224, False, 0),   # lists of 224 entries from hundreds of blocks
     (40000, 64, 30000, 1, 224, True, 0),
     (3000, 4096, 400, 33, 10, True, 0),     # 8 lanes per row
+    (3000, 4096, 400, 1, 10, True, 0),      # a warp per row
+    (600, 16384, 200, 1, 3, True, 0),       # the same, 32-warp blocks
+    (600, 16384, 200, 40, 3, False, 0),
 ])
 def test_grouped_queries_match_oracle(indexes, n, L, leaf, nq, k, lbsax, seed_leaves):
     X, Q, ix, oi = indexes(n, L, leaf)
