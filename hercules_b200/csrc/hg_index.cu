@@ -297,7 +297,7 @@ static void free_scratch(hg_index* ix) {
   dfree(s.sort_keys);
   dfree(s.list);
   dfree(s.stats);
-  dfree(s.err);
+  s.err = nullptr;  // in stats
   dfree(s.actl);
   s.slots = 0;
 }
@@ -316,6 +316,13 @@ static void free_device(hg_index* ix) {
   dfree(d.leaf_sk);
   dfree(d.nodes);
   free_scratch(ix);
+  dfree(ix->io.q);
+  dfree(ix->io.out);
+  ix->io = hg::HostIo{};
+  for (cudaEvent_t& e : ix->ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
   hg::BatchData& bd = ix->bd;
   dfree(bd.xbf);
   dfree(bd.xmeta);
@@ -1187,8 +1194,8 @@ static cudaError_t alloc_scratch(hg_index* ix, size_t slots) {
   get(&s.topk_count, slots);
   get(&s.sax_tab, slots * HG_PAA_SEGMENTS * HG_SAX_CARD);
   if (nl > (size_t)hg::kMaxLeavesSort) get(&s.sort_keys, slots * 4 * nl);
-  get(&s.stats, 8);
-  get(&s.err, 1);
+  get(&s.stats, 9);
+  s.err = reinterpret_cast<int*>(s.stats + 8);
   get(&s.actl, 4);
   if (e == cudaSuccess) s.slots = (int)slots;
   return e;
@@ -1632,9 +1639,26 @@ static hg_status knn_rounds(hg_index* ix, const float* d_q, uint32_t k, const hg
   return HG_OK;
 }
 
+constexpr size_t kHostIoKeep = 64u << 20;
+
+template <class T>
+static hg_status grow_io(T** p, size_t* cap, size_t bytes) {
+  if (*cap >= bytes && *p) return HG_OK;
+  dfree(*p);
+  *cap = 0;
+  unsigned char* b = nullptr;
+  CK(dalloc(&b, bytes));
+  *p = reinterpret_cast<T*>(b);
+  *cap = bytes;
+  return HG_OK;
+}
+
+// host_out: if set, host_bytes from device memory host_src (the answers) are
+// copied there with the call's counters, before its one synchronisation.
 static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t nq, uint32_t k,
                                  const hg_knn_opts* opts, float* d_dist, int64_t* d_id, cudaStream_t st,
-                                 hg_query_stats* stats) {
+                                 hg_query_stats* stats, void* host_out = nullptr, const void* host_src = nullptr,
+                                 size_t host_bytes = 0) {
   if (!ix || (!d_queries && nq)) return set_error(HG_ERR_ARG, "hg_knn: null argument");
   if (k == 0) return set_error(HG_ERR_ARG, "hg_knn: k must be positive");
   if (ix->L > 16384) return set_error(HG_ERR_LIMIT, "hg_knn: series longer than 16384");
@@ -1653,13 +1677,11 @@ static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t 
   const bool grouped = !approx && (int)k <= hg::kMaxK;
   HCK(ensure_scratch(ix, grouped ? group_slots(ix, nq) : 1));
   if (!st) st = ix->stream;
-  cudaEvent_t e0, e1;
-  CK(cudaEventCreate(&e0));
-  CK(cudaEventCreate(&e1));
-  CK(cudaMemsetAsync(ix->s.stats, 0, sizeof(unsigned long long) * 8, st));
-  CK(cudaMemsetAsync(ix->s.err, 0, sizeof(int), st));
+  for (cudaEvent_t& e : ix->ev)
+    if (!e) CK(cudaEventCreate(&e));
+  CK(cudaMemsetAsync(ix->s.stats, 0, sizeof(unsigned long long) * 9, st));
   Prof prof;
-  CK(cudaEventRecord(e0, st));
+  CK(cudaEventRecord(ix->ev[0], st));
   uint64_t launches = 0;
   const uint32_t per = grouped ? std::min<uint32_t>(group_slots(ix, nq), (uint32_t)ix->s.slots) : 1;
   for (uint32_t i = 0; i < nq; i += per) {
@@ -1671,16 +1693,14 @@ static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t 
     else if (grouped) HCK(knn_group(ix, qi, (int)std::min(per, nq - i), (int)k, o, di, ii, st, pr, &launches));
     else HCK(knn_rounds(ix, qi, k, o, di, ii, st, pr, &launches));
   }
-  CK(cudaEventRecord(e1, st));
-  unsigned long long hs[8];
-  int ferr = 0;
+  CK(cudaEventRecord(ix->ev[1], st));
+  unsigned long long hs[9];  // counters, error flag
   CK(cudaMemcpyAsync(hs, ix->s.stats, sizeof hs, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&ferr, ix->s.err, sizeof ferr, cudaMemcpyDeviceToHost, st));
+  if (host_out) CK(cudaMemcpyAsync(host_out, host_src, host_bytes, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  const int ferr = (int)(uint32_t)hs[8];
   float ms = 0;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  if (stats) cudaEventElapsedTime(&ms, ix->ev[0], ix->ev[1]);
   if (ferr) return set_error(HG_ERR_TIMEOUT, "hg_knn: an LB_SAX filter wait timed out");
   const size_t ed_launches = prof.ed.size(), filter_launches = prof.filter.size();
   const double scan_ms = drain(prof.ed);
@@ -2296,6 +2316,12 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   uint64_t launches = 0;
   hg::BatchCtl hc;
   int round = 0;
+  auto copy_answers = [&]() -> hg_status {
+    const cudaMemcpyKind kind = host_io ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
+    if (d_dist) CK(cudaMemcpyAsync(d_dist, b.out_dist, sizeof(float) * nq * kmax, kind, st));
+    if (d_id) CK(cudaMemcpyAsync(d_id, b.out_id, sizeof(int64_t) * nq * kmax, kind, st));
+    return HG_OK;
+  };
   for (;; ++round) {
     if (!b.graph[round]) {
       hg::QueryMaps qmaps;
@@ -2316,6 +2342,9 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
     }
     launches += b.graph_launches[round];
     CK(cudaGraphLaunch(b.graph[round], st));
+    // the answers with the counters, before the round's one synchronisation:
+    // nearly always they are final
+    HCK(copy_answers());
     CK(cudaMemcpyAsync(&hc, b.ctl, sizeof hc, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     // the queries left to retry, while rounds are left
@@ -2327,49 +2356,35 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   const uint32_t unverified = ctrl[3] + ctrl[4 + round + 1];
   if (dev_err) return set_error(HG_ERR_TIMEOUT, "hg_knn_batch: a tensor-core filter wait timed out");
   // queries that did not verify: the plain path
-  cudaEvent_t fb0 = nullptr, fb1 = nullptr;
-  CK(cudaEventCreate(&fb0));
-  CK(cudaEventCreate(&fb1));
-  CK(cudaEventRecord(fb0, st));
   uint64_t fallbacks = 0, fallback_launches = 0;
-  hg_status fs = HG_OK;
+  float tf = 0;
   if (unverified > 0) {
+    for (cudaEvent_t& e : ix->ev)
+      if (!e) CK(cudaEventCreate(&e));
     std::vector<int> ok(nq);
-    CK(cudaMemcpy(ok.data(), b.ok, sizeof(int) * nq, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(ok.data(), b.ok, sizeof(int) * nq, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     hg_knn_opts po{};
     po.mode = HG_MODE_PLAIN;
     po.use_lb_sax = 1;
     CK(cudaMemsetAsync(ix->s.err, 0, sizeof(int), st));
-    for (uint32_t q = 0; q < nq && fs == HG_OK; ++q) {
+    CK(cudaEventRecord(ix->ev[0], st));
+    for (uint32_t q = 0; q < nq; ++q) {
       if (ok[q] == 1) continue;
       ++fallbacks;
-      fs = knn_group(ix, b.qin + (uint64_t)q * L, 1, (int)kq[q], po, b.out_dist + (uint64_t)q * kmax,
-                     b.out_id + (uint64_t)q * kmax, st, nullptr, &fallback_launches);
+      HCK(knn_group(ix, b.qin + (uint64_t)q * L, 1, (int)kq[q], po, b.out_dist + (uint64_t)q * kmax,
+                    b.out_id + (uint64_t)q * kmax, st, nullptr, &fallback_launches));
     }
-  }
-  cudaEventRecord(fb1, st);
-  if (fs == HG_OK) {
-    const cudaMemcpyKind kind = host_io ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    cudaError_t ce = cudaSuccess;
-    if (d_dist) ce = cudaMemcpyAsync(d_dist, b.out_dist, sizeof(float) * nq * kmax, kind, st);
-    if (ce == cudaSuccess && d_id) ce = cudaMemcpyAsync(d_id, b.out_id, sizeof(int64_t) * nq * kmax, kind, st);
-    if (ce != cudaSuccess) fs = cuda_fail(ce, "hg_knn_batch");
-  }
-  int ferr = 0;
-  if (fallbacks && fs == HG_OK) {
-    const cudaError_t ce = cudaMemcpyAsync(&ferr, ix->s.err, sizeof ferr, cudaMemcpyDeviceToHost, st);
-    if (ce != cudaSuccess) fs = cuda_fail(ce, "hg_knn_batch");
-  }
-  cudaStreamSynchronize(st);
-  if (fs == HG_OK && ferr) fs = set_error(HG_ERR_TIMEOUT, "hg_knn_batch: an LB_SAX filter wait timed out");
-  if (fs != HG_OK) {
-    cudaEventDestroy(fb0);
-    cudaEventDestroy(fb1);
-    return fs;
+    CK(cudaEventRecord(ix->ev[1], st));
+    HCK(copy_answers());
+    int ferr = 0;
+    CK(cudaMemcpyAsync(&ferr, ix->s.err, sizeof ferr, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (ferr) return set_error(HG_ERR_TIMEOUT, "hg_knn_batch: an LB_SAX filter wait timed out");
+    cudaEventElapsedTime(&tf, ix->ev[0], ix->ev[1]);
   }
   if (stats) {
     auto span = [&](int i, int j) { return (double)(ts[j] - ts[i]) * 1e-6; };  // ms
-    float tf = 0;
     double gemm = 0, rerank = 0;
     uint64_t pairs = 0, retried = 0;
     const double t01 = span(0, 2);
@@ -2382,7 +2397,6 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
       // pass ran instead
       pairs += (i == 0 && prune) ? hc.pairs[0] + (uint64_t)pc[2] * ix->n : cnt * ix->n;
     }
-    cudaEventElapsedTime(&tf, fb0, fb1);
     const double t0e = span(0, 4 + 3 * round) + (fallbacks ? tf : 0.0);
     stats->queries = nq;
     stats->rows_visited = hs[0];
@@ -2405,8 +2419,6 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
     stats->leaf_pairs = prune ? (uint64_t)nq * nonempty : 0;
     stats->leaf_pairs_kept = prune ? pc[3] : 0;
   }
-  cudaEventDestroy(fb0);
-  cudaEventDestroy(fb1);
   return HG_OK;
 }
 
@@ -2545,28 +2557,36 @@ hg_status hg_knn(hg_index* ix, const float* queries, uint32_t nq, uint32_t k, co
   if (!ix || (!queries && nq)) return set_error(HG_ERR_ARG, "hg_knn: null argument");
   if (nq == 0) return HG_OK;
   CK(cudaSetDevice(ix->device));
-  float* d_q = nullptr;
-  float* d_dist = nullptr;
-  int64_t* d_id = nullptr;
-  CK(dalloc(&d_q, (size_t)nq * ix->L));
-  cudaError_t e = dalloc(&d_dist, (size_t)nq * k);
-  if (e == cudaSuccess) e = dalloc(&d_id, (size_t)nq * k);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_q, queries, sizeof(float) * nq * ix->L, cudaMemcpyHostToDevice, ix->stream);
+  const size_t nk = (size_t)nq * k, q_bytes = sizeof(float) * nq * ix->L, id_bytes = sizeof(int64_t) * nk;
+  const size_t out_bytes = id_bytes + sizeof(float) * nk;
+  hg::HostIo& io = ix->io;
+  HCK(grow_io(&io.q, &io.q_cap, q_bytes));
+  HCK(grow_io(&io.out, &io.out_cap, out_bytes));
+  // ids and distances side by side: one copy back
+  int64_t* d_id = reinterpret_cast<int64_t*>(io.out);
+  float* d_dist = reinterpret_cast<float*>(io.out + id_bytes);
+  std::vector<int64_t> ids(nk + (nk + 1) / 2);
+  const cudaError_t e = cudaMemcpyAsync(io.q, queries, q_bytes, cudaMemcpyHostToDevice, ix->stream);
   hg_status s = e == cudaSuccess ? HG_OK : cuda_fail(e, "hg_knn");
-  if (s == HG_OK) s = knn_device_impl(ix, d_q, nq, k, opts, d_dist, d_id, ix->stream, stats);
-  std::vector<int64_t> ids((size_t)nq * k);
-  if (s == HG_OK) {
-    e = cudaMemcpyAsync(ids.data(), d_id, sizeof(int64_t) * nq * k, cudaMemcpyDeviceToHost, ix->stream);
-    if (e == cudaSuccess && dist_out)
-      e = cudaMemcpyAsync(dist_out, d_dist, sizeof(float) * nq * k, cudaMemcpyDeviceToHost, ix->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ix->stream);
-    if (e != cudaSuccess) s = cuda_fail(e, "hg_knn");
+  const bool batch = opts && opts->mode == HG_MODE_BATCH;
+  if (s == HG_OK)
+    s = knn_device_impl(ix, io.q, nq, k, opts, d_dist, d_id, ix->stream, stats, batch ? nullptr : ids.data(), io.out,
+                        out_bytes);
+  if (s == HG_OK && batch) {
+    cudaError_t ce = cudaMemcpyAsync(ids.data(), io.out, out_bytes, cudaMemcpyDeviceToHost, ix->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(ix->stream);
+    if (ce != cudaSuccess) s = cuda_fail(ce, "hg_knn");
   }
-  cudaFree(d_q);
-  cudaFree(d_dist);
-  cudaFree(d_id);
+  if (io.q_cap > kHostIoKeep) {
+    dfree(io.q);
+    io.q_cap = 0;
+  }
+  if (io.out_cap > kHostIoKeep) {
+    dfree(io.out);
+    io.out_cap = 0;
+  }
   if (s != HG_OK) return s;
+  if (dist_out) memcpy(dist_out, ids.data() + nk, sizeof(float) * nk);
   if (id_out) memcpy(id_out, ids.data(), sizeof(int64_t) * nq * k);
   if (leaf_pos_out) {
     // answer id -> leaf-ordered row -> its leaf's file_pos

@@ -72,9 +72,10 @@ struct QueryScratch {
   float* sax_tab = nullptr;       // 16 x 256 LB_SAX terms of the query
   uint32_t* sort_keys = nullptr;  // 4 x leaves: candidate sort above kMaxLeavesSort leaves
   uint32_t* list = nullptr;       // LB_SAX survivors (rows), n entries
-  // shared by the slots
-  unsigned long long* stats = nullptr;  // counters of the call (knn_device_impl)
-  int* err = nullptr;             // device error flag
+  // shared by the slots, one block: counters of the call (knn_device_impl),
+  // then the device error flag
+  unsigned long long* stats = nullptr;
+  int* err = nullptr;             // stats + 8
   uint32_t* actl = nullptr;       // approximate searches: [0] stale k-th bound bits, [1] gate flag
 };
 
@@ -155,6 +156,15 @@ struct BatchScratch {
   float2* segstats = nullptr;            // [prune_nq][nu]
 };
 
+// Device copies of a host call's queries and answers, kept with the handle and
+// grown to the largest call (at most kHostIoKeep bytes outlive a call).
+struct HostIo {
+  float* q = nullptr;
+  size_t q_cap = 0;
+  unsigned char* out = nullptr;  // ids, then distances
+  size_t out_cap = 0;
+};
+
 }  // namespace hg
 
 struct hg_index {
@@ -169,6 +179,8 @@ struct hg_index {
   bool has_ids = false;         // false for an index built by the reference
   hg::DeviceIndex d;
   hg::QueryScratch s;
+  hg::HostIo io;
+  cudaEvent_t ev[2] = {nullptr, nullptr};  // around the device work of a call
   hg::BatchData bd;
   hg::BatchScratch bs;
   cudaStream_t stream = nullptr;
