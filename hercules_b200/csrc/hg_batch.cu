@@ -578,9 +578,51 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_merge(BatchRank a) {
   }
 }
 
-// Survivor pairs into their queries' buckets, 32 pairs per warp step: lanes
-// holding the same query share one atomic (pairs of a query cluster, since
-// the filter emits them tile by tile); empty slots (~0) are skipped.
+// Survivor pairs into their queries' buckets; empty slots (~0) are skipped.
+// Up to kScatterQueries queries: a block takes kScatterPairs pairs, ranks each
+// among the block's pairs of its query with a counter in shared memory and
+// reserves room with one global atomic per query.
+constexpr int kScatterThreads = 512, kScatterPer = 8, kScatterQueries = 8192;
+constexpr uint32_t kScatterPairs = kScatterThreads * kScatterPer;
+__global__ void __launch_bounds__(kScatterThreads) k_scatter_blocks(const unsigned long long* __restrict__ pairs,
+                                                                    const uint32_t* pairs_cnt, uint32_t pairs_cap,
+                                                                    uint32_t* __restrict__ bucket, uint32_t* bucket_cnt,
+                                                                    uint32_t bucket_cap, uint32_t nq,
+                                                                    unsigned long long* stamp) {
+  stamp_start(stamp);
+  extern __shared__ uint32_t s_cnt[];  // [nq] pairs of each query in the block, then its first position
+  const uint32_t n = min(*pairs_cnt, pairs_cap);
+  for (uint64_t base = (uint64_t)blockIdx.x * kScatterPairs; base < n; base += (uint64_t)gridDim.x * kScatterPairs) {
+    for (uint32_t q = threadIdx.x; q < nq; q += kScatterThreads) s_cnt[q] = 0;
+    __syncthreads();
+    unsigned long long e[kScatterPer];
+    uint32_t rank[kScatterPer];
+#pragma unroll
+    for (int i = 0; i < kScatterPer; ++i) {
+      const uint64_t p = base + i * kScatterThreads + threadIdx.x;
+      e[i] = p < n ? pairs[p] : ~0ull;
+    }
+#pragma unroll
+    for (int i = 0; i < kScatterPer; ++i)
+      if (e[i] != ~0ull) rank[i] = atomicAdd(&s_cnt[(uint32_t)(e[i] >> 32)], 1u);
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < nq; q += kScatterThreads) {
+      const uint32_t c = s_cnt[q];
+      if (c) s_cnt[q] = atomicAdd(&bucket_cnt[q], c);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kScatterPer; ++i)
+      if (e[i] != ~0ull) {
+        const uint32_t q = (uint32_t)(e[i] >> 32), pos = s_cnt[q] + rank[i];
+        if (pos < bucket_cap) bucket[(uint64_t)q * bucket_cap + pos] = (uint32_t)e[i];
+      }
+    __syncthreads();
+  }
+}
+
+// More queries: 32 pairs per warp step, lanes holding the same query share one
+// atomic (pairs of a query cluster, since the filter emits them tile by tile).
 __global__ void k_scatter_pairs(const unsigned long long* __restrict__ pairs, const uint32_t* pairs_cnt,
                                 uint32_t pairs_cap, uint32_t* __restrict__ bucket, uint32_t* bucket_cnt,
                                 uint32_t bucket_cap, unsigned long long* stamp) {
@@ -890,7 +932,12 @@ cudaError_t launch_tile_norms(const float4* meta, uint64_t n, float4* tile_meta,
 
 cudaError_t launch_scatter_pairs(const unsigned long long* pairs, const uint32_t* pairs_cnt, uint32_t pairs_cap,
                                  uint32_t* bucket, uint32_t* bucket_cnt, uint32_t bucket_cap,
-                                 unsigned long long* stamp, cudaStream_t s) {
+                                 uint32_t nq, unsigned long long* stamp, cudaStream_t s) {
+  if (nq <= (uint32_t)kScatterQueries) {
+    k_scatter_blocks<<<4 * 148, kScatterThreads, sizeof(uint32_t) * nq, s>>>(pairs, pairs_cnt, pairs_cap, bucket,
+                                                                            bucket_cnt, bucket_cap, nq, stamp);
+    return cudaGetLastError();
+  }
   // grid-stride, enough threads in flight to hide the bucket atomics' latency
   k_scatter_pairs<<<2048, 256, 0, s>>>(pairs, pairs_cnt, pairs_cap, bucket, bucket_cnt, bucket_cap, stamp);
   return cudaGetLastError();

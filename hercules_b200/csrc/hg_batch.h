@@ -175,7 +175,7 @@ cudaError_t launch_rerank(const BatchRank& r, int part_blocks, cudaStream_t s);
 // Distributes the filter's survivor pairs into per-query buckets
 // (bucket_cnt[q] counts every pair of q, also beyond bucket_cap).
 cudaError_t launch_scatter_pairs(const unsigned long long* pairs, const uint32_t* pairs_cnt, uint32_t pairs_cap,
-                                 uint32_t* bucket, uint32_t* bucket_cnt, uint32_t bucket_cap,
+                                 uint32_t* bucket, uint32_t* bucket_cnt, uint32_t bucket_cap, uint32_t nq,
                                  unsigned long long* stamp, cudaStream_t s);
 
 }  // namespace hg

@@ -2162,7 +2162,7 @@ static hg_status enqueue_round(hg_index* ix, int round, uint32_t nq, uint32_t km
     g.queue = c->queues + 2 + round;
     CK(screen(qmaps));
   }
-  CK(hg::launch_scatter_pairs(b.pairs, c->heads + 1, b.pairs_cap, b.bucket, b.bucket_cnt, bucket_cap,
+  CK(hg::launch_scatter_pairs(b.pairs, c->heads + 1, b.pairs_cap, b.bucket, b.bucket_cnt, bucket_cap, nq,
                               c->stamps + 3 + 3 * round, st));
   CK(hg::launch_rerank(r, sms * (int)ix->tune.rerank_blocks_per_sm, st));
   CK(hg::launch_collect_retry(b.ok, list, nq, n_dev, lists[round & 1], c->ctrl + 4 + round + 1, c->ctrl + 3,

@@ -252,6 +252,41 @@ __device__ __forceinline__ uint32_t screen32(const float* v, float h, int nv) {
   return mask;
 }
 
+// Survivor pairs of a warp's 32 rows (lane = row; masks: its columns 32 ci + j)
+// into the warp's reserved block [pcur, pend) of the pair list: plain stores,
+// one atomic per block.  The lanes' counts are scanned once per row tile: at 12
+// survivors per 128 x 256 tile (unit vectors) a ballot per survivor and chunk
+// made the epilogue, not the MMAs, pace the pass (tensor pipe 20% active).
+__device__ __forceinline__ void push_survivors(const BatchGemm& a, const uint32_t (&masks)[4], uint32_t row,
+                                               const uint32_t* qidx, uint32_t& pcur, uint32_t& pend) {
+  const int lane = threadIdx.x & 31;
+  if (!__any_sync(HG_FULL, (masks[0] | masks[1] | masks[2] | masks[3]) != 0)) return;
+  const uint32_t n = (uint32_t)(__popc(masks[0]) + __popc(masks[1]) + __popc(masks[2]) + __popc(masks[3]));
+  uint32_t x = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(HG_FULL, x, o);
+    if (lane >= o) x += y;
+  }
+  const uint32_t total = __shfl_sync(HG_FULL, x, 31);
+  if (pcur + total > pend) {
+    // close the block (sentinels in its tail) and reserve the next
+    for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
+    const uint32_t size = max(kBatchPairBlock, total);
+    uint32_t nb = 0;
+    if (lane == 0) nb = atomicAdd(a.pairs_cnt, size);
+    nb = __shfl_sync(HG_FULL, nb, 0);
+    pcur = nb;
+    pend = nb + size < a.pairs_cap ? nb + size : (nb < a.pairs_cap ? a.pairs_cap : nb);
+  }
+  uint32_t slot = pcur + x - n;
+#pragma unroll
+  for (int ci = 0; ci < 4; ++ci)
+    for (uint32_t m = masks[ci]; m; m &= m - 1, ++slot)
+      if (slot < pend) a.pairs[slot] = ((unsigned long long)qidx[32 * ci + __ffs(m) - 1] << 32) | row;
+  pcur += total;
+}
+
 __device__ __forceinline__ uint32_t ordered_key(float f) {
   const uint32_t b = __float_as_uint(f);
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
@@ -652,7 +687,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (screen && etid == 0) mbar_arrive(bfull_bar);
       // the two warp groups split the item's columns (32-column granules)
       const int half_cols = min(qtile / 2, (int)((it.qcnt + 63u) / 64u) * 32);
-      const int c_lo = half * half_cols;
+      // a bound-pass group of at most 32 queries is one chunk of columns: the
+      // two warp groups take alternate row tiles instead, so both reduce
+      // accumulators at once (a pass that its epilogue paces)
+      const bool alternate = !screen && a.mode == 0 && it.qcnt <= 32u;
+      const int c_lo = alternate ? 0 : half * half_cols;
       const int c_hi = min(c_lo + half_cols, (int)it.qcnt);
       // the bound pass (64-query tiles: one 32-column chunk per warp): half
       // the query norms of the warp's columns in registers; its keys order
@@ -691,6 +730,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         tc_fence_after();
+        if (kGroup == 1 && alternate && (int)(tcount & 1u) != half) {
+          // the other group's tile (waited for all the same, so that the
+          // arrival counts toward this use of the accumulator)
+          if (lane == 0) mbar_arrive(tempty_bar(b));
+          continue;
+        }
         // mode 1: survivor masks of the warp's (up to) four 32-column chunks
         // per row tile; the buckets are written after the accumulator is
         // handed back
@@ -698,6 +743,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint64_t rows_g[kGroup];
 #pragma unroll
         for (uint32_t gi = 0; gi < kGroup; ++gi) {
+        if (kGroup == 2 && alternate && (int)gi != half) continue;
         const uint32_t t = it.t_lo + jg * kGroup + gi;
         const uint64_t row = it.rb + (uint64_t)t * kUM + quarter * 32 + lane;
         const bool row_ok = t < it.t_hi && row >= it.vb && row < it.re && row < a.nrows;
@@ -815,39 +861,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(tempty_bar(b));
-        // survivor pairs into the warp's reserved block of the pair list:
-        // plain stores, one atomic per kBatchPairBlock pairs
+        if (screen) {
 #pragma unroll
-        for (uint32_t gi = 0; gi < kGroup; ++gi) {
-        const uint64_t row = rows_g[gi];
-#pragma unroll
-        for (int ci = 0; ci < 4; ++ci) {
-          uint32_t mask = masks[gi][ci];
-          while (__any_sync(HG_FULL, mask != 0)) {
-            const bool has = mask != 0;
-            unsigned long long e = 0;
-            if (has) {
-              const int j = __ffs(mask) - 1;
-              mask &= mask - 1;
-              e = ((unsigned long long)s_qidx[c_lo + 32 * ci + j] << 32) | (uint32_t)row;
-            }
-            const uint32_t bal = __ballot_sync(HG_FULL, has);
-            const uint32_t n = (uint32_t)__popc(bal);
-            if (pcur + n > pend) {
-              // close the block (sentinels in its tail) and reserve the next
-              for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
-              uint32_t nb = 0;
-              if (lane == 0) nb = atomicAdd(a.pairs_cnt, (uint32_t)kBatchPairBlock);
-              nb = __shfl_sync(HG_FULL, nb, 0);
-              pcur = nb;
-              pend = nb + kBatchPairBlock < a.pairs_cap ? nb + kBatchPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
-            }
-            const uint32_t slot = pcur + (uint32_t)__popc(bal & ((1u << lane) - 1));
-            if (has && slot < pend) a.pairs[slot] = e;
-            pcur += n;
-          }
+          for (uint32_t gi = 0; gi < kGroup; ++gi)
+            push_survivors(a, masks[gi], (uint32_t)rows_g[gi], s_qidx + c_lo, pcur, pend);
         }
-        }  // row tiles of the group
       }
     }
     for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;  // close the last block
@@ -1366,32 +1384,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (leader) mbar_arrive(tempty_bar(b));
           else mbar_arrive_cl(mapa(tempty_bar(b), 0));
         }
-#pragma unroll
-        for (int ci = 0; ci < 4; ++ci) {
-          uint32_t mask = masks[ci];
-          while (__any_sync(HG_FULL, mask != 0)) {
-            const bool has = mask != 0;
-            unsigned long long e = 0;
-            if (has) {
-              const int jj = __ffs(mask) - 1;
-              mask &= mask - 1;
-              e = ((unsigned long long)s_qidx[c_lo + 32 * ci + jj] << 32) | (uint32_t)row;
-            }
-            const uint32_t bal = __ballot_sync(HG_FULL, has);
-            const uint32_t cnt = (uint32_t)__popc(bal);
-            if (pcur + cnt > pend) {
-              for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
-              uint32_t nb = 0;
-              if (lane == 0) nb = atomicAdd(a.pairs_cnt, (uint32_t)kBatchPairBlock);
-              nb = __shfl_sync(HG_FULL, nb, 0);
-              pcur = nb;
-              pend = nb + kBatchPairBlock < a.pairs_cap ? nb + kBatchPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
-            }
-            const uint32_t slot = pcur + (uint32_t)__popc(bal & ((1u << lane) - 1));
-            if (has && slot < pend) a.pairs[slot] = e;
-            pcur += cnt;
-          }
-        }
+        push_survivors(a, masks, (uint32_t)row, s_qidx + c_lo, pcur, pend);
       }
     }
     for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
