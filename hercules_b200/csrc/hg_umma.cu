@@ -159,6 +159,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// true in one lane of the warp, the same at every call
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -497,77 +504,100 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer
-    if (lane == 0) {
-      uint32_t g = 0, tcount = 0, it_n = 0;
-      uint32_t s_cur = 0, ph = 0;  // stage g % nst and the parity of g / nst
+    // ---------------- MMA issuer: the whole warp walks the loop together and
+    // one elected lane issues.  Waits end in a vote and shared values come
+    // through shuffles, so control flow and descriptors are uniform over the
+    // warp and stay in uniform registers, which the MMA takes them from; with
+    // the loop inside `if (lane == 0)` a K = 16 step took about 100 cycles to
+    // issue whatever its width, and that paced narrow or short tiles (8M x 256,
+    // 4,096 queries: 1,200 -> 1,365 TFLOP/s; 1.5M x 256, 333: 745 -> 832; 3M x
+    // 96, 64: 184 -> 216).
+    const bool elected = elect_one();
+    auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+      bool r = mbar_try(bar, parity);
+      if (__all_sync(HG_FULL, r)) return true;
+      r = r || mbar_wait_slow(bar, parity, abort_flag, a.err, wns);
+      return __all_sync(HG_FULL, r);
+    };
+    {
+      uint32_t tcount = 0, it_n = 0;
+      uint32_t s_cur = 0, ph = 0;  // the stage and the parity of its use
       const uint64_t dae = sw32_desc(base + LY::kAext), dbe = sw32_desc(base + LY::kBext);
       const int last_steps = kTail ? (a.L - (nkb - 1) * kUK) / 16 : 0;  // 1..3: L is a multiple of 16
       bool ok = true;
       for (; ok; ++it_n) {
         const int sl = (int)(it_n & 1);
-        ok = mbar_wait(ifull_bar(sl), (it_n >> 1) & 1, abort_flag, a.err, wns);
+        ok = wait(ifull_bar(sl), (it_n >> 1) & 1);
         if (!ok) break;
-        const uint32_t w = s_item[sl];
-        mbar_arrive(iempty_bar(sl));
+        const uint32_t w = __shfl_sync(HG_FULL, s_item[sl], 0);
+        if (elected) mbar_arrive(iempty_bar(sl));
         if (w == kNoItem) break;
         const Item it = item_of(a, w, QT, ntiles, qtile, nq);
+        const uint32_t idesc = __shfl_sync(HG_FULL, idesc_for(item_n(it.qcnt, qtile)), 0);
+        const uint32_t ngroups =
+            __shfl_sync(HG_FULL, it.t_hi > it.t_lo ? (it.t_hi - it.t_lo + kGroup - 1) / kGroup : 0u, 0);
         if (resident) {
-          ok = mbar_wait(qfull_bar, it_n & 1, abort_flag, a.err, wns);
+          ok = wait(qfull_bar, it_n & 1);
           if (!ok) break;
           tc_fence_after();
         }
         if (screen) {
           // the item's thresholds in B_ext (written by the epilogue warps)
-          ok = mbar_wait(bfull_bar, it_n & 1, abort_flag, a.err, wns);
+          ok = wait(bfull_bar, it_n & 1);
           if (!ok) break;
           tc_fence_after();
         }
-        const uint32_t idesc = idesc_for(item_n(it.qcnt, qtile));
-        const uint32_t ngroups = it.t_hi > it.t_lo ? (it.t_hi - it.t_lo + kGroup - 1) / kGroup : 0u;
-        for (uint32_t jg = 0; ok && jg < ngroups; ++jg, ++tcount) {
+        for (uint32_t jg = 0; jg < ngroups; ++jg, ++tcount) {
           const int b = kGroup == 1 ? (int)(tcount & 1) : 0;
           const uint32_t tph = kGroup == 1 ? ((tcount >> 1) & 1) : (tcount & 1);
-          ok = mbar_wait(tempty_bar(b), tph ^ 1, abort_flag, a.err, wns);
+          ok = wait(tempty_bar(b), tph ^ 1);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d = tmem + (uint32_t)b * kUN;  // + gi * kUN for the group's row tile gi
           // screening: the accumulator starts as -(t_hi + t_lo) of its column
-          if (screen) {
+          if (screen && elected) {
 #pragma unroll
             for (uint32_t gi = 0; gi < kGroup; ++gi) tc_mma(d + gi * kUN, dae, dbe, idesc, 0u);
           }
-          for (int kb = 0; kb < nkb; ++kb, ++g) {
-            const int s = (int)s_cur;
-            const uint32_t par = ph;
+          for (int kb = 0; kb < nkb; ++kb) {
+            const uint32_t s = s_cur, par = ph;
             if (++s_cur == nst) {
               s_cur = 0;
               ph ^= 1u;
             }
-            ok = mbar_wait(full_bar(s), par, abort_flag, a.err, wns);
+            ok = wait(full_bar((int)s), par);
             if (!ok) break;
             tc_fence_after();
             // K step k16 is 32 bytes on: 2 in the descriptors' address field
-            const uint64_t dq = sw128_desc(base + LY::kQ + (resident ? (uint32_t)kb * LY::kQBlk : (uint32_t)s * kQBytes));
+            const uint64_t dq = sw128_desc(base + LY::kQ + (resident ? (uint32_t)kb * LY::kQBlk : s * kQBytes));
             const int steps = kTail && kb == nkb - 1 ? last_steps : kUK / 16;
+            if (elected) {
 #pragma unroll
-            for (uint32_t gi = 0; gi < kGroup; ++gi) {
-              const uint64_t da = sw128_desc(base + aBase + (s * kGroup + gi) * kABytes);
+              for (uint32_t gi = 0; gi < kGroup; ++gi) {
+                const uint64_t da = sw128_desc(base + aBase + (s * kGroup + gi) * kABytes);
 #pragma unroll
-              for (int k16 = 0; k16 < kUK / 16; ++k16)
-                if (!kTail || k16 < steps)
-                  tc_mma(d + gi * kUN, da + 2 * k16, dq + 2 * k16, idesc, (screen || kb || k16) ? 1u : 0u);
+                for (int k16 = 0; k16 < kUK / 16; ++k16)
+                  if (!kTail || k16 < steps)
+                    tc_mma(d + gi * kUN, da + 2 * k16, dq + 2 * k16, idesc, (screen || kb || k16) ? 1u : 0u);
+              }
+              tc_commit(empty_bar((int)s));
             }
-            tc_commit(empty_bar(s));
           }
-          if (ok) tc_commit(tfull_bar(b));
+          if (!ok) break;
+          if (elected) tc_commit(tfull_bar(b));
         }
-        if (ok && resident) tc_commit(qempty_bar);
-        if (ok && screen) tc_commit(bempty_bar);  // B_ext free once the item's MMAs are done
+        if (!ok) break;
+        if (elected) {
+          if (resident) tc_commit(qempty_bar);
+          if (screen) tc_commit(bempty_bar);  // B_ext free once the item's MMAs are done
+        }
       }
       // every MMA issued has completed before TMEM is freed
-      tc_commit(done_bar);
-      drain_wait(done_bar, 0, wns);
+      if (elected) {
+        tc_commit(done_bar);
+        drain_wait(done_bar, 0, wns);
+      }
+      __syncwarp();
     }
   } else if (warp >= 4) {
     // ---------------- epilogue
