@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kRankWarps * 32, 4) k_rerank_part(BatchRank a)
     uint32_t row = 0;
     int ch = 0;
     float dist = 0.0f;
-    const float4* x = nullptr;
+    const float* x = nullptr;
     const float4* qc = reinterpret_cast<const float4*>(qv) + 2 * j;
     for (;;) {
       const uint32_t need = __ballot_sync(HG_FULL, !valid) & leaders;
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kRankWarps * 32, 4) k_rerank_part(BatchRank a)
           valid = true;
           dist = 0.0f;
           ch = 0;
-          x = reinterpret_cast<const float4*>(a.rows + (uint64_t)row * a.L) + 2 * j;
+          x = a.rows + (uint64_t)row * a.L + 8 * j;
           if (j == 0) ++n_rows;
         }
         next += min((uint32_t)__popc(need), avail);
@@ -409,15 +409,23 @@ __global__ void __launch_bounds__(kRankWarps * 32, 4) k_rerank_part(BatchRank a)
 #pragma unroll
       for (int l = 0; l < kLines; ++l) {
         const bool in = valid && ch + kSlot * l + j < nch;
-        float4 x0, x1, q0, q1;
+        float xx[8];
+        float4 q0, q1;
         if (in) {
-          x0 = x[2 * kSlot * l];
-          x1 = x[2 * kSlot * l + 1];
+          if constexpr (kSlot == 8) {
+            load_chunk(x + 8 * kSlot * l, xx);
+          } else {
+            // short rows are read by several queries (5% slower when marked
+            // for early eviction)
+            const float4* p = reinterpret_cast<const float4*>(x + 8 * kSlot * l);
+            const float4 lo = p[0], hi = p[1];
+            xx[0] = lo.x; xx[1] = lo.y; xx[2] = lo.z; xx[3] = lo.w;
+            xx[4] = hi.x; xx[5] = hi.y; xx[6] = hi.z; xx[7] = hi.w;
+          }
           q0 = qc[2 * ch + 2 * kSlot * l];
           q1 = qc[2 * ch + 2 * kSlot * l + 1];
         }
         const float qq[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const float xx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
         const float d = hg_chunk_d2(qq, xx);
         dl[l] = in ? d : 0.0f;
       }
@@ -443,7 +451,7 @@ __global__ void __launch_bounds__(kRankWarps * 32, 4) k_rerank_part(BatchRank a)
         } else {
           dist = acc;
           ch += kStep;
-          x += 2 * kStep;
+          x += 8 * kStep;
           if (ch >= nch) {
             finished = true;
             valid = false;

@@ -23,6 +23,15 @@ __device__ __forceinline__ void stamp_start(unsigned long long* slot) {
   }
 }
 
+// A chunk of a row (8 floats) in one load, marked for early eviction: rows of
+// an index are 64-byte multiples from a device allocation, so their chunks are
+// 32-byte aligned (a caller's matrix may not be).
+__device__ __forceinline__ void load_chunk(const float* p, float (&v)[8]) {
+  asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(p));
+}
+
 // --- warp candidate list -----------------------------------------------------
 // A warp keeps its candidates as 64-bit keys (distance bits << 32 | id) in a
 // shared buffer of kWarpListCap entries.  Compaction sorts the buffer

@@ -1273,7 +1273,7 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
   uint32_t row = 0;
   int ch = 0;  // a multiple of kStep: the query offsets below stay inside one 32-chunk group
   float dist = 0.0f;
-  const float4* x = nullptr;
+  const float* x = nullptr;
   uint32_t n_chunks = 0, n_done = 0, n_rows = 0;  // this lane's (slot leaders only)
   constexpr int kStep = kSlot * kLines;  // chunks of a row per step
   static_assert(32 % kStep == 0, "a step stays inside one 32-chunk group of the staged query");
@@ -1306,7 +1306,7 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
         valid = true;
         dist = 0.0f;
         ch = 0;
-        x = reinterpret_cast<const float4*>(a.rows + (uint64_t)row * a.L) + 2 * j;
+        x = a.rows + (uint64_t)row * a.L + 8 * j;
         if (j == 0) ++n_rows;
       }
       cur_used += take;
@@ -1315,14 +1315,22 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
     if (!__any_sync(HG_FULL, valid)) break;
     // kLines chunks of every owned row in flight: lane j computes chunks
     // ch + kSlot l + j (l < kLines); chunks past the row's end count as 0
-    float4 xv[kLines][2];
+    float xa[kLines][8];
     bool in[kLines];
 #pragma unroll
     for (int l = 0; l < kLines; ++l) {
       in[l] = valid && ch + kSlot * l + j < nch;
       if (in[l]) {
-        xv[l][0] = __ldcs(x + 2 * kSlot * l);
-        xv[l][1] = __ldcs(x + 2 * kSlot * l + 1);
+        if constexpr (kRowIds || (kWarps != 32 && kSlot != 32)) {
+          // a caller's matrix is aligned to 16 bytes; and 8-warp blocks over
+          // medium lengths are up to 3% faster with these
+          const float4* p = reinterpret_cast<const float4*>(x + 8 * kSlot * l);
+          const float4 lo = __ldcs(p), hi = __ldcs(p + 1);
+          xa[l][0] = lo.x; xa[l][1] = lo.y; xa[l][2] = lo.z; xa[l][3] = lo.w;
+          xa[l][4] = hi.x; xa[l][5] = hi.y; xa[l][6] = hi.z; xa[l][7] = hi.w;
+        } else {
+          load_chunk(x + 8 * kSlot * l, xa[l]);
+        }
       }
     }
     // a slot without a row (its ch may equal nch) reads the first chunks:
@@ -1334,9 +1342,7 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
     for (int l = 0; l < kLines; ++l) {
       const float4 q0 = qs4[qb + qoff[l]], q1 = qs4[qb + qoff[l] + 1];
       const float qa[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-      const float xa[8] = {xv[l][0].x, xv[l][0].y, xv[l][0].z, xv[l][0].w,
-                           xv[l][1].x, xv[l][1].y, xv[l][1].z, xv[l][1].w};
-      const float d = hg_chunk_d2(qa, xa);
+      const float d = hg_chunk_d2(qa, xa[l]);
       dl[l] = in[l] ? d : 0.0f;
     }
     // the slot adds the step's chunk sums in order (adding 0 leaves a sum
@@ -1364,7 +1370,7 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
       } else {
         dist = acc;
         ch += kStep;
-        x += 2 * kStep;
+        x += 8 * kStep;
         if (ch >= nch) {
           finished = true;
           valid = false;
@@ -1382,8 +1388,8 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
   ed_finish<W>(a, lists, list, cnt, n_chunks, n_done, n_rows);
 }
 
-// The same for a group of queries over short series: a warp takes 8 rows (4
-// lanes each) together and stays with them until the last has finished or
+// The same for a group of queries over short series: a warp takes 32 / kSlot
+// rows (kSlot lanes each) together and stays with them until the last has finished or
 // abandoned, instead of giving a free slot the next row at every step.  Lanes
 // idle more (a row of 256 points abandons after 1.5 to 2.7 of its 4 steps), but
 // a step costs far fewer instructions (no refill; one place in the query for
@@ -1393,9 +1399,14 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
 // x 2048 0.85 -> 0.77.  A query alone waits for its loads instead, and the
 // other kernel's slots never idle: allocation-free scan of 1M x 256 127 us
 // there, 145 here.  (Loading the next rows' first step early spills at 64
-// registers: 5 to 20% slower.)
+// registers: 5 to 20% slower.)  Up to 256 points 16 rows of 128 bytes per step:
+// half the chain of sums per row and less read past the abandoning chunk
+// (PSCAN of 2M x 256, 4 queries 655 -> 555 us, of 2M x 96, 8 queries 740 -> 481,
+// 16 queries of 8M x 256 5.37 -> 5.10 ms); longer rows differ more, so 8 of 256
+// bytes (1M x 1024: 1.04 ms against 1.13).
+template <int kSlot, int kLines>
 __global__ void __launch_bounds__(32 * kEdWarps, kEdBlocksPerSm) k_ed_short(EdArgs a) {
-  constexpr int W = kEdWarps, kSlot = 4, kLines = 2, kStep = kSlot * kLines, kRows = 32 / kSlot;
+  constexpr int W = kEdWarps, kStep = kSlot * kLines, kRows = 32 / kSlot;
   extern __shared__ float4 ed_smem[];
   unsigned long long* lists = reinterpret_cast<unsigned long long*>(ed_smem);  // [W][kWarpListCap]
   float4* qs = ed_smem + W * kWarpListCap / 2;                                 // the query, whole steps, zero beyond L
@@ -1425,7 +1436,7 @@ __global__ void __launch_bounds__(32 * kEdWarps, kEdBlocksPerSm) k_ed_short(EdAr
   };
   uint32_t cur = entry(batch), cur_n = count_of(batch), used = 0;  // lane i holds entry i of the batch
   uint32_t nxt = entry(batch + nwarps), nxt_n = count_of(batch + nwarps);
-  // the next 8 rows; false: none left
+  // the next kRows rows; false: none left
   uint32_t row = 0;
   bool alive = false;  // slot-uniform
   auto fetch = [&]() -> bool {
@@ -1449,28 +1460,23 @@ __global__ void __launch_bounds__(32 * kEdWarps, kEdBlocksPerSm) k_ed_short(EdAr
   const float F = a.has_floor ? a.floor : -1.0f;  // distances are >= 0
   uint32_t n_chunks = 0, n_done = 0, n_rows = 0;  // this lane's (slot leaders only)
   for (uint32_t turn = 0; fetch(); ++turn) {
-    const float4* x = reinterpret_cast<const float4*>(a.rows + (uint64_t)row * a.L) + 2 * j;
+    const float* x = a.rows + (uint64_t)row * a.L + 8 * j;
     if (alive && j == 0) ++n_rows;
     float dist = 0.0f;
     for (int ch = 0;;) {
-      float4 xv[kLines][2];
+      float xa[kLines][8];
       bool in[kLines];
 #pragma unroll
       for (int l = 0; l < kLines; ++l) {
         in[l] = alive && ch + kSlot * l + j < nch;
-        if (in[l]) {
-          xv[l][0] = __ldcs(x + 2 * (ch + kSlot * l));
-          xv[l][1] = __ldcs(x + 2 * (ch + kSlot * l) + 1);
-        }
+        if (in[l]) load_chunk(x + 8 * (ch + kSlot * l), xa[l]);
       }
       float dl[kLines];
 #pragma unroll
       for (int l = 0; l < kLines; ++l) {
         const float4 q0 = qs[2 * (ch + kSlot * l + j)], q1 = qs[2 * (ch + kSlot * l + j) + 1];
         const float qa[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const float xa[8] = {xv[l][0].x, xv[l][0].y, xv[l][0].z, xv[l][0].w,
-                             xv[l][1].x, xv[l][1].y, xv[l][1].z, xv[l][1].w};
-        const float d = hg_chunk_d2(qa, xa);
+        const float d = hg_chunk_d2(qa, xa[l]);
         dl[l] = in[l] ? d : 0.0f;  // adding 0 leaves a sum unchanged
       }
       float part[kStep];
@@ -1900,12 +1906,13 @@ static cudaError_t launch_ed(K kernel, SmemLimit& attr, const EdArgs& args, int 
 // 8 lanes: 528 us, 348 us with 32; with rows for every warp 8 lanes are faster,
 // PSCAN of 60k x 16384 619 us against 1,007).
 cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
-  static SmemLimit wide, lng, mid, shrt, few_wide, few_lng;
+  static SmemLimit wide, lng, mid, shrt, shrt2, few_wide, few_lng;
   if (a.few_rows) {
     if (ed_wide(a.L)) return launch_ed(k_ed_stream<false, 1, 32, 32>, few_wide, a, 32, slots, blocks, s);
     return launch_ed(k_ed_stream<false, 1, 32, kEdWarps>, few_lng, a, kEdWarps, slots, blocks, s);
   }
-  if (slots > 1 && a.L <= kEdShortL) return launch_ed(k_ed_short, shrt, a, kEdWarps, slots, blocks, s);
+  if (slots > 1 && a.L <= 256) return launch_ed(k_ed_short<2, 2>, shrt, a, kEdWarps, slots, blocks, s);
+  if (slots > 1 && a.L <= kEdShortL) return launch_ed(k_ed_short<4, 2>, shrt2, a, kEdWarps, slots, blocks, s);
   if (ed_wide(a.L)) return launch_ed(k_ed_stream<false, 2, 8, 32>, wide, a, 32, slots, blocks, s);
   if (a.L >= 4096) return launch_ed(k_ed_stream<false, 2, 8, kEdWarps>, lng, a, kEdWarps, slots, blocks, s);
   return launch_ed(k_ed_stream<false, 2, 4, kEdWarps>, mid, a, kEdWarps, slots, blocks, s);
