@@ -286,6 +286,7 @@ static void free_scratch(hg_index* ix) {
   dfree(s.cand_lb);
   dfree(s.cand_count);
   dfree(s.unit_prefix);
+  dfree(s.row_prefix);
   dfree(s.counters);
   dfree(s.bound);
   dfree(s.kslots);
@@ -1186,6 +1187,7 @@ static cudaError_t alloc_scratch(hg_index* ix, size_t slots) {
   get(&s.cand_lb, slots * (nl + 1));
   get(&s.cand_count, slots);
   get(&s.unit_prefix, slots * (nl + 2));
+  get(&s.row_prefix, slots * (nl + 2));
   get(&s.bound, slots);
   get(&s.kslots, slots * hg::kMaxK);
   get(&s.parts, slots * s.nparts * hg::kWarpListCap);
@@ -1375,6 +1377,7 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
   sel.cand_lb = s.cand_lb;
   sel.cand_count = s.cand_count;
   sel.unit_prefix = s.unit_prefix;
+  sel.row_prefix = o.use_lb_sax ? nullptr : s.row_prefix;
   sel.gkeys = s.sort_keys;
   CK(hg::launch_merge_select(merge_args(ix, a_blocks, k), sel, slots, st));
   hg::FilterArgs f{};
@@ -1387,8 +1390,8 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
   f.cand_lb = s.cand_lb;
   f.cand_count = s.cand_count;
   f.unit_prefix = s.unit_prefix;
+  f.row_prefix = s.row_prefix;
   f.sax_tab = s.sax_tab;
-  f.use_lbsax = o.use_lb_sax ? 1 : 0;
   f.bound = s.bound;
   f.list = s.list;
   f.list_stride = ix->n;
@@ -1396,13 +1399,14 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
   f.err = s.err;
   e.ident_leaf = nullptr;
   e.list = s.list;
-  // one filter block is resident per SM: a query alone takes them all, a
-  // group a share each, with some to spare for its larger queries
-  const int f_blocks = std::min(sms, std::max(1, 4 * sms / slots));
+  // one LB_SAX filter block is resident per SM (eight that only list rows): a
+  // query alone takes them all, a group a share each, with some to spare for
+  // its larger queries
+  const int f_blocks = std::min(sms, std::max(1, 4 * sms / slots)) * (o.use_lb_sax ? 1 : 8);
   auto filter_scan_merge = [&](uint32_t* count, float* dist, int64_t* id) -> hg_status {
     f.list_count = count;
     HCK(timed_begin(prof ? &prof->filter : nullptr, st));
-    CK(hg::launch_lbsax_filter(f, slots, f_blocks, st));
+    CK(o.use_lb_sax ? hg::launch_lbsax_filter(f, slots, f_blocks, st) : hg::launch_list_rows(f, slots, f_blocks, st));
     HCK(timed_end(prof ? &prof->filter : nullptr, st));
     e.list_count = count;
     HCK(scan(ed_blocks));

@@ -697,9 +697,10 @@ __device__ void select_sort(const SelectArgs& a, uint32_t slot, float B, uint32_
     vo = x;
   }
   // 3. outputs and tile prefix
-  uint32_t tiles = 0;
+  uint32_t tiles = 0, rows = 0;
   for (int i = r0; i < r1; ++i) {
     const int leaf = (int)vi[i];
+    rows += leaf_size[leaf];
     cand[i] = leaf;
     cand_lb[i] = __uint_as_float(ki[i]);
     tiles += tiles_of_leaf(leaf_start[leaf], leaf_size[leaf]);
@@ -710,8 +711,19 @@ __device__ void select_sort(const SelectArgs& a, uint32_t slot, float B, uint32_
     unit_prefix[i] = tp;
     tp += tiles_of_leaf(leaf_start[leaf], leaf_size[leaf]);
   }
-  if (t == 0) {
+  if (a.row_prefix) {
+    uint32_t* row_prefix = a.row_prefix + (uint64_t)slot * (nleaves + 2);
+    if (t == 0) unit_prefix[n] = total;
+    uint32_t rp = block_exclusive_scan<kSortThreads>(rows, tmp, &total);
+    for (int i = r0; i < r1; ++i) {
+      row_prefix[i] = rp;
+      rp += leaf_size[vi[i]];
+    }
+    if (t == 0) row_prefix[n] = total;
+  } else if (t == 0) {
     unit_prefix[n] = total;
+  }
+  if (t == 0) {
     a.cand_count[slot] = n;
   }
 }
@@ -817,17 +829,71 @@ __device__ __forceinline__ bool fl_wait(uint32_t bar, uint32_t parity, volatile 
   return fl_try(bar, parity) || fl_wait_slow(bar, parity, abort_flag, err);
 }
 
-__global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a) {
-  extern __shared__ __align__(16) unsigned char fsm[];
+// The launch's arguments moved to the block's query, and the units [ubase,
+// ubase + total) of its candidates [clo, chi) (all of them by default).
+__device__ __forceinline__ void filter_range(FilterArgs& a, int& ncand, int& clo, int& chi, uint32_t& ubase,
+                                             uint32_t& total) {
   const uint32_t slot = blockIdx.x;
   a.cand += (uint64_t)slot * (a.nleaves + 1);
   a.cand_lb += (uint64_t)slot * (a.nleaves + 1);
-  a.cand_count += slot;
   a.unit_prefix += (uint64_t)slot * (a.nleaves + 2);
+  a.row_prefix += (uint64_t)slot * (a.nleaves + 2);
   a.sax_tab += (uint64_t)slot * (HG_PAA_SEGMENTS * HG_SAX_CARD);
   a.bound += slot;
   a.list += (uint64_t)slot * a.list_stride;
   a.list_count += 8 * slot;
+  ncand = a.cand_count[slot];
+  clo = min(a.cand_lo, ncand);
+  chi = a.cand_hi > 0 ? min(a.cand_hi, ncand) : ncand;
+  ubase = clo < chi ? a.unit_prefix[clo] : 0u;
+  total = clo < chi ? a.unit_prefix[chi] - ubase : 0u;
+}
+
+// Stage 1 without LB_SAX: every row of the leaves within the bound, in LB
+// order (a row's place in the list is its leaf's row prefix plus its place in
+// the leaf).  A warp lists a contiguous range of units, at least kListUnits of
+// them; the one that meets the last leaf within the bound writes the count.
+// Bound by its stores, 4 bytes per row: 16 queries of 8M x 256, 56.5M rows,
+// 57 us; the LB_SAX filter's kernel, which did this too, took 332 us (one block
+// of 21 warps per SM, the words copied and not read, an atomicAdd per 96 rows),
+// and its list, in no order, made the scan behind it slower (100 queries of
+// 1M x 256: 5.79 ms per call, now 5.38; 12 of 100k x 16384 3.99, now 3.71).
+constexpr int kListWarps = 8, kListUnits = 8;
+__global__ void __launch_bounds__(32 * kListWarps) k_list_rows(FilterArgs a) {
+  int ncand, clo, chi;
+  uint32_t ubase, total;
+  filter_range(a, ncand, clo, chi, ubase, total);
+  const uint32_t lane = threadIdx.x & 31, w = blockIdx.y * kListWarps + (threadIdx.x >> 5);
+  const uint32_t nwarps = gridDim.y * kListWarps;
+  const uint32_t per_warp = max((uint32_t)kListUnits, (total + nwarps - 1) / nwarps);
+  if ((uint64_t)w * per_warp >= total) return;
+  const uint32_t u0 = ubase + w * per_warp, u1 = min(ubase + total, u0 + per_warp);
+  const float B = __int_as_float((int)ld_volatile(a.bound));
+  const uint32_t base = a.row_prefix[clo];
+  uint32_t n_leaves = 0;
+  for (int c = unit_candidate_warp(a.unit_prefix, ncand, clo, u0, (int)lane); c < chi; ++c) {
+    const uint32_t first_unit = a.unit_prefix[c], next = a.unit_prefix[c + 1];
+    if (first_unit >= u1 || a.cand_lb[c] > B) break;  // LBs ascend: no later leaf is within the bound
+    const uint32_t from = max(u0, first_unit), to = min(u1, next);
+    n_leaves += from == first_unit ? 1u : 0u;
+    const int leaf = a.cand[c];
+    const uint32_t lstart = (uint32_t)a.leaf_start[leaf], lend = lstart + a.leaf_size[leaf];
+    uint32_t* out = a.list + (a.row_prefix[c] - base);
+    const uint32_t row1 = min(lend, ((lstart >> 5) + (to - first_unit)) << 5);
+#pragma unroll 4
+    for (uint32_t r = (((lstart >> 5) + (from - first_unit)) << 5) + lane; r < row1; r += 32)
+      if (r >= lstart) out[r - lstart] = r;
+    if (to == next && (c + 1 == chi || a.cand_lb[c + 1] > B) && lane == 0) {
+      const uint32_t count = a.row_prefix[c + 1] - base;
+      *a.list_count = count;
+      atomicAdd(&a.stats[0], (unsigned long long)count);
+    }
+  }
+  if (lane == 0 && n_leaves) atomicAdd(&a.stats[3], (unsigned long long)n_leaves);
+}
+
+__global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a) {
+  extern __shared__ __align__(16) unsigned char fsm[];
   uint32_t* qtab = reinterpret_cast<uint32_t*>(fsm);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(fsm);
@@ -835,14 +901,10 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a
   auto empty_bar = [&](int st) { return sbase + kFiltSmBar + 8u * (kFiltStages + st); };
   volatile uint32_t* s_uend = reinterpret_cast<volatile uint32_t*>(fsm + kFiltSmMeta);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(fsm + kFiltSmMeta + 4);
+  int ncand, clo, chi;
+  uint32_t ubase, total;
+  filter_range(a, ncand, clo, chi, ubase, total);
   const float B = __int_as_float((int)ld_volatile(a.bound));
-  // candidates [clo, chi) of the sorted list (all of them by default); this
-  // block's contiguous range of their units
-  const int ncand = *a.cand_count;
-  const int clo = min(a.cand_lo, ncand);
-  const int chi = a.cand_hi > 0 ? min(a.cand_hi, ncand) : ncand;
-  const uint32_t ubase = clo < chi ? a.unit_prefix[clo] : 0u;
-  const uint32_t total = clo < chi ? a.unit_prefix[chi] - ubase : 0u;
   // at least one full stage per block: fewer units leave blocks without a
   // range, which return before they build a table
   const uint32_t per_block = max((uint32_t)kStageUnits, (total + gridDim.y - 1) / gridDim.y);
@@ -884,7 +946,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a
     }
     __syncwarp();
     asm volatile("bar.arrive 1, %0;" ::"r"(kFilterThreads) : "memory");
-  } else if (a.use_lbsax) {
+  } else {
     const float Bs = __fadd_rn(__fmul_rn(B, 1.0009765625f), 1e-6f);
     const float T = __fdiv_ru(Bs, (float)(a.L / HG_PAA_SEGMENTS));
     const float scale = __fdiv_rd(254.0f, T);  // 0 when the bound is +inf: nothing is pruned
@@ -981,7 +1043,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a
         rr[i] = (((lstart >> 5) + tile_in) << 5) + lane;
         bool pass = rr[i] >= lstart && rr[i] < lend;
         n_rows += (uint32_t)__popc(__ballot_sync(HG_FULL, pass));
-        if (pass && a.use_lbsax) {
+        if (pass) {
           // byte j of word q is the symbol s of segment t = 4 q + j; the
           // permute puts s in byte 1 and 4 lane in byte 0: 256 s + 4 lane,
           // the lookup's offset from segment t's fixed base
@@ -1874,6 +1936,10 @@ cudaError_t launch_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count
   return cudaGetLastError();
 }
 
+cudaError_t launch_list_rows(const FilterArgs& a, int slots, int blocks, cudaStream_t s) {
+  k_list_rows<<<dim3(slots, blocks), 32 * kListWarps, 0, s>>>(a);
+  return cudaGetLastError();
+}
 cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cudaStream_t s) {
   static SmemLimit attr;
   const cudaError_t ea = attr.ensure((const void*)k_lbsax_filter, (int)lbsax_filter_smem());

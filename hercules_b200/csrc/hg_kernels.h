@@ -78,7 +78,8 @@ struct PrepArgs {
   uint32_t* counters;    // [slot][8] reset to 0
 };
 
-// Stage 1 of the leaf scan: candidate leaves -> LB_SAX survivors.
+// Stage 1 of the leaf scan: candidate leaves -> their rows, with LB_SAX its survivors
+// (launch_lbsax_filter) or all of them (launch_list_rows).
 struct FilterArgs {
   const uint8_t* sax;
   int L;
@@ -89,8 +90,8 @@ struct FilterArgs {
   const float* cand_lb;         // [slot][nleaves + 1]
   const int* cand_count;        // [slot]
   const uint32_t* unit_prefix;  // [slot][nleaves + 2] exclusive prefix of 32-row units per candidate
+  const uint32_t* row_prefix;   // [slot][nleaves + 2] the same of rows (launch_list_rows)
   const float* sax_tab;  // [slot][16 x 256] the query's LB_SAX terms (k_query_prep), 16-byte aligned
-  int use_lbsax;
   int cand_lo, cand_hi;  // candidates [cand_lo, cand_hi) of the sorted list; cand_hi <= 0: to the end
   const uint32_t* bound;  // [slot]
   uint32_t* list;         // [slot][list_stride] surviving rows
@@ -155,6 +156,7 @@ struct SelectArgs {
   float* cand_lb;
   int* cand_count;
   uint32_t* unit_prefix;
+  uint32_t* row_prefix;   // [slot][nleaves + 2] exclusive prefix of rows; NULL: not wanted
   uint32_t* gkeys;        // [slot][4 x nleaves], needed above kMaxLeavesSort leaves
 };
 
@@ -215,6 +217,7 @@ cudaError_t launch_route_queries(const float* Q, int nq, int L, Tree t, int* lea
                                  uint32_t nb = 0, unsigned long long* stamp = nullptr);
 cudaError_t launch_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count, int slots, cudaStream_t s);
 // blocks: per slot
+cudaError_t launch_list_rows(const FilterArgs& a, int slots, int blocks, cudaStream_t s);
 cudaError_t launch_lbsax_filter(const FilterArgs& a, int slots, int blocks, cudaStream_t s);
 size_t lbsax_filter_smem();
 // blocks: per slot, at most EdArgs::parts_stride
