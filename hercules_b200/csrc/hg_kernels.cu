@@ -623,14 +623,20 @@ __device__ void select_sort(const SelectArgs& a, uint32_t slot, float B, uint32_
     }
   }
   __syncthreads();
-  // 2. sort by LB.  Up to kSortThreads candidates (the usual case): one
+  // 2. sort by LB, unless the leaves may stay in file order (by_file, all of
+  //    them within a finite bound, so none is met that ends the list: their
+  //    LBs read 0).  Up to kSortThreads candidates (the usual case): one
   //    bitonic sort of (LB bits, leaf) keys; the leaves are in index order on
   //    input, so equal LBs end in the order the stable radix sort below gives
   //    them, which handles larger counts.
   const int per2 = (n + kSortThreads - 1) / kSortThreads;
   const int r0 = min(n, t * per2), r1 = min(n, r0 + per2);
   uint32_t *ki = keys0, *vi = vals0, *ko = keys1, *vo = vals1;
-  if (n <= kSortThreads) {
+  const bool by_file = a.by_file && B < __int_as_float(0x7f800000);
+  if (by_file) {
+    for (int i = t; i < n; i += kSortThreads) keys0[i] = 0;
+    __syncthreads();
+  } else if (n <= kSortThreads) {
     unsigned long long* kv = reinterpret_cast<unsigned long long*>(keys1);  // 8-byte aligned, 2 x cap words (n <= 1024)
     int np = 2;
     while (np < n) np <<= 1;
@@ -657,7 +663,7 @@ __device__ void select_sort(const SelectArgs& a, uint32_t slot, float B, uint32_
     }
     __syncthreads();
   }
-  for (int pass = 0; n > kSortThreads && pass < 8; ++pass) {
+  for (int pass = 0; !by_file && n > kSortThreads && pass < 8; ++pass) {
     const int shift = pass * 4;
     uint32_t c[16];
 #pragma unroll

@@ -87,7 +87,7 @@ struct FilterArgs {
   const uint64_t* leaf_start;
   const uint32_t* leaf_size;
   const int* cand;              // [slot][nleaves + 1]
-  const float* cand_lb;         // [slot][nleaves + 1]
+  const float* cand_lb;         // [slot][nleaves + 1] ascending
   const int* cand_count;        // [slot]
   const uint32_t* unit_prefix;  // [slot][nleaves + 2] exclusive prefix of 32-row units per candidate
   const uint32_t* row_prefix;   // [slot][nleaves + 2] the same of rows (launch_list_rows)
@@ -156,6 +156,7 @@ struct SelectArgs {
   float* cand_lb;
   int* cand_count;
   uint32_t* unit_prefix;
+  int by_file;            // leaves within a finite bound may stay in file order
   uint32_t* row_prefix;   // [slot][nleaves + 2] exclusive prefix of rows; NULL: not wanted
   uint32_t* gkeys;        // [slot][4 x nleaves], needed above kMaxLeavesSort leaves
 };

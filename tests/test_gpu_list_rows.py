@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
     (97, 64, 10, 1, 3, 0),
     (3001, 64, 7, 3, 5, 0),
     (3001, 64, 7, 1, 5, 4),
+    (3001, 64, 7, 3, 50, 0),  # the approximate leaf leaves the bound open
     (60013, 96, 701, 1, 10, 0),
     (60013, 96, 701, 7, 10, 3),
     (400009, 64, 20000, 2, 100, 0),
