@@ -7,7 +7,8 @@
 //               per stage) and the query tile (B, up to 256 queries x L in
 //               boxes of 64, resident in shared memory for L <= 256, else
 //               streamed with A);
-//   warp 1      MMA issuer (one lane): per 128-row tile, L/16 MMAs of
+//   warp 1      MMA issuer (one elected lane of a uniform warp): per 128-row
+//               tile, L/16 MMAs of
 //               M=128, N=256, K=16 into one of two TMEM accumulators;
 //   warp 2      allocates / frees the 512 TMEM columns;
 //   warps 4-11  epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (the
@@ -252,46 +253,52 @@ __device__ __forceinline__ uint32_t screen32(const float* v, float h, int nv) {
     for (int q = 0; q < 4; ++q) {
       if (g[q] >= h) {
 #pragma unroll
-        for (int j = 8 * q; j < 8 * q + 8; ++j) mask |= (j < nv && v[j] >= h) ? (1u << j) : 0u;
+        for (int j = 8 * q; j < 8 * q + 8; ++j) mask |= v[j] >= h ? (1u << j) : 0u;
       }
     }
+    if (nv < 32) mask &= (1u << nv) - 1u;
   }
   return mask;
 }
 
 // Survivor pairs of a warp's 32 rows (lane = row; masks: its columns 32 ci + j)
 // into the warp's reserved block [pcur, pend) of the pair list: plain stores,
-// one atomic per block.  The lanes' counts are scanned once per row tile: at 12
-// survivors per 128 x 256 tile (unit vectors) a ballot per survivor and chunk
-// made the epilogue, not the MMAs, pace the pass (tensor pipe 20% active).
+// one atomic per block.  Every vote places one survivor of each lane that has
+// any left, whichever chunk it is in: at 12 survivors per 128 x 256 tile (unit
+// vectors) that is one vote and a last one.  Such passes are paced by the
+// epilogue; with the lanes' counts scanned by shuffles and a loop per chunk this
+// took 28% of its time (3M x 96, 333 queries: filter 439 -> 388 us; 8M x 256,
+// 4,096 queries: 6.15 -> 6.06 ms, with screen32's test of the last column once per mask).
 __device__ __forceinline__ void push_survivors(const BatchGemm& a, const uint32_t (&masks)[4], uint32_t row,
                                                const uint32_t* qidx, uint32_t& pcur, uint32_t& pend) {
+  uint32_t m0 = masks[0], m1 = masks[1], m2 = masks[2], m3 = masks[3];
+  uint32_t left = __ballot_sync(HG_FULL, (m0 | m1 | m2 | m3) != 0);
+  if (!left) return;
   const int lane = threadIdx.x & 31;
-  if (!__any_sync(HG_FULL, (masks[0] | masks[1] | masks[2] | masks[3]) != 0)) return;
-  const uint32_t n = (uint32_t)(__popc(masks[0]) + __popc(masks[1]) + __popc(masks[2]) + __popc(masks[3]));
-  uint32_t x = n;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(HG_FULL, x, o);
-    if (lane >= o) x += y;
-  }
-  const uint32_t total = __shfl_sync(HG_FULL, x, 31);
-  if (pcur + total > pend) {
-    // close the block (sentinels in its tail) and reserve the next
-    for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
-    const uint32_t size = max(kBatchPairBlock, total);
-    uint32_t nb = 0;
-    if (lane == 0) nb = atomicAdd(a.pairs_cnt, size);
-    nb = __shfl_sync(HG_FULL, nb, 0);
-    pcur = nb;
-    pend = nb + size < a.pairs_cap ? nb + size : (nb < a.pairs_cap ? a.pairs_cap : nb);
-  }
-  uint32_t slot = pcur + x - n;
-#pragma unroll
-  for (int ci = 0; ci < 4; ++ci)
-    for (uint32_t m = masks[ci]; m; m &= m - 1, ++slot)
-      if (slot < pend) a.pairs[slot] = ((unsigned long long)qidx[32 * ci + __ffs(m) - 1] << 32) | row;
-  pcur += total;
+  const uint32_t lt = (1u << lane) - 1;
+  do {
+    const uint32_t n = (uint32_t)__popc(left);
+    if (pcur + n > pend) {
+      // close the block (sentinels in its tail) and reserve the next
+      for (uint32_t i = pcur + lane; i < pend; i += 32) a.pairs[i] = ~0ull;
+      uint32_t nb = 0;
+      if (lane == 0) nb = atomicAdd(a.pairs_cnt, kBatchPairBlock);
+      nb = __shfl_sync(HG_FULL, nb, 0);
+      pcur = nb;
+      pend = nb + kBatchPairBlock < a.pairs_cap ? nb + kBatchPairBlock : (nb < a.pairs_cap ? a.pairs_cap : nb);
+    }
+    const uint32_t slot = pcur + (uint32_t)__popc(left & lt);
+    const uint32_t m = m0 ? m0 : (m1 ? m1 : (m2 ? m2 : m3));  // the first chunk with survivors
+    const int c = m0 ? 0 : (m1 ? 32 : (m2 ? 64 : 96));
+    if (m && slot < pend) a.pairs[slot] = ((unsigned long long)qidx[c + __ffs(m) - 1] << 32) | row;
+    const uint32_t rest = m & (m - 1);
+    if (c == 0) m0 = rest;
+    else if (c == 32) m1 = rest;
+    else if (c == 64) m2 = rest;
+    else m3 = rest;
+    pcur += n;
+    left = __ballot_sync(HG_FULL, (m0 | m1 | m2 | m3) != 0);
+  } while (left);
 }
 
 __device__ __forceinline__ uint32_t ordered_key(float f) {
