@@ -126,7 +126,6 @@ __global__ void k_tile_norms(const float4* __restrict__ meta, uint64_t n, float4
 // kMaxK smallest are ranked exactly (hg_ed, reference order) and the k-th
 // distinct distance among them bounds the query's k-th neighbour distance
 // (more rows than k: a tighter bound, and k distinct distances despite ties).
-constexpr int kSelThreads = 256;
 constexpr int kRankLongSeries = 4096;  // L from which the exact ranking uses 8 lanes per row
 
 // Exact distances of the rows named by the first nrank keys of `buf` (~0: no
@@ -137,14 +136,18 @@ constexpr int kRankLongSeries = 4096;  // L from which the exact ranking uses 8 
 // before the current ones are summed.  One row per warp, its 32 chunk sums
 // added one shuffle after the other, was bound by that chain: 428 us for 128
 // queries of 16,384 points (52 rows each), 58 us for 512 queries of 1,024.
-template <int kSlot>
+// A long series' step waits for its loads whatever the other warps do, so its
+// block has 16 warps, a round of 64 rows, not 8 (205 us for those 128 queries,
+// 120 with 16; 16 lanes per row and 32 warps are no faster there and slower for
+// 512 queries of 4,096 points).
+template <int kSlot, int kThreads>
 __device__ __forceinline__ void rank_rows(const BatchRank& a, const float* qv, const unsigned long long* buf, int nrank,
                                           unsigned long long* list) {
   constexpr int kLines = 2, kStep = kSlot * kLines, kRows = 32 / kSlot;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int slot = lane / kSlot, slot_lead = lane & ~(kSlot - 1), j = lane & (kSlot - 1);
   const int nch = a.L >> 3;
-  for (int i0 = warp * kRows; i0 < nrank; i0 += (kSelThreads / 32) * kRows) {
+  for (int i0 = warp * kRows; i0 < nrank; i0 += (kThreads / 32) * kRows) {
     const int i = i0 + slot;
     const unsigned long long key = i < nrank ? buf[i] : ~0ull;
     const bool valid = key != ~0ull;
@@ -192,8 +195,8 @@ __device__ __forceinline__ void rank_rows(const BatchRank& a, const float* qv, c
   }
 }
 
-template <int kSlot>
-__global__ void __launch_bounds__(kSelThreads) k_bound_select(BatchRank a) {
+template <int kSlot, int kThreads>
+__global__ void __launch_bounds__(kThreads) k_bound_select(BatchRank a) {
   extern __shared__ unsigned long long ssel[];
   unsigned long long* buf = ssel;                    // bm_pow2 keys
   __shared__ unsigned long long list[kWarpListCap];  // exact (distance, id) keys
@@ -203,11 +206,11 @@ __global__ void __launch_bounds__(kSelThreads) k_bound_select(BatchRank a) {
   const uint32_t ns = min(a.slots_of_query[q], a.bm_cap);
   int n = 32;
   while (n < (int)ns) n <<= 1;
-  for (int i = tid; i < n; i += kSelThreads) buf[i] = i < (int)ns ? a.bm[(uint64_t)q * a.bm_cap + i] : ~0ull;
+  for (int i = tid; i < n; i += kThreads) buf[i] = i < (int)ns ? a.bm[(uint64_t)q * a.bm_cap + i] : ~0ull;
   __syncthreads();
   for (int size = 2; size <= n; size <<= 1)
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < (n >> 1); i += kSelThreads) {
+      for (int i = tid; i < (n >> 1); i += kThreads) {
         const int pos = 2 * i - (i & (stride - 1));
         const int partner = pos + stride;
         const bool asc = (pos & size) == 0;
@@ -223,9 +226,9 @@ __global__ void __launch_bounds__(kSelThreads) k_bound_select(BatchRank a) {
   // the 2k + 32 best slots by d~ (at most kMaxK) are ranked exactly: the k-th
   // distinct exact distance among them bounds the query's k-th neighbour
   const int nrank = min(min(kMaxK, 2 * k + 32), n);
-  for (int i = tid; i < kWarpListCap; i += kSelThreads) list[i] = ~0ull;
+  for (int i = tid; i < kWarpListCap; i += kThreads) list[i] = ~0ull;
   __syncthreads();
-  rank_rows<kSlot>(a, qv, buf, nrank, list);
+  rank_rows<kSlot, kThreads>(a, qv, buf, nrank, list);
   __syncthreads();
   if (tid < 32) {
     // the valid keys are a prefix (rows of the sorted prefix), the rest ~0
@@ -997,14 +1000,15 @@ cudaError_t launch_bound_select(const BatchRank& r, cudaStream_t s) {
   if (!r.nq) return cudaSuccess;
   int n = 32;
   while (n < (int)r.bm_cap) n <<= 1;
-  auto run = [&](auto kernel, SmemLimit& attr) {
+  auto run = [&](auto kernel, SmemLimit& attr, int threads) {
     const cudaError_t ea = attr.ensure((const void*)kernel, (int)(sizeof(unsigned long long) * kBatchMaxSlots));
     if (ea != cudaSuccess) return ea;
-    kernel<<<r.nq, kSelThreads, sizeof(unsigned long long) * n, s>>>(r);
+    kernel<<<r.nq, threads, sizeof(unsigned long long) * n, s>>>(r);
     return cudaGetLastError();
   };
   static SmemLimit attr_long, attr_short;
-  return r.L >= kRankLongSeries ? run(k_bound_select<8>, attr_long) : run(k_bound_select<4>, attr_short);
+  return r.L >= kRankLongSeries ? run(k_bound_select<8, 512>, attr_long, 512)
+                                : run(k_bound_select<4, 256>, attr_short, 256);
 }
 
 cudaError_t launch_rerank(const BatchRank& r, int part_blocks, cudaStream_t s) {
