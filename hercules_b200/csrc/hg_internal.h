@@ -62,6 +62,8 @@ struct QueryScratch {
   float* cand_lb = nullptr;       // leaves + 1
   int* cand_count = nullptr;      // 1
   uint32_t* unit_prefix = nullptr;  // leaves + 2 (32-row units per candidate, exclusive scan)
+  float* group_q = nullptr;         // slots x L: queries gathered from a batch
+  uint32_t* group_row = nullptr;    // slots: their places in it
   uint32_t* row_prefix = nullptr;   // leaves + 2 (rows per candidate, exclusive scan)
   uint32_t* counters = nullptr;   // 8: [2] filter survivors, [4] the seeding stage's
   uint32_t* bound = nullptr;      // float bits of the current k-th distance bound

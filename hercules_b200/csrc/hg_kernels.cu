@@ -1676,11 +1676,12 @@ __device__ float merge_parts(const MergeArgs& a, uint32_t slot, unsigned long lo
     a.bound[slot] = B;
   }
   if (a.dist_out || a.id_out) {
+    const uint64_t out_at = a.out_row ? (uint64_t)a.out_row[slot] * a.out_stride : (uint64_t)slot * k;
     for (int i = t; i < k; i += kMergeThreads) {
       const unsigned long long v = i < cnt ? buf[i] : ~0ull;
       if (a.dist_out)
-        a.dist_out[(uint64_t)slot * k + i] = i < cnt ? __uint_as_float((uint32_t)(v >> 32)) : __int_as_float(0x7f800000);
-      if (a.id_out) a.id_out[(uint64_t)slot * k + i] = i < cnt ? (int64_t)(uint32_t)v : -1;
+        a.dist_out[out_at + i] = i < cnt ? __uint_as_float((uint32_t)(v >> 32)) : __int_as_float(0x7f800000);
+      if (a.id_out) a.id_out[out_at + i] = i < cnt ? (int64_t)(uint32_t)v : -1;
     }
   }
   return __uint_as_float(B);

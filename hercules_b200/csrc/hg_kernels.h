@@ -143,6 +143,8 @@ struct MergeArgs {
   uint32_t* bound;           // [slot]
   float* dist_out;           // [slot][k] answers; both NULL: none written
   int64_t* id_out;
+  const uint32_t* out_row;   // [slot] row of the answers in dist_out / id_out; NULL: the slot
+  uint32_t out_stride;       // entries per row with out_row
 };
 
 // Candidate leaves of a group (LB_EAPCA within the bound, in LB order).
