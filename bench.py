@@ -621,7 +621,7 @@ def main():
     pscan = {"value": round(npq / (pscan_ms / 1000.0), 2), "unit": UNIT, "queries": npq, "k": pk,
              "path": "hg_knn_device, HG_MODE_PSCAN (every row, early abandon at the running k-th distance)",
              "answers_equal_plain_path": pscan_same,
-             "scan": {"kernel": "k_ed_stream", "achieved": round(pscan_gbs, 1), "unit": "GB/s",
+             "scan": {"kernel": "k_ed_short" if args.L <= 2048 else "k_ed_stream", "achieved": round(pscan_gbs, 1), "unit": "GB/s",
                       "frac": round(pscan_gbs / measured_peaks_all()["hbm"], 4),
                       "algorithmic_bytes_per_query": pscan_bytes / npq}}
 
@@ -661,7 +661,7 @@ def main():
                 "peak_source": peaks["source"] + " sustained bf16 (the filter runs inside seconds-long steps)",
                 "traffic": traffic, "algorithmic_flops_per_step": flops / steps,
                 "avg_ms_per_step": agg["gemm_ms"] / steps, "pairs_per_step": agg["bf16_pairs"] / steps}
-    # leaf scan of the plain path: k_ed_stream's algorithmic bytes = 32 B per
+    # leaf scan of the plain path: the distance stream's algorithmic bytes = 32 B per
     # 8-float chunk computed + 4 B list entry per row started + 8 B id per
     # finished row, over its summed launch time
     pst = plain_st
@@ -669,11 +669,11 @@ def main():
     alg_bytes = 32.0 * pst["chunks_loaded"] + 4.0 * pst["rows_visited"] + 8.0 * pst["rows_completed"]
     scan_s = pst["scan_ms"] / 1000.0
     ed_gbs = alg_bytes / scan_s / 1e9 if scan_s > 0 else 0.0
-    tre = profile_json("k_ed_stream_traffic.json")
+    tre = profile_json("k_ed_short_traffic.json")
     ed_traffic = None
     if tre and tre.get("dram_bytes_per_algorithmic_byte"):
         ed_traffic = tre["dram_bytes_per_algorithmic_byte"] * alg_bytes / max(launches, 1)
-    leaf_scan = {"bound": "hbm", "kernel": "k_ed_stream", "achieved": round(ed_gbs, 1), "peak": peaks["hbm"],
+    leaf_scan = {"bound": "hbm", "kernel": "k_ed_short" if args.L <= 2048 else "k_ed_stream", "achieved": round(ed_gbs, 1), "peak": peaks["hbm"],
                  "unit": "GB/s", "frac": round(ed_gbs / peaks["hbm"], 4), "peak_source": peaks["source"],
                  "traffic": ed_traffic, "algorithmic_bytes_per_launch": alg_bytes / max(launches, 1),
                  "avg_launch_ms": pst["scan_ms"] / max(launches, 1), "launches": launches}
