@@ -751,7 +751,8 @@ __global__ void k_pscan_prep(uint32_t* bound, uint32_t* kslots, int* topk_count)
 // stream over that list.
 // ---------------------------------------------------------------------------
 
-// Stage 1.  Work: the candidate leaves in ascending LB_EAPCA order, cut into
+// Stage 1.  Work: the candidate leaves (file order, or ascending LB_EAPCA:
+// select_sort), cut into
 // 32-row units (32-aligned rows; a unit's rows outside its leaf are skipped).
 // One persistent block per SM owns a contiguous range of units, ending at the
 // first leaf whose LB exceeds the bound (found by the producer warp while
@@ -1094,15 +1095,15 @@ __global__ void __launch_bounds__(kFilterThreads, 1) k_lbsax_filter(FilterArgs a
 // Stage 2: the early-abandoning squared distance (ts_euclidean_distance_SIMD,
 // ts.c:83-109) over a row list, or over a row range when there is no list.
 //
-// A warp works on 8 rows at a time, 4 lanes per row ("slot").  Per step the
-// 4 lanes of a slot load one 128-byte line of their row (chunk ch + j in
-// lane j), each computes its 8-float chunk sum, and the slot adds the 4 chunk
-// sums to the running distance in chunk order (shuffles), testing the bound
-// after each (a strict test: a row whose distance equals the bound finishes,
-// so ties keep the lowest id).  A slot whose row abandoned or finished takes
-// the next row of its warp's batch: warp w of W owns the 32-entry batches w,
-// w + W, w + 2W, ... of the list, and the next batch's entries are loaded
-// while the current one is consumed.  Finished rows within the bound enter
+// A warp works on 8 rows at a time, 4 lanes per row ("slot"; wider slots for
+// long series).  Per step the lanes of a slot load kLines lines of their row
+// (chunk ch + j of a line in lane j), each computes its 8-float chunk sums, and
+// the slot adds them to the running distance in chunk order (shuffles) and
+// tests the bound once (a strict test: a row whose distance equals the bound
+// finishes, so ties keep the lowest id).  A slot whose row abandoned or
+// finished takes the next row of its warp's batch: warp w of W owns the
+// batches w, w + W, w + 2W, ... of the list (up to 32 entries each), and the
+// next batch's entries are loaded while the current one is consumed.  Finished rows within the bound enter
 // the warp's top-k list, which lowers the global bound (atomicMin) once it
 // holds k distances.  The query lives in shared memory in blocks of 32
 // chunks (40 float4 pairs each): chunk r of a block sits at pair r + r / 4,
@@ -1467,7 +1468,8 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
 // x 2048 0.85 -> 0.77.  A query alone waits for its loads instead, and the
 // other kernel's slots never idle: allocation-free scan of 1M x 256 127 us
 // there, 145 here.  (Loading the next rows' first step early spills at 64
-// registers: 5 to 20% slower.)  Up to 256 points 16 rows of 128 bytes per step:
+// registers, 5 to 20% slower; through shared memory with cp.async it does not,
+// and is 1 to 11% slower: issue, load pipe and DRAM are each half busy.)  Up to 256 points 16 rows of 128 bytes per step:
 // half the chain of sums per row and less read past the abandoning chunk
 // (PSCAN of 2M x 256, 4 queries 655 -> 555 us, of 2M x 96, 8 queries 740 -> 481,
 // 16 queries of 8M x 256 5.37 -> 5.10 ms); longer rows differ more, so 8 of 256
