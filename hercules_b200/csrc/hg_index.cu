@@ -1164,8 +1164,11 @@ static hg_status read_impl(const char* dir, int device, hg_index** out) {
 // queries' scans and fills the GPU from indexes whose leaves are too small to
 // (per query, one at a time -> in groups: 1M x 256, leaf 100,000, k = 10:
 // 139 -> 28 us; 100k x 16384: 480 -> 92 us; 8M x 256, k = 100: 800 -> 390 us).
+// 4 GB of lists, 2% of the GPU's memory, hold 32 queries of 33M rows; with
+// 512 MB 25M rows left groups of five (64 queries of 25M x 256: 63.0 ms, 54.9
+// now, with LB_SAX 22.2 and 19.0; 32 of 30M x 96 15.2 and 13.6).
 constexpr uint32_t kGroupSlots = 32;
-constexpr uint64_t kGroupListBytes = 512ull << 20;
+constexpr uint64_t kGroupListBytes = 4ull << 30;
 static uint32_t group_slots(const hg_index* ix, uint32_t nq) {
   const uint64_t by_list = std::max<uint64_t>(4, kGroupListBytes / (4 * std::max<uint64_t>(ix->n, 1)));
   const uint32_t most = (uint32_t)std::min<uint64_t>(kGroupSlots, by_list);
