@@ -662,15 +662,15 @@ __global__ void k_scatter_pairs(const unsigned long long* __restrict__ pairs, co
 // Queries grouped by approximate leaf (one block): per leaf its query count
 // and offset (counting sort; the order inside a leaf is arbitrary), each
 // query's bound slots, and the bound pass's item offsets per leaf (groups of
-// at most kBatchBoundQueries queries x chunks of nitems[1] tiles: btpi, or
-// fewer, down to 2, until there are kBatchItemTarget items).
+// at most kBatchBoundQueries queries x chunks of nitems[1] tiles:
+// bound_item_tiles).
 constexpr int kGroupThreads = 1024;
 __global__ void __launch_bounds__(kGroupThreads) k_group_queries(const int* __restrict__ approx, int nq,
                                                                  const LeafPlan* __restrict__ plan, int nleaves,
                                                                  uint32_t btpi, uint32_t* perm, uint32_t* slots,
                                                                  uint32_t* leaf_qoff, uint32_t* leaf_qcnt,
                                                                  uint32_t* item_off, uint32_t* nitems,
-                                                                 uint32_t* gcnt) {
+                                                                 uint32_t items_cap, uint32_t* gcnt) {
   // per-leaf counters in shared memory, or in gcnt (2 x nleaves words of
   // global memory) above kMaxLeavesSort leaves
   extern __shared__ uint32_t gsh[];
@@ -686,15 +686,21 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_queries(const int* __re
   // thread owns a run of consecutive leaves
   const int per = (nleaves + kGroupThreads - 1) / kGroupThreads;
   const int l0 = min(tid * per, nleaves), l1 = min(l0 + per, nleaves);
-  __shared__ unsigned long long s_work;
-  if (tid == 0) s_work = 0;
+  __shared__ unsigned long long s_work, s_groups;
+  if (tid == 0) s_work = s_groups = 0;
   __syncthreads();
-  unsigned long long work = 0;  // (group, tile) pairs
-  for (int l = l0; l < l1; ++l)
-    work += (unsigned long long)((cnt[l] + kBatchBoundQueries - 1) / kBatchBoundQueries) * plan[l].use_tiles;
-  if (work) atomicAdd(&s_work, work);
+  unsigned long long work = 0, groups = 0;  // (group, tile) pairs, groups
+  for (int l = l0; l < l1; ++l) {
+    const uint32_t g = (cnt[l] + kBatchBoundQueries - 1) / kBatchBoundQueries;
+    groups += g;
+    work += (unsigned long long)g * plan[l].use_tiles;
+  }
+  if (groups) {
+    atomicAdd(&s_work, work);
+    atomicAdd(&s_groups, groups);
+  }
   __syncthreads();
-  btpi = (uint32_t)min((unsigned long long)btpi, max(2ull, s_work / kBatchItemTarget));
+  btpi = bound_item_tiles(s_work, s_groups, btpi, items_cap);
   auto items_of = [&](int l) -> uint32_t {
     const uint32_t c = cnt[l], use = plan[l].use_tiles;
     if (c == 0 || use == 0) return 0u;
@@ -956,8 +962,8 @@ cudaError_t launch_scatter_pairs(const unsigned long long* pairs, const uint32_t
 
 cudaError_t launch_group_queries(const int* approx, int nq, const LeafPlan* plan, int nleaves, uint32_t btpi,
                                  uint32_t* perm, uint32_t* slots, uint32_t* leaf_qoff, uint32_t* leaf_qcnt,
-                                 uint32_t* item_off, uint32_t* nitems, BatchItem* items, cudaStream_t s,
-                                 uint32_t* gcnt) {
+                                 uint32_t* item_off, uint32_t* nitems, BatchItem* items, uint32_t items_cap,
+                                 cudaStream_t s, uint32_t* gcnt) {
   const bool global_cnt = nleaves > kMaxLeavesSort;
   if (global_cnt && !gcnt) return cudaErrorInvalidValue;
   const size_t smem = global_cnt ? 0 : sizeof(uint32_t) * 2 * (size_t)nleaves;
@@ -965,7 +971,7 @@ cudaError_t launch_group_queries(const int* approx, int nq, const LeafPlan* plan
   const cudaError_t ea = attr.ensure((const void*)k_group_queries, (int)(sizeof(uint32_t) * 2 * kMaxLeavesSort));
   if (ea != cudaSuccess) return ea;
   k_group_queries<<<1, kGroupThreads, smem, s>>>(approx, nq, plan, nleaves, btpi, perm, slots, leaf_qoff, leaf_qcnt,
-                                                 item_off, nitems, global_cnt ? gcnt : nullptr);
+                                                 item_off, nitems, items_cap, global_cnt ? gcnt : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_group_items<<<nblk((uint64_t)nleaves * 32, 256), 256, 0, s>>>(plan, nleaves, nitems, leaf_qoff, leaf_qcnt,

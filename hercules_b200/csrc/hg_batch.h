@@ -5,13 +5,13 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "hg_items.h"
 #include "hg_kernels.h"
 
 namespace hg {
 
 constexpr int kBatchTileRows = 128;   // rows per tensor-core tile (and per tile norm)
 constexpr int kBatchQueryTile = 256;  // queries per tensor-core tile (filter pass)
-constexpr int kBatchBoundQueries = 64;  // queries per tile in the bound pass (MMA N = 64)
 constexpr int kBatchMaxSlots = 4096;  // bound slots per query (sorted in one block)
 // re-rank segments over all queries of a round, beyond one per query: five for
 // each of the 32 warps resident on each of 148 SMs
@@ -126,10 +126,6 @@ struct BatchRank {
 constexpr uint32_t kBatchPairBlock = 1024;  // survivor pairs a filter warp reserves at a time
 constexpr uint32_t kBatchPairWarps = 8;     // filter warps per SM that do
 
-// Work items that even out over the SMs: the filter's work lists are cut into
-// at least this many items where their tiles allow it
-constexpr uint32_t kBatchItemTarget = 8 * 148;
-
 // TMA descriptors of one BF16 query matrix: boxes of 256 and of 64 queries
 // (narrow query tiles), and of 128 (the CTA-pair filter)
 struct QueryMaps {
@@ -141,10 +137,11 @@ struct QueryMaps {
 cudaError_t launch_rows_to_bf16(const float* rows, const uint32_t* idx, uint64_t n, int L, void* out, float4* meta,
                                 cudaStream_t s, const uint32_t* n_dev = nullptr);
 // nitems[0]: items, nitems[1]: tiles per item (at most btpi; fewer where that
-// would leave SMs without an item)
+// would leave SMs without an item and the list fits items_cap)
 cudaError_t launch_group_queries(const int* approx, int nq, const LeafPlan* plan, int nleaves, uint32_t btpi,
                                  uint32_t* perm, uint32_t* slots, uint32_t* leaf_qoff, uint32_t* leaf_qcnt,
-                                 uint32_t* item_off, uint32_t* nitems, BatchItem* items, cudaStream_t s,
+                                 uint32_t* item_off, uint32_t* nitems, BatchItem* items, uint32_t items_cap,
+                                 cudaStream_t s,
                                  uint32_t* gcnt = nullptr);  // 2 x nleaves words above kMaxLeavesSort leaves
 // the pruned filter's query panel list and work items from the kept
 // (leaf, query) pairs (k_group_pruned, k_emit_pruned); ctl[2] = the query

@@ -2108,7 +2108,8 @@ static hg_status enqueue_round(hg_index* ix, int round, uint32_t nq, uint32_t km
     CK(hg::launch_route_queries(b.qin, (int)nq, (int)L, index_tree(ix), b.approx, st, b.bucket_cnt, nq,
                                 prune ? b.leaf_cnt : nullptr, prune ? (uint32_t)nl : 0u, c->stamps + 0));
     CK(hg::launch_group_queries(b.approx, (int)nq, b.leaf_plan, nl, ix->tune.bound_tiles_per_item, b.qperm, b.slots,
-                                b.leaf_qoff, b.leaf_qcnt, b.item_off, c->ctrl + 0, b.items, st, b.group_cnt));
+                                b.leaf_qoff, b.leaf_qcnt, b.item_off, c->ctrl + 0, b.items, b.items_cap, st,
+                                b.group_cnt));
     CK(hg::launch_rows_to_bf16(b.qin, b.qperm, nq, (int)L, b.qbf, b.qmeta, st));
     // 2. bound pass
     g.qperm = b.qperm;
@@ -2306,12 +2307,10 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   const uint32_t bucket_cap = o.bucket_cap > 0 ? (uint32_t)o.bucket_cap : kDefaultBucket;
   hg::BatchScratch& b = ix->bs;
   HCK(ensure_leaf_plan(ix, std::max<uint64_t>(2ull * kmax + 32, 256), st));
-  const uint32_t btpi = ix->tune.bound_tiles_per_item;
-  const uint32_t items_cap =
-      (uint32_t)(((uint64_t)(nq + hg::kBatchBoundQueries - 1) / hg::kBatchBoundQueries + ix->leaves.size()) *
-                 ((b.plan_max_use + btpi - 1) / btpi)) +
-      hg::kBatchItemTarget + nq;
-  HCK(ensure_batch_scratch(ix, std::max(nq, b.nq_cap), bucket_cap, b.plan_bm_cap, items_cap, kmax));
+  const uint64_t items_cap =
+      hg::bound_items_room(nq, ix->leaves.size(), b.plan_max_use, ix->tune.bound_tiles_per_item);
+  if (items_cap > UINT32_MAX) return set_error(HG_ERR_NOMEM, "hg_knn_batch: bound pass work list");
+  HCK(ensure_batch_scratch(ix, std::max(nq, b.nq_cap), bucket_cap, b.plan_bm_cap, (uint32_t)items_cap, kmax));
   if (!b.qlist2 || !b.qin || b.out_kmax < kmax) {
     dfree(b.qlist2);
     dfree(b.qin);
