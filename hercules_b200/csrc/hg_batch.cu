@@ -269,13 +269,9 @@ __global__ void __launch_bounds__(1024) k_rerank_plan(BatchRank a) {
   __syncthreads();
   const float inf = __int_as_float(0x7f800000);
   const int nlist = a.nlist_dev ? (int)*a.nlist_dev : a.nlist;
-  // a pair list that overflowed lost rows of any query: all of the round's
-  // count as overflowed
-  const bool lost = *a.pairs_cnt > a.pairs_cap;
   unsigned long long mine = 0;
   for (int i = tid; i < nlist; i += 1024) {
     const int q = a.qlist ? (int)a.qlist[i] : i;
-    if (lost) a.bucket_cnt[q] = max(a.bucket_cnt[q], a.bucket_cap + 1);
     mine += a.bound[q] < inf ? min(a.bucket_cnt[q], a.bucket_cap) : 0u;
   }
   if (mine) atomicAdd(&s_rows, mine);
@@ -508,8 +504,11 @@ __global__ void __launch_bounds__(kRankWarps * 32, 4) k_rerank_part(BatchRank a)
 // Merge: one block per query folds its starting list and its parts into the
 // answer (k distinct distances, lowest id per distance) and verifies it:
 //   ok 1: the filter kept every row within B_q and the k-th distance is <= B_q;
-//   ok 0: the bucket overflowed but its first rows gave k distances below
-//         B_q: B_q is lowered to the k-th, the list kept, the query retried;
+//   ok 0: the bucket overflowed, or the pair list did, which may have lost rows
+//         of any query of the round, but the rows that are there gave k
+//         distances below B_q: B_q is lowered to the k-th, the list kept, the
+//         query retried (its bucket holds bucket_cnt rows and no more: nothing
+//         beyond what was scattered is read);
 //   ok -1: neither: the plain path answers it.
 // A warp takes 32 parts at a time (a lane per part: the parts hold few
 // entries), so only queries with more than 32 parts occupy the other warps,
@@ -570,7 +569,8 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_rerank_merge(BatchRank a) {
   const float Bq = a.bound[q];
   const uint32_t nb = a.bucket_cnt[q];
   const float dk = cnt == k ? __uint_as_float((uint32_t)(list[k - 1] >> 32)) : inf;
-  const int ok = (Bq < inf && nb <= a.bucket_cap && dk <= Bq) ? 1 : ((Bq < inf && dk < Bq) ? 0 : -1);
+  const bool whole = nb <= a.bucket_cap && *a.pairs_cnt <= a.pairs_cap;
+  const int ok = (Bq < inf && whole && dk <= Bq) ? 1 : ((Bq < inf && dk < Bq) ? 0 : -1);
   for (int i = lane; i < a.kmax; i += 32) {
     const bool have = i < cnt;
     a.dist_out[(uint64_t)q * a.kmax + i] = have ? __uint_as_float((uint32_t)(list[i] >> 32)) : inf;

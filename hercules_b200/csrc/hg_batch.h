@@ -103,9 +103,9 @@ struct BatchRank {
   unsigned long long* init;        // [q][kMaxK] exact keys of the bound rows
   int* init_cnt;
   const uint32_t* bucket;
-  uint32_t* bucket_cnt;            // raised past bucket_cap for every query when the pair list overflowed
+  const uint32_t* bucket_cnt;      // rows scattered to the bucket, those beyond bucket_cap among them
   uint32_t bucket_cap;
-  const uint32_t* pairs_cnt;       // pair slots the filter reserved
+  const uint32_t* pairs_cnt;       // pair slots the filter reserved; above pairs_cap: rows were lost
   uint32_t pairs_cap;
   float* dist_out;  // [q][kmax]
   int64_t* id_out;
