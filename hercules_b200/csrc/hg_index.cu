@@ -1826,6 +1826,11 @@ static hg_status ensure_batch_scratch(hg_index* ix, uint32_t nq, uint32_t bucket
     dfree(b.init_cnt);
     dfree(b.bucket_cnt);
     dfree(b.ok);
+    // sized for nq_cap queries too, allocated by the caller
+    dfree(b.qlist2);
+    dfree(b.qin);
+    dfree(b.out_dist);
+    dfree(b.out_id);
     uint16_t* q = nullptr;
     CK(dalloc(&q, (size_t)nq * ix->L));
     b.qbf = q;
