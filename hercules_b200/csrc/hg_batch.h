@@ -123,9 +123,6 @@ struct BatchRank {
   uint32_t* heads;            // [0] segment counter
 };
 
-constexpr uint32_t kBatchPairBlock = 1024;  // survivor pairs a filter warp reserves at a time
-constexpr uint32_t kBatchPairWarps = 8;     // filter warps per SM that do
-
 // TMA descriptors of one BF16 query matrix: boxes of 256 and of 64 queries
 // (narrow query tiles), and of 128 (the CTA-pair filter)
 struct QueryMaps {

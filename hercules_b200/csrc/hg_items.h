@@ -34,4 +34,19 @@ HG_HD uint32_t bound_item_tiles(uint64_t work, uint64_t groups, uint32_t btpi, u
   return b < btpi && work / b + groups <= room ? (uint32_t)b : btpi;
 }
 
+constexpr uint32_t kBatchPairBlock = 1024;  // survivor pairs a filter warp reserves at a time
+constexpr uint32_t kBatchPairWarps = 8;     // filter warps per SM that do
+
+// The block of the pair list (pairs_cap slots) that a filter warp got for the
+// counter's value nb: slots [*cur, *end).  Past the list's end *cur is
+// pairs_cap + 1, and the warp reserves no more: the counter then says that pairs
+// were lost, and ends within a block per warp of that.  (A warp that went on
+// took 1,024 counts for every 32 survivors it dropped: 134M of them wrapped the
+// counter, and the list could look whole.)
+HG_HD void pair_block(uint32_t nb, uint32_t pairs_cap, uint32_t* cur, uint32_t* end) {
+  *cur = nb < pairs_cap ? nb : pairs_cap + 1;
+  *end = nb + kBatchPairBlock < pairs_cap ? nb + kBatchPairBlock : (nb < pairs_cap ? pairs_cap : pairs_cap + 1);
+}
+HG_HD bool pair_list_full(uint32_t cur, uint32_t pairs_cap) { return cur > pairs_cap; }
+
 }  // namespace hg

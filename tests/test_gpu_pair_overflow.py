@@ -29,6 +29,7 @@ def mixed(hg, gpu_available):
 
 @pytest.mark.parametrize("far,near,k", [
     (1, 9, 10),     # one query fills the list, nine lose rows to it
+    (100, 28, 10),  # 160M survivors for 3.3M slots: the slot counter's range
 ])
 def test_lost_pairs_are_found_again(mixed, far, near, k):
     import torch

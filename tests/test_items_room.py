@@ -1,7 +1,13 @@
-"""The bound pass's work list (hg_items.h): whatever chunk length the device
-chooses, the items it then writes fit the room the host gave the list.  The
-header is compiled for the CPU and both sides are run over explicit leaf
-layouts and over random ones, for every chunk length that the tuning takes."""
+"""Sizes that the host's buffers and the kernels agree on (hg_items.h), compiled
+for the CPU.
+
+The bound pass's work list: whatever chunk length the device chooses, the items
+it then writes fit the room the host gave the list, over explicit leaf layouts
+and over random ones, for every chunk length that the tuning takes.
+
+The survivor-pair list: warps that reserve blocks of it past its end leave a
+counter that tells so, however many pairs they drop, and no slot is written
+twice."""
 import os
 import shutil
 import subprocess
@@ -72,12 +78,68 @@ int main() {
 """
 
 
-def test_bound_pass_items_fit_their_room(tmp_path):
+PAIRS = r"""
+#include <cstdio>
+#include <vector>
+#include "hg_items.h"
+using namespace hg;
+
+// `warps` warps push `votes` votes of n pairs each, in turn
+static int run(uint32_t cap, uint32_t warps, uint64_t votes, uint32_t n) {
+  std::vector<uint32_t> cur(warps, 0), end(warps, 0);
+  std::vector<uint8_t> slots(cap, 0);
+  uint32_t counter = 0;  // the device's, 32 bits
+  uint64_t stored = 0;
+  for (uint64_t v = 0; v < votes; ++v) {
+    uint32_t &c = cur[v % warps], &e = end[v % warps];
+    if (c + n > e) {
+      if (pair_list_full(c, cap)) continue;
+      for (uint32_t i = c; i < e; ++i) ++slots[i];  // closed with sentinels
+      const uint32_t nb = counter;
+      counter += kBatchPairBlock;
+      pair_block(nb, cap, &c, &e);
+    }
+    for (uint32_t i = 0; i < n; ++i)
+      if (c + i < e) {
+        if (c + i >= cap) return printf("slot %u of %u\n", c + i, cap), 1;
+        ++slots[c + i];
+        ++stored;
+      }
+    c += n;
+  }
+  for (uint32_t w = 0; w < warps; ++w)
+    for (uint32_t i = cur[w]; i < end[w]; ++i) ++slots[i];
+  for (uint32_t i = 0; i < cap; ++i)
+    if (slots[i] != (i < counter ? 1 : 0)) return printf("slot %u of %u written %d times\n", i, cap, slots[i]), 1;
+  // the last block inside the list begins below cap; after it a warp takes one
+  // more at most.  A list that is no multiple of a block (the library's are) says
+  // "lost" as soon as its last block is begun.
+  const bool lost = counter > cap, dropped = stored < votes * n;
+  if ((dropped && !lost) || (lost && !dropped && cap % kBatchPairBlock == 0) ||
+      counter > (uint64_t)cap + ((uint64_t)warps + 1) * kBatchPairBlock)
+    return printf("cap %u, %u warps, %llu votes of %u: %llu stored, counter %u\n", cap, warps,
+                  (unsigned long long)votes, n, (unsigned long long)stored, counter), 1;
+  return 0;
+}
+
+int main() {
+  int bad = 0;
+  for (uint32_t cap : {1u, 1000u, 1024u, 4096u, 16384u + 1184u * 1024u})
+    for (uint32_t n : {1u, 5u, 32u})
+      for (uint64_t votes : {1ull, 31ull, 4096ull, 200000ull, 9000000ull})  // the last: past 2^32 blocks of counts
+        for (uint32_t warps : {1u, 1184u}) bad += run(cap, warps, votes, n);
+  return bad ? 1 : 0;
+}
+"""
+
+
+@pytest.mark.parametrize("source", [SOURCE, PAIRS], ids=["bound pass items", "survivor pairs"])
+def test_sizes_agree(tmp_path, source):
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no g++")
     src = tmp_path / "items.cpp"
-    src.write_text(SOURCE)
+    src.write_text(source)
     exe = str(tmp_path / "items")
     subprocess.run([cxx, "-O2", "-std=c++17", "-I" + os.path.join(ROOT, "hercules_b200", "csrc"), str(src), "-o", exe],
                    check=True)
