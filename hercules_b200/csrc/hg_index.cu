@@ -1365,10 +1365,11 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
   // group's approximate leaves may hold against the GPU's 32 warps per SM
   // (12 queries, leaf 1,562, L = 16384: 0.93 ms at 4 entries, 1.20 at 8; 20
   // queries, leaf 2,000, L = 4096: 0.74 at 4, 0.67 at 8)
+  const uint64_t warps = 32ull * sms;
   if (ix->L >= 4096) {
-    const uint64_t rows = (uint64_t)slots * std::min<uint64_t>(ix->leaf_size, ix->n), warps = 32ull * sms;
-    e.few_rows = slots == 1 && 2 * rows <= warps ? 1 : 0;
-    e.min_batch = e.few_rows ? 1u : (slots > 1 && rows >= 6 * warps ? 8u : 4u);
+    const uint64_t rows = (uint64_t)slots * std::min<uint64_t>(ix->leaf_size, ix->n);
+    e.few_rows = slots == 1 && 2 * rows <= warps ? UINT32_MAX : 0;
+    e.min_batch = slots > 1 && rows >= 6 * warps ? 8u : 4u;
   } else {
     e.min_batch = slots > 1 ? 32u : 8u;
   }
@@ -1416,6 +1417,14 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
   f.err = s.err;
   e.ident_leaf = nullptr;
   e.list = s.list;
+  // the rows left for one query over long series: a warp each while there are
+  // warps for all, 8 lanes above.  LB_SAX often leaves a thousand rows; without
+  // it, or for a query unlike any row, most of the collection is left, and only
+  // the device knows.  One query of 100k x 16384, leaf 1,562, whole calls: a warp
+  // per row whatever the count / 8 lanes / by the count: 30k rows 0.84 / 0.61 /
+  // 0.61 ms, white noise (99k rows) 2.22 / 1.36 / 1.36, 1,500 rows 0.341 / 0.407 /
+  // 0.345.  The launch that returns at once takes 4 us.
+  e.few_rows = ix->L >= 4096 && slots == 1 ? (uint32_t)warps : 0;
   // one LB_SAX filter block is resident per SM (eight that only list rows): a
   // query alone takes them all, a group a share each, with some to spare for
   // its larger queries
@@ -1432,7 +1441,7 @@ static hg_status knn_group(hg_index* ix, const float* d_q, int slots, int k, con
     m.out_row = out_row;
     m.out_stride = out_stride;
     CK(hg::launch_merge(m, slots, st));
-    *launches += 3;
+    *launches += e.few_rows ? 4 : 3;
     return HG_OK;
   };
   // greedy seeding (the paper's L_max): the next approx_leaves - 1

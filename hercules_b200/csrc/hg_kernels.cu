@@ -1306,6 +1306,12 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_ed_stream(EdArgs a
   const int nch = a.L >> 3;
   uint64_t first;
   uint32_t total, bs;
+  if (!kRowIds && kSlot >= 8 && a.few_rows && a.few_rows != UINT32_MAX) {
+    // one of two launches over the same list, and the other one's list (looked
+    // at here and not in ed_range, where it made this kernel spill)
+    const uint32_t n = a.list_count[8 * blockIdx.x];
+    if (kSlot == 32 ? n > a.few_rows : n <= a.few_rows) return;
+  }
   if (!ed_range<W>(a, first, total, bs)) return;
   const uint32_t nwarps = gridDim.y * W;
   const uint32_t gw = blockIdx.y * W + wib;
@@ -1979,12 +1985,16 @@ static cudaError_t launch_ed(K kernel, SmemLimit& attr, const EdArgs& args, int 
 // row in flight -- all 32 where there are fewer rows than warps (one query over
 // a leaf of a thousand rows of 64 KB reads each row in 128 dependent steps with
 // 8 lanes: 528 us, 348 us with 32; with rows for every warp 8 lanes are faster,
-// PSCAN of 60k x 16384 619 us against 1,007).
+// PSCAN of 60k x 16384 619 us against 1,007).  Where the device alone knows how
+// many rows there are, both are launched and one of them returns at once.
 cudaError_t launch_ed_stream(const EdArgs& a, int slots, int blocks, cudaStream_t s) {
   static SmemLimit wide, lng, mid, shrt, shrt2, few_wide, few_lng;
   if (a.few_rows) {
-    if (ed_wide(a.L)) return launch_ed(k_ed_stream<false, 1, 32, 32>, few_wide, a, 32, slots, blocks, s);
-    return launch_ed(k_ed_stream<false, 1, 32, kEdWarps>, few_lng, a, kEdWarps, slots, blocks, s);
+    EdArgs f = a;
+    f.min_batch = 1;
+    const cudaError_t e = ed_wide(a.L) ? launch_ed(k_ed_stream<false, 1, 32, 32>, few_wide, f, 32, slots, blocks, s)
+                                       : launch_ed(k_ed_stream<false, 1, 32, kEdWarps>, few_lng, f, kEdWarps, slots, blocks, s);
+    if (e != cudaSuccess || a.few_rows == UINT32_MAX) return e;
   }
   if (slots > 1 && a.L <= 256) return launch_ed(k_ed_short<2, 2>, shrt, a, kEdWarps, slots, blocks, s);
   if (slots > 1 && a.L <= kEdShortL) return launch_ed(k_ed_short<4, 2>, shrt2, a, kEdWarps, slots, blocks, s);

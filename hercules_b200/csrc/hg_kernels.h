@@ -115,7 +115,8 @@ struct EdArgs {
   const uint64_t* leaf_start;
   const uint32_t* leaf_size;
   uint32_t min_batch;          // entries a warp takes at least, 1..32: with fewer in all, blocks stay idle
-  int few_rows;                // 1: one query, fewer rows than half the warps of the GPU: a warp per row
+  uint32_t few_rows;           // one query over long rows: a warp each up to this many rows, 8 lanes each
+                               // above (two launches); 0: 8 lanes, UINT32_MAX: a warp, whatever the count
   const float* q;              // [slot][L]
   int k;
   uint32_t* bound;             // [slot] float bits of the running k-th bound (atomicMin)
