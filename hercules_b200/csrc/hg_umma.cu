@@ -1096,6 +1096,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t bempty_bar = done_bar + 48u;  // the item's MMAs have read B_ext (both CTAs)
   volatile uint32_t* s_item = reinterpret_cast<volatile uint32_t*>(sm + kPSmItem);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + kPSmAbort);
+  stamp_start(a.stamp);
   const uint32_t peer_abort = mapa(base + kPSmAbort, peer);
   uint32_t* s_qidx = reinterpret_cast<uint32_t*>(sm + kPSmQidx);
   volatile int* s_okw = reinterpret_cast<volatile int*>(sm + kPSmOkw);
