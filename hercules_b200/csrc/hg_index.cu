@@ -41,6 +41,7 @@ static hg_status set_error(hg_status s, const char* what) {
 void hg_record_error(const char* msg) { set_error(HG_OK, msg); }
 
 static hg_status cuda_fail(cudaError_t e, const char* where) {
+  cudaGetLastError();  // reported here: not again by the next call's first launch
   char buf[512];
   snprintf(buf, sizeof buf, "%s: %s", where, cudaGetErrorString(e));
   return set_error(e == cudaErrorMemoryAllocation ? HG_ERR_NOMEM : HG_ERR_CUDA, buf);
@@ -305,32 +306,7 @@ static void free_scratch(hg_index* ix) {
   s.slots = 0;
 }
 
-static void free_device(hg_index* ix) {
-  hg::DeviceIndex& d = ix->d;
-  dfree(d.rows);
-  dfree(d.rows_rm);
-  dfree(d.ids);
-  dfree(d.sax);
-  dfree(d.bp);
-  dfree(d.leaf_start);
-  dfree(d.leaf_size);
-  dfree(d.leaf_seg_off);
-  dfree(d.leaf_points);
-  dfree(d.leaf_sk);
-  dfree(d.nodes);
-  free_scratch(ix);
-  dfree(ix->io.q);
-  dfree(ix->io.out);
-  ix->io = hg::HostIo{};
-  for (cudaEvent_t& e : ix->ev) {
-    if (e) cudaEventDestroy(e);
-    e = nullptr;
-  }
-  hg::BatchData& bd = ix->bd;
-  dfree(bd.xbf);
-  dfree(bd.xmeta);
-  dfree(bd.tile_meta);
-  hg::BatchScratch& b = ix->bs;
+static void free_batch_scratch(hg::BatchScratch& b) {
   dfree(b.qbf);
   dfree(b.qmeta);
   dfree(b.qperm);
@@ -375,6 +351,34 @@ static void free_device(hg_index* ix) {
   dfree(b.seg_uid);
   dfree(b.segstats);
   b = hg::BatchScratch{};
+}
+
+static void free_device(hg_index* ix) {
+  hg::DeviceIndex& d = ix->d;
+  dfree(d.rows);
+  dfree(d.rows_rm);
+  dfree(d.ids);
+  dfree(d.sax);
+  dfree(d.bp);
+  dfree(d.leaf_start);
+  dfree(d.leaf_size);
+  dfree(d.leaf_seg_off);
+  dfree(d.leaf_points);
+  dfree(d.leaf_sk);
+  dfree(d.nodes);
+  free_scratch(ix);
+  dfree(ix->io.q);
+  dfree(ix->io.out);
+  ix->io = hg::HostIo{};
+  for (cudaEvent_t& e : ix->ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
+  hg::BatchData& bd = ix->bd;
+  dfree(bd.xbf);
+  dfree(bd.xmeta);
+  dfree(bd.tile_meta);
+  free_batch_scratch(ix->bs);
 }
 
 // Routing tree in the final encoding: internal nodes renumbered densely,
@@ -1799,19 +1803,31 @@ static hg_status encode_query_maps(hg::QueryMaps* m, const void* base, uint64_t 
   return encode_bf16_map(&m->q64, base, n, L, hg::kBatchBoundQueries);
 }
 
+static hg_status make_batch_data(hg_index* ix, cudaStream_t st, uint16_t** x) {
+  hg::BatchData& b = ix->bd;
+  const uint64_t nt = (ix->n + hg::kBatchTileRows - 1) / hg::kBatchTileRows;
+  CK(dalloc(x, ix->n * ix->L));
+  CK(dalloc(&b.xmeta, ix->n));
+  CK(dalloc(&b.tile_meta, nt));
+  CK(hg::launch_rows_to_bf16(ix->d.rows, nullptr, ix->n, (int)ix->L, *x, b.xmeta, st));
+  CK(hg::launch_tile_norms(b.xmeta, ix->n, b.tile_meta, st));
+  return encode_bf16_map(&b.rows_map, *x, ix->n, ix->L, 128);
+}
+
+// b.xbf says that all of it is there
 static hg_status ensure_batch_data(hg_index* ix, cudaStream_t st) {
   hg::BatchData& b = ix->bd;
   if (b.xbf) return HG_OK;
-  const uint64_t nt = (ix->n + hg::kBatchTileRows - 1) / hg::kBatchTileRows;
   uint16_t* x = nullptr;
-  CK(dalloc(&x, ix->n * ix->L));
-  b.xbf = x;
-  CK(dalloc(&b.xmeta, ix->n));
-  CK(dalloc(&b.tile_meta, nt));
-  CK(hg::launch_rows_to_bf16(ix->d.rows, nullptr, ix->n, (int)ix->L, b.xbf, b.xmeta, st));
-  CK(hg::launch_tile_norms(b.xmeta, ix->n, b.tile_meta, st));
-  HCK(encode_bf16_map(&b.rows_map, b.xbf, ix->n, ix->L, 128));
-  return HG_OK;
+  const hg_status s = make_batch_data(ix, st, &x);
+  if (s == HG_OK) {
+    b.xbf = x;
+    return HG_OK;
+  }
+  dfree(x);
+  dfree(b.xmeta);
+  dfree(b.tile_meta);
+  return s;
 }
 
 static hg_status ensure_batch_scratch(hg_index* ix, uint32_t nq, uint32_t bucket_cap, uint32_t bm_cap,
@@ -2281,6 +2297,33 @@ static hg_status knn_batch_plain(hg_index* ix, const float* Q, uint32_t nq, cons
   return status;
 }
 
+// Every buffer of a batch of nq queries with at most kmax answers each.
+static hg_status ensure_batch_buffers(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_t bucket_cap, bool want_prune,
+                                      bool* prune, cudaStream_t st) {
+  hg::BatchScratch& b = ix->bs;
+  HCK(ensure_scratch(ix, 1));
+  HCK(ensure_batch_data(ix, st));
+  HCK(ensure_leaf_plan(ix, std::max<uint64_t>(2ull * kmax + 32, 256), st));
+  const uint64_t items_cap =
+      hg::bound_items_room(nq, ix->leaves.size(), b.plan_max_use, ix->tune.bound_tiles_per_item);
+  if (items_cap > UINT32_MAX) return set_error(HG_ERR_NOMEM, "hg_knn_batch: bound pass work list");
+  HCK(ensure_batch_scratch(ix, std::max(nq, b.nq_cap), bucket_cap, b.plan_bm_cap, (uint32_t)items_cap, kmax));
+  if (!b.qlist2 || !b.qin || b.out_kmax < kmax) {
+    dfree(b.qlist2);
+    dfree(b.qin);
+    dfree(b.out_dist);
+    dfree(b.out_id);
+    CK(dalloc(&b.qlist2, b.nq_cap));
+    CK(dalloc(&b.qin, (size_t)b.nq_cap * ix->L));
+    CK(dalloc(&b.out_dist, (size_t)b.nq_cap * kmax));
+    CK(dalloc(&b.out_id, (size_t)b.nq_cap * kmax));
+    b.out_kmax = kmax;
+    ++b.gen;
+  }
+  if (want_prune) HCK(ensure_prune_scratch(ix, prune));
+  return HG_OK;
+}
+
 // Batched exact k-NN; ks is a host array (or null).  Queries and answers are
 // device buffers, or host buffers with host_io (copied straight into and out
 // of the handle's fixed buffers: no allocation per call).
@@ -2314,36 +2357,23 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   if (nq == 0) return HG_OK;
   CK(cudaSetDevice(ix->device));
   if (!st) st = ix->stream;
-  HCK(ensure_scratch(ix, 1));
   const bool data_built = ix->bd.xbf == nullptr;
-  HCK(ensure_batch_data(ix, st));
   const uint32_t L = ix->L;
   const uint32_t bucket_cap = o.bucket_cap > 0 ? (uint32_t)o.bucket_cap : kDefaultBucket;
   hg::BatchScratch& b = ix->bs;
-  HCK(ensure_leaf_plan(ix, std::max<uint64_t>(2ull * kmax + 32, 256), st));
-  const uint64_t items_cap =
-      hg::bound_items_room(nq, ix->leaves.size(), b.plan_max_use, ix->tune.bound_tiles_per_item);
-  if (items_cap > UINT32_MAX) return set_error(HG_ERR_NOMEM, "hg_knn_batch: bound pass work list");
-  HCK(ensure_batch_scratch(ix, std::max(nq, b.nq_cap), bucket_cap, b.plan_bm_cap, (uint32_t)items_cap, kmax));
-  if (!b.qlist2 || !b.qin || b.out_kmax < kmax) {
-    dfree(b.qlist2);
-    dfree(b.qin);
-    dfree(b.out_dist);
-    dfree(b.out_id);
-    CK(dalloc(&b.qlist2, b.nq_cap));
-    CK(dalloc(&b.qin, (size_t)b.nq_cap * L));
-    CK(dalloc(&b.out_dist, (size_t)b.nq_cap * kmax));
-    CK(dalloc(&b.out_id, (size_t)b.nq_cap * kmax));
-    b.out_kmax = kmax;
-    ++b.gen;
+  bool prune = false;
+  const hg_status bst = ensure_batch_buffers(ix, nq, kmax, bucket_cap, o.dense_filter == 0, &prune, st);
+  if (bst != HG_OK) {
+    // sets that are half there, or sized for a batch that did not fit, must not
+    // meet the next call
+    free_batch_scratch(b);
+    return bst;
   }
   // inputs at fixed addresses: the queries and their k
   CK(cudaMemcpyAsync(b.qin, d_Q, sizeof(float) * nq * L,
                      host_io ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
   CK(cudaMemcpyAsync(b.kq, kq.data(), sizeof(uint32_t) * nq, cudaMemcpyHostToDevice, st));
   // the rounds, each captured once per shape in a CUDA graph and replayed
-  bool prune = false;
-  if (!o.dense_filter) HCK(ensure_prune_scratch(ix, &prune));
   const uint64_t key[8] = {nq, kmax, bucket_cap, b.gen, ix->tune.filter_tiles_per_item, ix->tune.bound_tiles_per_item,
                            ix->tune.rerank_blocks_per_sm, (prune ? 2u : 1u) | (ix->tune.filter_cta_pair << 4)};
   if (memcmp(key, b.graph_key, sizeof key) != 0) {
