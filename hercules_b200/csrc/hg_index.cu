@@ -299,11 +299,15 @@ static void free_scratch(hg_index* ix) {
   dfree(s.topk_count);
   dfree(s.sax_tab);
   dfree(s.sort_keys);
-  dfree(s.list);
   dfree(s.stats);
   s.err = nullptr;  // in stats
   dfree(s.actl);
   s.slots = 0;
+}
+
+static void free_lists(hg_index* ix) {
+  dfree(ix->s.list);
+  ix->s.list_slots = 0;
 }
 
 static void free_batch_scratch(hg::BatchScratch& b) {
@@ -367,6 +371,7 @@ static void free_device(hg_index* ix) {
   dfree(d.leaf_sk);
   dfree(d.nodes);
   free_scratch(ix);
+  free_lists(ix);
   dfree(ix->io.q);
   dfree(ix->io.out);
   ix->io = hg::HostIo{};
@@ -1170,7 +1175,9 @@ static hg_status read_impl(const char* dir, int device, hg_index** out) {
 // 139 -> 28 us; 100k x 16384: 480 -> 92 us; 8M x 256, k = 100: 800 -> 390 us).
 // 4 GB of lists, 2% of the GPU's memory, hold 32 queries of 33M rows; with
 // 512 MB 25M rows left groups of five (64 queries of 25M x 256: 63.0 ms, 54.9
-// now, with LB_SAX 22.2 and 19.0; 32 of 30M x 96 15.2 and 13.6).
+// now, with LB_SAX 22.2 and 19.0; 32 of 30M x 96 15.2 and 13.6).  PSCAN, which
+// reads no lists, keeps to the same groups: 32 queries of 80M x 64 take 60.0 ms
+// in groups of 11, 61.5 together.
 constexpr uint32_t kGroupSlots = 32;
 constexpr uint64_t kGroupListBytes = 4ull << 30;
 static uint32_t group_slots(const hg_index* ix, uint32_t nq) {
@@ -1189,7 +1196,6 @@ static cudaError_t alloc_scratch(hg_index* ix, size_t slots) {
     if (e == cudaSuccess) e = dalloc(p, count);
   };
   get(&s.lb, slots * nl);
-  get(&s.list, slots * ix->n);
   get(&s.counters, slots * 8);
   get(&s.approx_leaf, slots);
   get(&s.cand, slots * (nl + 1));
@@ -1214,21 +1220,52 @@ static cudaError_t alloc_scratch(hg_index* ix, size_t slots) {
   return e;
 }
 
-// Scratch for groups of `want` queries; where the device has no room for so
-// many, for half as many, down to one (the caller reads s.slots).
-static hg_status ensure_scratch(hg_index* ix, uint32_t want) {
+// Scratch for groups of `want` queries, with a list of rows each if `lists`;
+// where the device has no room for so many, for half as many, down to one (the
+// caller reads group_room).  PSCAN, the epsilon and the nprobes search read no
+// lists, which are most of the scratch of a large collection.
+static hg_status ensure_scratch(hg_index* ix, uint32_t want, bool lists) {
   hg::QueryScratch& s = ix->s;
-  if (s.slots > 0 && want <= s.asked) return HG_OK;
-  free_scratch(ix);
-  for (uint32_t slots = want;; slots = std::max<uint32_t>(1, slots / 2)) {
-    const cudaError_t e = alloc_scratch(ix, slots);
-    if (e == cudaSuccess) break;
+  if (s.slots == 0 || want > s.asked) {
     free_scratch(ix);
-    if (e != cudaErrorMemoryAllocation || slots == 1) return cuda_fail(e, "query scratch");
-    cudaGetLastError();  // the failed allocation
+    for (uint32_t slots = want;; slots = std::max<uint32_t>(1, slots / 2)) {
+      const cudaError_t e = alloc_scratch(ix, slots);
+      if (e == cudaSuccess) break;
+      free_scratch(ix);
+      if (e != cudaErrorMemoryAllocation || slots == 1) return cuda_fail(e, "query scratch");
+      cudaGetLastError();  // the failed allocation
+    }
+    s.asked = want;  // a smaller group was all there was room for: not tried again on each call
   }
-  s.asked = want;  // a smaller group was all there was room for: not tried again on each call
+  if (!lists || (s.list_slots > 0 && want <= s.list_asked)) return HG_OK;
+  free_lists(ix);
+  for (uint32_t slots = std::min<uint32_t>(want, (uint32_t)s.slots);; slots = std::max<uint32_t>(1, slots / 2)) {
+    const cudaError_t e = dalloc(&s.list, (size_t)slots * ix->n);
+    if (e == cudaSuccess) {
+      s.list_slots = (int)slots;
+      break;
+    }
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "query scratch");
+    cudaGetLastError();
+    if (slots > 1) continue;
+    // not one list beside this group's other scratch: a query at a time
+    if (s.slots == 1) return cuda_fail(e, "query scratch");
+    const uint32_t asked = s.asked;
+    free_scratch(ix);
+    const cudaError_t e1 = alloc_scratch(ix, 1);
+    if (e1 != cudaSuccess) {
+      free_scratch(ix);
+      return cuda_fail(e1, "query scratch");
+    }
+    s.asked = asked;
+  }
+  s.list_asked = want;
   return HG_OK;
+}
+
+// queries per group, at most, of what ensure_scratch could get
+static uint32_t group_room(const hg_index* ix, bool lists) {
+  return (uint32_t)(lists ? std::min(ix->s.slots, ix->s.list_slots) : ix->s.slots);
 }
 
 static hg::Tree index_tree(const hg_index* ix) { return hg::Tree{ix->d.nodes, ix->d.root}; }
@@ -1711,8 +1748,9 @@ static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t 
     return set_error(HG_ERR_LIMIT, "hg_knn: k above 224 with epsilon or nprobes");
   CK(cudaSetDevice(ix->device));
   // rounds and approximate searches follow one query at a time
-  const bool grouped = !approx && (int)k <= hg::kMaxK;
-  HCK(ensure_scratch(ix, grouped ? group_slots(ix, nq) : 1));
+  const bool grouped = !approx && (int)k <= hg::kMaxK, lists = !approx && o.mode != HG_MODE_PSCAN;
+  const uint32_t want = grouped ? group_slots(ix, nq) : 1;
+  HCK(ensure_scratch(ix, want, lists));
   if (!st) st = ix->stream;
   for (cudaEvent_t& e : ix->ev)
     if (!e) CK(cudaEventCreate(&e));
@@ -1720,7 +1758,7 @@ static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t 
   Prof prof;
   CK(cudaEventRecord(ix->ev[0], st));
   uint64_t launches = 0;
-  const uint32_t per = grouped ? std::min<uint32_t>(group_slots(ix, nq), (uint32_t)ix->s.slots) : 1;
+  const uint32_t per = std::min(want, group_room(ix, lists));
   for (uint32_t i = 0; i < nq; i += per) {
     const float* qi = d_queries + (uint64_t)i * ix->L;
     float* di = d_dist ? d_dist + (uint64_t)i * k : nullptr;
@@ -2301,7 +2339,7 @@ static hg_status knn_batch_plain(hg_index* ix, const float* Q, uint32_t nq, cons
 static hg_status ensure_batch_buffers(hg_index* ix, uint32_t nq, uint32_t kmax, uint32_t bucket_cap, bool want_prune,
                                       bool* prune, cudaStream_t st) {
   hg::BatchScratch& b = ix->bs;
-  HCK(ensure_scratch(ix, 1));
+  HCK(ensure_scratch(ix, 1, true));
   HCK(ensure_batch_data(ix, st));
   HCK(ensure_leaf_plan(ix, std::max<uint64_t>(2ull * kmax + 32, 256), st));
   const uint64_t items_cap =
@@ -2362,7 +2400,15 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   const uint32_t bucket_cap = o.bucket_cap > 0 ? (uint32_t)o.bucket_cap : kDefaultBucket;
   hg::BatchScratch& b = ix->bs;
   bool prune = false;
-  const hg_status bst = ensure_batch_buffers(ix, nq, kmax, bucket_cap, o.dense_filter == 0, &prune, st);
+  hg_status bst = ensure_batch_buffers(ix, nq, kmax, bucket_cap, o.dense_filter == 0, &prune, st);
+  if (bst == HG_ERR_NOMEM && std::max(ix->s.slots, ix->s.list_slots) > 1) {
+    // the scratch of an earlier plain call's groups (lists of 4 GB at most) may
+    // hold what the batch lacks
+    free_batch_scratch(b);
+    free_scratch(ix);
+    free_lists(ix);
+    bst = ensure_batch_buffers(ix, nq, kmax, bucket_cap, o.dense_filter == 0, &prune, st);
+  }
   if (bst != HG_OK) {
     // sets that are half there, or sized for a batch that did not fit, must not
     // meet the next call
@@ -2442,12 +2488,12 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
       if (ok[q] != 1) left.push_back(q);
     std::stable_sort(left.begin(), left.end(), [&](uint32_t x, uint32_t y) { return kq[x] < kq[y]; });
     fallbacks = left.size();
-    HCK(ensure_scratch(ix, group_slots(ix, (uint32_t)fallbacks)));
+    HCK(ensure_scratch(ix, group_slots(ix, (uint32_t)fallbacks), true));
     CK(cudaMemsetAsync(ix->s.err, 0, sizeof(int), st));
     CK(cudaEventRecord(ix->ev[0], st));
     for (size_t i = 0, n; i < left.size(); i += n) {
       const int k = (int)kq[left[i]];
-      const size_t most = std::min<size_t>(left.size() - i, (size_t)ix->s.slots);
+      const size_t most = std::min<size_t>(left.size() - i, group_room(ix, true));
       for (n = 1; n < most && (int)kq[left[i + n]] == k;) ++n;
       const uint32_t q = left[i];
       if (n == 1) {

@@ -55,6 +55,8 @@ struct DeviceIndex {
 struct QueryScratch {
   int slots = 0;                  // 0: not allocated
   uint32_t asked = 0;             // the slots asked for (slots of them fitted)
+  int list_slots = 0;             // slots with a list (searches of the leaves alone need one)
+  uint32_t list_asked = 0;
   int nparts = 0;                 // lists per slot
   float* lb = nullptr;            // leaves
   int* approx_leaf = nullptr;     // 1
@@ -74,7 +76,7 @@ struct QueryScratch {
   int* topk_count = nullptr;      // 1
   float* sax_tab = nullptr;       // 16 x 256 LB_SAX terms of the query
   uint32_t* sort_keys = nullptr;  // 4 x leaves: candidate sort above kMaxLeavesSort leaves
-  uint32_t* list = nullptr;       // LB_SAX survivors (rows), n entries
+  uint32_t* list = nullptr;       // [list_slots] LB_SAX survivors (rows), n entries
   // shared by the slots, one block: counters of the call (knn_device_impl),
   // then the device error flag
   unsigned long long* stats = nullptr;
