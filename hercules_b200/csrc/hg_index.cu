@@ -1727,6 +1727,18 @@ static hg_status grow_io(T** p, size_t* cap, size_t bytes) {
   return HG_OK;
 }
 
+// frees the copies that are larger than `keep`
+static void trim_io(hg::HostIo& io, size_t keep) {
+  if (io.q_cap > keep) {
+    dfree(io.q);
+    io.q_cap = 0;
+  }
+  if (io.out_cap > keep) {
+    dfree(io.out);
+    io.out_cap = 0;
+  }
+}
+
 // host_out: if set, host_bytes from device memory host_src (the answers) are
 // copied there with the call's counters, before its one synchronisation.
 static hg_status knn_device_impl(hg_index* ix, const float* d_queries, uint32_t nq, uint32_t k,
@@ -2401,12 +2413,15 @@ static hg_status knn_batch_impl(hg_index* ix, const float* d_Q, uint32_t nq, con
   hg::BatchScratch& b = ix->bs;
   bool prune = false;
   hg_status bst = ensure_batch_buffers(ix, nq, kmax, bucket_cap, o.dense_filter == 0, &prune, st);
-  if (bst == HG_ERR_NOMEM && std::max(ix->s.slots, ix->s.list_slots) > 1) {
-    // the scratch of an earlier plain call's groups (lists of 4 GB at most) may
-    // hold what the batch lacks
+  hg::HostIo& io = ix->io;
+  const bool own_io = d_Q != io.q && io.q_cap + io.out_cap > 0;
+  if (bst == HG_ERR_NOMEM && (std::max(ix->s.slots, ix->s.list_slots) > 1 || own_io)) {
+    // the scratch of an earlier plain call's groups (lists of 4 GB at most) and
+    // its copies of queries and answers may hold what the batch lacks
     free_batch_scratch(b);
     free_scratch(ix);
     free_lists(ix);
+    if (own_io) trim_io(io, 0);
     bst = ensure_batch_buffers(ix, nq, kmax, bucket_cap, o.dense_filter == 0, &prune, st);
   }
   if (bst != HG_OK) {
@@ -2692,14 +2707,18 @@ hg_status hg_knn(hg_index* ix, const float* queries, uint32_t nq, uint32_t k, co
   const size_t nk = (size_t)nq * k, q_bytes = sizeof(float) * nq * ix->L, id_bytes = sizeof(int64_t) * nk;
   const size_t out_bytes = id_bytes + sizeof(float) * nk;
   hg::HostIo& io = ix->io;
-  HCK(grow_io(&io.q, &io.q_cap, q_bytes));
-  HCK(grow_io(&io.out, &io.out_cap, out_bytes));
+  hg_status s = grow_io(&io.q, &io.q_cap, q_bytes);
+  if (s == HG_OK) s = grow_io(&io.out, &io.out_cap, out_bytes);
+  if (s != HG_OK) {
+    trim_io(io, 0);
+    return s;
+  }
   // ids and distances side by side: one copy back
   int64_t* d_id = reinterpret_cast<int64_t*>(io.out);
   float* d_dist = reinterpret_cast<float*>(io.out + id_bytes);
   std::vector<int64_t> ids(nk + (nk + 1) / 2);
   const cudaError_t e = cudaMemcpyAsync(io.q, queries, q_bytes, cudaMemcpyHostToDevice, ix->stream);
-  hg_status s = e == cudaSuccess ? HG_OK : cuda_fail(e, "hg_knn");
+  if (e != cudaSuccess) s = cuda_fail(e, "hg_knn");
   const bool batch = opts && opts->mode == HG_MODE_BATCH;
   if (s == HG_OK)
     s = knn_device_impl(ix, io.q, nq, k, opts, d_dist, d_id, ix->stream, stats, batch ? nullptr : ids.data(), io.out,
@@ -2709,14 +2728,7 @@ hg_status hg_knn(hg_index* ix, const float* queries, uint32_t nq, uint32_t k, co
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(ix->stream);
     if (ce != cudaSuccess) s = cuda_fail(ce, "hg_knn");
   }
-  if (io.q_cap > kHostIoKeep) {
-    dfree(io.q);
-    io.q_cap = 0;
-  }
-  if (io.out_cap > kHostIoKeep) {
-    dfree(io.out);
-    io.out_cap = 0;
-  }
+  trim_io(io, kHostIoKeep);
   if (s != HG_OK) return s;
   if (dist_out) memcpy(dist_out, ids.data() + nk, sizeof(float) * nk);
   if (id_out) memcpy(id_out, ids.data(), sizeof(int64_t) * nq * k);

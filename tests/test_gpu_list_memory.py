@@ -1,6 +1,7 @@
 """The survivor lists of a group (a word per row of the collection and query):
 searches that read none do not allocate them, and a batched call that lacks
-room gets theirs."""
+room gets theirs.  The same for the device copies of a host call's queries and
+answers."""
 import numpy as np
 import pytest
 
@@ -59,4 +60,28 @@ def test_lists_beside_a_large_group(hg, gpu_available):
     with Filled(4 * MiB):
         d, ids = ix.knn(Q, 10)
         assert np.array_equal(d.view(np.uint32), pd.view(np.uint32)) and np.array_equal(ids, pi)
+    ix.close()
+
+
+def test_host_copies_are_given_back(hg, gpu_available):
+    """The copies of a call's queries and answers: those of a call that fails
+    are freed, and a batch gets the room of those kept."""
+    import torch
+    ix, Q = make(hg)
+    big = np.resize(Q, (600000, L))  # 154 MB, above what is kept
+    ix.knn(Q[:1], 10)
+    free = torch.cuda.mem_get_info()[0]
+    with Filled(200 * MiB):
+        with pytest.raises(hg.HerculesError) as e:
+            ix.knn(big, 100)         # answers of 720 MB
+        assert e.value.status == -5
+    assert free - torch.cuda.mem_get_info()[0] < 32 * MiB
+    kept = np.resize(Q, (250000, L))  # 64 MB
+    ix.pscan(kept[:1], 10)
+    with pytest.raises(hg.HerculesError):
+        ix.knn(kept, 0)              # refused, its copy kept
+    d0, i0 = ix.pscan(Q[:8], 10)
+    with Filled(270 * MiB):          # BF16 rows and norms 288 MB
+        d, ids = ix.knn_batch(Q[:8], 10)
+    assert np.array_equal(d.view(np.uint32), d0.view(np.uint32)) and np.array_equal(ids, i0)
     ix.close()
