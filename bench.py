@@ -699,7 +699,8 @@ def main():
               "ms_per_step": agg["rerank_ms"] / steps}
     plain.update({"value": plain_qps, "unit": UNIT, "k": pk,
                   "batched_over_plain": round(value / plain_qps, 2) if plain_qps > 0 else None,
-                  "path": "hg_knn_device (one query at a time, LB_SAX on); value = the k = %d leg" % pk})
+                  "path": "hg_knn_device (the queries of a call in groups of up to 32 that share each launch, "
+                          "LB_SAX on); value = the k = %d leg" % pk})
     line = {
         "metric": METRIC, "value": round(value, 2), "unit": UNIT, "n_gpus": world, "steps": steps, "warmup": warm,
         "ms_per_step": ms / steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

@@ -471,9 +471,10 @@ namespace {
 // The waiting rows are counted again, until none waits.  The tree is the one
 // that splits one at a time give.  Splitting one leaf at a time and routing
 // the rest of the window again after it, with the member lists on the host,
-// took 74 ms for 1M x 256, leaf 10,000 (193 leaves; 24 ms of it routing), and
-// 1.37 s for 1M x 64, leaf 200 (8,468 leaves); this takes
-// 20 and 60 ms.
+// took 72 to 81 ms for 1M x 256, leaf 10,000 (193 leaves; 24 ms of it routing),
+// and 1.35 to 1.41 s for 1M x 64, leaf 200 (8,468 leaves); this takes 20 to 21 and
+// 52 to 63 ms (medians of three processes of 25 builds each; the rest is host
+// memory management, and single builds take up to 58 ms where that is slow).
 struct BuildCtx {
   hg_index* ix;
   const float* X;  // device, n x L row-major, original order
