@@ -17,10 +17,10 @@ constexpr uint32_t kBatchItemTarget = 8 * 148;
 // The bound pass's work list holds, for every group of at most
 // kBatchBoundQueries queries of one leaf, the leaf's tiles in chunks.  Room for
 // any batch of nq queries over `leaves` leaves of at most max_use tiles: chunks
-// of btpi tiles, and what shorter chunks (bound_item_tiles) add.  Those have
-// work / b tiles each for b = max(2, floor(work / kBatchItemTarget)), fewer than
-// 1.5 kBatchItemTarget chunks (work just below 3 kBatchItemTarget), and one
-// partly filled per group, of which there are at most nq.
+// of btpi tiles, and what shorter chunks (bound_item_tiles) add.  Of b =
+// max(2, floor(work / kBatchItemTarget)) tiles there are work / b, fewer than 1.5
+// kBatchItemTarget (most for work just below 3 kBatchItemTarget), and at most one
+// more per group, of which there are at most nq.
 inline uint64_t bound_items_room(uint32_t nq, uint64_t leaves, uint32_t max_use, uint32_t btpi) {
   const uint64_t groups = ((uint64_t)nq + kBatchBoundQueries - 1) / kBatchBoundQueries + leaves;
   return groups * ((max_use + btpi - 1) / btpi) + 2 * kBatchItemTarget + nq;

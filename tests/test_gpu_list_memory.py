@@ -56,6 +56,9 @@ def test_batch_gets_the_room_of_the_lists(hg, gpu_available):
 def test_lists_beside_a_large_group(hg, gpu_available):
     """A group's scratch without lists took the room: a query at a time then."""
     ix, Q = make(hg)
+    small = hg.HerculesIndex.build(hg.generate_walks(1, 3000, L), 500)
+    small.knn(Q[:2], 10)   # the kernels are loaded while there is room
+    small.close()
     pd, pi = ix.pscan(Q, 10)
     with Filled(4 * MiB):
         d, ids = ix.knn(Q, 10)
